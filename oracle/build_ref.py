@@ -222,9 +222,10 @@ def run_pins(exe: str):
 
 
 def reference_tree():
-    """The reference tree to build from, or None where it does not exist."""
+    """The reference tree to build from, or None where it does not exist or
+    holds no headers (an empty mount)."""
     path = os.environ.get("BTE_REFERENCE_TREE", _MOUNT)
-    return path if os.path.isdir(path) else None
+    return path if os.path.isdir(os.path.join(path, "external", "eigen")) else None
 
 
 def build(reference: str) -> str:
