@@ -1,16 +1,15 @@
 """Autotuner of the production grid kernel.
 
 Tries block shapes, resident blocks per SM (the register/residency variants
-of rta_prod_grid), shared-memory tally privatisation and the particles each
-thread carries at once (1, or 2 in the interleaved kernel) on a short slice
-of the real workload, measures device time per flight event, and leaves the
+of rta_prod_grid) and shared-memory tally privatisation on a short slice of
+the real workload, measures device time per flight event, and leaves the
 fastest setting on the engine.  Runs before any timed region.
 """
 import btegpu
 
 # (threads per block, blocks per SM, shared-memory tally, particles per thread)
 CANDIDATES = [(256, 4, 0, 1), (128, 8, 0, 1), (256, 3, 0, 1), (256, 2, 0, 1), (128, 6, 0, 1), (128, 4, 0, 1),
-              (256, 1, 1, 1), (256, 1, 0, 2), (128, 3, 0, 2), (256, 2, 0, 2), (128, 4, 0, 2)]
+              (256, 1, 1, 1)]
 
 
 def tune(engine, run, trial_particles: int, smem_bytes: int, repeats: int = 2):

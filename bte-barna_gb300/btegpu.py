@@ -640,6 +640,22 @@ def split_frames(data: bytes):
     return out
 
 
+def debug_fixwalk(gx, gy, vmax, step, nbins, p, e, tau, vx, vy, cap=100000):
+    """The grid kernel's integer walk of one particle on the host: rows
+    (flight, kind, x, y, ticks) and the scales (kx, kt, sub)."""
+    lib = load_library()
+    gx, gy, tau, vx, vy = (np.ascontiguousarray(a, dtype=np.float64) for a in (gx, gy, tau, vx, vy))
+    e = np.ascontiguousarray(e, dtype=np.float32)
+    out = np.zeros((cap, 5), dtype=np.int64)
+    sc = (C.c_int * 3)()
+    fn = lib.btegpu_debug_fixwalk
+    fn.restype = C.c_longlong
+    n = fn(_dptr(gx), gx.size - 1, _dptr(gy), gy.size - 1, C.c_double(vmax), C.c_double(step), int(nbins),
+           C.c_double(p[0]), C.c_double(p[1]), C.c_longlong(e.size), e.ctypes.data_as(C.POINTER(C.c_float)), _dptr(tau),
+           _dptr(vx), _dptr(vy), sc, out.ctypes.data_as(C.POINTER(C.c_longlong)), C.c_longlong(cap))
+    return out[:min(n, cap)], tuple(sc)
+
+
 def debug_log(x: np.ndarray) -> np.ndarray:
     lib = load_library()
     x = np.ascontiguousarray(x, dtype=np.float64)

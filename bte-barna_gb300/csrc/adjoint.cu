@@ -33,18 +33,22 @@ bte_status bte_rta_adjoint(bte_ctx* c, const bte_rta_params* p, const double* we
         const bte_status st = prepared_grid_run(c, p, &r, &why);
         if (st != BTE_OK) throw Error(st, why);
         // time grid, src/RTA_MC2D.cpp:2118-2124
-        c->d_time.upload(time_grid_with_widths(r.ntime, r.maxtime, r.step), c->stream);
+        c->d_time.upload(time_grid_with_widths(r.ntime, r.maxtime, r.step, r.A.fx.kt - r.A.fx.sub), c->stream);
         r.T.timegrid = c->d_time.as<double>();
         const std::size_t nk = std::size_t(r.nboxes) * std::size_t(r.nbins);
         const std::size_t n = c->modes.n();
         const long long np = r.T.pend - r.T.pbegin;
-        DBuf dW, dphi, dg, ds, dtal, dcnt, derr, dwork;
-        std::vector<double> W(weights, weights + nk * 3);
+        DBuf dW, dphi, dg, ds, dcnt, derr, dwork;
+        std::vector<double> W(weights, weights + nk * 3);  // in the walk's units
+        for (std::size_t k = 0; k < nk; ++k) {
+            W[3 * k] *= r.A.fx.per_tick();
+            W[3 * k + 1] *= r.A.fx.per_unit();
+            W[3 * k + 2] *= r.A.fx.per_unit();
+        }
         dW.upload(W, c->stream);
         dphi.alloc(size_t(np > 0 ? np : 1) * sizeof(double));
         dg.alloc(n * sizeof(double));
         ds.alloc(4 * sizeof(double));
-        dtal.alloc(nk * 3 * sizeof(double));
         dcnt.alloc(16 * sizeof(unsigned long long));
         derr.alloc(4 * sizeof(int));
         dwork.alloc(sizeof(unsigned long long));
@@ -56,11 +60,10 @@ bte_status bte_rta_adjoint(bte_ctx* c, const bte_rta_params* p, const double* we
         float ms_total = 0.f;
         unsigned long long ev = 0;
         for (int pass = 1; pass <= 2; ++pass) {
-            ck(cudaMemsetAsync(dtal.p, 0, nk * 3 * sizeof(double), s), "memset");
             ck(cudaMemsetAsync(dcnt.p, 0, 16 * sizeof(unsigned long long), s), "memset");
             ck(cudaMemsetAsync(dwork.p, 0, sizeof(unsigned long long), s), "memset");
             ck(cudaEventRecord(c->ev0, s), "cudaEventRecord");
-            if (!launch_prod_grid(r.T, r.A, dtal.as<double>(), dcnt.as<unsigned long long>(), derr.as<int>(),
+            if (!launch_prod_grid(r.T, r.A, nullptr, dcnt.as<unsigned long long>(), derr.as<int>(),
                                   dwork.as<unsigned long long>(), r.tune, r.nsm, s, pass, &a))
                 throw Error(BTE_ERR_INPUT, "tuning not supported by the grid kernel");
             ck(cudaGetLastError(), "adjoint launch");

@@ -702,7 +702,7 @@ constexpr unsigned BRANCH_CAP = 1u << 20;
 __global__ void __launch_bounds__(256) be_advance(PArr in, const unsigned long long* n_in, PArr out,
                                                   unsigned long long* dc, long long ocap, int advect,
                                                   AdvectArgs aa, int rta, const PAlias* pal, const BoxProp* bprop,
-                                                  int nm, const double* w, const float* rprob, const int* ralt,
+                                                  int nm, const double* w, const int2* resample,
                                                   int nmodes, unsigned long long skey, int* H, int* err) {
     const long long n = min((long long)*n_in, ocap);  // places beyond the buffers (an overflow) are not read
     const int lane = threadIdx.x & 31;
@@ -773,7 +773,8 @@ __global__ void __launch_bounds__(256) be_advance(PArr in, const unsigned long l
             if (u < 1. - exp(-__ldg(w + mode) * aa.dt)) {
                 const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
                 const float acc = float(g.next32() >> 8) * 0x1p-24f;
-                nmode = acc < __ldg(rprob + j) ? j : __ldg(ralt + j);
+                const int2 e = __ldg(resample + j);
+                nmode = acc < __int_as_float(e.x) ? j : e.y;
             }
         } else if (act && valid) {
             // one table for every box (pal), or the box's own
@@ -1763,7 +1764,7 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             be_advance<<<pblocks, 256, 0, s>>>(arr(B.a_x, B.a_y, B.a_mode, B.a_box, B.a_sign), dc + DC_NP,
                                                arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc, cap, 1, a_step,
                                                p->rta, pal, bprop, B.nm, c->d_w.as<double>(),
-                                               c->d_rprob.as<float>(), c->d_ralt.as<int>(), n,
+                                               c->d_resample.as<int2>(), n,
                                                mix_key(p->seed, istep, 64), B.d_H.as<int>(), err);
             ck(cudaEventRecord(ev[1], s), "event");
             // 2-4 the step's sources, made at A[0..) (A is free now) and each
@@ -1812,7 +1813,7 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             ck(cudaMemsetAsync(dc + DC_WORK, 0, sizeof(unsigned long long), s), "memset");
             be_advance<<<pblocks, 256, 0, s>>>(A, dc + DC_NGEN, arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc,
                                                cap, 0, a_step, p->rta, pal, bprop, B.nm, c->d_w.as<double>(),
-                                               c->d_rprob.as<float>(), c->d_ralt.as<int>(), n,
+                                               c->d_resample.as<int2>(), n,
                                                mix_key(p->seed, istep, 65), B.d_H.as<int>(), err);
             ck(cudaEventRecord(ev[3], s), "event");
             ck(cudaEventRecord(ev[4], s), "event");  // the histogram is made in the passes above

@@ -25,6 +25,18 @@ long long btegpu_debug_lambert(const bte_mode_table* m, const bte_geometry* g,
 long long btegpu_debug_frame(double time, double Eeff, const double* temps, const int* H, int nboxes,
                              int nmodes, char* out, long long cap);
 
+/* The integer walk of the grid kernel (fixed_walk.cuh), on the host: one
+ * particle from (px, py) through free flights k of tau[k] e[k] ps at
+ * (vx[k], vy[k]) over the cells of the lines gx[0..nx], gy[0..ny], nbins time
+ * bins of `step` ps, until it leaves the grid or the bins end.  Per segment
+ * five values: flight, kind (1 / 2: crosses a line in x / y, 4: flight ends,
+ * 8: part of a bin ends), x, y, ticks; scales: kx, kt, sub.  Returns the
+ * number of segments. */
+long long btegpu_debug_fixwalk(const double* gx, int nx, const double* gy, int ny, double vmax, double step,
+                               int nbins, double px, double py, long long nflights, const float* e,
+                               const double* tau, const double* vx, const double* vy, int* scales, long long* out,
+                               long long cap);
+
 /* The host build of bte_log. */
 int btegpu_debug_log(const double* x, double* y, long long n);
 

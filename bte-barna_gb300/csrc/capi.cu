@@ -57,6 +57,10 @@ void ensure_static(bte_ctx* c) {
         c->d_w.upload(wall, c->stream);
         c->d_tau.upload(tau, c->stream);
         c->d_mv.upload(mv, c->stream);
+        c->d_mf.alloc(n * sizeof(bte::ModeFix));
+        c->vmax = 0.;
+        for (std::size_t k = 0; k < n; ++k) c->vmax = std::max({c->vmax, std::fabs(m.vxc[k]), std::fabs(m.vyc[k])});
+        c->fix_dev = false;
         sync(c);
         c->modes_dev = true;
     }
@@ -89,6 +93,18 @@ void ensure_static(bte_ctx* c) {
                     if (b >= 0) bc[std::size_t(b)] = make_int2(i, j);
                 }
             c->d_boxcell.upload(bc, c->stream);
+            c->d_gxf.alloc(g.gx.size() * sizeof(long long));
+            c->d_gyf.alloc(g.gy.size() * sizeof(long long));
+            c->d_wxf.alloc(g.gx.size() * sizeof(long long));
+            c->d_wyf.alloc(g.gy.size() * sizeof(long long));
+            std::vector<int> map(std::size_t(g.gnx + 2) * std::size_t(g.gny + 2), -1);
+            for (int i = 0; i < g.gnx; ++i)
+                for (int j = 0; j < g.gny; ++j)
+                    map[std::size_t(i + 1) * std::size_t(g.gny + 2) + std::size_t(j + 1)] =
+                        g.gcell[std::size_t(i) * g.gny + j];
+            c->d_map.upload(map, c->stream);
+            sync(c);
+            c->fix_dev = false;
         }
         {
             // border lines and neighbour pieces of the convex-polygon path
@@ -239,6 +255,14 @@ void ensure_static(bte_ctx* c) {
         }
         c->nclass = L.nclass;
         c->d_row_ptr.upload(L.row_ptr, c->stream);
+        std::vector<unsigned long long> lrow(std::size_t(L.nclass) * m.n());
+        for (int k = 0; k < L.nclass; ++k)
+            for (std::size_t j = 0; j < m.n(); ++j) {
+                const long long* r = L.row_ptr.data() + std::size_t(k) * (m.n() + 1) + j;
+                if (r[0] >> 36 || (r[1] - r[0]) >> 28) throw Error(BTE_ERR_INPUT, "Lambert table too large");
+                lrow[std::size_t(k) * m.n() + j] = (unsigned long long)r[0] | ((unsigned long long)(r[1] - r[0]) << 36);
+            }
+        c->d_lrow.upload(lrow, c->stream);
         c->d_lcol.upload(L.col, c->stream);
         c->d_lcdf.upload(L.cdf, c->stream);
         c->d_lalias.upload(L.alias, c->stream);
@@ -363,15 +387,9 @@ void ensure_resample(bte_ctx* c, double T0) {
     } else {
         bte::build_resample(c->modes, T0, cdf, al);
     }
-    std::vector<float> prob(al.size());
-    std::vector<int> alt(al.size());
-    for (std::size_t i = 0; i < al.size(); ++i) {
-        prob[i] = al[i].prob;
-        alt[i] = al[i].alt;
-    }
+    static_assert(sizeof(bte::Alias) == sizeof(int2) && offsetof(bte::Alias, alt) == 4, "an alias slot is an int2");
     c->d_rcdf.upload(cdf, c->stream);
-    c->d_rprob.upload(prob, c->stream);
-    c->d_ralt.upload(alt, c->stream);
+    c->d_resample.upload(al, c->stream);
     sync(c);
     c->resample_T0 = T0;
 }
@@ -1097,8 +1115,11 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         if (ntime < 2) throw Error(BTE_ERR_INPUT, "maxtime shorter than one time bin");
         const double maxtime = double(ntime - 1) * p->dt;
         const double step = (maxtime - 0.0) / double(ntime - 1);
+        bte::GridArgs A{};
+        if (g.rect_grid) bte::prepare_fixed(c, step, A);
         {
-            const std::vector<double> tg = bte::time_grid_with_widths(int(ntime), maxtime, step);
+            const std::vector<double> tg =
+                bte::time_grid_with_widths(int(ntime), maxtime, step, A.fx.kt - A.fx.sub);
             c->h_time.assign(tg.begin(), tg.begin() + std::ptrdiff_t(ntime));
             c->d_time.upload(tg, c->stream);
         }
@@ -1143,8 +1164,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         T.w = c->d_w.as<double>();
         T.tau = c->d_tau.as<double>();
         T.resample_cdf = c->d_rcdf.as<double>();
-        T.resample_prob = c->d_rprob.as<float>();
-        T.resample_alt = c->d_ralt.as<int>();
+        T.resample = c->d_resample.as<int2>();
         T.nboxes = nbx;
         T.boxes = c->d_boxes.as<bte::GBox>();
         T.hull = c->d_hull.as<bte::V2>();
@@ -1159,6 +1179,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         T.row_ptr = c->d_row_ptr.as<long long>();
         T.lcol = c->d_lcol.as<int>();
         T.lcdf = c->d_lcdf.as<double>();
+        T.lrow = c->d_lrow.as<unsigned long long>();
         T.lalias = c->d_lalias.as<int4>();
         T.mirror = c->have_mirror ? c->d_mirror.as<int>() : nullptr;
         T.box_mat = c->nmat > 0 ? c->d_boxmat.as<int>() : nullptr;
@@ -1203,26 +1224,15 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         }
         c->spec_valid = false;
 
+        // the grid kernel's tallies are in its integer units (powers of two)
+        const bool grid_run = !replay && g.rect_grid && c->ncrys == 0;
+        const double unit_t = grid_run ? A.fx.per_tick() : 1., unit_x = grid_run ? A.fx.per_unit() : 1.;
         auto* counters = c->d_counters.as<unsigned long long>();
         auto* err = c->d_err.as<int>();
         ck(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
         if (replay) {
             bte::launch_replay(T, c->d_tally.as<unsigned long long>(), counters, err, c->nsm, c->stream);
-        } else if (g.rect_grid && c->ncrys == 0) {
-            bte::GridArgs A{};
-            A.G.nx = g.gnx;
-            A.G.ny = g.gny;
-            A.G.gx = c->d_gx.as<double>();
-            A.G.gy = c->d_gy.as<double>();
-            A.G.cell = c->d_gcell.as<int>();
-            A.boxcell = c->d_boxcell.as<int2>();
-            A.mv = c->d_mv.as<bte::ModeVel>();
-            const bte::V2 want[4] = {bte::v2(1, 0), bte::v2(-1, 0), bte::v2(0, 1), bte::v2(0, -1)};
-            for (int w = 0; w < 4; ++w) {
-                A.cls[w] = -1;
-                for (std::size_t k = 0; k < g.normals.size(); ++k)
-                    if (g.normals[k].x == want[w].x && g.normals[k].y == want[w].y) A.cls[w] = int(k);
-            }
+        } else if (grid_run) {
             if (!bte::launch_prod_grid(T, A, c->d_tally.as<double>(), counters, err,
                                        c->d_work.as<unsigned long long>(), c->tune, c->nsm, c->stream))
                 throw Error(BTE_ERR_INPUT, "tuning not supported by the grid kernel");
@@ -1230,12 +1240,12 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
             bte::launch_prod_general(T, c->d_tally.as<double>(), counters, err,
                                      c->d_work.as<unsigned long long>(), c->nsm, c->stream);
         } else {
-            const bte::PolyArgs A{c->d_pborders.as<bte::PolyBorder>(), c->d_ppieces.as<bte::PolyPiece>(),
+            const bte::PolyArgs PA{c->d_pborders.as<bte::PolyBorder>(), c->d_ppieces.as<bte::PolyPiece>(),
                                   c->d_mv.as<bte::ModeVel>(), c->d_invden.as<double>(),
                                   c->d_prect.as<bte::PolyRect>(),
                                   c->ncrys > 0 ? c->d_dmm_row.as<long long>() : nullptr,
                                   c->ncrys > 0 ? c->d_dmm_ent.as<bte::DmmEnt>() : nullptr};
-            if (!bte::launch_prod_poly(T, A, c->d_tally.as<double>(), counters, err,
+            if (!bte::launch_prod_poly(T, PA, c->d_tally.as<double>(), counters, err,
                                        c->d_work.as<unsigned long long>(), c->nsm, c->stream))
                 throw Error(BTE_ERR_CUDA, "polygon kernel does not fit on the device");
         }
@@ -1270,6 +1280,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
                     c->spec_raw[i] = double(v) / bte::FIX_SCALE;
                 } else {
                     std::memcpy(&c->spec_raw[i], &hspec[i], sizeof(double));
+                    c->spec_raw[i] *= unit_t;
                 }
             }
             c->spec_nbins = nbins;
@@ -1294,10 +1305,14 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         std::vector<double> sum;
         if (ngroups > 1) {
             // keep the groups; the run's outputs are their sum, in group order
-            c->group_raw.assign(htal, htal + nk * 3 * std::size_t(ngroups));
+            c->group_raw.resize(nk * 3 * std::size_t(ngroups));
             sum.assign(nk * 3, 0.);
             for (int gi = 0; gi < ngroups; ++gi)
-                for (std::size_t k = 0; k < nk * 3; ++k) sum[k] += htal[std::size_t(gi) * nk * 3 + k];
+                for (std::size_t k = 0; k < nk * 3; ++k) {
+                    const std::size_t i = std::size_t(gi) * nk * 3 + k;
+                    c->group_raw[i] = htal[i] * (k % 3 == 0 ? unit_t : unit_x);
+                    sum[k] += htal[i];
+                }
             htal = sum.data();
             c->group_n = ngroups;
             c->group_nbx = nbx;
@@ -1326,9 +1341,9 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
             if (out->exact) std::memcpy(out->exact, hex.data(), nk * 6 * sizeof(long long));
         } else {
             for (std::size_t k = 0; k < nk; ++k) {
-                gz[k] = htal[3 * k];
-                jx[k] = htal[3 * k + 1];
-                jy[k] = htal[3 * k + 2];
+                gz[k] = htal[3 * k] * unit_t;
+                jx[k] = htal[3 * k + 1] * unit_x;
+                jy[k] = htal[3 * k + 2] * unit_x;
             }
         }
         out->nboxes = nbx;
@@ -1424,6 +1439,61 @@ long long btegpu_debug_frame(double time, double Eeff, const double* temps, cons
     return (long long)f.size();
 }
 
+long long btegpu_debug_fixwalk(const double* gx, int nx, const double* gy, int ny, double vmax, double step,
+                               int nbins, double px, double py, long long nflights, const float* e,
+                               const double* tau, const double* vx, const double* vy, int* scales, long long* out,
+                               long long cap) {
+    const bte::FixScale f = bte::choose_scale(gx[0], gx[nx], gy[0], gy[ny], vmax, step);
+    scales[0] = f.kx;
+    scales[1] = f.kt;
+    scales[2] = f.sub;
+    auto line = [&](const double* g, int k, double o) { return bte::fix_round(g[k] - o, f.kx); };
+    int i = 0, j = 0;
+    while (i + 1 < nx && px >= gx[i + 1]) ++i;
+    while (j + 1 < ny && py >= gy[j + 1]) ++j;
+    int64_t x = bte::fix_round(px - f.x0, f.kx), y = bte::fix_round(py - f.y0, f.kx);
+    const uint64_t w = uint64_t(bte::fix_round(step, f.kt - f.sub));
+    uint64_t rb = w;
+    long long part = 0, m = 0;
+    for (long long k = 0; k < nflights; ++k) {
+        bte::ModeFix v;
+        bte::fix_velocity(vx[k], f, v.vx, v.rx);
+        bte::fix_velocity(vy[k], f, v.vy, v.ry);
+        const bool ux = !(v.vx & bte::FIX_DOWN), uy = !(v.vy & bte::FIX_DOWN);
+        uint32_t hi;
+        uint64_t lo = bte::fix_flight(e[k], tau[k], f.kt, hi);
+        for (;;) {
+            const uint64_t ax = uint64_t(ux ? line(gx, i + 1, f.x0) - x : x - line(gx, i, f.x0));
+            const uint64_t ay = uint64_t(uy ? line(gy, j + 1, f.y0) - y : y - line(gy, j, f.y0));
+            const bte::FixSeg q = bte::fix_segment(ax, ay, v, lo, hi, rb);
+            hi -= lo < q.seg ? 1u : 0u;
+            lo -= q.seg;
+            rb -= q.seg;
+            x += ux ? int64_t(q.dx) : -int64_t(q.dx);
+            y += uy ? int64_t(q.dy) : -int64_t(q.dy);
+            const int kind = (q.cross_x ? 1 : 0) | (q.cross_y ? 2 : 0) | (q.flight_end ? 4 : 0) | (q.bin_end ? 8 : 0);
+            if (m < cap) {
+                long long* o = out + 5 * m;
+                o[0] = k;
+                o[1] = kind;
+                o[2] = x;
+                o[3] = y;
+                o[4] = (long long)q.seg;
+            }
+            ++m;
+            if (q.bin_end) {
+                if (++part >= ((long long)nbins << f.sub)) return m;
+                rb = w;
+            }
+            if (q.cross_x) i += ux ? 1 : -1;
+            if (q.cross_y) j += uy ? 1 : -1;
+            if (i < 0 || j < 0 || i >= nx || j >= ny) return m;
+            if (q.flight_end) break;
+        }
+    }
+    return m;
+}
+
 int btegpu_debug_log(const double* x, double* y, long long n) {
     for (long long i = 0; i < n; ++i) y[i] = bte::bte_log(x[i]);
     return 0;
@@ -1503,8 +1573,7 @@ bte_status prepared_grid_run(bte_ctx* c, const bte_rta_params* p, PreparedRun* r
     T.w = c->d_w.as<double>();
     T.tau = c->d_tau.as<double>();
     T.resample_cdf = c->d_rcdf.as<double>();
-    T.resample_prob = c->d_rprob.as<float>();
-    T.resample_alt = c->d_ralt.as<int>();
+    T.resample = c->d_resample.as<int2>();
     T.nboxes = r->nboxes;
     T.boxes = c->d_boxes.as<GBox>();
     T.hull = c->d_hull.as<V2>();
@@ -1519,6 +1588,7 @@ bte_status prepared_grid_run(bte_ctx* c, const bte_rta_params* p, PreparedRun* r
     T.row_ptr = c->d_row_ptr.as<long long>();
     T.lcol = c->d_lcol.as<int>();
     T.lcdf = c->d_lcdf.as<double>();
+    T.lrow = c->d_lrow.as<unsigned long long>();
     T.lalias = c->d_lalias.as<int4>();
     T.mirror = c->have_mirror ? c->d_mirror.as<int>() : nullptr;
     T.box_mat = c->nmat > 0 ? c->d_boxmat.as<int>() : nullptr;
@@ -1545,20 +1615,13 @@ bte_status prepared_grid_run(bte_ctx* c, const bte_rta_params* p, PreparedRun* r
     T.pbegin = pbeg;
     T.pend = pend;
     T.nbins = r->nbins;
-    GridArgs& A = r->A;
-    A = GridArgs{};
-    A.G.nx = g.gnx;
-    A.G.ny = g.gny;
-    A.G.gx = c->d_gx.as<double>();
-    A.G.gy = c->d_gy.as<double>();
-    A.G.cell = c->d_gcell.as<int>();
-    A.boxcell = c->d_boxcell.as<int2>();
-    A.mv = c->d_mv.as<ModeVel>();
-    const V2 want[4] = {v2(1, 0), v2(-1, 0), v2(0, 1), v2(0, -1)};
-    for (int w = 0; w < 4; ++w) {
-        A.cls[w] = -1;
-        for (std::size_t k = 0; k < g.normals.size(); ++k)
-            if (g.normals[k].x == want[w].x && g.normals[k].y == want[w].y) A.cls[w] = int(k);
+    r->A = GridArgs{};
+    try {
+        ck(cudaSetDevice(c->device), "cudaSetDevice");
+        prepare_fixed(c, r->step, r->A);
+    } catch (const Error& e) {
+        *why = e.what();
+        return e.code;
     }
     r->stream = c->stream;
     r->ev0 = c->ev0;
@@ -1569,10 +1632,65 @@ bte_status prepared_grid_run(bte_ctx* c, const bte_rta_params* p, PreparedRun* r
     return BTE_OK;
 }
 
-std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step) {
-    std::vector<double> g(std::size_t(2 * ntime - 1));
+// Scales of the integer walk (fixed_walk.cuh): a bin below 2^61 ticks, the
+// domain below 2^58 units, and the fastest velocity below 2^63 units per
+// 2^64 ticks, which costs the positions at most three bits once a bin (or its
+// 2^sub parts) is no longer than eight flights across the domain.
+FixScale choose_scale(double x0, double x1, double y0, double y1, double vmax, double step) {
+    FixScale f{};
+    f.x0 = x0;
+    f.y0 = y0;
+    const double ext = std::max(x1 - x0, y1 - y0);
+    double w = step * (1.0 + 0x1p-20);  // no bin is longer (they differ by rounding)
+    while (vmax * w > 8.0 * ext && f.sub < 24) {
+        w *= 0.5;
+        ++f.sub;
+    }
+    f.kt = 60 - std::ilogb(w);
+    f.kx = 57 - std::ilogb(ext);
+    if (vmax > 0.) f.kx = std::min(f.kx, f.kt - 2 - std::ilogb(vmax));
+    return f;
+}
+
+void prepare_fixed(bte_ctx* c, double step, GridArgs& A) {
+    const HostGeometry& g = c->geom;
+    A.G.nx = g.gnx;
+    A.G.ny = g.gny;
+    A.G.gx = c->d_gx.as<double>();
+    A.G.gy = c->d_gy.as<double>();
+    A.G.cell = c->d_gcell.as<int>();
+    A.boxcell = c->d_boxcell.as<int2>();
+    A.mv = c->d_mv.as<ModeVel>();
+    A.mf = c->d_mf.as<ModeFix>();
+    A.gxf = c->d_gxf.as<long long>();
+    A.gyf = c->d_gyf.as<long long>();
+    A.wxf = c->d_wxf.as<unsigned long long>();
+    A.wyf = c->d_wyf.as<unsigned long long>();
+    A.map = c->d_map.as<int>();
+    A.fx = choose_scale(g.gx.front(), g.gx.back(), g.gy.front(), g.gy.back(), c->vmax, step);
+    const V2 want[4] = {v2(1, 0), v2(-1, 0), v2(0, 1), v2(0, -1)};
+    for (int w = 0; w < 4; ++w) {
+        A.cls[w] = -1;
+        for (std::size_t k = 0; k < g.normals.size(); ++k)
+            if (g.normals[k].x == want[w].x && g.normals[k].y == want[w].y) A.cls[w] = int(k);
+    }
+    const FixScale& f = A.fx;
+    if (c->fix_dev && c->fix.x0 == f.x0 && c->fix.y0 == f.y0 && c->fix.kx == f.kx && c->fix.kt == f.kt) return;
+    launch_fix_tables(f, A.mv, int(c->modes.n()), c->d_mf.as<ModeFix>(), A.G, c->d_gxf.as<long long>(),
+                      c->d_gyf.as<long long>(), c->d_wxf.as<long long>(), c->d_wyf.as<long long>(), c->stream);
+    ck(cudaGetLastError(), "integer tables launch");
+    c->fix = f;
+    c->fix_dev = true;
+}
+
+std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step, int tick_exp) {
+    std::vector<double> g(std::size_t(3 * ntime - 2));
     for (int i = 0; i < ntime; ++i) g[std::size_t(i)] = (i == ntime - 1) ? maxtime : 0.0 + double(i) * step;
-    for (int i = 0; i + 1 < ntime; ++i) g[std::size_t(ntime + i)] = g[std::size_t(i + 1)] - g[std::size_t(i)];
+    for (int i = 0; i + 1 < ntime; ++i) {
+        const double w = g[std::size_t(i + 1)] - g[std::size_t(i)];
+        g[std::size_t(ntime + i)] = w;
+        g[std::size_t(2 * ntime - 1 + i)] = bitsd(uint64_t(std::llrint(std::ldexp(w, tick_exp))));
+    }
     return g;
 }
 
@@ -1584,8 +1702,7 @@ void fill_static_tables(bte_ctx* c, DevTables& T) {
     T.w = c->d_w.as<double>();
     T.tau = c->d_tau.as<double>();
     T.resample_cdf = c->d_rcdf.as<double>();
-    T.resample_prob = c->d_rprob.as<float>();
-    T.resample_alt = c->d_ralt.as<int>();
+    T.resample = c->d_resample.as<int2>();
     T.nboxes = int(c->geom.boxes.size());
     T.boxes = c->d_boxes.as<GBox>();
     T.hull = c->d_hull.as<V2>();
@@ -1600,6 +1717,7 @@ void fill_static_tables(bte_ctx* c, DevTables& T) {
     T.row_ptr = c->d_row_ptr.as<long long>();
     T.lcol = c->d_lcol.as<int>();
     T.lcdf = c->d_lcdf.as<double>();
+    T.lrow = c->d_lrow.as<unsigned long long>();
     T.lalias = c->d_lalias.as<int4>();
     T.mirror = c->have_mirror ? c->d_mirror.as<int>() : nullptr;
     T.box_mat = c->nmat > 0 ? c->d_boxmat.as<int>() : nullptr;

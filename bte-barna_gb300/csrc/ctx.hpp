@@ -115,8 +115,14 @@ struct bte_ctx {
     bte::DBuf d_dmm_row, d_dmm_ent;
     bte::DBuf d_cdmm, d_crysoff;  // per contact its interface table (-1: none); crystals' first modes
     bte::DBuf d_gx, d_gy, d_gcell, d_boxcell;
+    // integer tables of the grid walk (fixed_walk.cuh) and the scales they
+    // were made for (remade on the device when a run asks for others)
+    bte::DBuf d_mf, d_gxf, d_gyf, d_wxf, d_wyf, d_map;
+    bte::FixScale fix{};
+    bool fix_dev = false;
+    double vmax = 0.;  // largest velocity component of the loaded modes
     bte::DBuf d_pborders, d_ppieces;  // convex-polygon path (geometries that are not a grid)
-    bte::DBuf d_row_ptr, d_lcol, d_lcdf, d_lalias, d_mirror;
+    bte::DBuf d_row_ptr, d_lrow, d_lcol, d_lcdf, d_lalias, d_mirror;
     int nclass = 0;
     bool have_mirror = false;
     // materials of batched runs (0: the mode table's own rates at the run's T0)
@@ -133,7 +139,7 @@ struct bte_ctx {
     bte::DBuf d_boxmat;
     // per-T0 (or per-material) resampling
     double resample_T0 = -1;
-    bte::DBuf d_rcdf, d_rprob, d_ralt;
+    bte::DBuf d_rcdf, d_resample;
     // generators
     int gen_key_source = -1;
     long long gen_key_n = -1;
@@ -198,7 +204,11 @@ void set_crystal_tables(const bte_ctx* c, DevTables& T);
 double crystal_thickness(const bte_ctx* c, int k);
 double box_thickness(const bte_ctx* c, int b);
 // The ntime points of the time grid (src/RTA_MC2D.cpp:2118-2124: i * step,
-// the last exactly maxtime) followed by the ntime - 1 bin widths, the
-// layout DevTables::timegrid points to.
-std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step);
+// the last exactly maxtime), the ntime - 1 bin widths, and the bit patterns
+// of the integers width 2^tick_exp: the layout DevTables::timegrid points to.
+std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step, int tick_exp);
+FixScale choose_scale(double x0, double x1, double y0, double y1, double vmax, double step);
+// The integer units of a grid run with bins of `step` ps, and their tables
+// on the device: fills the grid arguments (no allocation).
+void prepare_fixed(bte_ctx* c, double step, GridArgs& A);
 }  // namespace bte

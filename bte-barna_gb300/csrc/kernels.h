@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include "fixed_walk.cuh"
 #include "rta_flight.cuh"
 
 namespace bte {
@@ -19,7 +20,7 @@ struct ProdTuning {
     int block_threads;
     int blocks_per_sm;
     int smem_tally;
-    int particles_per_thread;  // 1 or 2 (the interleaved grid kernel)
+    int particles_per_thread;  // accepted; every lane carries one
 };
 
 void launch_replay(const DevTables& T, unsigned long long* ex, unsigned long long* counters,
@@ -52,6 +53,13 @@ struct GridArgs {
     DevGrid G;
     const int2* boxcell;     // box -> (i, j)
     const ModeVel* mv;       // per mode velocities and inverses
+    FixScale fx;             // the run's integer units,
+    const ModeFix* mf;       //   the modes' velocities in them
+    const long long* gxf;    //   the grid lines
+    const long long* gyf;
+    const unsigned long long* wxf;  // and the widths between them
+    const unsigned long long* wyf;
+    const int* map;          // the cells with a void rim: [nx + 2][ny + 2], as G.cell
     int cls[4];              // normal classes of the +x, -x, +y, -y walls (-1: none)
 };
 
@@ -112,7 +120,8 @@ struct AdjArgs {
 };
 
 // Axis-aligned grid production kernel (persistent, warp-refilled work).
-// adj_pass 1 / 2 runs the forward / adjoint pass of the adjoint with `adj`.
+// adj_pass 1 / 2 runs the forward / adjoint pass of the adjoint with `adj`
+// (no tally).  The tally comes out in the units of A.fx.
 // Returns false when the tuning cannot be honoured (e.g. smem too small).
 // Production kernel of geometries that are not a grid: exit times from the
 // convex box's border lines, neighbours from the border pieces.
@@ -125,6 +134,12 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A, double* tally,
                       unsigned long long* counters, int* err, unsigned long long* work,
                       const ProdTuning& tune, int nsm, cudaStream_t s, int adj_pass = 0,
                       const AdjArgs* adj = nullptr);
+
+// The integer tables of the scales f: mf[n] from mv, the lines and widths from G.
+void launch_fix_tables(const FixScale& f, const ModeVel* mv, int n, ModeFix* mf, const DevGrid& G, long long* gxf,
+                       long long* gyf, long long* wxf, long long* wyf, cudaStream_t s);
+// A tally in the walk's units (nk keys of three sums) to ps and nm, in place.
+void launch_scale_tally(double* tally, long long nk, const FixScale& f, int nsm, cudaStream_t s);
 
 // Kernel arguments of a context already prepared for one set of run
 // parameters (see prepared_grid_run in capi.cu).

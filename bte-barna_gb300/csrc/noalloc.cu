@@ -45,7 +45,7 @@ void set_ctx_error(bte_ctx* c, const std::string& m);
 namespace {
 
 constexpr int kHeaderBytes = 256;  // counters (8 x u64), error word (4 x int), work counter
-constexpr size_t kScratchBytes = kHeaderBytes + sizeof(double) * (2 * BTE_NOALLOC_MAX_BINS + 1);
+constexpr size_t kScratchBytes = kHeaderBytes + sizeof(double) * (3 * BTE_NOALLOC_MAX_BINS + 1);
 
 // The scratch of every allocation-free call.  Host code must not use the
 // symbol as an address; it asks the runtime for the device address below.
@@ -77,16 +77,19 @@ bool scratch_address(int device, unsigned char** out, std::string* why) {
 }
 
 // The time grid of src/RTA_MC2D.cpp:2118-2124 (LinSpaced: i * step, the
-// last point exactly maxtime) and its ntime - 1 bin widths after it, written
-// into the scratch.
+// last point exactly maxtime), its ntime - 1 bin widths and their ticks
+// (width 2^tick_exp as integers) after it, written into the scratch.
 __device__ __forceinline__ double noalloc_point(int i, int ntime, double maxtime, double step) {
     return (i == ntime - 1) ? maxtime : 0.0 + double(i) * step;
 }
-__global__ void noalloc_time_grid(double* grid, int ntime, double maxtime, double step) {
+__global__ void noalloc_time_grid(double* grid, int ntime, double maxtime, double step, int tick_exp) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < ntime) grid[i] = noalloc_point(i, ntime, maxtime, step);
-    if (i + 1 < ntime)
-        grid[ntime + i] = noalloc_point(i + 1, ntime, maxtime, step) - noalloc_point(i, ntime, maxtime, step);
+    if (i + 1 < ntime) {
+        const double w = noalloc_point(i + 1, ntime, maxtime, step) - noalloc_point(i, ntime, maxtime, step);
+        grid[ntime + i] = w;
+        grid[2 * ntime - 1 + i] = bte::bitsd(uint64_t(bte::fix_round(w, tick_exp)));
+    }
 }
 
 bte_status fail(bte_ctx* c, bte_status s, const std::string& m) {
@@ -122,7 +125,7 @@ extern "C" bte_status bte_rta_run_noalloc(bte_ctx* ctx, const bte_rta_params* pa
     if (cudaMemsetAsync(base, 0, kHeaderBytes, s) != cudaSuccess ||
         cudaMemsetAsync(d_tally, 0, tally_bytes, s) != cudaSuccess)
         return fail(ctx, BTE_ERR_CUDA, "cudaMemsetAsync failed (is d_tally a device pointer?)");
-    noalloc_time_grid<<<(r.ntime + 255) / 256, 256, 0, s>>>(grid, r.ntime, r.maxtime, r.step);
+    noalloc_time_grid<<<(r.ntime + 255) / 256, 256, 0, s>>>(grid, r.ntime, r.maxtime, r.step, r.A.fx.kt - r.A.fx.sub);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ctx, BTE_ERR_CUDA, std::string("time grid launch: ") + cudaGetErrorString(e));
     r.T.timegrid = grid;
@@ -131,6 +134,9 @@ extern "C" bte_status bte_rta_run_noalloc(bte_ctx* ctx, const bte_rta_params* pa
         return fail(ctx, BTE_ERR_INPUT, "tuning not supported by the grid kernel");
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ctx, BTE_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
+    bte::launch_scale_tally(d_tally, (long long)r.nboxes * r.nbins, r.A.fx, r.nsm, s);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return fail(ctx, BTE_ERR_CUDA, std::string("scale launch: ") + cudaGetErrorString(e));
     if (cudaEventRecord(r.ev1, s) != cudaSuccess) return fail(ctx, BTE_ERR_CUDA, "cudaEventRecord failed");
     unsigned long long hc[8];
     int herr[4];

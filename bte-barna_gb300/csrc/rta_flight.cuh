@@ -47,8 +47,7 @@ struct DevTables {
     const double* tau;
     const int* box_mat;     // [box] material (null: one material)
     const double* resample_cdf;
-    const float* resample_prob;
-    const int* resample_alt;
+    const int2* resample;   // post-scattering alias slots {prob bits, alt} (production)
     // geometry
     int nboxes;
     const GBox* boxes;
@@ -69,11 +68,12 @@ struct DevTables {
     const long long* row_ptr;
     const int* lcol;
     const double* lcdf;
+    const unsigned long long* lrow;  // [class][mode] first entry (36 bits) and length of the row in lalias
     const int4* lalias;   // {prob bits, keep, alt, pad}
     const int* mirror;    // [nclass][n] or null
     // time grid
     int ntime;
-    const double* timegrid;   // ntime points, then the ntime - 1 bin widths
+    const double* timegrid;   // ntime points, the ntime - 1 bin widths, then their integer ticks (grid path)
     double maxtime;
     double inv_dt;        // 1 / bin width (production)
     // generators

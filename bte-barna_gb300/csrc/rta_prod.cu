@@ -2,8 +2,9 @@
 //
 // Draws come from counter-based Philox4x32-10 streams keyed by (seed,
 // particle); mode distributions and Lambert rows are sampled through alias
-// tables; positions, times and tallies stay FP64, with tallies reduced by FP64
-// atomics.  Three kernels:
+// tables; positions and times are doubles, or on the grid path 64-bit
+// integers of a finer resolution (fixed_walk.cuh); tallies are reduced by
+// FP64 atomics.  Three kernels:
 //   rta_prod_general  any convex-box geometry, the flight logic of
 //                     rta_flight.cuh (one evolparticle step per pass);
 //   rta_prod_grid     boxes that tile an axis-aligned grid: a persistent
@@ -49,6 +50,17 @@ __device__ __forceinline__ int alias_draw(Philox& g, const float* prob, const in
     return a < __ldg(prob + j) ? j : __ldg(alt + j);
 }
 
+// The Lambert row of (class, mode) r: its first entry and length, packed as
+// 36 and 28 bits in one word.
+struct LambertRow {
+    uint64_t off;
+    uint32_t len;
+};
+__device__ __forceinline__ LambertRow lambert_row(const DevTables& T, long long r) {
+    const uint64_t w = __ldg(T.lrow + r);
+    return LambertRow{w & 0xfffffffffull, uint32_t(w >> 36)};
+}
+
 struct ProdPolicy {
     Philox g;
     double* out;
@@ -60,7 +72,10 @@ struct ProdPolicy {
         return double(-logf(g.uniformf())) * __ldg(T.tau + k);  // k: material offset + mode
     }
     __device__ int resample(const DevTables& T, int mo) {
-        return alias_draw(g, T.resample_prob + mo, T.resample_alt + mo, T.n);
+        const int j = int(mulhi32(g.next32(), uint32_t(T.n)));
+        const float a = float(g.next32() >> 8) * 0x1p-24f;
+        const int2 e = __ldg(T.resample + mo + j);
+        return a < __int_as_float(e.x) ? j : e.y;
     }
     __device__ int gen_mode(const DevTables& T, int gi) {
         const long long o = (long long)gi * T.n;
@@ -68,12 +83,9 @@ struct ProdPolicy {
         return j;
     }
     __device__ int bounce(const DevTables& T, int cls, int mode) {
-        const long long a = __ldg(T.row_ptr + (long long)cls * (T.n + 1) + mode);
-        const long long b = __ldg(T.row_ptr + (long long)cls * (T.n + 1) + mode + 1);
-        const int len = int(b - a);
-        if (len <= 0) return -1;
-        const int j = int(mulhi32(g.next32(), uint32_t(len)));
-        const int4 e = __ldg(T.lalias + a + j);
+        const LambertRow r = lambert_row(T, (long long)cls * T.n + mode);
+        if (r.len == 0) return -1;
+        const int4 e = __ldg(T.lalias + r.off + mulhi32(g.next32(), r.len));
         const float acc = float(g.next32() >> 8) * 0x1p-24f;
         return acc < __int_as_float(e.x) ? e.y : e.z;
     }
@@ -328,7 +340,7 @@ void launch_prod_general(const DevTables& T, double* tally, unsigned long long* 
 // ------------------------------------------------------------------ grid path
 
 struct GridParticle {
-    double x, y, t;
+    double x, y;   // generated position, nm
     int i, j;      // cell
     int mode;
     int sign;
@@ -380,9 +392,10 @@ struct Pending {
     }
 };
 
-__device__ __forceinline__ int grid_cell(const DevGrid& G, int i, int j) {
-    if (i < 0 || j < 0 || i >= G.nx || j >= G.ny) return -1;
-    return __ldg(G.cell + i * G.ny + j);
+// Ticks of the time bins (of each of their 2^sub parts), after the grid's
+// points and widths.
+__device__ __forceinline__ const uint64_t* bin_ticks(const DevTables& T) {
+    return reinterpret_cast<const uint64_t*>(T.timegrid + 2 * T.ntime - 1);
 }
 
 // Generate particle `pid` on the grid.  Returns 0 or an error code.
@@ -423,7 +436,6 @@ __device__ int grid_generate(const DevTables& T, const DevGrid& G, const int2* b
     p.j = ij.y;
     p.box = box;
     p.mo = mat_off(T, box);
-    p.t = 0.;
     return 0;
 }
 
@@ -446,21 +458,29 @@ __device__ __forceinline__ uint4 pass_block(uint32_t pass, uint64_t pid, uint64_
 // One lane carries one particle; each pass of the loop advances every active
 // lane by exactly one segment, which ends at the first of: the end of the
 // free flight, the next cell line, the next time-bin border (the last one is
-// maxtime).  Every pass therefore runs one fixed FP64 sequence on all lanes
-// -- the two exit times, the bin border, the advance and the three
-// differences of the pending tally -- and a lane flushes at most once per
-// pass, at the segment end; the FP64 pipe, the limit of this kernel on
-// GB300, never sees the same operation issued twice for different lanes.
+// maxtime).  Positions and times are 64-bit integers (fixed_walk.cuh): the
+// particle's cell, the distance (ax, ay) to the cell's borders ahead of it,
+// and the pending tally as time and signed displacement since its (box, bin)
+// key opened, so a segment is two exit times, two products and a few
+// subtractions on the integer units.  In doubles the same segment held the
+// SM's two FP64 lanes for 200 cycles a pass and bounded the kernel at 75 %
+// busy; now the FP64 pipe only turns the three pending sums into doubles
+// (17 cycles each), and the kernel is bound by instruction issue: 2e6
+// particles of the porous transient (36864 modes, 2422 cells, 200 bins) take
+// 115 ms instead of 151, the 1e6-particle ribbon 4.04 instead of 4.51.  A lane
+// flushes at most once per pass; a sum of zero (a mode without velocity) adds
+// nothing and is not sent.  The tally is left in the walk's units (ticks, and
+// position units), which the reader scales by powers of two.
 // Idle lanes take new particles from a global counter, one atomic per warp.
-// Comparisons, min/max and the float -> double widening run on the integer
-// pipe.  The random words of a pass come from one Philox block per lane
+// The random words of a pass come from one Philox block per lane
 // (pass_block); a flight that ends at a void wall or by scattering draws
 // its next mode in one block for both cases (Lambert row or post-scattering
 // alias table) and draws the next flight length there.
 //
-// ADJ selects the two passes of the adjoint (ADJ = 0 is the plain kernel):
-// 1 forward: also accumulates each particle's contribution to a linear
-//   functional Phi = sum W[box][bin][q] tally[box][bin][q] and stores it;
+// ADJ selects the two passes of the adjoint (ADJ = 0 is the plain kernel),
+// which need no tally:
+// 1 forward: accumulates each particle's contribution to a linear functional
+//   Phi = sum W[box][bin][q] tally[box][bin][q] (W in the walk's units);
 // 2 adjoint: replays every particle from its Philox counter (the same draws
 //   as pass 1) and adds likelihood-ratio terms, each weighted by the
 //   particle's future contribution R = Phi_total - Phi so far:
@@ -471,6 +491,7 @@ __device__ __forceinline__ uint4 pass_block(uint32_t pass, uint64_t pid, uint64_
 // CHECK: the checked variant (BTE_FLAG_CHECKS): every table, tally and grid
 // index is tested before use; a violation stops the particle with E_CHECK.
 // The checks draw nothing, so the trajectories are the plain variant's.
+// A particle that stops with an error leaves its pending sums: the run fails.
 template <bool SMEM_TALLY, int MINB, int ADJ, bool CHECK = false>
 __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs A, double* gtally,
                                                      unsigned long long* counters, int* err,
@@ -486,301 +507,274 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
     Counters c = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     const int lane = threadIdx.x & 31;
     const long long total = T.pend - T.pbegin;
-    const int last_bin = T.nbins - 1;
-    // specular draw on the integer pipe: u32 < p 2^32 (p >= 1: always);
-    // 0 when the walls are diffuse
+    const FixScale& F = A.fx;
+    const int last_bin = T.nbins - 1, last_part = (1 << F.sub) - 1;
+    const int row = A.G.ny + 2;  // cells of a column of the padded map
+    // a particle's flights fit 32 bits: a larger cap is never met
+    const uint32_t cap = T.flight_cap < 0xffffffffll ? uint32_t(T.flight_cap) : 0xffffffffu;
+    // specular draw on the integer pipe: u32 < p 2^32 (p >= 1: always)
     const unsigned long long spec_thr =
         T.specularity >= 1.0 ? (1ull << 32)
                              : (T.specularity > 0. ? (unsigned long long)(T.specularity * 4294967296.0) : 0ull);
-    Pending pd;
-    pd.key = -1;
-    pd.flushes = 0;
-    pd.r0 = pd.x0 = pd.y0 = 0.;
-    GridParticle p;
-    p.i = p.j = p.mode = p.box = p.mo = 0;
-    p.sign = 1;
-    p.x = p.y = p.t = 0.;
-    Philox g;
-    g.init(0, 0);
-    ModeVel mv = {0., 0., 0., 0.};
-    // dt: time left in the free flight; rb: time left to the end of the
-    // current time bin (bin widths follow the ntime grid points)
-    const double* binw = T.timegrid + T.ntime;
-    double dt = 0., rb = 0.;
-    long long pid = -1, nev = 0;
+    const double score_spec = 1.0 / T.specularity, score_diff = -1.0 / (1.0 - T.specularity);
+    const uint64_t* binw = bin_ticks(T);
+    // the particle: mode, box and its column, line and place in the padded
+    // map, material offset, time bin and which of its 2^sub parts
+    int mode = 0, box = 0, ci = 0, cj = 0, cell = 0, mo = 0, bin = 0, part = 0;
+    uint64_t flip = 0;  // FIX_DOWN for a particle of negative sign
+    ModeFix mv = {0, 0, ~0ull, ~0ull};
+    uint64_t ax = 0, ay = 0;
+    // ticks left in the free flight (96 bits) and to the end of the bin part
+    uint64_t dt_lo = 0, rb = 0;
+    uint32_t dt_hi = 0;
+    uint64_t pt = 0;  // pending: ticks, and displacement times the sign
+    int64_t px = 0, py = 0;
+    long long pid = -1;
+    uint32_t nev = 0, npass = 0;
     double* tgrp = tally;  // the tally of the particle's replica group
-    uint32_t npass = 0;
-    int bin = 0;
-    unsigned long long signbit = 0;
     bool active = false, done = false;
     // adjoint state: Phi so far, the particle's total, pending score terms
     double phi_run = 0., phi_tot = 0., spec_score = 0.;
     double sum_r = 0., g_p = 0., phi_all = 0.;
     long long slot = 0;
     int pend_kind = 0;
-    // A new free flight of the current mode from one random word:
-    // dt = -tau ln u (FP32 log), u = (k + 1/2) 2^-23 from 23 bits, never 0
-    // or 1; its velocities stay in registers for the segments that follow.
-    // Returns false when the particle stops with an error.
-    // a failed index check stops the particle (checked variant only)
-    auto check_fail = [&]() {
-        record_error(err, E_CHECK, pid);
+    // the particle stops with an error
+    auto stop = [&](int e) {
+        record_error(err, e, pid);
         active = false;
         done = true;
     };
-    auto new_flight = [&](uint32_t word) -> bool {
-        const int k = p.mode;
-        if (CHECK && (k < 0 || k >= T.n || p.mo < 0)) {
-            check_fail();
-            return false;
+    // The functional's part of the pending sums.
+    auto weighted = [&]() -> double {
+        const double* Wk = adj.W + 3ll * (box * T.nbins + bin);
+        const double t = double((long long)pt);
+        return __ldg(Wk) * (flip ? -t : t) + __ldg(Wk + 1) * double((long long)px) +
+               __ldg(Wk + 2) * double((long long)py);
+    };
+    // A new free flight of the current mode from one random word:
+    // dt = -tau ln u (FP32 log), u = (k + 1/2) 2^-23 from 23 bits, never 0
+    // or 1; its velocities stay in registers for the segments that follow.
+    // Where a direction turns, the border ahead is the other one.
+    auto new_flight = [&](uint32_t word) {
+        if (CHECK && (mode < 0 || mode >= T.n || mo < 0)) {
+            stop(E_CHECK);
+            return;
         }
-        mv = A.mv[k];
+        const ModeFix m = A.mf[mode];
         const float ef = -logf((float(word >> 9) + 0.5f) * 0x1p-23f);
-        const double tau_k = __ldg(T.tau + p.mo + k);
-        dt = widen_pos(ef) * tau_k;
+        const double tau_k = __ldg(T.tau + mo + mode);
+        if ((m.vx ^ mv.vx) & FIX_DOWN) ax = __ldg(A.wxf + ci) - ax;
+        if ((m.vy ^ mv.vy) & FIX_DOWN) ay = __ldg(A.wyf + cj) - ay;
+        mv = m;
+        dt_lo = fix_flight(ef, tau_k, F.kt, dt_hi);
         c.events++;
         if (ADJ == 2) {
             // future contribution from here: Phi_total - (flushed + pending part)
-            const double* Wk = adj.W + 3ll * pd.key;
-            const double part = __ldg(Wk) * (pd.r0 - rb) + __ldg(Wk + 1) * (p.x - pd.x0) +
-                                __ldg(Wk + 2) * (p.y - pd.y0);
-            const double R = phi_tot - (phi_run + (p.sign < 0 ? -part : part));
-            double gk = (widen_pos(ef) - 1.0) / tau_k * R;
-            if (pend_kind & 1) {  // this mode came from a post-scattering draw
-                gk -= R / tau_k;
-                sum_r += R;
-            }
+            const double R = phi_tot - (phi_run + weighted());
+            // the flight's (e - 1) / tau and, for a mode from a
+            // post-scattering draw, that draw's -1 / tau
+            const double gk = (widen_pos(ef) - ((pend_kind & 1) ? 2.0 : 1.0)) * (R * __ldg(T.w + mo + mode));
+            if (pend_kind & 1) sum_r += R;
             if (pend_kind & 2) g_p += spec_score * R;
             pend_kind = 0;
-            atomicAdd(adj.g_tau + k, gk);
+            atomicAdd(adj.g_tau + mode, gk);
         }
-        if (ob(dt) <= 0 || ++nev > T.flight_cap) {  // zero rate or runaway particle
-            record_error(err, ob(dt) > 0 ? E_LIMIT : E_VALUE, pid);
-            active = false;
-            done = true;
-            pd.flush(tgrp, signbit, rb, p.x, p.y);
-            return false;
-        }
-        return true;
+        // zero rate or runaway particle
+        if (++nev > cap || tau_k <= 0.) stop(tau_k > 0. ? E_LIMIT : E_VALUE);
     };
     for (;;) {
-        // refill idle lanes of the warp with new particles
-        const unsigned idle = __ballot_sync(0xffffffffu, !active && !done);
-        if (idle) {
+        // refill idle lanes of the warp with new particles; a lane is done when
+        // the counter has run out or its particle stopped with an error
+        if (!__all_sync(0xffffffffu, active)) {
+            const unsigned idle = __ballot_sync(0xffffffffu, !active && !done);
             unsigned long long base = 0;
-            const int leader = __ffs(idle) - 1;
-            if (lane == leader) base = atomicAdd(work, (unsigned long long)__popc(idle));
+            const int leader = idle ? __ffs(idle) - 1 : 0;
+            if (idle && lane == leader) base = atomicAdd(work, (unsigned long long)__popc(idle));
             base = __shfl_sync(0xffffffffu, base, leader);
             if (!active && !done) {
                 const long long mine = (long long)base + __popc(idle & ((1u << lane) - 1u));
                 if (mine < total) {
                     pid = T.pbegin + mine;
                     tgrp = T.ngroups > 1 ? tally + (long long)(pid % T.ngroups) * T.group_stride : tally;
+                    Philox g;
                     g.init(T.seed, (uint64_t)pid);
+                    GridParticle p;
                     int e = grid_generate(T, A.G, A.boxcell, g, pid, p);
                     if (CHECK && !e &&
                         (p.box < 0 || p.box >= T.nboxes || p.i < 0 || p.i >= A.G.nx || p.j < 0 || p.j >= A.G.ny))
                         e = E_CHECK;
                     if (e) {
-                        record_error(err, e, pid);
-                        done = true;
+                        stop(e);
                     } else {
                         active = true;
-                        nev = 0;
-                        npass = 0;
+                        mode = p.mode;
+                        box = p.box;
+                        mo = p.mo;
+                        ci = p.i;
+                        cj = p.j;
+                        cell = (ci + 1) * row + cj + 1;
+                        flip = p.sign < 0 ? FIX_DOWN : 0;
+                        nev = npass = 0;
                         if (ADJ) {
                             slot = mine;
                             phi_run = 0.;
                             pend_kind = 0;
                             if (ADJ == 2) phi_tot = adj.phi_total[mine];
                         }
-                        bin = 0;
+                        bin = part = 0;
                         rb = __ldg(binw);
-                        signbit = p.sign < 0 ? 0x8000000000000000ull : 0ull;
-                        pd.start(p.box * T.nbins, rb, p.x, p.y);
+                        pt = 0;
+                        px = py = 0;
+                        // the distances as for a flight towards larger
+                        // coordinates; the flight turns them where it goes
+                        mv.vx = mv.vy = 0;
+                        const long long dx = A.gxf[ci + 1] - fix_round(p.x - F.x0, F.kx);
+                        const long long dy = A.gyf[cj + 1] - fix_round(p.y - F.y0, F.kx);
+                        const long long wx = A.wxf[ci], wy = A.wyf[cj];
+                        ax = dx < 0 ? 0 : dx > wx ? wx : dx;
+                        ay = dy < 0 ? 0 : dy > wy ? wy : dy;
                         new_flight(g.next32());  // the first flight, from the generation stream
                     }
                 } else {
                     done = true;
                 }
             }
+            if (__all_sync(0xffffffffu, !active)) {
+                // a lane whose first flight already failed leaves others to refill
+                if (__all_sync(0xffffffffu, done)) break;
+                continue;
+            }
         }
-        if (__all_sync(0xffffffffu, done)) break;
-        if (!active) continue;
-        // this pass's random words (used at its end); computed ahead of the
-        // segment, with which it shares no data
-        const uint4 rr = pass_block(npass++, (uint64_t)pid, T.seed);
-        // segment end.  A zero velocity component takes the upper cell line,
-        // so (line - position) >= 0 times its +inf inverse gives +inf (or NaN
-        // on the line, ordered above +inf); a negative value (a position that
-        // rounded past its line) orders below 0 and ends the segment at once.
-        if (CHECK && (p.i < 0 || p.i >= A.G.nx || p.j < 0 || p.j >= A.G.ny || p.box < 0 || p.box >= T.nboxes ||
-                      bin < 0 || bin > last_bin)) {
-            check_fail();
-            continue;
-        }
-        const int upx = ob(mv.vx) >= 0 ? 1 : 0;
-        const int upy = ob(mv.vy) >= 0 ? 1 : 0;
-        const double xw = __ldg(A.G.gx + p.i + upx);
-        const double yw = __ldg(A.G.gy + p.j + upy);
-        const double tx = (xw - p.x) * mv.ivx;
-        const double ty = (yw - p.y) * mv.ivy;
-        const double tb = rb;
-        const bool xfirst = ob(tx) <= ob(ty);
-        long long te_b = xfirst ? ob(tx) : ob(ty);
-        long long tb_b = ob(tb);
-        te_b = te_b > 0 ? te_b : 0;
-        tb_b = tb_b > 0 ? tb_b : 0;
-        const long long dt_b = ob(dt);
-        const long long lim_b = te_b < tb_b ? te_b : tb_b;
-        const bool flight_end = !(dt_b > lim_b);             // the flight ends first (or ties)
-        const long long seg_b = flight_end ? dt_b : lim_b;
-        const bool wall = !flight_end && te_b <= tb_b;         // reaches a cell line
-        const bool bin_end = tb_b <= seg_b;                    // reaches the bin border
-        const double seg = obd(seg_b);
-        double r1 = rb - seg;
-        double nx = fma(seg, mv.vx, p.x);
-        double ny = fma(seg, mv.vy, p.y);
-        dt -= seg;
-        if (bin_end) r1 = 0.;
-        int ni = p.i, nj = p.j, wside = 0;
-        if (wall) {  // the crossed coordinate is the grid line
-            if (xfirst) {
-                nx = xw;
-                ni = p.i + (upx ? 1 : -1);
-                wside = upx ? 0 : 1;
+        if (active) {
+            // this pass's random words (used at its end); computed ahead of
+            // the segment, with which it shares no data
+            const uint4 rr = pass_block(npass++, (uint64_t)pid, T.seed);
+            if (CHECK && (ci < 0 || ci >= A.G.nx || cj < 0 || cj >= A.G.ny || box < 0 || box >= T.nboxes || bin < 0 ||
+                          bin > last_bin)) {
+                stop(E_CHECK);
+                continue;
+            }
+            const FixSeg q = fix_segment(ax, ay, mv, dt_lo, dt_hi, rb);
+            const bool border = q.cross_x || q.cross_y;
+            const bool downx = (long long)mv.vx < 0, downy = (long long)mv.vy < 0;
+            // what lies across the border
+            const int step = q.cross_x ? (downx ? -row : row) : (downy ? -1 : 1);
+            int nb = box;
+            if (border) nb = __ldg(A.map + cell + step);
+            ax -= q.dx;
+            ay -= q.dy;
+            const int64_t fx = (int64_t)(mv.vx ^ flip) >> 63, fy = (int64_t)(mv.vy ^ flip) >> 63;
+            px += ((int64_t)q.dx ^ fx) - fx;
+            py += ((int64_t)q.dy ^ fy) - fy;
+            pt += q.seg;
+            rb -= q.seg;
+            dt_hi -= dt_lo < q.seg ? 1u : 0u;
+            dt_lo -= q.seg;
+            // spectral decomposition: the segment's time per mode at selected boxes
+            if (ADJ == 0 && T.spec_loc) {
+                const int loc = __ldg(T.spec_loc + box);
+                if (loc >= 0) {
+                    const double ds = double((long long)q.seg);
+                    atomicAdd(T.spec + (long long)(loc * T.nbins + bin) * T.n + mode, flip ? -ds : ds);
+                }
+            }
+            const bool reflect = nb == -1;              // void: reflection, a new flight follows
+            const bool leave = border && !reflect;      // into the next cell or a reservoir
+            if (CHECK && (box * T.nbins + bin >= T.nboxes * T.nbins || nb >= T.nboxes)) {
+                stop(E_CHECK);
+                continue;
+            }
+            if (leave || q.bin_end) {
+                if (ADJ) {
+                    phi_run += weighted();
+                } else {
+                    double* b = tgrp + 3ll * (box * T.nbins + bin);
+                    const double t = double((long long)pt);
+                    if (pt) atomicAdd(b + 0, flip ? -t : t);
+                    if (px) atomicAdd(b + 1, double((long long)px));
+                    if (py) atomicAdd(b + 2, double((long long)py));
+                }
+                if (leave || part == last_part) c.tallies++;
+                pt = 0;
+                px = py = 0;
+                if (leave) {
+                    if (nb >= 0) {
+                        box = nb;
+                        cell += step;
+                        if (q.cross_x) {
+                            ci += downx ? -1 : 1;
+                            ax = __ldg(A.wxf + ci);
+                        } else {
+                            cj += downy ? -1 : 1;
+                            ay = __ldg(A.wyf + cj);
+                        }
+                        c.crossings++;
+                    } else {
+                        c.absorbed++;
+                        active = false;
+                    }
+                } else {
+                    if (part == last_part) {
+                        part = 0;
+                        active = ++bin <= last_bin;
+                    } else {
+                        ++part;
+                    }
+                    if (active) rb = __ldg(binw + bin);
+                }
+                if (ADJ == 1 && !active) {
+                    adj.phi_total[slot] = phi_run;
+                    phi_all += phi_run;
+                }
             } else {
-                ny = yw;
-                nj = p.j + (upy ? 1 : -1);
-                wside = upy ? 2 : 3;
-            }
-        }
-        // spectral decomposition: the segment's time per mode at selected boxes
-        if (ADJ == 0 && T.spec_loc) {
-            const int loc = __ldg(T.spec_loc + p.box);
-            if (loc >= 0) {
-                const double ds = rb - r1;
-                atomicAdd(T.spec + (long long)(loc * T.nbins + bin) * T.n + p.mode, p.sign < 0 ? -ds : ds);
-            }
-        }
-        // differences of the pending tally at the segment end (telescoping)
-        const double d0 = pd.r0 - r1, d1 = nx - pd.x0, d2 = ny - pd.y0;
-        rb = r1;
-        p.x = nx;
-        p.y = ny;
-        int nb = p.box;
-        if (wall) nb = grid_cell(A.G, ni, nj);
-        const bool move = wall && nb >= 0;        // into the next cell
-        const bool absorbed = wall && nb <= -2;   // into a reservoir
-        const bool reflect = wall && nb == -1;    // void: reflection, a new flight follows
-        const bool last = bin_end && bin == last_bin;
-        if (ADJ && (move || absorbed || bin_end)) {
-            const double* Wk = adj.W + 3ll * pd.key;
-            const double cphi = __ldg(Wk) * d0 + __ldg(Wk + 1) * d1 + __ldg(Wk + 2) * d2;
-            phi_run += p.sign < 0 ? -cphi : cphi;
-        }
-        if (CHECK && (move || absorbed || bin_end) && (pd.key < 0 || pd.key >= T.nboxes * T.nbins)) {
-            check_fail();
-            continue;
-        }
-        if (CHECK && move && nb >= T.nboxes) {
-            check_fail();
-            continue;
-        }
-        if (move || absorbed || bin_end) {
-            double* b = tgrp + 3ll * pd.key;
-            atomicAdd(b + 0, __longlong_as_double(__double_as_longlong(d0) ^ signbit));
-            atomicAdd(b + 1, __longlong_as_double(__double_as_longlong(d1) ^ signbit));
-            atomicAdd(b + 2, __longlong_as_double(__double_as_longlong(d2) ^ signbit));
-            pd.flushes++;
-            pd.key = -1;
-        }
-        if (absorbed || last) {
-            if (absorbed) c.absorbed++;
-            active = false;
-            if (ADJ == 1) {
-                adj.phi_total[slot] = phi_run;
-                phi_all += phi_run;
-            }
-            continue;
-        }
-        if (bin_end) {
-            ++bin;
-            rb = __ldg(binw + bin);
-        }
-        if (move) {
-            p.i = ni;
-            p.j = nj;
-            p.box = nb;
-            c.crossings++;
-        }
-        if (move || bin_end) pd.start(p.box * T.nbins + bin, rb, nx, ny);
-        if (reflect || flight_end) {
-            // the next mode: a Lambert row at a void wall (or the mirror
-            // mode on a specular draw), the post-scattering table after a
-            // scattering (none for ballistic runs)
-            const int k = p.mode;
-            int nm = k;
-            if (reflect || !T.ballistic) {
-                float pr = 0.f;
-                int keep = k, alt = k;
+                // the next mode: a Lambert row at a void wall (or the mirror
+                // mode on a specular draw), the post-scattering table after a
+                // scattering (none for ballistic runs)
+                float pr = 2.f;  // keep whatever the acceptance word
+                int keep = mode, alt = mode;
                 if (reflect) {
                     // (selects, not an indexed parameter array, which would live in local memory)
-                    const int cls =
-                        wside == 0 ? A.cls[0] : wside == 1 ? A.cls[1] : wside == 2 ? A.cls[2] : A.cls[3];
-                    if (cls < 0) {
-                        record_error(err, E_GEOM, pid);
-                        active = false;
-                        done = true;
-                        pd.flush(tgrp, signbit, rb, p.x, p.y);
+                    const int cls = q.cross_x ? (downx ? A.cls[1] : A.cls[0]) : (downy ? A.cls[3] : A.cls[2]);
+                    if (cls < 0 || (CHECK && cls >= T.nclass)) {
+                        stop(cls < 0 ? E_GEOM : E_CHECK);
                         continue;
                     }
-                    if (CHECK && cls >= T.nclass) {
-                        check_fail();
-                        continue;
-                    }
+                    const long long r = (long long)cls * T.n + mode;
                     int mirror_mode = -1;
                     if (spec_thr) {
-                        const bool spec = (unsigned long long)rr.w < spec_thr;
+                        const bool spec = rr.w < spec_thr;
                         if (ADJ == 2) {
-                            spec_score = spec ? 1.0 / T.specularity : -1.0 / (1.0 - T.specularity);
+                            spec_score = spec ? score_spec : score_diff;
                             pend_kind |= 2;
                         }
-                        if (spec && T.mirror) mirror_mode = __ldg(T.mirror + (long long)cls * T.n + k);
+                        if (spec && T.mirror) mirror_mode = __ldg(T.mirror + r);
                     }
                     if (mirror_mode >= 0) {
                         c.specular++;
-                        pr = 2.f;  // keep = the mirror mode whatever the acceptance word
                         keep = mirror_mode;
                     } else {
-                        const long long a = __ldg(T.row_ptr + (long long)cls * (T.n + 1) + k);
-                        const long long bb = __ldg(T.row_ptr + (long long)cls * (T.n + 1) + k + 1);
-                        const int len = int(bb - a);
-                        if (len <= 0) {
-                            record_error(err, E_GEOM, pid);
-                            active = false;
-                            done = true;
-                            pd.flush(tgrp, signbit, rb, p.x, p.y);
+                        const LambertRow lr = lambert_row(T, r);
+                        if (lr.len == 0) {
+                            stop(E_GEOM);
                             continue;
                         }
-                        const int4 e = __ldg(T.lalias + a + int(mulhi32(rr.y, uint32_t(len))));
+                        const int4 e = __ldg(T.lalias + lr.off + mulhi32(rr.y, lr.len));
                         pr = __int_as_float(e.x);
                         keep = e.y;
                         alt = e.z;
                     }
                     c.wall_hits++;
-                } else {
-                    const int j = int(mulhi32(rr.y, uint32_t(T.n)));
-                    pr = __ldg(T.resample_prob + p.mo + j);
-                    keep = j;
-                    alt = __ldg(T.resample_alt + p.mo + j);
+                } else if (!T.ballistic) {
+                    keep = int(mulhi32(rr.y, uint32_t(T.n)));
+                    const int2 e = __ldg(T.resample + mo + keep);
+                    pr = __int_as_float(e.x);
+                    alt = e.y;
                     if (ADJ == 2) pend_kind |= 1;
                 }
                 const float acc = float(rr.z >> 8) * 0x1p-24f;
-                nm = acc < pr ? keep : alt;
+                mode = acc < pr ? keep : alt;
+                new_flight(rr.x);
             }
-            p.mode = nm;
-            if (!new_flight(rr.x)) continue;
         }
     }
     if (ADJ) {
@@ -795,291 +789,51 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
             atomicAdd(adj.g_scalar + 2, phi_all);
         }
     }
-    c.tallies = pd.flushes;
     flush_counters_p<8>(c, counters);  // no periodic boxes on the grid path
     if (SMEM_TALLY) {
         __syncthreads();
         for (int k = threadIdx.x; k < nk3; k += blockDim.x) {
-            const double x = stally[k];
-            if (x != 0.) atomicAdd(gtally + k, x);
+            const double v = stally[k];
+            if (v != 0.) atomicAdd(gtally + k, v);
         }
     }
 }
 
-// ------------------------------------------------ grid path, PPT per thread
-
-// One particle slot of the interleaved grid kernel.
-struct GridSlot {
-    GridParticle p;
-    Pending pd;
-    Philox g;
-    ModeVel mv;
-    double* tb;  // the tally of the particle's replica group
-    double dt, rb;
-    long long pid, nev;
-    uint32_t npass;
-    int bin;
-    unsigned long long signbit;
-    bool active, done;
-};
-
-// The segment one slot takes in one pass.
-struct GridSeg {
-    uint4 rr;
-    double r1, nx, ny, dt, d0, d1, d2;
-    int ni, nj, wside;
-    bool xfirst, flight_end, wall, bin_end;
-};
-
-// The plain production grid kernel (global tally, no spectral locations)
-// with PPT particles per thread.  It follows rta_prod_grid's loop (same
-// draws, same segments, same tallies) but splits every pass in two phases:
-// first the segment of each slot, a straight-line FP64 sequence computed for
-// every slot (a slot without a particle computes on its last state, whose
-// indices stay in range, and drops the result), so that the FP64 chains of
-// the PPT particles interleave and hide each other's latency; then, slot
-// by slot, the branchy end of the segment (tally flush, crossing, wall or
-// scattering redraw).  Each slot refills from the global particle counter
-// on its own ballot.
-template <int PPT, int MINB>
-__global__ void __launch_bounds__(256, MINB) rta_prod_grid_ilp(DevTables T, GridArgs A, double* tally,
-                                                         unsigned long long* counters, int* err,
-                                                         unsigned long long* work) {
-    Counters c = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const int lane = threadIdx.x & 31;
-    const long long total = T.pend - T.pbegin;
-    const int last_bin = T.nbins - 1;
-    const unsigned long long spec_thr =
-        T.specularity >= 1.0 ? (1ull << 32)
-                             : (T.specularity > 0. ? (unsigned long long)(T.specularity * 4294967296.0) : 0ull);
-    const double* binw = T.timegrid + T.ntime;
-    GridSlot S[PPT];
-#pragma unroll
-    for (int s = 0; s < PPT; ++s) {
-        GridSlot& L = S[s];
-        L.pd.key = -1;
-        L.pd.flushes = 0;
-        L.pd.r0 = L.pd.x0 = L.pd.y0 = 0.;
-        L.p.i = L.p.j = L.p.mode = L.p.box = L.p.mo = 0;
-        L.p.sign = 1;
-        L.p.x = L.p.y = L.p.t = 0.;
-        L.g.init(0, 0);
-        L.mv = ModeVel{0., 0., 0., 0.};
-        L.dt = L.rb = 0.;
-        L.pid = -1;
-        L.tb = tally;
-        L.nev = 0;
-        L.npass = 0;
-        L.bin = 0;
-        L.signbit = 0;
-        L.active = L.done = false;
+// The integer tables of a run's scales: every mode's velocity record, the
+// grid lines and the widths between them (fixed_walk.cuh).
+__global__ void fix_tables(FixScale f, const ModeVel* mv, int n, ModeFix* mf, DevGrid G, long long* gxf,
+                           long long* gyf, long long* wxf, long long* wyf) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    auto line = [&](const double* g, int k, double o) { return fix_round(g[k] - o, f.kx); };
+    if (i < n) {
+        ModeFix m;
+        fix_velocity(mv[i].vx, f, m.vx, m.rx);
+        fix_velocity(mv[i].vy, f, m.vy, m.ry);
+        mf[i] = m;
     }
-    // a new free flight of the slot's current mode from one random word (as
-    // rta_prod_grid's new_flight); false when the particle stops with an error
-    auto new_flight = [&](GridSlot& L, uint32_t word) -> bool {
-        const int k = L.p.mode;
-        L.mv = A.mv[k];
-        const float ef = -logf((float(word >> 9) + 0.5f) * 0x1p-23f);
-        L.dt = widen_pos(ef) * __ldg(T.tau + L.p.mo + k);
-        c.events++;
-        if (ob(L.dt) <= 0 || ++L.nev > T.flight_cap) {
-            record_error(err, ob(L.dt) > 0 ? E_LIMIT : E_VALUE, L.pid);
-            L.active = false;
-            L.done = true;
-            L.pd.flush(L.tb, L.signbit, L.rb, L.p.x, L.p.y);
-            return false;
-        }
-        return true;
-    };
-    // the branchy end of one slot's segment
-    auto finish = [&](GridSlot& L, const GridSeg& G) {
-        L.dt = G.dt;
-        L.rb = G.r1;
-        L.p.x = G.nx;
-        L.p.y = G.ny;
-        int nb = L.p.box;
-        if (G.wall) nb = grid_cell(A.G, G.ni, G.nj);
-        const bool move = G.wall && nb >= 0;
-        const bool absorbed = G.wall && nb <= -2;
-        const bool reflect = G.wall && nb == -1;
-        const bool last = G.bin_end && L.bin == last_bin;
-        if (move || absorbed || G.bin_end) {
-            double* b = L.tb + 3ll * L.pd.key;
-            atomicAdd(b + 0, __longlong_as_double(__double_as_longlong(G.d0) ^ L.signbit));
-            atomicAdd(b + 1, __longlong_as_double(__double_as_longlong(G.d1) ^ L.signbit));
-            atomicAdd(b + 2, __longlong_as_double(__double_as_longlong(G.d2) ^ L.signbit));
-            L.pd.flushes++;
-            L.pd.key = -1;
-        }
-        if (absorbed || last) {
-            if (absorbed) c.absorbed++;
-            L.active = false;
-            return;
-        }
-        if (G.bin_end) {
-            ++L.bin;
-            L.rb = __ldg(binw + L.bin);
-        }
-        if (move) {
-            L.p.i = G.ni;
-            L.p.j = G.nj;
-            L.p.box = nb;
-            c.crossings++;
-        }
-        if (move || G.bin_end) L.pd.start(L.p.box * T.nbins + L.bin, L.rb, G.nx, G.ny);
-        if (reflect || G.flight_end) {
-            const int k = L.p.mode;
-            int nm = k;
-            if (reflect || !T.ballistic) {
-                float pr = 0.f;
-                int keep = k, alt = k;
-                if (reflect) {
-                    const int cls = G.wside == 0   ? A.cls[0]
-                                    : G.wside == 1 ? A.cls[1]
-                                    : G.wside == 2 ? A.cls[2]
-                                                   : A.cls[3];
-                    if (cls < 0) {
-                        record_error(err, E_GEOM, L.pid);
-                        L.active = false;
-                        L.done = true;
-                        L.pd.flush(L.tb, L.signbit, L.rb, L.p.x, L.p.y);
-                        return;
-                    }
-                    int mirror_mode = -1;
-                    if (spec_thr && (unsigned long long)G.rr.w < spec_thr && T.mirror)
-                        mirror_mode = __ldg(T.mirror + (long long)cls * T.n + k);
-                    if (mirror_mode >= 0) {
-                        c.specular++;
-                        pr = 2.f;
-                        keep = mirror_mode;
-                    } else {
-                        const long long a = __ldg(T.row_ptr + (long long)cls * (T.n + 1) + k);
-                        const long long bb = __ldg(T.row_ptr + (long long)cls * (T.n + 1) + k + 1);
-                        const int len = int(bb - a);
-                        if (len <= 0) {
-                            record_error(err, E_GEOM, L.pid);
-                            L.active = false;
-                            L.done = true;
-                            L.pd.flush(L.tb, L.signbit, L.rb, L.p.x, L.p.y);
-                            return;
-                        }
-                        const int4 e = __ldg(T.lalias + a + int(mulhi32(G.rr.y, uint32_t(len))));
-                        pr = __int_as_float(e.x);
-                        keep = e.y;
-                        alt = e.z;
-                    }
-                    c.wall_hits++;
-                } else {
-                    const int j = int(mulhi32(G.rr.y, uint32_t(T.n)));
-                    pr = __ldg(T.resample_prob + L.p.mo + j);
-                    keep = j;
-                    alt = __ldg(T.resample_alt + L.p.mo + j);
-                }
-                const float acc = float(G.rr.z >> 8) * 0x1p-24f;
-                nm = acc < pr ? keep : alt;
-            }
-            L.p.mode = nm;
-            new_flight(L, G.rr.x);
-        }
-    };
-    for (;;) {
-#pragma unroll
-        for (int s = 0; s < PPT; ++s) {
-            GridSlot& L = S[s];
-            const unsigned idle = __ballot_sync(0xffffffffu, !L.active && !L.done);
-            if (idle) {
-                unsigned long long base = 0;
-                const int leader = __ffs(idle) - 1;
-                if (lane == leader) base = atomicAdd(work, (unsigned long long)__popc(idle));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (!L.active && !L.done) {
-                    const long long mine = (long long)base + __popc(idle & ((1u << lane) - 1u));
-                    if (mine < total) {
-                        L.pid = T.pbegin + mine;
-                        L.tb = T.ngroups > 1 ? tally + (long long)(L.pid % T.ngroups) * T.group_stride : tally;
-                        L.g.init(T.seed, (uint64_t)L.pid);
-                        const int e = grid_generate(T, A.G, A.boxcell, L.g, L.pid, L.p);
-                        if (e) {
-                            record_error(err, e, L.pid);
-                            L.done = true;
-                        } else {
-                            L.active = true;
-                            L.nev = 0;
-                            L.npass = 0;
-                            L.bin = 0;
-                            L.rb = __ldg(binw);
-                            L.signbit = L.p.sign < 0 ? 0x8000000000000000ull : 0ull;
-                            L.pd.start(L.p.box * T.nbins, L.rb, L.p.x, L.p.y);
-                            new_flight(L, L.g.next32());
-                        }
-                    } else {
-                        L.done = true;
-                    }
-                }
-            }
-        }
-        bool finished = true;
-#pragma unroll
-        for (int s = 0; s < PPT; ++s) finished = finished && S[s].done;
-        if (__all_sync(0xffffffffu, finished)) break;
-        // phase 1: every slot's segment, straight-line
-        GridSeg G[PPT];
-#pragma unroll
-        for (int s = 0; s < PPT; ++s) {
-            GridSlot& L = S[s];
-            GridSeg& q = G[s];
-            q.rr = pass_block(L.npass, (uint64_t)L.pid, T.seed);
-            L.npass += L.active ? 1u : 0u;
-            const int upx = ob(L.mv.vx) >= 0 ? 1 : 0;
-            const int upy = ob(L.mv.vy) >= 0 ? 1 : 0;
-            const double xw = __ldg(A.G.gx + L.p.i + upx);
-            const double yw = __ldg(A.G.gy + L.p.j + upy);
-            const double tx = (xw - L.p.x) * L.mv.ivx;
-            const double ty = (yw - L.p.y) * L.mv.ivy;
-            q.xfirst = ob(tx) <= ob(ty);
-            long long te_b = q.xfirst ? ob(tx) : ob(ty);
-            long long tb_b = ob(L.rb);
-            te_b = te_b > 0 ? te_b : 0;
-            tb_b = tb_b > 0 ? tb_b : 0;
-            const long long dt_b = ob(L.dt);
-            const long long lim_b = te_b < tb_b ? te_b : tb_b;
-            q.flight_end = !(dt_b > lim_b);
-            const long long seg_b = q.flight_end ? dt_b : lim_b;
-            q.wall = !q.flight_end && te_b <= tb_b;
-            q.bin_end = tb_b <= seg_b;
-            const double seg = obd(seg_b);
-            q.r1 = q.bin_end ? 0. : L.rb - seg;
-            q.nx = fma(seg, L.mv.vx, L.p.x);
-            q.ny = fma(seg, L.mv.vy, L.p.y);
-            q.dt = L.dt - seg;
-            q.ni = L.p.i;
-            q.nj = L.p.j;
-            q.wside = 0;
-            if (q.wall) {
-                if (q.xfirst) {
-                    q.nx = xw;
-                    q.ni = L.p.i + (upx ? 1 : -1);
-                    q.wside = upx ? 0 : 1;
-                } else {
-                    q.ny = yw;
-                    q.nj = L.p.j + (upy ? 1 : -1);
-                    q.wside = upy ? 2 : 3;
-                }
-            }
-            q.d0 = L.pd.r0 - q.r1;
-            q.d1 = q.nx - L.pd.x0;
-            q.d2 = q.ny - L.pd.y0;
-        }
-        // phase 2: the ends of the segments, slot by slot
-#pragma unroll
-        for (int s = 0; s < PPT; ++s)
-            if (S[s].active) finish(S[s], G[s]);
+    if (i <= G.nx) gxf[i] = line(G.gx, i, f.x0);
+    if (i <= G.ny) gyf[i] = line(G.gy, i, f.y0);
+    if (i < G.nx) wxf[i] = line(G.gx, i + 1, f.x0) - line(G.gx, i, f.x0);
+    if (i < G.ny) wyf[i] = line(G.gy, i + 1, f.y0) - line(G.gy, i, f.y0);
+}
+
+void launch_fix_tables(const FixScale& f, const ModeVel* mv, int n, ModeFix* mf, const DevGrid& G, long long* gxf,
+                       long long* gyf, long long* wxf, long long* wyf, cudaStream_t s) {
+    const int g = G.nx > G.ny ? G.nx + 1 : G.ny + 1, m = n > g ? n : g;
+    fix_tables<<<(m + 255) / 256, 256, 0, s>>>(f, mv, n, mf, G, gxf, gyf, wxf, wyf);
+}
+
+__global__ void scale_tally_k(double* t, long long nk, double st, double sx) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nk; i += (long long)gridDim.x * blockDim.x) {
+        t[3 * i] *= st;
+        t[3 * i + 1] *= sx;
+        t[3 * i + 2] *= sx;
     }
-    unsigned flushes = 0;
-#pragma unroll
-    for (int s = 0; s < PPT; ++s) flushes += S[s].pd.flushes;
-    c.tallies = flushes;
-    flush_counters_p<8>(c, counters);
+}
+void launch_scale_tally(double* tally, long long nk, const FixScale& f, int nsm, cudaStream_t s) {
+    long long b = (nk + 255) / 256;
+    if (b > nsm * 8ll) b = nsm * 8ll;
+    scale_tally_k<<<unsigned(b), 256, 0, s>>>(tally, nk, f.per_tick(), f.per_unit());
 }
 
 // ------------------------------------------------------------ polygon path
@@ -1456,16 +1210,14 @@ __global__ void __launch_bounds__(256) rta_prod_poly(DevTables T, PolyArgs A, do
                         pr = 2.f;
                         keep = mirror_mode;
                     } else {
-                        const long long a = __ldg(T.row_ptr + (long long)cls * (T.n + 1) + k);
-                        const long long bb = __ldg(T.row_ptr + (long long)cls * (T.n + 1) + k + 1);
-                        const int len = int(bb - a);
-                        if (len <= 0) {
+                        const LambertRow lr = lambert_row(T, (long long)cls * T.n + k);
+                        if (lr.len == 0) {
                             record_error(err, E_GEOM, pid);
                             active = false;
                             done = true;
                             continue;
                         }
-                        const int4 e = __ldg(T.lalias + a + int(mulhi32(rr.y, uint32_t(len))));
+                        const int4 e = __ldg(T.lalias + lr.off + mulhi32(rr.y, lr.len));
                         pr = __int_as_float(e.x);
                         keep = e.y;
                         alt = e.z;
@@ -1473,9 +1225,10 @@ __global__ void __launch_bounds__(256) rta_prod_poly(DevTables T, PolyArgs A, do
                     c.wall_hits++;
                 } else {
                     const int j = int(mulhi32(rr.y, uint32_t(T.n)));
-                    pr = __ldg(T.resample_prob + p.mo + j);
+                    const int2 e = __ldg(T.resample + p.mo + j);
+                    pr = __int_as_float(e.x);
                     keep = j;
-                    alt = __ldg(T.resample_alt + p.mo + j);
+                    alt = e.y;
                 }
                 const float acc = float(rr.z >> 8) * 0x1p-24f;
                 nm = acc < pr ? keep : alt;
@@ -1758,26 +1511,6 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A, double* tally,
         const long long need = (n + 255) / 256;
         if (blocks > need) blocks = need;
         rta_prod_grid<false, 2, 0, true><<<unsigned(blocks), 256, 0, s>>>(T, A, tally, counters, err, work, aa);
-        return true;
-    }
-    if (tune.particles_per_thread == 2 && adj_pass == 0 && !use_smem && !T.spec_loc) {
-        // two particles per thread: the register cap follows the resident
-        // threads (152 registers up to 384 threads per SM, 128 above)
-        const bool capped = threads * bps > 384;
-        const void* f2 = capped ? reinterpret_cast<const void*>(rta_prod_grid_ilp<2, 2>)
-                                : reinterpret_cast<const void*>(rta_prod_grid_ilp<2, 1>);
-        int maxb = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, f2, threads, 0);
-        if (maxb < 1) return false;
-        const int b2 = bps > maxb ? maxb : bps;
-        long long blocks = (long long)nsm * b2;
-        const long long need = (n + 2ll * threads - 1) / (2ll * threads);
-        if (blocks > need) blocks = need;
-        if (blocks < 1) blocks = 1;
-        if (capped)
-            rta_prod_grid_ilp<2, 2><<<unsigned(blocks), threads, 0, s>>>(T, A, tally, counters, err, work);
-        else
-            rta_prod_grid_ilp<2, 1><<<unsigned(blocks), threads, 0, s>>>(T, A, tally, counters, err, work);
         return true;
     }
     const void* fn;

@@ -293,10 +293,10 @@ typedef struct bte_tuning {
     int32_t block_threads;   /* threads per block                              */
     int32_t blocks_per_sm;   /* resident blocks per SM of the persistent grid  */
     int32_t smem_tally;      /* 1: privatise tallies in shared memory           */
-    int32_t particles_per_thread; /* particles each thread carries at once in
-                                the grid kernel: 1, or 2 for the interleaved
-                                variant (plain production runs with a global
-                                tally and no spectral locations; others use 1) */
+    int32_t particles_per_thread; /* 0, 1 or 2, accepted and without effect: each
+                                thread carries one particle (two at once hid
+                                the latency of FP64 chains that the walk no
+                                longer has)                                   */
 } bte_tuning;
 
 /* ------------------------------------------------------------------------ */
