@@ -1131,13 +1131,24 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         if (c->ngroups > 1 && (replay || !g.rect_grid))
             throw Error(BTE_ERR_INPUT, "replica groups need production mode on boxes that tile a grid");
         const int ngroups = c->ngroups > 1 ? c->ngroups : 1;
+        const bool grid_run = !replay && g.rect_grid && c->ncrys == 0;
         const std::size_t tally_bytes =
             replay ? nk * 6 * sizeof(unsigned long long) : nk * 3 * sizeof(double) * std::size_t(ngroups);
-        c->d_tally.alloc(tally_bytes);
+        // A small tally is hit by all SMs at few places (the cells next to the
+        // reservoirs, the first bins), and reductions on one address serialise
+        // in L2: 1.25e5 B took 4.25 ms with one copy, 3.54 with two, 3.41 with
+        // four, 3.38 with eight and no less with more (1e6 particles, 5200
+        // keys; 2e5 particles, 1080 keys: 1.17, 0.75, 0.58, 0.53).  Copies
+        // beyond 16 MB in all only fill L2 (11.6 MB: 118.0 ms with one, 118.8
+        // with eight).
+        int ncopies = 1;
+        if (grid_run && ngroups == 1)
+            ncopies = int(std::clamp<std::size_t>((std::size_t(16) << 20) / tally_bytes, 1, 8));
+        c->d_tally.alloc(tally_bytes * std::size_t(ncopies));
         c->d_counters.alloc(16 * sizeof(unsigned long long));
         c->d_err.alloc(4 * sizeof(int));
         c->d_work.alloc(sizeof(unsigned long long));
-        ck(cudaMemsetAsync(c->d_tally.p, 0, tally_bytes, c->stream), "memset");
+        ck(cudaMemsetAsync(c->d_tally.p, 0, tally_bytes * std::size_t(ncopies), c->stream), "memset");
         ck(cudaMemsetAsync(c->d_counters.p, 0, 16 * sizeof(unsigned long long), c->stream), "memset");
         ck(cudaMemsetAsync(c->d_err.p, 0, 4 * sizeof(int), c->stream), "memset");
         ck(cudaMemsetAsync(c->d_work.p, 0, sizeof(unsigned long long), c->stream), "memset");
@@ -1208,6 +1219,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         T.nbins = nbins;
         T.ngroups = ngroups;
         T.group_stride = (long long)(nk * 3);
+        T.ncopies = ncopies;
         // spectral decomposition: per-mode time at the selected boxes
         const std::size_t nloc = c->spec_boxes.size();
         const std::size_t spec_vals = nloc * std::size_t(nbins) * m.n();
@@ -1224,9 +1236,6 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         }
         c->spec_valid = false;
 
-        // the grid kernel's tallies are in its integer units (powers of two)
-        const bool grid_run = !replay && g.rect_grid && c->ncrys == 0;
-        const double unit_t = grid_run ? A.fx.per_tick() : 1., unit_x = grid_run ? A.fx.per_unit() : 1.;
         auto* counters = c->d_counters.as<unsigned long long>();
         auto* err = c->d_err.as<int>();
         ck(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
@@ -1236,6 +1245,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
             if (!bte::launch_prod_grid(T, A, c->d_tally.as<double>(), counters, err,
                                        c->d_work.as<unsigned long long>(), c->tune, c->nsm, c->stream))
                 throw Error(BTE_ERR_INPUT, "tuning not supported by the grid kernel");
+            bte::launch_gather_tally(c->d_tally.as<double>(), (long long)(nk * 3) * ngroups, ncopies, A.fx, c->nsm, c->stream);
         } else if (p->flags & BTE_FLAG_GENERAL) {
             bte::launch_prod_general(T, c->d_tally.as<double>(), counters, err,
                                      c->d_work.as<unsigned long long>(), c->nsm, c->stream);
@@ -1280,7 +1290,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
                     c->spec_raw[i] = double(v) / bte::FIX_SCALE;
                 } else {
                     std::memcpy(&c->spec_raw[i], &hspec[i], sizeof(double));
-                    c->spec_raw[i] *= unit_t;
+                    if (grid_run) c->spec_raw[i] *= A.fx.per_tick();
                 }
             }
             c->spec_nbins = nbins;
@@ -1305,14 +1315,10 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         std::vector<double> sum;
         if (ngroups > 1) {
             // keep the groups; the run's outputs are their sum, in group order
-            c->group_raw.resize(nk * 3 * std::size_t(ngroups));
+            c->group_raw.assign(htal, htal + nk * 3 * std::size_t(ngroups));
             sum.assign(nk * 3, 0.);
             for (int gi = 0; gi < ngroups; ++gi)
-                for (std::size_t k = 0; k < nk * 3; ++k) {
-                    const std::size_t i = std::size_t(gi) * nk * 3 + k;
-                    c->group_raw[i] = htal[i] * (k % 3 == 0 ? unit_t : unit_x);
-                    sum[k] += htal[i];
-                }
+                for (std::size_t k = 0; k < nk * 3; ++k) sum[k] += htal[std::size_t(gi) * nk * 3 + k];
             htal = sum.data();
             c->group_n = ngroups;
             c->group_nbx = nbx;
@@ -1341,9 +1347,9 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
             if (out->exact) std::memcpy(out->exact, hex.data(), nk * 6 * sizeof(long long));
         } else {
             for (std::size_t k = 0; k < nk; ++k) {
-                gz[k] = htal[3 * k] * unit_t;
-                jx[k] = htal[3 * k + 1] * unit_x;
-                jy[k] = htal[3 * k + 2] * unit_x;
+                gz[k] = htal[3 * k];
+                jx[k] = htal[3 * k + 1];
+                jy[k] = htal[3 * k + 2];
             }
         }
         out->nboxes = nbx;

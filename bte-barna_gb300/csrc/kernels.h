@@ -138,8 +138,9 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A, double* tally,
 // The integer tables of the scales f: mf[n] from mv, the lines and widths from G.
 void launch_fix_tables(const FixScale& f, const ModeVel* mv, int n, ModeFix* mf, const DevGrid& G, long long* gxf,
                        long long* gyf, long long* wxf, long long* wyf, cudaStream_t s);
-// A tally in the walk's units (nk keys of three sums) to ps and nm, in place.
-void launch_scale_tally(double* tally, long long nk, const FixScale& f, int nsm, cudaStream_t s);
+// The copies of a grid-kernel tally of n sums added into the first and turned
+// from the walk's units into ps and nm.
+void launch_gather_tally(double* tally, long long n, int ncopies, const FixScale& f, int nsm, cudaStream_t s);
 
 // Kernel arguments of a context already prepared for one set of run
 // parameters (see prepared_grid_run in capi.cu).

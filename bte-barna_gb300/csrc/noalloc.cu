@@ -134,7 +134,7 @@ extern "C" bte_status bte_rta_run_noalloc(bte_ctx* ctx, const bte_rta_params* pa
         return fail(ctx, BTE_ERR_INPUT, "tuning not supported by the grid kernel");
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ctx, BTE_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
-    bte::launch_scale_tally(d_tally, (long long)r.nboxes * r.nbins, r.A.fx, r.nsm, s);
+    bte::launch_gather_tally(d_tally, 3ll * r.nboxes * r.nbins, 1, r.A.fx, r.nsm, s);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(ctx, BTE_ERR_CUDA, std::string("scale launch: ") + cudaGetErrorString(e));
     if (cudaEventRecord(r.ev1, s) != cudaSuccess) return fail(ctx, BTE_ERR_CUDA, "cudaEventRecord failed");

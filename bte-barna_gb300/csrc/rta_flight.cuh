@@ -105,6 +105,10 @@ struct DevTables {
     // <= 1: one tally)
     int ngroups;
     long long group_stride;
+    // copies of the grid kernel's tally that share its reductions: block b
+    // adds to copy b mod ncopies, group_stride doubles after the previous one
+    // (one copy with replica groups)
+    int ncopies;
     // crystals joined by mismatch interfaces (null: one crystal): per
     // contact the interface table of (its box's crystal, the neighbour's,
     // the contact normal), -1 within a crystal; the tables' rows

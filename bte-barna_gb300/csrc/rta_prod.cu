@@ -499,6 +499,7 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
     extern __shared__ double stally[];
     const int nk3 = 3 * T.nboxes * T.nbins;
     double* tally = gtally;
+    if (T.ncopies > 1) tally = gtally += (long long)(blockIdx.x % T.ncopies) * T.group_stride;
     if (SMEM_TALLY) {
         for (int k = threadIdx.x; k < nk3; k += blockDim.x) stally[k] = 0.;
         __syncthreads();
@@ -823,17 +824,18 @@ void launch_fix_tables(const FixScale& f, const ModeVel* mv, int n, ModeFix* mf,
     fix_tables<<<(m + 255) / 256, 256, 0, s>>>(f, mv, n, mf, G, gxf, gyf, wxf, wyf);
 }
 
-__global__ void scale_tally_k(double* t, long long nk, double st, double sx) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nk; i += (long long)gridDim.x * blockDim.x) {
-        t[3 * i] *= st;
-        t[3 * i + 1] *= sx;
-        t[3 * i + 2] *= sx;
+// The copies of a tally summed into the first, in ps and nm.
+__global__ void gather_tally_k(double* t, long long n, int ncopies, double st, double sx) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        double v = t[i];
+        for (int k = 1; k < ncopies; ++k) v += t[i + k * n];
+        t[i] = v * (i % 3 == 0 ? st : sx);
     }
 }
-void launch_scale_tally(double* tally, long long nk, const FixScale& f, int nsm, cudaStream_t s) {
-    long long b = (nk + 255) / 256;
+void launch_gather_tally(double* tally, long long n, int ncopies, const FixScale& f, int nsm, cudaStream_t s) {
+    long long b = (n + 255) / 256;
     if (b > nsm * 8ll) b = nsm * 8ll;
-    scale_tally_k<<<unsigned(b), 256, 0, s>>>(tally, nk, f.per_tick(), f.per_unit());
+    gather_tally_k<<<unsigned(b), 256, 0, s>>>(tally, n, ncopies, f.per_tick(), f.per_unit());
 }
 
 // ------------------------------------------------------------ polygon path
@@ -1497,10 +1499,14 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A, double* tally,
     const size_t smem = size_t(3) * T.nboxes * T.nbins * sizeof(double);
     // the adjoint passes run with the tally in global memory
     const bool use_smem = tune.smem_tally != 0 && smem <= 200 * 1024 && adj_pass == 0 && T.ngroups <= 1;
-    // residency variants: 4 blocks of 256 threads per SM (64 registers, a
-    // few spills), 3 (80 registers) or 2 (no register cap); the
-    // shared-memory tally allows one block per SM
-    int bps = tune.blocks_per_sm > 0 ? tune.blocks_per_sm : (use_smem ? 1 : 3);
+    // residency variants: 4 blocks of 256 threads per SM (64 registers), 3 (76
+    // registers) or 2 (no register cap); the shared-memory tally allows one
+    // block per SM.  Four hide the table reads better once every lane carries
+    // several particles in turn (2e6 on 36864 modes: 111 ms against 118 with
+    // three), three leave fewer lanes idle at the end of a short run (2e5:
+    // 0.53 ms against 0.61; 1e6: 3.36 and 3.38, the same).
+    const bool long_run = n >= 8ll * 1024 * nsm;
+    int bps = tune.blocks_per_sm > 0 ? tune.blocks_per_sm : (use_smem ? 1 : long_run ? 4 : 3);
     const AdjArgs none{};
     const AdjArgs& aa = adj ? *adj : none;
     if (T.checks && adj_pass == 0) {  // the checked variant, at its own residency
