@@ -397,6 +397,9 @@ void ensure_resample(bte_ctx* c, double T0) {
 }  // namespace bte
 
 namespace {
+// Header of a run's device buffer: 16 counters, the work counter at 128, four
+// error words at RUN_ERR; the tally follows.
+constexpr std::size_t RUN_ERR = 136, RUN_HEAD = 256;
 using bte::ensure_resample;
 using bte::ensure_static;
 using bte::sync;
@@ -554,8 +557,139 @@ void prepare_run(bte_ctx* c, const bte_rta_params* p) {
 }
 }  // namespace bte
 
+namespace {
+
+// Per box: 1 / V_box times the energy (and flux) factor, the temperature per
+// energy density, and the reference temperature.
+struct BoxPost {
+    double e, j, t, T0;
+};
+struct PostArgs {
+    const double* tally;     // [ncopies][box][bin][3]
+    int ncopies;
+    long long stride;        // doubles from one copy to the next
+    double unit_t, unit_x;   // of the raw sums
+    int nboxes, nbins, integrate;
+    const BoxPost* box;
+    double* raw[3];          // outputs [box][bin], null: not asked for
+    double* post[3];
+};
+
+// The outputs of a production run from its tally (src/RTA_MC2D.cpp:2336-2435):
+// the copies summed, per box the energy and flux factors, and for a walls
+// source the sum over the time bins so far.  One warp per box and quantity
+// takes 32 bins at a time; the running sum is a warp scan.  The host took
+// 2 ms for it on the 1e6-particle ribbon's 5200 keys and 25 ms on the sweep's
+// 333 000 with eight groups (copying every group's tally back first).
+__global__ void __launch_bounds__(128) post_tally(PostArgs a) {
+    const int w = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int b = w / 3, q = w % 3;
+    if (b >= a.nboxes || !(a.raw[q] || a.post[q])) return;
+    const BoxPost f = a.box[b];
+    const double unit = q == 0 ? a.unit_t : a.unit_x, fac = q == 0 ? f.e : f.j;
+    double carry = 0.;
+    for (int i0 = 0; i0 < a.nbins; i0 += 32) {
+        const int i = i0 + lane;
+        const long long k = (long long)b * a.nbins + i;
+        double v = 0.;
+        if (i < a.nbins)
+            for (int c = 0; c < a.ncopies; ++c) v += a.tally[c * a.stride + 3 * k + q];
+        v *= unit;
+        if (a.raw[q] && i < a.nbins) a.raw[q][k] = v;
+        if (!a.post[q]) continue;
+        v *= fac;
+        if (a.integrate) {
+            for (int o = 1; o < 32; o <<= 1) {
+                const double u = __shfl_up_sync(0xffffffffu, v, o);
+                if (lane >= o) v += u;
+            }
+            v += carry;
+            carry = __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (i < a.nbins) a.post[q][k] = q == 0 ? v * f.t + f.T0 : v;
+    }
+}
+
+}  // namespace
+
 namespace bte {
-// The post-processing of one run's raw tallies into its outputs
+// C_v per material (per crystal: over its own modes, q points and cell),
+// cached while the tables and temperatures stay.
+const std::vector<double>& heat_capacities(bte_ctx* c, double T0) {
+    std::vector<double> T0s(std::size_t(std::max(c->nmat, 1)));
+    for (std::size_t k = 0; k < T0s.size(); ++k) T0s[k] = c->nmat > 0 ? c->mat_T0[k] : T0;
+    if (c->cv_version != c->tables_version || c->cv_T0s != T0s) {
+        c->cv_cache.resize(T0s.size());
+        for (std::size_t k = 0; k < T0s.size(); ++k)
+            c->cv_cache[k] = bte::calc_cv(c->ncrys > 0 ? c->crys[k] : c->modes, T0s[k]);
+        c->cv_T0s = T0s;
+        c->cv_version = c->tables_version;
+    }
+    return c->cv_cache;
+}
+
+// The outputs `out` asks for, formed on the device from the tally at
+// `tally` and read back with `head` bytes of the run's header in front of
+// them (into *hdr): one launch, one copy, one synchronisation.
+void device_post(bte_ctx* c, const bte_rta_params* p, int nbx, int nbins, double Eeff, double step,
+                 const double* tally, int ncopies, PostUnits u, std::size_t head, bte_rta_result* out) {
+    const HostGeometry& g = c->geom;
+    const std::size_t nk = std::size_t(nbx) * std::size_t(nbins);
+    const bool initial = p->source != BTE_SOURCE_WALLS;
+    const bool shares = !c->mat_share.empty() && !initial;
+    const std::vector<double>* cvm = out->temperature ? &heat_capacities(c, p->T0) : nullptr;
+    std::vector<double> bp(std::size_t(nbx) * 4);
+    for (int b = 0; b < nbx; ++b) {
+        const std::size_t m = std::size_t(c->nmat > 0 ? g.mat[std::size_t(b)] : 0);
+        // Eeff_m = E_m / (share_m N) per material with shares
+        double E = Eeff;
+        if (shares) E = c->mat_share[m] > 0. ? c->mat_energy[m] / (c->mat_share[m] * double(p->nparticles)) : 0.;
+        if (initial) E /= step;  // relaxation of an initial deviation: bin averages
+        const double thick = box_thickness(c, b), vbox = g.boxes[std::size_t(b)].area * thick;
+        const double vcorr = thick / (c->ncrys > 0 ? c->crys[m].c : c->modes.c);
+        double* f = bp.data() + std::size_t(b) * 4;
+        f[0] = E / vbox;
+        f[1] = E * 1e12 * 1e9 * 1e9 / vbox;
+        f[2] = cvm ? vcorr / (*cvm)[m] : 0.;
+        f[3] = box_T0(c, b, p->T0);
+    }
+    if (c->h_boxpost != bp) {
+        c->h_boxpost.swap(bp);  // (stays until the copy is done)
+        c->d_boxpost.upload(c->h_boxpost, c->stream);
+    }
+    PostArgs a{};
+    a.tally = tally;
+    a.ncopies = ncopies;
+    a.stride = (long long)(nk * 3);
+    a.unit_t = u.t;
+    a.unit_x = u.x;
+    a.nboxes = nbx;
+    a.nbins = nbins;
+    a.integrate = initial ? 0 : 1;
+    a.box = c->d_boxpost.as<BoxPost>();
+    double* host[6] = {out->gz, out->gz_jx, out->gz_jy, out->temperature, out->jx, out->jy};
+    std::size_t n = 0;
+    for (int q = 0; q < 6; ++q)
+        if (host[q]) ++n;
+    const std::size_t bytes = head + n * nk * sizeof(double);
+    c->d_out.alloc(bytes);
+    c->h_out.reserve(bytes);
+    double* d = reinterpret_cast<double*>(c->d_out.as<char>() + head);
+    for (int q = 0, k = 0; q < 6; ++q)
+        if (host[q]) (q < 3 ? a.raw[q] : a.post[q - 3]) = d + nk * std::size_t(k++);
+    if (n) post_tally<<<unsigned((3 * nbx + 3) / 4), 128, 0, c->stream>>>(a);
+    ck(cudaGetLastError(), "post-processing launch");
+    char* h = static_cast<char*>(c->h_out.p);
+    if (head) ck(cudaMemcpyAsync(h, c->d_run.p, head, cudaMemcpyDeviceToHost, c->stream), "d2h");
+    if (n) ck(cudaMemcpyAsync(h + head, d, n * nk * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "d2h");
+    sync(c);
+    if (head && *reinterpret_cast<const int*>(h + RUN_ERR) != 0) return;  // the run failed
+    const double* r = reinterpret_cast<const double*>(h + head);
+    for (int q = 0, k = 0; q < 6; ++q)
+        if (host[q]) std::memcpy(host[q], r + nk * std::size_t(k++), nk * sizeof(double));
+}
+
+// The post-processing of a replay run's raw tallies on the host
 // (src/RTA_MC2D.cpp:2336-2435): / V_box, x Eeff (per material with shares),
 // the flux factor, the time integration of a walls source (or bin averages
 // of an initial deviation) and T = gz / (C_v / vcorr) + T0.
@@ -614,18 +748,7 @@ void rta_post(bte_ctx* c, const bte_rta_params* p, int nbx, int nbins, double Ee
         });
     }
     if (out->temperature) {
-        // C_v per material (per crystal: over its own modes, q points and
-        // cell), cached while the tables and temperatures stay
-        std::vector<double> T0s(std::size_t(std::max(c->nmat, 1)));
-        for (std::size_t k = 0; k < T0s.size(); ++k) T0s[k] = c->nmat > 0 ? c->mat_T0[k] : p->T0;
-        if (c->cv_version != c->tables_version || c->cv_T0s != T0s) {
-            c->cv_cache.resize(T0s.size());
-            for (std::size_t k = 0; k < T0s.size(); ++k)
-                c->cv_cache[k] = bte::calc_cv(c->ncrys > 0 ? c->crys[k] : m, T0s[k]);
-            c->cv_T0s = T0s;
-            c->cv_version = c->tables_version;
-        }
-        const std::vector<double>& cvm = c->cv_cache;
+        const std::vector<double>& cvm = heat_capacities(c, p->T0);
         for (int ir = 0; ir < nbx; ++ir) {
             const std::size_t mk = std::size_t(c->nmat > 0 ? g.mat[std::size_t(ir)] : 0);
             const double cv = cvm[mk];
@@ -1062,20 +1185,10 @@ bte_status bte_get_group_result(bte_ctx* c, int32_t group, bte_rta_result* out) 
         return BTE_ERR_INPUT;
     }
     try {
+        ck(cudaSetDevice(c->device), "cudaSetDevice");
         const std::size_t nk = std::size_t(c->group_nbx) * std::size_t(c->group_nbins);
-        const double* raw = c->group_raw.data() + std::size_t(group) * nk * 3;
-        const double G = double(c->group_n);
         // the group holds 1/G of the run's particles: x G estimates the whole run
-        const bool want[3] = {out->gz || out->temperature, out->gz_jx || out->jx, out->gz_jy || out->jy};
-        std::vector<double> v[3];
-        for (int q = 0; q < 3; ++q) {
-            if (!want[q]) continue;
-            v[q].resize(nk);
-            for (std::size_t k = 0; k < nk; ++k) v[q][k] = raw[3 * k + std::size_t(q)] * G;
-        }
-        std::vector<double>& gz = v[0];
-        std::vector<double>& jx = v[1];
-        std::vector<double>& jy = v[2];
+        const double G = double(c->group_n);
         out->nboxes = c->group_nbx;
         out->nbins = c->group_nbins;
         out->Eeff = c->group_Eeff;
@@ -1083,12 +1196,12 @@ bte_status bte_get_group_result(bte_ctx* c, int32_t group, bte_rta_result* out) 
         out->events = out->wall_hits = out->crossings = out->absorbed = 0;
         out->specular_hits = out->tally_updates = out->translations = 0;
         out->kernel_ms = 0.;
-        if (out->gz) std::copy(gz.begin(), gz.end(), out->gz);
-        if (out->gz_jx) std::copy(jx.begin(), jx.end(), out->gz_jx);
-        if (out->gz_jy) std::copy(jy.begin(), jy.end(), out->gz_jy);
-        bte::rta_post(c, &c->group_params, c->group_nbx, c->group_nbins, c->group_Eeff, c->group_step, gz, jx, jy,
-                      out);
+        const double* tally = reinterpret_cast<const double*>(c->d_run.as<char>() + RUN_HEAD) + std::size_t(group) * nk * 3;
+        bte::device_post(c, &c->group_params, c->group_nbx, c->group_nbins, c->group_Eeff, c->group_step, tally, 1,
+                         bte::PostUnits{c->group_units.t * G, c->group_units.x * G}, 0, out);
         return BTE_OK;
+    } catch (const Error& e) {
+        return fail(c, e);
     } catch (const std::exception& e) {
         c->err = e.what();
         return BTE_ERR_INPUT;
@@ -1117,12 +1230,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         const double step = (maxtime - 0.0) / double(ntime - 1);
         bte::GridArgs A{};
         if (g.rect_grid) bte::prepare_fixed(c, step, A);
-        {
-            const std::vector<double> tg =
-                bte::time_grid_with_widths(int(ntime), maxtime, step, A.fx.kt - A.fx.sub);
-            c->h_time.assign(tg.begin(), tg.begin() + std::ptrdiff_t(ntime));
-            c->d_time.upload(tg, c->stream);
-        }
+        bte::upload_time_grid(c, int(ntime), maxtime, step, A.fx.kt - A.fx.sub);
         const int nbins = int(ntime - 1);
         const int nbx = int(g.boxes.size());
         const std::size_t nk = std::size_t(nbx) * std::size_t(nbins);
@@ -1144,14 +1252,14 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         int ncopies = 1;
         if (grid_run && ngroups == 1)
             ncopies = int(std::clamp<std::size_t>((std::size_t(16) << 20) / tally_bytes, 1, 8));
-        c->d_tally.alloc(tally_bytes * std::size_t(ncopies));
-        c->d_counters.alloc(16 * sizeof(unsigned long long));
-        c->d_err.alloc(4 * sizeof(int));
-        c->d_work.alloc(sizeof(unsigned long long));
-        ck(cudaMemsetAsync(c->d_tally.p, 0, tally_bytes * std::size_t(ncopies), c->stream), "memset");
-        ck(cudaMemsetAsync(c->d_counters.p, 0, 16 * sizeof(unsigned long long), c->stream), "memset");
-        ck(cudaMemsetAsync(c->d_err.p, 0, 4 * sizeof(int), c->stream), "memset");
-        ck(cudaMemsetAsync(c->d_work.p, 0, sizeof(unsigned long long), c->stream), "memset");
+        const std::size_t run_bytes = RUN_HEAD + tally_bytes * std::size_t(ncopies);
+        c->d_run.alloc(run_bytes);
+        ck(cudaMemsetAsync(c->d_run.p, 0, run_bytes, c->stream), "memset");
+        char* base = c->d_run.as<char>();
+        auto* counters = reinterpret_cast<unsigned long long*>(base);
+        auto* work = reinterpret_cast<unsigned long long*>(base + 128);
+        auto* err = reinterpret_cast<int*>(base + RUN_ERR);
+        auto* tally = reinterpret_cast<double*>(base + RUN_HEAD);
 
         // Eeff (src/RTA_MC2D.cpp:2177) and the particle range
         double Eeff;
@@ -1236,52 +1344,47 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         }
         c->spec_valid = false;
 
-        auto* counters = c->d_counters.as<unsigned long long>();
-        auto* err = c->d_err.as<int>();
+        bte::PostUnits units;
         ck(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
         if (replay) {
-            bte::launch_replay(T, c->d_tally.as<unsigned long long>(), counters, err, c->nsm, c->stream);
+            bte::launch_replay(T, reinterpret_cast<unsigned long long*>(tally), counters, err, c->nsm, c->stream);
         } else if (grid_run) {
-            if (!bte::launch_prod_grid(T, A, c->d_tally.as<double>(), counters, err,
-                                       c->d_work.as<unsigned long long>(), c->tune, c->nsm, c->stream))
+            if (!bte::launch_prod_grid(T, A, tally, counters, err, work, c->tune, c->nsm, c->stream))
                 throw Error(BTE_ERR_INPUT, "tuning not supported by the grid kernel");
-            bte::launch_gather_tally(c->d_tally.as<double>(), (long long)(nk * 3) * ngroups, ncopies, A.fx, c->nsm, c->stream);
         } else if (p->flags & BTE_FLAG_GENERAL) {
-            bte::launch_prod_general(T, c->d_tally.as<double>(), counters, err,
-                                     c->d_work.as<unsigned long long>(), c->nsm, c->stream);
+            bte::launch_prod_general(T, tally, counters, err, work, c->nsm, c->stream);
         } else {
             const bte::PolyArgs PA{c->d_pborders.as<bte::PolyBorder>(), c->d_ppieces.as<bte::PolyPiece>(),
                                   c->d_mv.as<bte::ModeVel>(), c->d_invden.as<double>(),
                                   c->d_prect.as<bte::PolyRect>(),
                                   c->ncrys > 0 ? c->d_dmm_row.as<long long>() : nullptr,
                                   c->ncrys > 0 ? c->d_dmm_ent.as<bte::DmmEnt>() : nullptr};
-            if (!bte::launch_prod_poly(T, PA, c->d_tally.as<double>(), counters, err,
-                                       c->d_work.as<unsigned long long>(), c->nsm, c->stream))
+            if (!bte::launch_prod_poly(T, PA, tally, counters, err, work, c->nsm, c->stream))
                 throw Error(BTE_ERR_CUDA, "polygon kernel does not fit on the device");
         }
         ck(cudaGetLastError(), "kernel launch");
         ck(cudaEventRecord(c->ev1, c->stream), "cudaEventRecord");
-        std::vector<unsigned long long> hc(16);
-        int herr[4];
-        std::vector<unsigned long long> hex;
-        const double* htal = nullptr;  // the production tally, in the page-locked readback buffer
-        if (replay) {
-            hex.resize(nk * 6);
-            ck(cudaMemcpyAsync(hex.data(), c->d_tally.p, tally_bytes, cudaMemcpyDeviceToHost, c->stream), "d2h");
-        } else {
-            c->h_tally.reserve(tally_bytes);
-            htal = static_cast<const double*>(c->h_tally.p);
-            ck(cudaMemcpyAsync(c->h_tally.p, c->d_tally.p, tally_bytes, cudaMemcpyDeviceToHost, c->stream), "d2h");
-        }
-        ck(cudaMemcpyAsync(hc.data(), counters, 16 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, c->stream), "d2h");
-        ck(cudaMemcpyAsync(herr, err, 4 * sizeof(int), cudaMemcpyDeviceToHost, c->stream), "d2h");
-        std::vector<unsigned long long> hspec;
+        std::vector<unsigned long long> hspec, hex;
         if (nloc > 0) {
             hspec.resize(replay ? 2 * spec_vals : spec_vals);
             ck(cudaMemcpyAsync(hspec.data(), c->d_spec.p, hspec.size() * sizeof(unsigned long long),
                                cudaMemcpyDeviceToHost, c->stream), "d2h");
         }
-        sync(c);
+        if (replay) {
+            hex.resize(nk * 6);
+            ck(cudaMemcpyAsync(hex.data(), tally, tally_bytes, cudaMemcpyDeviceToHost, c->stream), "d2h");
+            c->h_out.reserve(RUN_HEAD);
+            ck(cudaMemcpyAsync(c->h_out.p, base, RUN_HEAD, cudaMemcpyDeviceToHost, c->stream), "d2h");
+            sync(c);
+        } else {
+            // the outputs' sum over replica groups or copies, in their order
+            if (grid_run) units = bte::PostUnits{A.fx.per_tick(), A.fx.per_unit()};
+            bte::device_post(c, p, nbx, nbins, Eeff, step, tally, ngroups > 1 ? ngroups : ncopies, units, RUN_HEAD, out);
+        }
+        unsigned long long hc[16];
+        int herr[4];
+        std::memcpy(hc, c->h_out.p, sizeof hc);
+        std::memcpy(herr, static_cast<const char*>(c->h_out.p) + RUN_ERR, sizeof herr);
         if (nloc > 0) {
             c->spec_raw.resize(spec_vals);
             for (std::size_t i = 0; i < spec_vals; ++i) {
@@ -1312,30 +1415,18 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
                                                       : "geometry error");
             throw Error(bte_status(herr[0]), msg);
         }
-        std::vector<double> sum;
-        if (ngroups > 1) {
-            // keep the groups; the run's outputs are their sum, in group order
-            c->group_raw.assign(htal, htal + nk * 3 * std::size_t(ngroups));
-            sum.assign(nk * 3, 0.);
-            for (int gi = 0; gi < ngroups; ++gi)
-                for (std::size_t k = 0; k < nk * 3; ++k) sum[k] += htal[std::size_t(gi) * nk * 3 + k];
-            htal = sum.data();
+        if (ngroups > 1) {  // the groups' tallies stay on the device
             c->group_n = ngroups;
             c->group_nbx = nbx;
             c->group_nbins = nbins;
             c->group_Eeff = Eeff;
             c->group_step = step;
             c->group_params = *p;
+            c->group_units = units;
             c->group_valid = true;
         }
-        // raw tallies
-        std::vector<double>& gz = c->post_gz;
-        std::vector<double>& jx = c->post_jx;
-        std::vector<double>& jy = c->post_jy;
-        gz.resize(nk);
-        jx.resize(nk);
-        jy.resize(nk);
-        if (replay) {
+        if (replay) {  // raw tallies
+            std::vector<double> gz(nk), jx(nk), jy(nk);
             for (std::size_t k = 0; k < nk; ++k) {
                 double* dst[3] = {&gz[k], &jx[k], &jy[k]};
                 for (int q = 0; q < 3; ++q) {
@@ -1345,12 +1436,10 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
                 }
             }
             if (out->exact) std::memcpy(out->exact, hex.data(), nk * 6 * sizeof(long long));
-        } else {
-            for (std::size_t k = 0; k < nk; ++k) {
-                gz[k] = htal[3 * k];
-                jx[k] = htal[3 * k + 1];
-                jy[k] = htal[3 * k + 2];
-            }
+            if (out->gz) std::copy(gz.begin(), gz.end(), out->gz);
+            if (out->gz_jx) std::copy(jx.begin(), jx.end(), out->gz_jx);
+            if (out->gz_jy) std::copy(jy.begin(), jy.end(), out->gz_jy);
+            bte::rta_post(c, p, nbx, nbins, Eeff, step, gz, jx, jy, out);
         }
         out->nboxes = nbx;
         out->nbins = nbins;
@@ -1366,10 +1455,6 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         out->translations = (int64_t)hc[8];
         out->interface_hits = (int64_t)hc[11];
         out->interface_transmissions = (int64_t)hc[12];
-        if (out->gz) std::copy(gz.begin(), gz.end(), out->gz);
-        if (out->gz_jx) std::copy(jx.begin(), jx.end(), out->gz_jx);
-        if (out->gz_jy) std::copy(jy.begin(), jy.end(), out->gz_jy);
-        bte::rta_post(c, p, nbx, nbins, Eeff, step, gz, jx, jy, out);
         return BTE_OK;
     } catch (const Error& e) {
         return fail(c, e);
@@ -1687,6 +1772,16 @@ void prepare_fixed(bte_ctx* c, double step, GridArgs& A) {
     ck(cudaGetLastError(), "integer tables launch");
     c->fix = f;
     c->fix_dev = true;
+}
+
+void upload_time_grid(bte_ctx* c, int ntime, double maxtime, double step, int tick_exp) {
+    if (c->time_n == ntime && c->time_max == maxtime && c->time_step == step && c->time_exp == tick_exp) return;
+    c->h_time = time_grid_with_widths(ntime, maxtime, step, tick_exp);  // (stays until the copy is done)
+    c->d_time.upload(c->h_time, c->stream);
+    c->time_n = ntime;
+    c->time_max = maxtime;
+    c->time_step = step;
+    c->time_exp = tick_exp;
 }
 
 std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step, int tick_exp) {

@@ -69,6 +69,11 @@ struct Pinned {
 };
 
 
+// What turns a raw tally into ps and nm, and the group estimate's factor.
+struct PostUnits {
+    double t = 1., x = 1.;
+};
+
 inline int hw_threads() {
     unsigned n = std::thread::hardware_concurrency();
     return n ? int(n < 64u ? n : 64u) : 4;
@@ -165,14 +170,15 @@ struct bte_ctx {
     int group_n = 0, group_nbx = 0, group_nbins = 0;
     double group_Eeff = 0., group_step = 0.;
     bte_rta_params group_params{};
-    std::vector<double> group_raw;
-    // the production tally's readback (page-locked) and the raw tallies
-    // handed to the post-processing, kept across runs
-    bte::Pinned h_tally;
-    std::vector<double> post_gz, post_jx, post_jy;
-    // run buffers
-    bte::DBuf d_time, d_tally, d_counters, d_err, d_work;
-    std::vector<double> h_time;
+    bte::PostUnits group_units{};
+    // run buffers: the header of a run (counters, error word, work counter)
+    // with the tally behind it, the outputs formed on the device with the
+    // per-box factors they take, and their page-locked readback
+    bte::DBuf d_time, d_run, d_out, d_boxpost, d_err;
+    bte::Pinned h_out;
+    std::vector<double> h_boxpost, h_time;   // what d_boxpost and d_time hold
+    int time_n = 0, time_exp = 0;            // and for which grid
+    double time_max = 0., time_step = 0.;
     // beyond-RTA (berta.cu)
     bte::BertaState* berta = nullptr;
     // periodic / gradient steady state (steady.cu)
@@ -207,6 +213,8 @@ double box_thickness(const bte_ctx* c, int b);
 // the last exactly maxtime), the ntime - 1 bin widths, and the bit patterns
 // of the integers width 2^tick_exp: the layout DevTables::timegrid points to.
 std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step, int tick_exp);
+// That grid into c->d_time, unless it is there already.
+void upload_time_grid(bte_ctx* c, int ntime, double maxtime, double step, int tick_exp);
 FixScale choose_scale(double x0, double x1, double y0, double y1, double vmax, double step);
 // The integer units of a grid run with bins of `step` ps, and their tables
 // on the device: fills the grid arguments (no allocation).
