@@ -30,6 +30,7 @@ UNITS = [
     ("berta.cu", []),
     ("steady.cu", []),
     ("adjoint.cu", []),
+    ("spectral.cu", []),
 ]
 
 

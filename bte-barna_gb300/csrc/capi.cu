@@ -804,6 +804,7 @@ bte_status bte_destroy(bte_ctx* c) {
     cudaStream_t s = c->stream;
     bte::destroy_berta(c);
     bte::destroy_steady(c);
+    bte::destroy_spectral(c);
     delete c;
     if (s) cudaStreamDestroy(s);
     return BTE_OK;
@@ -1035,134 +1036,6 @@ bte_status bte_set_spectral(bte_ctx* c, int32_t nloc, const int32_t* boxes, int3
     }
 }
 
-bte_status bte_get_spectral(bte_ctx* c, bte_spectral_result* out) {
-    if (!c || !out) return BTE_ERR_INPUT;
-    try {
-        if (!c->spec_valid) throw Error(BTE_ERR_STATE, "no run with spectral locations yet");
-        const bte::HostGeometry& g = c->geom;
-        const std::size_t n = c->modes.n();  // global modes (the crystals' one after the other)
-        const std::size_t nloc = c->spec_boxes.size(), nbins = std::size_t(c->spec_nbins);
-        const std::size_t nw = std::size_t(c->spec_nomega);
-        // each location's crystal (the reference takes the location's
-        // material's grid, :1987-2048): its modes and their first global index
-        auto crystal_of = [&](std::size_t l) -> int {
-            return c->ncrys > 0 ? g.mat[std::size_t(c->spec_boxes[l])] : -1;
-        };
-        auto modes_of = [&](int k) -> const bte::HostModes& {
-            return k >= 0 ? c->crys[std::size_t(k)] : c->modes;
-        };
-        const bte::HostModes& m0 = modes_of(nloc > 0 ? crystal_of(0) : -1);
-        const std::size_t nq = std::size_t(m0.nq);
-        for (std::size_t l = 1; l < nloc; ++l) {
-            const bte::HostModes& ml = modes_of(crystal_of(l));
-            if (ml.nq != m0.nq || ml.grid[0] != m0.grid[0] || ml.grid[1] != m0.grid[1])
-                throw Error(BTE_ERR_INPUT, "spectral locations in crystals of different q grids");
-        }
-        out->nloc = int32_t(nloc);
-        out->nbins = int32_t(nbins);
-        out->nomega = int32_t(nw);
-        out->nq = int32_t(nq);
-        const double hbar = 1.054571726e-34;
-        for (std::size_t l = 0; l < nloc; ++l) {
-            const int kc = crystal_of(l);
-            const bte::HostModes& m = modes_of(kc);
-            const std::size_t off = kc >= 0 ? c->crys_off[std::size_t(kc)] : 0, nk = m.n();
-            const std::size_t nb = std::size_t(m.nb);
-            // omega ticks of the location's crystal: LinSpaced(nomega, 0,
-            // max omega) + delta/2 (:2041-2045)
-            double maxw = 0.;
-            for (double w : m.omega) maxw = std::max(maxw, w);
-            std::vector<double> grid(nw);
-            for (std::size_t i = 0; i < nw; ++i)
-                grid[i] = (nw > 1 ? maxw * double(i) / double(nw - 1) : 0.) + 0.5 * maxw / double(nw);
-            if (out->omega) std::copy(grid.begin(), grid.end(), out->omega + l * nw);
-            // Gamma pdf of every mode over the ticks, shape k = w^2 / sigma,
-            // scale theta = sigma / w (gamma_pdf, :61-63), kept where it is not
-            // negligible
-            const std::vector<double> sig = bte::mode_sigmas(m);
-            std::vector<std::vector<std::pair<int, double>>> gw(nk);
-            for (std::size_t k = 0; k < nk; ++k) {
-                const double w = m.omega[k];
-                if (!(w > 0.)) continue;
-                const double kk = w * w / sig[k], th = sig[k] / w;
-                const double lg = std::lgamma(kk);
-                for (std::size_t i = 0; i < nw; ++i) {
-                    const double x = grid[i] / th;
-                    const double lp = (kk - 1.0) * std::log(x) - x - lg - std::log(th);
-                    if (lp > -700.) {
-                        const double pdf = std::exp(lp);
-                        if (pdf > 0.) gw[k].emplace_back(int(i), pdf);
-                    }
-                }
-            }
-            const int box = c->spec_boxes[l];
-            const double tb = bte::box_thickness(c, box);
-            const double vcorr = tb / m.c;
-            const double vbox = g.boxes[std::size_t(box)].area * tb;
-            const double T0b = bte::box_T0(c, box, c->spec_T0);
-            const double cv = bte::calc_cv(m, T0b);
-            const double Eeff = c->spec_Eeff;
-            std::vector<double> dT(nbins * nw, 0.), jx(nbins * nw, 0.), jy(nbins * nw, 0.), fq(nbins * nq, 0.);
-            const bool steady = c->spec_steady;
-            for (std::size_t b = 0; b < nbins; ++b) {
-                const double* Tm = c->spec_raw.data() + (l * nbins + b) * n + off;
-                for (std::size_t k = 0; k < nk; ++k) {
-                    const double t = Tm[k];
-                    // fd_qmesh: time / omega (transient, :757), sign / omega
-                    // per segment (steady, :829)
-                    const double f = steady ? double(c->spec_cnt[l * n + off + k]) : t;
-                    if (f != 0. && m.omega[k] > 0.) fq[b * nq + k / nb] += f / m.omega[k];
-                    if (t == 0.) continue;
-                    for (auto& [i, wgt] : gw[k]) {
-                        dT[b * nw + std::size_t(i)] += t * wgt;
-                        jx[b * nw + std::size_t(i)] += m.vxc[k] * t * wgt;
-                        jy[b * nw + std::size_t(i)] += m.vyc[k] * t * wgt;
-                    }
-                }
-            }
-            // scaling (:2350-2376) and integration in time (:2386-2413)
-            const double sdT = Eeff / vbox, sj = Eeff * 1e12 * 1e9 * 1e9 / vbox;
-            const double sq = Eeff * vcorr * double(nq) / (vbox * 1.0e+12 * hbar);
-            for (auto& x : dT) x *= sdT;
-            for (auto& x : jx) x *= sj;
-            for (auto& x : jy) x *= sj;
-            for (auto& x : fq) x *= sq;
-            for (std::size_t b = 1; b < nbins && !steady; ++b) {
-                for (std::size_t i = 0; i < nw; ++i) {
-                    dT[b * nw + i] += dT[(b - 1) * nw + i];
-                    jx[b * nw + i] += jx[(b - 1) * nw + i];
-                    jy[b * nw + i] += jy[(b - 1) * nw + i];
-                }
-                for (std::size_t q = 0; q < nq; ++q) fq[b * nq + q] += fq[(b - 1) * nq + q];
-            }
-            for (auto& x : dT) x = x / (cv / vcorr);
-            if (out->dT_omega) std::copy(dT.begin(), dT.end(), out->dT_omega + l * nbins * nw);
-            if (out->jx_omega) std::copy(jx.begin(), jx.end(), out->jx_omega + l * nbins * nw);
-            if (out->jy_omega) std::copy(jy.begin(), jy.end(), out->jy_omega + l * nbins * nw);
-            if (out->fd_q) std::copy(fq.begin(), fq.end(), out->fd_q + l * nbins * nq);
-        }
-        if (out->raw) std::copy(c->spec_raw.begin(), c->spec_raw.end(), out->raw);
-        out->steady = c->spec_steady ? 1 : 0;
-        if (out->counts && c->spec_steady)
-            for (std::size_t i = 0; i < c->spec_cnt.size(); ++i) out->counts[i] = double(c->spec_cnt[i]);
-        if (out->q1bz) {
-            // q points in Cartesian coordinates, reduced coordinates wrapped
-            // to [-1/2, 1/2) (a Gamma-centred n1 x n2 grid, iq = i n2 + j)
-            const bte::HostModes& m = m0;
-            const int n1 = m.grid[0] > 0 ? m.grid[0] : 1, n2 = m.grid[1] > 0 ? m.grid[1] : 1;
-            for (std::size_t iq = 0; iq < nq; ++iq) {
-                const int i = int(iq) / n2, j = int(iq) % n2;
-                const int ii = (i + n1 / 2) % n1 - n1 / 2, jj = (j + n2 / 2) % n2 - n2 / 2;
-                out->q1bz[2 * iq + 0] = ii * m.dq[0] + jj * m.dq[3];
-                out->q1bz[2 * iq + 1] = ii * m.dq[1] + jj * m.dq[4];
-            }
-        }
-        return BTE_OK;
-    } catch (const Error& e) {
-        return fail(c, e);
-    }
-}
-
 bte_status bte_set_groups(bte_ctx* c, int32_t ngroups) {
     if (!c) return BTE_ERR_INPUT;
     if (ngroups < 0 || ngroups > 4096) {
@@ -1332,7 +1205,8 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         const std::size_t nloc = c->spec_boxes.size();
         const std::size_t spec_vals = nloc * std::size_t(nbins) * m.n();
         if (nloc > 0) {
-            std::vector<int> loc(std::size_t(nbx), -1);
+            std::vector<int>& loc = c->h_specloc;  // (stays until the copy is done)
+            loc.assign(std::size_t(nbx), -1);
             for (std::size_t i = 0; i < nloc; ++i) loc[std::size_t(c->spec_boxes[i])] = int(i);
             c->d_specloc.upload(loc, c->stream);
             const std::size_t bytes = spec_vals * (replay ? 2 * sizeof(unsigned long long) : sizeof(double));
@@ -1364,12 +1238,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         }
         ck(cudaGetLastError(), "kernel launch");
         ck(cudaEventRecord(c->ev1, c->stream), "cudaEventRecord");
-        std::vector<unsigned long long> hspec, hex;
-        if (nloc > 0) {
-            hspec.resize(replay ? 2 * spec_vals : spec_vals);
-            ck(cudaMemcpyAsync(hspec.data(), c->d_spec.p, hspec.size() * sizeof(unsigned long long),
-                               cudaMemcpyDeviceToHost, c->stream), "d2h");
-        }
+        std::vector<unsigned long long> hex;
         if (replay) {
             hex.resize(nk * 6);
             ck(cudaMemcpyAsync(hex.data(), tally, tally_bytes, cudaMemcpyDeviceToHost, c->stream), "d2h");
@@ -1385,21 +1254,12 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         int herr[4];
         std::memcpy(hc, c->h_out.p, sizeof hc);
         std::memcpy(herr, static_cast<const char*>(c->h_out.p) + RUN_ERR, sizeof herr);
-        if (nloc > 0) {
-            c->spec_raw.resize(spec_vals);
-            for (std::size_t i = 0; i < spec_vals; ++i) {
-                if (replay) {
-                    const __int128 v = (__int128)(((unsigned __int128)hspec[2 * i] << 64) | hspec[2 * i + 1]);
-                    c->spec_raw[i] = double(v) / bte::FIX_SCALE;
-                } else {
-                    std::memcpy(&c->spec_raw[i], &hspec[i], sizeof(double));
-                    if (grid_run) c->spec_raw[i] *= A.fx.per_tick();
-                }
-            }
+        if (nloc > 0) {  // the tally stays on the device for bte_get_spectral
+            if (replay) bte::spec_from_exact(c, spec_vals);
+            c->spec_unit = grid_run ? A.fx.per_tick() : 1.;
             c->spec_nbins = nbins;
             c->spec_T0 = p->T0;
             c->spec_steady = false;
-            c->spec_cnt.clear();
             c->spec_valid = true;
         }
         float ms = 0;
@@ -1793,6 +1653,19 @@ std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step
         g[std::size_t(2 * ntime - 1 + i)] = bitsd(uint64_t(std::llrint(std::ldexp(w, tick_exp))));
     }
     return g;
+}
+
+// A replay run's 128-bit per-mode tally in c->d_spec, replaced by its values
+// as doubles.
+void spec_from_exact(bte_ctx* c, std::size_t vals) {
+    std::vector<unsigned long long> h(2 * vals);
+    std::vector<double> v(vals);
+    ck(cudaMemcpyAsync(h.data(), c->d_spec.p, h.size() * sizeof(h[0]), cudaMemcpyDeviceToHost, c->stream), "d2h");
+    sync(c);
+    for (std::size_t i = 0; i < vals; ++i)
+        v[i] = double((__int128)(((unsigned __int128)h[2 * i] << 64) | h[2 * i + 1])) / FIX_SCALE;
+    c->d_spec.upload(v, c->stream);
+    sync(c);
 }
 
 void fill_static_tables(bte_ctx* c, DevTables& T) {

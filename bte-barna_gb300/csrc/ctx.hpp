@@ -81,6 +81,7 @@ inline int hw_threads() {
 
 struct BertaState;   // berta.cu
 struct SteadyState;  // steady.cu
+struct SpectralState;  // spectral.cu
 
 }  // namespace bte
 
@@ -153,12 +154,11 @@ struct bte_ctx {
     double gen_Eeff = 0;
     bte::DBuf d_gcdf, d_gprob, d_galt, d_walls, d_wcum, d_ifirst, d_ibox, d_isign;
     // spectral decomposition: selected boxes, ticks, the last run's tally
-    std::vector<int> spec_boxes;
+    std::vector<int> spec_boxes, h_specloc;
     int spec_nomega = 0;
-    bte::DBuf d_specloc, d_spec;
-    std::vector<double> spec_raw;      // [nloc][nbins][n] of the last run
-    bte::DBuf d_speccnt;
-    std::vector<long long> spec_cnt;   // steady runs: signed segments [nloc][n]
+    bte::DBuf d_specloc, d_spec;       // the last run's [nloc][nbins][n], in spec_unit ps
+    bte::DBuf d_speccnt;               // steady runs: signed segments [nloc][n]
+    double spec_unit = 1.;
     bool spec_steady = false;
     int spec_nbins = 0;
     double spec_Eeff = 0., spec_T0 = 0.;
@@ -183,6 +183,8 @@ struct bte_ctx {
     bte::BertaState* berta = nullptr;
     // periodic / gradient steady state (steady.cu)
     bte::SteadyState* steady = nullptr;
+    // device buffers of the spectral outputs (spectral.cu)
+    bte::SpectralState* spectral = nullptr;
 };
 
 namespace bte {
@@ -194,6 +196,8 @@ void destroy_berta(bte_ctx* c);
 // Forget the loaded propagators (they refer to the previous mode table).
 void reset_propagators(bte_ctx* c);
 void destroy_steady(bte_ctx* c);
+void destroy_spectral(bte_ctx* c);
+void spec_from_exact(bte_ctx* c, std::size_t vals);
 // T0 of box b's material (the run's T0 without materials).
 double box_T0(const bte_ctx* c, int b, double T0);
 // Validation and tables of one RTA run (capi.cu).
