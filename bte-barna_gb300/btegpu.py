@@ -640,6 +640,21 @@ def split_frames(data: bytes):
     return out
 
 
+def debug_links(g: dict, cap=100000):
+    """The linked cells of a geometry: None, or x lines, y lines, sides
+    [cell][4] (cell, box, flags) and cycles [cell][4]."""
+    lib = load_library()
+    s, keep = geom_struct(g)
+    lines, out = np.zeros(2 * cap), np.zeros(2 + 16 * cap, dtype=np.int32)
+    lib.btegpu_debug_links.restype = C.c_longlong
+    n = lib.btegpu_debug_links(C.byref(s), _dptr(lines), _iptr(out), C.c_longlong(cap))
+    if n <= 0:
+        return None
+    nx, ny = int(out[0]), int(out[1])
+    t = out[2:2 + 16 * n].reshape(n, 4, 4)
+    return lines[:nx + 1], lines[nx + 1:nx + ny + 2], t[:, :, :3].copy(), t[:, :, 3].copy()
+
+
 def debug_fixwalk(gx, gy, vmax, step, nbins, p, e, tau, vx, vy, cap=100000):
     """The grid kernel's integer walk of one particle on the host: rows
     (flight, kind, x, y, ticks) and the scales (kx, kt, sub)."""

@@ -25,6 +25,7 @@ UNITS = [
     # (source, extra nvcc flags)
     ("rta_replay.cu", ["-fmad=false"]),
     ("rta_prod.cu", []),
+    ("rta_link.cu", []),
     ("capi.cu", []),
     ("noalloc.cu", []),
     ("berta.cu", []),

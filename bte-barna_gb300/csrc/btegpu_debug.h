@@ -25,6 +25,12 @@ long long btegpu_debug_lambert(const bte_mode_table* m, const bte_geometry* g,
 long long btegpu_debug_frame(double time, double Eeff, const double* temps, const int* H, int nboxes,
                              int nmodes, char* out, long long cap);
 
+/* The linked cells of a geometry (build_link_grid): returns their number, 0
+ * where the boxes cannot be linked, minus the number needed when above cap.
+ * lines: the x lines, then the y lines; out: nx, ny, then per cell four rows
+ * (+x, -x, +y, -y) of cell, box, flags, and the cell's four period limits. */
+long long btegpu_debug_links(const bte_geometry* g, double* lines, int* out, long long cap);
+
 /* The integer walk of the grid kernel (fixed_walk.cuh), on the host: one
  * particle from (px, py) through free flights k of tau[k] e[k] ps at
  * (vx[k], vy[k]) over the cells of the lines gx[0..nx], gy[0..ny], nbins time

@@ -81,9 +81,17 @@ void ensure_static(bte_ctx* c) {
                 c->d_tfast_u.upload(tf.u, c->stream);
             }
         }
+        c->link = bte::build_link_grid(g);
+        const std::vector<double>& gx = g.rect_grid ? g.gx : c->link.gx;
+        const std::vector<double>& gy = g.rect_grid ? g.gy : c->link.gy;
+        if (g.rect_grid || c->link.ok) {
+            c->d_gx.upload(gx, c->stream);
+            c->d_gy.upload(gy, c->stream);
+            for (bte::DBuf* d : {&c->d_gxf, &c->d_wxf}) d->alloc(gx.size() * sizeof(long long));
+            for (bte::DBuf* d : {&c->d_gyf, &c->d_wyf}) d->alloc(gy.size() * sizeof(long long));
+            c->fix_dev = false;
+        }
         if (g.rect_grid) {
-            c->d_gx.upload(g.gx, c->stream);
-            c->d_gy.upload(g.gy, c->stream);
             c->d_gcell.upload(g.gcell, c->stream);
             std::vector<int2> bc(g.boxes.size(), make_int2(-1, -1));
             for (int i = 0; i < g.gnx; ++i)
@@ -93,10 +101,6 @@ void ensure_static(bte_ctx* c) {
                     if (b >= 0) bc[std::size_t(b)] = make_int2(i, j);
                 }
             c->d_boxcell.upload(bc, c->stream);
-            c->d_gxf.alloc(g.gx.size() * sizeof(long long));
-            c->d_gyf.alloc(g.gy.size() * sizeof(long long));
-            c->d_wxf.alloc(g.gx.size() * sizeof(long long));
-            c->d_wyf.alloc(g.gy.size() * sizeof(long long));
             std::vector<int> map(std::size_t(g.gnx + 2) * std::size_t(g.gny + 2), -1);
             for (int i = 0; i < g.gnx; ++i)
                 for (int j = 0; j < g.gny; ++j)
@@ -104,7 +108,6 @@ void ensure_static(bte_ctx* c) {
                         g.gcell[std::size_t(i) * g.gny + j];
             c->d_map.upload(map, c->stream);
             sync(c);
-            c->fix_dev = false;
         }
         {
             // border lines and neighbour pieces of the convex-polygon path
@@ -233,6 +236,39 @@ void ensure_static(bte_ctx* c) {
                 rect[a] = R;
             }
             c->d_prect.upload(rect, c->stream);
+            if (c->link.ok) {
+                bte::LinkGrid& L = c->link;
+                std::vector<unsigned char> per(g.boxes.size());
+                for (std::size_t a = 0; a < per.size(); ++a) {
+                    const int* r = L.range.data() + 4 * a;
+                    per[a] = (unsigned char)((rect[a].kx1 >= 0 && rect[a].perx ? 1 : 0) |
+                                             (rect[a].kx1 >= 0 && rect[a].pery ? 2 : 0));
+                    // (a wrap by the box's width needs it to be one cell there)
+                    if (((per[a] & 1) && r[1] - r[0] != 1) || ((per[a] & 2) && r[3] - r[2] != 1)) L.ok = false;
+                }
+                c->link_corner = false;
+                std::vector<int> pbox(L.side.size(), -1);
+                for (std::size_t k = 0; k < pbox.size(); ++k) {
+                    if (!(L.side[k].flags & bte::LINK_TRANSLATE)) continue;
+                    // the periodic box itself: the cell across the side
+                    const int cell = int(k / 4), sd = int(k % 4), i = cell / L.ny, j = cell % L.ny;
+                    const int pi = i + (sd == 0) - (sd == 1), pj = j + (sd == 2) - (sd == 3);
+                    for (std::size_t b = 0; b < g.boxes.size(); ++b) {
+                        const int* r = L.range.data() + 4 * b;
+                        if (pi >= r[0] && pi < r[1] && pj >= r[2] && pj < r[3]) pbox[k] = int(b);
+                        // a box that spans this period wraps instead
+                        if (i >= r[0] && i < r[1] && j >= r[2] && j < r[3] && !(per[b] & (sd < 2 ? 1 : 2)))
+                            c->link_corner = true;
+                    }
+                }
+                c->d_lrange.upload(L.range, c->stream);
+                c->d_lper.upload(per, c->stream);
+                c->d_lcycle.upload(L.cycle, c->stream);
+                c->d_lpbox.upload(pbox, c->stream);
+                c->d_lbox.upload(L.box, c->stream);
+                c->d_lside.upload(L.side, c->stream);  // (interfaces: filled in with their tables)
+                sync(c);
+            }
         }
         sync(c);
         c->geom_dev = true;
@@ -362,6 +398,10 @@ void ensure_static(bte_ctx* c) {
         c->d_cdmm.upload(cdmm, c->stream);
         c->d_crysoff.upload(coff, c->stream);
         c->d_ppieces.upload(pcs, c->stream);
+        std::vector<bte::LinkSide> side = c->link.side;
+        for (bte::LinkSide& k : side)
+            if (k.flags >> 8) k.flags = (k.flags & 255) | ((cdmm[std::size_t((k.flags >> 8) - 1)] + 1) << 8);
+        if (c->link.ok) c->d_lside.upload(side, c->stream);
         c->ndmm = int(tab_of.size());
         sync(c);
         c->dmm_dev = true;
@@ -1101,18 +1141,29 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         if (ntime < 2) throw Error(BTE_ERR_INPUT, "maxtime shorter than one time bin");
         const double maxtime = double(ntime - 1) * p->dt;
         const double step = (maxtime - 0.0) / double(ntime - 1);
+        const bool replay = p->mode == BTE_MODE_REPLAY;
+        const bool grid_run = !replay && g.rect_grid && c->ncrys == 0;
+        // linked cells, unless particles start inside a periodic box or a
+        // reservoir (an initial deviation there), which the cells do not model
+        bool link_run = !replay && !grid_run && c->link.ok && !(p->flags & BTE_FLAG_GENERAL);
+        if (p->source == BTE_SOURCE_INITIAL)
+            for (int b : c->gens.init_box)
+                if (g.tto[std::size_t(b)] >= 0 || g.reservoir[std::size_t(b)]) link_run = false;
         bte::GridArgs A{};
-        if (g.rect_grid) bte::prepare_fixed(c, step, A);
+        bte::LinkArgs LA{};
+        if (grid_run) bte::prepare_fixed(c, step, A);
+        if (link_run) {
+            bte::prepare_link(c, step, LA);
+            A.fx = LA.fx;
+        }
         bte::upload_time_grid(c, int(ntime), maxtime, step, A.fx.kt - A.fx.sub);
         const int nbins = int(ntime - 1);
         const int nbx = int(g.boxes.size());
         const std::size_t nk = std::size_t(nbx) * std::size_t(nbins);
-        const bool replay = p->mode == BTE_MODE_REPLAY;
         c->group_valid = false;
         if (c->ngroups > 1 && (replay || !g.rect_grid))
             throw Error(BTE_ERR_INPUT, "replica groups need production mode on boxes that tile a grid");
         const int ngroups = c->ngroups > 1 ? c->ngroups : 1;
-        const bool grid_run = !replay && g.rect_grid && c->ncrys == 0;
         const std::size_t tally_bytes =
             replay ? nk * 6 * sizeof(unsigned long long) : nk * 3 * sizeof(double) * std::size_t(ngroups);
         // A small tally is hit by all SMs at few places (the cells next to the
@@ -1123,7 +1174,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         // beyond 16 MB in all only fill L2 (11.6 MB: 118.0 ms with one, 118.8
         // with eight).
         int ncopies = 1;
-        if (grid_run && ngroups == 1)
+        if ((grid_run || link_run) && ngroups == 1)
             ncopies = int(std::clamp<std::size_t>((std::size_t(16) << 20) / tally_bytes, 1, 8));
         const std::size_t run_bytes = RUN_HEAD + tally_bytes * std::size_t(ncopies);
         c->d_run.alloc(run_bytes);
@@ -1225,6 +1276,9 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         } else if (grid_run) {
             if (!bte::launch_prod_grid(T, A, tally, counters, err, work, c->tune, c->nsm, c->stream))
                 throw Error(BTE_ERR_INPUT, "tuning not supported by the grid kernel");
+        } else if (link_run) {
+            if (!bte::launch_prod_link(T, LA, tally, counters, err, work, c->nsm, c->stream))
+                throw Error(BTE_ERR_CUDA, "linked-cell kernel does not fit on the device");
         } else if (p->flags & BTE_FLAG_GENERAL) {
             bte::launch_prod_general(T, tally, counters, err, work, c->nsm, c->stream);
         } else {
@@ -1247,7 +1301,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
             sync(c);
         } else {
             // the outputs' sum over replica groups or copies, in their order
-            if (grid_run) units = bte::PostUnits{A.fx.per_tick(), A.fx.per_unit()};
+            if (grid_run || link_run) units = bte::PostUnits{A.fx.per_tick(), A.fx.per_unit()};
             bte::device_post(c, p, nbx, nbins, Eeff, step, tally, ngroups > 1 ? ngroups : ncopies, units, RUN_HEAD, out);
         }
         unsigned long long hc[16];
@@ -1256,7 +1310,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         std::memcpy(herr, static_cast<const char*>(c->h_out.p) + RUN_ERR, sizeof herr);
         if (nloc > 0) {  // the tally stays on the device for bte_get_spectral
             if (replay) bte::spec_from_exact(c, spec_vals);
-            c->spec_unit = grid_run ? A.fx.per_tick() : 1.;
+            c->spec_unit = grid_run || link_run ? A.fx.per_tick() : 1.;
             c->spec_nbins = nbins;
             c->spec_T0 = p->T0;
             c->spec_steady = false;
@@ -1388,6 +1442,28 @@ long long btegpu_debug_frame(double time, double Eeff, const double* temps, cons
     const std::string f = bte::berta_frame(time, Eeff, t, H, std::size_t(nboxes), std::size_t(nmodes));
     if ((long long)f.size() <= cap) std::memcpy(out, f.data(), f.size());
     return (long long)f.size();
+}
+
+long long btegpu_debug_links(const bte_geometry* gm, double* lines, int* out, long long cap) {
+    try {
+        const bte::LinkGrid L = bte::build_link_grid(bte::build_geometry(gm));
+        if (!L.ok) return 0;
+        const long long n = (long long)L.nx * L.ny;
+        if (cap < n) return -n;
+        out[0] = L.nx;
+        out[1] = L.ny;
+        std::copy(L.gx.begin(), L.gx.end(), lines);
+        std::copy(L.gy.begin(), L.gy.end(), lines + L.gx.size());
+        for (long long k = 0; k < 4 * n; ++k) {
+            out[2 + 4 * k] = L.side[std::size_t(k)].cell;
+            out[3 + 4 * k] = L.side[std::size_t(k)].box;
+            out[4 + 4 * k] = L.side[std::size_t(k)].flags;
+            out[5 + 4 * k] = L.cycle[std::size_t(k)];
+        }
+        return n;
+    } catch (const std::exception&) {
+        return 0;
+    }
 }
 
 long long btegpu_debug_fixwalk(const double* gx, int nx, const double* gy, int ny, double vmax, double step,
@@ -1603,6 +1679,8 @@ FixScale choose_scale(double x0, double x1, double y0, double y1, double vmax, d
     return f;
 }
 
+void fix_on_device(bte_ctx* c, const FixScale& f);
+
 void prepare_fixed(bte_ctx* c, double step, GridArgs& A) {
     const HostGeometry& g = c->geom;
     A.G.nx = g.gnx;
@@ -1625,9 +1703,50 @@ void prepare_fixed(bte_ctx* c, double step, GridArgs& A) {
         for (std::size_t k = 0; k < g.normals.size(); ++k)
             if (g.normals[k].x == want[w].x && g.normals[k].y == want[w].y) A.cls[w] = int(k);
     }
-    const FixScale& f = A.fx;
+    // Generating a particle is a long divergent block with FP64 draws: where
+    // particles are absorbed soon (walls), a warp waits for four idle lanes
+    // (1e6 particles, 61 flights each: 3.36 ms with one, 3.19 two, 3.14 four,
+    // 3.27 eight); an initial deviation keeps its particles to the end (1800
+    // flights each: 112.1 ms with one, 114.6 four).
+    A.refill = c->gen_key_source == BTE_SOURCE_WALLS ? 4 : 1;
+    fix_on_device(c, A.fx);
+}
+
+void prepare_link(bte_ctx* c, double step, LinkArgs& A) {
+    const LinkGrid& L = c->link;
+    A.mf = c->d_mf.as<ModeFix>();
+    A.gxf = c->d_gxf.as<long long>();
+    A.gyf = c->d_gyf.as<long long>();
+    A.wxf = c->d_wxf.as<unsigned long long>();
+    A.wyf = c->d_wyf.as<unsigned long long>();
+    A.ny = L.ny;
+    A.side = c->d_lside.as<int4>();
+    A.range = c->d_lrange.as<int4>();
+    A.per = c->d_lper.as<unsigned char>();
+    A.cellbox = c->d_lbox.as<int>();
+    A.cycle = c->d_lcycle.as<int4>();
+    A.pbox = c->link_corner ? c->d_lpbox.as<int>() : nullptr;
+    A.dmm_row = c->d_dmm_row.as<long long>();
+    A.dmm_ent = c->d_dmm_ent.as<DmmEnt>();
+    // (as in prepare_fixed; generation on convex boxes costs more: the bar's
+    // particles live five flights, 3.63 ms with one idle lane, 2.17 four, 1.89
+    // eight, 1.84 sixteen; the crystals' 25, 1.07, 0.80, 0.77, 0.82)
+    A.refill = c->gen_key_source == BTE_SOURCE_WALLS ? 8 : 1;
+    A.fx = choose_scale(L.gx.front(), L.gx.back(), L.gy.front(), L.gy.back(), c->vmax, step);
+    A.margin = (unsigned long long)std::llrint(std::ldexp(2.0e-6, A.fx.kx));
+    fix_on_device(c, A.fx);
+}
+
+// The integer tables for the scales f, unless they are on the device already.
+void fix_on_device(bte_ctx* c, const FixScale& f) {
+    const bool rect = c->geom.rect_grid;
+    DevGrid G{};
+    G.nx = rect ? c->geom.gnx : c->link.nx;
+    G.ny = rect ? c->geom.gny : c->link.ny;
+    G.gx = c->d_gx.as<double>();
+    G.gy = c->d_gy.as<double>();
     if (c->fix_dev && c->fix.x0 == f.x0 && c->fix.y0 == f.y0 && c->fix.kx == f.kx && c->fix.kt == f.kt) return;
-    launch_fix_tables(f, A.mv, int(c->modes.n()), c->d_mf.as<ModeFix>(), A.G, c->d_gxf.as<long long>(),
+    launch_fix_tables(f, c->d_mv.as<ModeVel>(), int(c->modes.n()), c->d_mf.as<ModeFix>(), G, c->d_gxf.as<long long>(),
                       c->d_gyf.as<long long>(), c->d_wxf.as<long long>(), c->d_wyf.as<long long>(), c->stream);
     ck(cudaGetLastError(), "integer tables launch");
     c->fix = f;

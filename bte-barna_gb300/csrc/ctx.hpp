@@ -127,6 +127,11 @@ struct bte_ctx {
     bte::FixScale fix{};
     bool fix_dev = false;
     double vmax = 0.;  // largest velocity component of the loaded modes
+    // linked cells (rta_link.cu); d_gx .. d_wyf hold these lines where the
+    // boxes tile no grid
+    bte::LinkGrid link;
+    bool link_corner = false;  // some side leads through a periodic box
+    bte::DBuf d_lside, d_lrange, d_lper, d_lcycle, d_lpbox, d_lbox;
     bte::DBuf d_pborders, d_ppieces;  // convex-polygon path (geometries that are not a grid)
     bte::DBuf d_row_ptr, d_lrow, d_lcol, d_lcdf, d_lalias, d_mirror;
     int nclass = 0;
@@ -223,4 +228,6 @@ FixScale choose_scale(double x0, double x1, double y0, double y1, double vmax, d
 // The integer units of a grid run with bins of `step` ps, and their tables
 // on the device: fills the grid arguments (no allocation).
 void prepare_fixed(bte_ctx* c, double step, GridArgs& A);
+// The same for a run over linked cells.
+void prepare_link(bte_ctx* c, double step, LinkArgs& A);
 }  // namespace bte

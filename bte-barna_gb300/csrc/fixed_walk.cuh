@@ -141,6 +141,19 @@ BTE_HD uint64_t fix_flight(float e, double tau, int kt, uint32_t& hi) {
     return x < 32 ? p << x : 0;
 }
 
+// t ps (a positive double) in ticks, truncated, as 96 bits; beyond them it
+// never ends.  Returns the low 64.
+BTE_HD uint64_t fix_ticks(double t, int kt, uint32_t& hi) {
+    const uint64_t b = dbits(t), m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL;
+    const int x = int((b >> 52) & 0x7ff) - 1075 + kt;
+    if (x <= 0) {
+        hi = 0;
+        return x > -64 ? m >> (-x) : 0;
+    }
+    hi = x < 12 ? 0 : x < 44 ? uint32_t(m >> (64 - x)) : 0xffffffffu;
+    return x < 64 ? m << x : 0;
+}
+
 // v 2^k to the nearest integer.
 BTE_HD int64_t fix_round(double v, int k) {
     const double s = bitsd(uint64_t(1023 + k) << 52);

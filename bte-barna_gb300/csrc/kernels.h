@@ -60,6 +60,7 @@ struct GridArgs {
     const unsigned long long* wxf;  // and the widths between them
     const unsigned long long* wyf;
     const int* map;          // the cells with a void rim: [nx + 2][ny + 2], as G.cell
+    int refill;              // idle lanes of a warp before new particles are generated
     int cls[4];              // normal classes of the +x, -x, +y, -y walls (-1: none)
 };
 
@@ -107,6 +108,36 @@ struct PolyArgs {
     const long long* dmm_row;
     const DmmEnt* dmm_ent;
 };
+
+// Linked cells of axis-aligned boxes (rta_link.cu, build_link_grid): in the
+// run's integer units the lines, widths and mode velocities, and per cell and
+// side (+x, -x, +y, -y) what lies across it.
+struct LinkEntry {
+    int cell, box, flags, cls;  // LK_*; above bit 8 the mismatch table + 1 of an interface
+};
+constexpr int LK_VOID = 1, LK_RESERVOIR = 2, LK_TRANSLATE = 4, LK_INNER = 8;
+struct LinkArgs {
+    FixScale fx;
+    const ModeFix* mf;
+    const long long* gxf;
+    const long long* gyf;
+    const unsigned long long* wxf;
+    const unsigned long long* wyf;
+    int ny, refill;
+    const int4* side;            // [cell = i ny + j][4] LinkEntry
+    const int4* range;           // [box] columns [x, y) and rows [z, w)
+    const unsigned char* per;    // [box] 1: spans the period in x, 2: in y
+    const int* cellbox;          // [cell] its box
+    const int4* cycle;           // [cell] columns of its x period, rows of its y period (-1: none)
+    const int* pbox;             // [cell][4] the periodic box across a side (null: none that is entered)
+    unsigned long long margin;   // 2e-6 nm
+    const long long* dmm_row;
+    const DmmEnt* dmm_ent;
+};
+bool launch_steady_link(const DevTables& T, const SteadyArgs& S, const LinkArgs& A, double* tally,
+                        unsigned long long* counters, int* err, int nsm, cudaStream_t s);
+bool launch_prod_link(const DevTables& T, const LinkArgs& A, double* tally, unsigned long long* counters, int* err,
+                      unsigned long long* work, int nsm, cudaStream_t s);
 
 // Adjoint passes of the grid kernel: the functional's weights per tally
 // value, each particle's total contribution (slot = particle - first),

@@ -311,6 +311,20 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
                           nullptr, nullptr,
                           crystals ? c->d_dmm_row.as<long long>() : nullptr,
                           crystals ? c->d_dmm_ent.as<DmmEnt>() : nullptr};
+        // rectangular boxes walk linked cells, in time units that hold the
+        // fastest mode's flight across the domain a few times over
+        const bool linked = !replay && c->link.ok && !(p->flags & BTE_FLAG_GENERAL);
+        LinkArgs LA{};
+        double unit_t = 1., unit_x = 1.;
+        if (linked) {
+            const double ext = std::max(c->link.gx.back() - c->link.gx.front(), c->link.gy.back() - c->link.gy.front());
+            prepare_link(c, c->vmax > 0. ? 4.0 * ext / c->vmax : 1.0, LA);
+            LA.pbox = c->d_lpbox.as<int>();
+            LA.refill = 8;
+            if (!crystals) LA.dmm_row = nullptr;
+            unit_t = LA.fx.per_tick();
+            unit_x = LA.fx.per_unit();
+        }
         const int max_gen = p->max_generations > 0 ? p->max_generations : 100000;
         std::vector<double> oldv(size_t(3) * nbx, 0.), cur(size_t(3) * nbx, 0.);
         std::vector<unsigned long long> hex, hphi(static_cast<size_t>(nbx));
@@ -340,7 +354,11 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
             else if (p->flags & BTE_FLAG_GENERAL)
                 launch_steady_prod(T, A, S.tally.as<double>(), S.counters.as<unsigned long long>(),
                                    S.err.as<int>(), nullptr, c->nsm, st);
-            else if (!launch_steady_poly(T, A, PA, S.tally.as<double>(), S.counters.as<unsigned long long>(),
+            else if (linked) {
+                if (!launch_steady_link(T, A, LA, S.tally.as<double>(), S.counters.as<unsigned long long>(),
+                                        S.err.as<int>(), c->nsm, st))
+                    throw Error(BTE_ERR_CUDA, "steady linked-cell kernel does not fit on the device");
+            } else if (!launch_steady_poly(T, A, PA, S.tally.as<double>(), S.counters.as<unsigned long long>(),
                                          S.err.as<int>(), c->nsm, st))
                 throw Error(BTE_ERR_CUDA, "steady polygon kernel does not fit on the device");
             ck(cudaGetLastError(), "steady launch");
@@ -383,7 +401,7 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
                         const unsigned long long hi = hex[6 * b + 2 * q], lo = hex[6 * b + 2 * q + 1];
                         v = double((__int128)(((unsigned __int128)hi << 64) | lo)) / FIX_SCALE;
                     } else {
-                        v = htal[3 * b + q];
+                        v = htal[3 * b + q] * (q == 0 ? unit_t : unit_x);
                     }
                     cur[size_t(q) * nbx + b] = v;
                 }

@@ -883,6 +883,141 @@ TranslationFast build_translation_fast(const HostGeometry& g, double margin) {
     return R;
 }
 
+LinkGrid build_link_grid(const HostGeometry& g) {
+    LinkGrid L;
+    const std::size_t nbx = g.boxes.size();
+    std::vector<std::array<double, 4>> r(nbx);  // x0, y0, x1, y1
+    for (std::size_t b = 0; b < nbx; ++b) {
+        const GBox& B = g.boxes[b];
+        const std::vector<V2> hull(g.hull.begin() + B.hull_off, g.hull.begin() + B.hull_off + B.nhull);
+        if (!as_rect(hull, r[b][0], r[b][1], r[b][2], r[b][3])) return L;
+        L.gx.insert(L.gx.end(), {r[b][0], r[b][2]});
+        L.gy.insert(L.gy.end(), {r[b][1], r[b][3]});
+    }
+    for (std::vector<double>* v : {&L.gx, &L.gy}) {
+        std::sort(v->begin(), v->end());
+        v->erase(std::unique(v->begin(), v->end()), v->end());
+    }
+    const int nx = L.nx = int(L.gx.size()) - 1, ny = L.ny = int(L.gy.size()) - 1;
+    if (nx < 1 || ny < 1 || double(nx) * ny > 4.0e6) return L;
+    const double ext = std::max(L.gx.back() - L.gx.front(), L.gy.back() - L.gy.front());
+    for (int i = 0; i < nx; ++i)
+        if (!(L.gx[std::size_t(i) + 1] - L.gx[std::size_t(i)] > 1e-9 * ext)) return L;
+    for (int j = 0; j < ny; ++j)
+        if (!(L.gy[std::size_t(j) + 1] - L.gy[std::size_t(j)] > 1e-9 * ext)) return L;
+    auto line = [](const std::vector<double>& v, double x) {
+        return int(std::lower_bound(v.begin(), v.end(), x) - v.begin());
+    };
+    std::vector<int>& box = L.box;
+    box.assign(std::size_t(nx) * ny, -1);
+    auto at = [&](int i, int j) { return i < 0 || j < 0 || i >= nx || j >= ny ? -1 : box[std::size_t(i) * ny + j]; };
+    L.range.resize(4 * nbx);
+    for (std::size_t b = 0; b < nbx; ++b) {
+        int* q = L.range.data() + 4 * b;
+        q[0] = line(L.gx, r[b][0]);
+        q[1] = line(L.gx, r[b][2]);
+        q[2] = line(L.gy, r[b][1]);
+        q[3] = line(L.gy, r[b][3]);
+        for (int i = q[0]; i < q[1]; ++i)
+            for (int j = q[2]; j < q[3]; ++j) {
+                int& c = box[std::size_t(i) * ny + j];
+                if (c != -1) return L;
+                c = int(b);
+            }
+    }
+    const V2 normal[4] = {v2(1, 0), v2(-1, 0), v2(0, 1), v2(0, -1)};
+    int cls[4];
+    for (int s = 0; s < 4; ++s) {
+        cls[s] = -1;
+        for (std::size_t k = 0; k < g.normals.size(); ++k)
+            if (g.normals[k].x == normal[s].x && g.normals[k].y == normal[s].y) cls[s] = int(k);
+    }
+    // the contact of box a with box b across a side with this normal, -1: none
+    auto contact = [&](int a, int b, V2 n) {
+        const GBox& A = g.boxes[std::size_t(a)];
+        for (int i = 0; i < A.ncontacts; ++i) {
+            const std::size_t ci = std::size_t(A.contact_off + i);
+            if (g.contacts[ci].id == b && g.contacts[ci].np.x == n.x && g.contacts[ci].np.y == n.y) return int(ci);
+        }
+        return -1;
+    };
+    L.side.assign(box.size() * 4, LinkSide{-1, -1, LINK_VOID, -1});
+    for (int i = 0; i < nx; ++i)
+        for (int j = 0; j < ny; ++j) {
+            const int a = at(i, j);
+            if (a < 0 || g.reservoir[std::size_t(a)] || g.tto[std::size_t(a)] >= 0) continue;
+            for (int s = 0; s < 4; ++s) {
+                LinkSide& k = L.side[(std::size_t(i) * ny + j) * 4 + std::size_t(s)];
+                k.cls = cls[s];
+                const int ti = i + int(normal[s].x), tj = j + int(normal[s].y);
+                int b = at(ti, tj);
+                if (b < 0) {
+                    if (cls[s] < 0) return L;
+                    continue;
+                }
+                k.flags = 0;
+                k.cell = ti * ny + tj;
+                k.box = b;
+                if (b == a) {
+                    k.flags = LINK_INNER;
+                    continue;
+                }
+                const int ci = contact(a, b, normal[s]);
+                if (ci < 0) return L;
+                if (g.mat[std::size_t(a)] != g.mat[std::size_t(b)]) k.flags |= (ci + 1) << 8;
+                if (g.reservoir[std::size_t(b)]) {
+                    k.flags |= LINK_RESERVOIR;
+                } else if (g.tto[std::size_t(b)] >= 0) {
+                    // translated onto the far line of the target box
+                    const V2 t = g.translation[std::size_t(b)];
+                    const bool x = s < 2, up = s % 2 == 0;
+                    if (x ? !(t.y == 0. && (up ? t.x < 0. : t.x > 0.)) : !(t.x == 0. && (up ? t.y < 0. : t.y > 0.))) return L;
+                    const std::vector<double>& v = x ? L.gx : L.gy;
+                    const double to = v[std::size_t((x ? i : j) + (up ? 1 : 0))] + (x ? t.x : t.y);
+                    int m = line(v, to - 1e-9 * ext);
+                    if (m >= int(v.size()) || std::fabs(v[std::size_t(m)] - to) > 1e-9 * ext) return L;
+                    const int in = up ? m : m - 1, q = up ? m - 1 : m;  // entered, and the target's side of the line
+                    const int bi = x ? in : i, bj = x ? j : in;
+                    b = at(bi, bj);
+                    if (b < 0 || g.reservoir[std::size_t(b)] || g.tto[std::size_t(b)] >= 0) return L;
+                    if (at(x ? q : i, x ? j : q) != g.tto[std::size_t(k.box)]) return L;
+                    if (contact(g.tto[std::size_t(k.box)], b, normal[s]) < 0) return L;
+                    k.flags |= LINK_TRANSLATE;
+                    k.cell = bi * ny + bj;
+                    k.box = b;
+                }
+            }
+        }
+    // periods: a run of cells of one column or row whose last leads back to
+    // its first through a translation, within one crystal
+    L.cycle.assign(box.size() * 4, -1);
+    for (int ax = 0; ax < 2; ++ax) {
+        const int n = ax ? ny : nx, m = ax ? nx : ny;
+        for (int o = 0; o < m; ++o)
+            for (int last = 0; last < n; ++last) {
+                const int cl = ax ? o * ny + last : last * ny + o;
+                const LinkSide& k = L.side[std::size_t(cl) * 4 + std::size_t(ax ? 2 : 0)];
+                if (k.flags != LINK_TRANSLATE) continue;
+                const int first = ax ? k.cell % ny : k.cell / ny;
+                if (first > last) continue;
+                const LinkSide& back = L.side[std::size_t(k.cell) * 4 + std::size_t(ax ? 3 : 1)];
+                bool ok = back.flags == LINK_TRANSLATE && back.cell == cl;
+                for (int q = first; q < last && ok; ++q) {
+                    const int c0 = ax ? o * ny + q : q * ny + o, c1 = ax ? o * ny + q + 1 : (q + 1) * ny + o;
+                    const LinkSide& f = L.side[std::size_t(c0) * 4 + std::size_t(ax ? 2 : 0)];
+                    ok = (f.flags == 0 || f.flags == LINK_INNER) && f.cell == c1;
+                }
+                for (int q = first; q <= last && ok; ++q) {
+                    const int c = ax ? o * ny + q : q * ny + o;
+                    L.cycle[std::size_t(c) * 4 + std::size_t(2 * ax)] = first;
+                    L.cycle[std::size_t(c) * 4 + std::size_t(2 * ax + 1)] = last;
+                }
+            }
+    }
+    L.ok = true;
+    return L;
+}
+
 Generators build_initial_generators(const HostModes& m, const HostGeometry& g, const GenEmbed* e) {
     Generators R;
     const std::size_t n = m.n();

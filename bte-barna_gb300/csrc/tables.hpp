@@ -71,6 +71,30 @@ struct TranslationFast {
 };
 TranslationFast build_translation_fast(const HostGeometry& g, double margin = 1.0e-2);
 
+// Boxes that are all axis-aligned rectangles, cut into the cells of the lines
+// through all their edges: what lies across each side of each cell.  `ok`
+// only where every side has one definite answer (no sliver between lines, a
+// contact behind every shared side, periodic boxes that translate along the
+// axis they are entered on into a box next to their target).
+struct LinkSide {  // the layout of int4
+    int cell;      // the cell entered
+    int box;       // its box (a reservoir's where it is one)
+    int flags;     // LINK_*, and contact index + 1 above bit 8 where the crystals differ
+    int cls;       // wall class of the side
+};
+enum { LINK_VOID = 1, LINK_RESERVOIR = 2, LINK_TRANSLATE = 4, LINK_INNER = 8 };
+struct LinkGrid {
+    bool ok = false;
+    int nx = 0, ny = 0;
+    std::vector<double> gx, gy;       // lines, nx + 1 and ny + 1
+    std::vector<LinkSide> side;       // [cell = i ny + j][+x, -x, +y, -y]
+    std::vector<int> range;           // [box][4] its columns [i0, i1) and rows [j0, j1)
+    std::vector<int> box;             // [cell] its box, -1: void
+    std::vector<int> cycle;           // [cell][4] first and last column of the x period the cell
+                                      // lies in (-1: none), first and last row of the y period
+};
+LinkGrid build_link_grid(const HostGeometry& g);
+
 // Alias entry of a Lambert row: pick slot j, keep its mode with probability
 // prob, else take alt (Walker / Vose).
 struct AliasRow {
