@@ -107,6 +107,8 @@ void upload_pinned(DBuf& d, Pinned& h, const std::vector<T>& v, cudaStream_t s) 
     ck(cudaMemcpyAsync(d.p, h.p, bytes, cudaMemcpyHostToDevice, s), "h2d");
 }
 
+struct BertaPlan;
+
 struct BertaState {
     bool have_prop = false;
     int nm = 0;
@@ -131,11 +133,14 @@ struct BertaState {
     Pinned h_gens[1];                       // staging: descriptors of the initial particles
     // device-resident step loop: counters, planned sources, per-step records
     DBuf d_dc, d_span, d_gdesc, d_ggenf, d_gcnt, d_idesc, d_igenf, d_icnt, d_adi, d_adesc, d_acnt;
-    DBuf d_phist, d_nhist, d_sa, d_sb, d_sc, d_sd, d_sx0, d_sxs;
+    DBuf d_phist, d_nhist, d_res, d_sa, d_sb, d_sc, d_sd, d_sx0, d_sxs;
 
-    std::vector<Spline1D> spl;
-    std::vector<char> spl_ok;
-    long long spl_version = -1;   // tables the splines were built for
+    // what a run takes from the tables alone, kept while they stay: sources,
+    // adiabatic borders and their splines (BertaPlan); the phase events
+    BertaPlan* plan = nullptr;
+    DBuf d_wallreq, d_wallsum;
+    std::vector<cudaEvent_t> events;
+    ~BertaState();
 };
 
 void reset_propagators(bte_ctx* c) {
@@ -415,6 +420,31 @@ __device__ __forceinline__ float wall_pmf_f(float w, float vn, float ce, float q
     else
         diff = 1.f / expm1f(xw) - 1.f / expm1f(xe);
     return vn * w * fabsf(diff);
+}
+
+// Energy flux (per 1e12 hbar) of an isothermal wall at `Tw` against a box at
+// `Te` with inward normal (nx, ny): sum over modes of v_n omega
+// |n(omega, Tw) - n(omega, Te)| (src/sampling.cpp:189-269), in FP64.  One block
+// per request; the 400 requests of a ribbon's four walls over 6144 modes took
+// the host 8 ms at every run, this 0.2 ms once per mode table and geometry.
+__global__ void __launch_bounds__(256) be_wall_sums(const double* om, const double* vx, const double* vy, int n,
+                                                    const WallReq* req, double* sum) {
+    const WallReq R = req[blockIdx.x];
+    constexpr double pre = 1e12 * 1.054571726e-34 / 1.3806488e-23;
+    double s = 0.;
+    for (int k = threadIdx.x; k < n; k += 256) {
+        const double w = om[k], vn = R.nx * vx[k] + R.ny * vy[k];
+        if (vn <= 0. || almost_equal(0., w)) continue;
+        s += vn * w * fabs(1. / (exp(pre * w / R.Tw) - 1.) - 1. / (exp(pre * w / R.Te) - 1.));
+    }
+    __shared__ double part[8];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) s += part[k];
+        sum[blockIdx.x] = s;
+    }
 }
 
 // pass 1: the chunk's running sums in place and its total
@@ -1165,6 +1195,203 @@ double Spline1D::interp(double x) const {
 
 }  // namespace bte
 
+namespace bte {
+
+// What the runs on one mode table and geometry share: the sources' tables,
+// the adiabatic borders, and the J(T) -> T splines of their walls.  Built for
+// a table version; the gradient source also for its parameters.
+struct BertaPlan {
+    long long version = -1;
+    Generators iso, ini;
+    bool have_ini = false;
+    int nk = 0;                                  // spline intervals
+    std::vector<AdiBorder> adi;
+    int grad_mode = -1;
+    double gx = 0., gy = 0.;
+    GradGenerators grad;
+};
+
+BertaState::~BertaState() {
+    delete plan;
+    for (auto e : events) cudaEventDestroy(e);
+}
+
+namespace {
+
+// The adiabatic borders (src/beyondRTA_MC2d.cpp:294-350): segment, inward
+// normal, Teq and the J(T) -> T spline of the wall, one per normal and Teq,
+// over 10 to 1000 K.
+void plan_adiabatic_borders(bte_ctx* c, BertaState& B, BertaPlan& P) {
+    const HostModes& m = c->modes;
+    const HostGeometry& g = c->geom;
+    const double vuc = m.V * g.thickness / m.c;
+    const std::size_t nborders = g.borders.size();
+    std::vector<int> border_box(nborders, -1);
+    for (std::size_t b = 0; b < g.boxes.size(); ++b)
+        for (int k = 0; k < g.boxes[b].nborders; ++k) border_box[std::size_t(g.boxes[b].border_off + k)] = int(b);
+    constexpr int NT = 100;
+    P.adi.assign(nborders, AdiBorder{});
+    std::map<std::tuple<double, double, double>, int> spline_of;
+    std::vector<WallReq> req;
+    for (std::size_t gb = 0; gb < nborders; ++gb) {
+        AdiBorder& A = P.adi[gb];
+        const int b = border_box[gb];
+        const GBorder& br = g.borders[gb];
+        A.x0 = br.p1.x;
+        A.y0 = br.p1.y;
+        A.dx = br.nd.x;
+        A.dy = br.nd.y;
+        A.nx = -br.np.x;
+        A.ny = -br.np.y;
+        A.len = norm(sub(br.p2, br.p1));
+        A.box = b;
+        A.spline = -1;
+        if (b < 0 || g.reservoir[std::size_t(b)] || g.tto[std::size_t(b)] >= 0) continue;
+        A.Teq = g.Teq[std::size_t(b)];
+        const auto it = spline_of.emplace(std::make_tuple(A.nx, A.ny, A.Teq), int(spline_of.size()));
+        A.spline = it.first->second;
+        if (it.second)
+            for (int t = 0; t < NT; ++t) req.push_back(WallReq{A.nx, A.ny, 10.0 + 10.0 * t, A.Teq});
+    }
+    P.nk = 0;
+    if (!req.empty()) {
+        std::vector<double> sum(req.size());
+        B.d_wallreq.upload(req, c->stream);
+        B.d_wallsum.alloc(req.size() * sizeof(double));
+        DBuf om;
+        om.upload(m.omega, c->stream);
+        B.d_rvx.upload(m.vx, c->stream);
+        B.d_rvy.upload(m.vy, c->stream);
+        be_wall_sums<<<unsigned(req.size()), 256, 0, c->stream>>>(om.as<double>(), B.d_rvx.as<double>(), B.d_rvy.as<double>(),
+                                                                  int(m.n()), B.d_wallreq.as<WallReq>(),
+                                                                  B.d_wallsum.as<double>());
+        ck(cudaGetLastError(), "wall sums launch");
+        ck(cudaMemcpyAsync(sum.data(), B.d_wallsum.p, sum.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "d2h");
+        sync(c);
+        std::vector<double> sa, sb, sc, sd, sx0, sxs, J(NT), Tv(NT);
+        for (std::size_t s0 = 0; s0 < req.size(); s0 += NT) {
+            for (int t = 0; t < NT; ++t) {
+                const WallReq& R = req[s0 + std::size_t(t)];
+                Tv[std::size_t(t)] = R.Tw;
+                J[std::size_t(t)] = ((R.Tw - R.Te) >= 0 ? 1 : -1) *
+                                    (1.0e+12 * 1.054571726e-34 * sum[s0 + std::size_t(t)] / (double(m.nq) * vuc));
+            }
+            Spline1D sp;
+            sp.build(J, Tv);
+            P.nk = int(sp.a.size());
+            sa.insert(sa.end(), sp.a.begin(), sp.a.end());
+            sb.insert(sb.end(), sp.b.begin(), sp.b.end());
+            sc.insert(sc.end(), sp.c.begin(), sp.c.end());
+            sd.insert(sd.end(), sp.d.begin(), sp.d.end());
+            sx0.insert(sx0.end(), sp.x0.begin(), sp.x0.end());
+            sxs.insert(sxs.end(), sp.xs.begin(), sp.xs.end());
+        }
+        B.d_sa.upload(sa, c->stream);
+        B.d_sb.upload(sb, c->stream);
+        B.d_sc.upload(sc, c->stream);
+        B.d_sd.upload(sd, c->stream);
+        B.d_sx0.upload(sx0, c->stream);
+        B.d_sxs.upload(sxs, c->stream);
+    }
+    B.d_adi.upload(P.adi, c->stream);
+    sync(c);
+}
+
+// The tables of the sources and walls for the loaded modes and geometry.
+BertaPlan& berta_plan(bte_ctx* c, BertaState& B, const bte_berta_params* p) {
+    const HostModes& m = c->modes;
+    const HostGeometry& g = c->geom;
+    cudaStream_t s = c->stream;
+    if (!B.plan) B.plan = new BertaPlan();
+    BertaPlan& P = *B.plan;
+    if (P.version != c->tables_version) {
+        P.version = -1;
+        P.grad_mode = -1;
+        try {
+            P.iso = build_wall_generators(m, g);
+        } catch (const Error&) {
+            P.iso = Generators();
+        }
+        try {
+            P.ini = build_initial_generators(m, g);
+            P.have_ini = true;
+        } catch (const Error&) {
+            P.have_ini = false;
+        }
+        plan_adiabatic_borders(c, B, P);
+        // the isothermal walls' alias rows do not change during a run
+        std::vector<float> ip(P.iso.alias.size());
+        std::vector<int> ia(P.iso.alias.size());
+        for (std::size_t i = 0; i < ip.size(); ++i) {
+            ip[i] = P.iso.alias[i].prob;
+            ia[i] = P.iso.alias[i].alt;
+        }
+        B.d_isoprob.upload(ip, s);
+        B.d_isoalt.upload(ia, s);
+        // FP32 copies for the adiabatic walls' pmf (omega = 0 where
+        // almost_equal(0, omega): those modes take no part)
+        std::vector<float> omf(m.omega.size()), vxf(m.omega.size()), vyf(m.omega.size());
+        for (std::size_t k = 0; k < omf.size(); ++k) {
+            omf[k] = almost_equal(0., m.omega[k]) ? 0.f : float(m.omega[k]);
+            vxf[k] = float(m.vx[k]);
+            vyf[k] = float(m.vy[k]);
+        }
+        B.d_om.upload(omf, s);
+        B.d_vx.upload(vxf, s);
+        B.d_vy.upload(vyf, s);
+        B.d_rvx.upload(m.vx, s);
+        B.d_rvy.upload(m.vy, s);
+        // walls of each box: global border index of its +x, -x, +y, -y border
+        std::vector<int4> boxwall(g.boxes.size(), make_int4(-1, -1, -1, -1));
+        for (std::size_t b = 0; b < g.boxes.size(); ++b) {
+            const GBox& bx = g.boxes[b];
+            for (int k = 0; k < bx.nborders; ++k) {
+                const V2 np = g.borders[std::size_t(bx.border_off + k)].np;
+                const int gb = bx.border_off + k;
+                if (np.x == 1. && np.y == 0.) boxwall[b].x = gb;
+                if (np.x == -1. && np.y == 0.) boxwall[b].y = gb;
+                if (np.x == 0. && np.y == 1.) boxwall[b].z = gb;
+                if (np.x == 0. && np.y == -1.) boxwall[b].w = gb;
+            }
+        }
+        B.d_boxwall.upload(boxwall, s);
+        std::vector<int> hres(g.reservoir.begin(), g.reservoir.end());
+        B.d_res.upload(hres, s);
+        sync(c);
+        P.version = c->tables_version;
+    }
+    // the gradient source term (source_term_gradient,
+    // src/beyondRTA_MC2d.cpp:597-676): a homogeneous <gradient> on every
+    // box that is neither a reservoir nor periodic, or the least-squares
+    // gradients of the boxes' Teq (calculate_gradientT, the reference's
+    // default, src/beyondRTA_MC2d.cpp:1441-1458); Nabla_T rows at each
+    // box's Teq for the boxes with a gradient
+    if (P.grad_mode != p->gradient_mode || (p->gradient_mode == 1 && (P.gx != p->gradient[0] || P.gy != p->gradient[1]))) {
+        P.grad_mode = -1;
+        P.grad = p->gradient_mode == 1 ? build_gradient_generators(m, g, p->gradient[0], p->gradient[1])
+                                       : build_gradient_generators_boxes(m, g, calculate_gradientT(g));
+        if (!P.grad.box.empty()) {
+            std::vector<float> gp(P.grad.alias.size());
+            std::vector<int> ga(P.grad.alias.size());
+            for (std::size_t i = 0; i < gp.size(); ++i) {
+                gp[i] = P.grad.alias[i].prob;
+                ga[i] = P.grad.alias[i].alt;
+            }
+            B.d_gprob.upload(gp, s);
+            B.d_galt.upload(ga, s);
+            B.d_gsign.upload(P.grad.sign, s);
+            sync(c);
+        }
+        P.gx = p->gradient[0];
+        P.gy = p->gradient[1];
+        P.grad_mode = p->gradient_mode;
+    }
+    return P;
+}
+
+}  // namespace
+}  // namespace bte
+
 using bte::Error;
 
 extern "C" bte_status bte_load_propagator(bte_ctx* c, const bte_propagator* P) {
@@ -1305,23 +1532,6 @@ std::size_t n_to_generate(double gen, bte::Pcg64& rng) {
     return np;
 }
 
-// Isothermal_wall_distribution pmf for normal n (src/sampling.cpp:189-269);
-// returns cumulsum = 1e12 hbar sum(pmf).
-double wall_pmf(const bte::HostModes& m, bte::V2 n, double Tw, double Te, std::vector<double>& pmf) {
-    pmf.assign(m.n(), 0.);
-    for (std::size_t k = 0; k < m.n(); ++k) {
-        const double vn = n.x * m.vx[k] + n.y * m.vy[k] + 0. * m.vz[k];
-        if (vn <= 0. || bte::almost_equal(0., m.omega[k]))
-            pmf[k] = 0.;
-        else
-            pmf[k] = vn * m.omega[k] *
-                     std::fabs(bte::bose_einstein(m.omega[k], Tw) - bte::bose_einstein(m.omega[k], Te));
-    }
-    double s = 0.;
-    for (double x : pmf) s += x;
-    return 1.0e+12 * 1.054571726e-34 * s;
-}
-
 [[noreturn]] void throw_step_error(int e) {
     throw Error(bte_status(e), e == BTE_ERR_LIMIT      ? "particle capacity or step cap exceeded"
                                : e == BTE_ERR_GEOMETRY ? "geometry error in the advection"
@@ -1367,24 +1577,10 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         const int nborders = int(g.borders.size());
         const double vuc = m.V * g.thickness / m.c;
         cudaStream_t s = c->stream;
-        // walls of each box: global border index of its +x, -x, +y, -y border
-        std::vector<int4> boxwall(std::size_t(nbx), make_int4(-1, -1, -1, -1));
-        for (int b = 0; b < nbx; ++b) {
-            const GBox& bx = g.boxes[std::size_t(b)];
-            for (int k = 0; k < bx.nborders; ++k) {
-                const V2 np = g.borders[std::size_t(bx.border_off + k)].np;
-                const int gb = bx.border_off + k;
-                if (np.x == 1. && np.y == 0.) boxwall[std::size_t(b)].x = gb;
-                if (np.x == -1. && np.y == 0.) boxwall[std::size_t(b)].y = gb;
-                if (np.x == 0. && np.y == 1.) boxwall[std::size_t(b)].z = gb;
-                if (np.x == 0. && np.y == -1.) boxwall[std::size_t(b)].w = gb;
-            }
-        }
-        std::vector<int> border_box(std::size_t(nborders), -1);
-        for (int b = 0; b < nbx; ++b)
-            for (int k = 0; k < g.boxes[std::size_t(b)].nborders; ++k)
-                border_box[std::size_t(g.boxes[std::size_t(b)].border_off + k)] = b;
-        B.d_boxwall.upload(boxwall, s);
+        const BertaPlan& PL = berta_plan(c, B, p);
+        const Generators &iso = PL.iso, &ini = PL.ini;
+        const GradGenerators& grad = PL.grad;
+        const bool have_ini = PL.have_ini;
         B.d_Eb.alloc(std::size_t(nborders) * sizeof(int));
         // per-step buffers at their largest size (one request per border),
         // so that no step reallocates
@@ -1393,38 +1589,13 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         B.d_cdftot.alloc(std::size_t(nborders) * sizeof(double));
         B.d_ctot.alloc(std::size_t(nborders) * ((m.n() + WCDF_CHUNK - 1) / WCDF_CHUNK) * sizeof(double));
         ck(cudaMemsetAsync(B.d_Eb.p, 0, std::size_t(nborders) * sizeof(int), s), "memset");
-        if (int(B.spl.size()) != nborders || B.spl_version != c->tables_version) {
-            B.spl.assign(std::size_t(nborders), Spline1D());
-            B.spl_ok.assign(std::size_t(nborders), 0);
-            B.spl_version = c->tables_version;
-        }
-        B.d_rvx.upload(m.vx, s);
-        B.d_rvy.upload(m.vy, s);
         B.d_H.alloc(std::size_t(nbx) * n * sizeof(int));
         B.d_cnt.alloc(std::size_t(nbx) * n * sizeof(int));
         B.d_props.alloc(std::size_t(nbx) * 3 * sizeof(double));
         c->d_err.alloc(4 * sizeof(int));
         ck(cudaMemsetAsync(c->d_err.p, 0, 4 * sizeof(int), s), "memset");
-        std::vector<int> hres(g.reservoir.begin(), g.reservoir.end());
-        DBuf d_res;
-        d_res.upload(hres, s);
         const long long cap = p->capacity > 0 ? p->capacity : (1ll << 24);
         alloc_particles(B, cap);
-        // sources: isothermal walls (static tables) and the initial deviation
-        Generators iso;
-        try {
-            iso = build_wall_generators(m, g);
-        } catch (const Error&) {
-            iso = Generators();
-        }
-        Generators ini;
-        bool have_ini = false;
-        try {
-            ini = build_initial_generators(m, g);
-            have_ini = true;
-        } catch (const Error&) {
-            have_ini = false;
-        }
         std::vector<std::pair<int, int>> cellof(std::size_t(nbx), {-1, -1});
         for (int i = 0; i < g.gnx; ++i)
             for (int j = 0; j < g.gny; ++j) {
@@ -1486,50 +1657,6 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             d.cdf = -1;
             return d;
         };
-        // the gradient source term (source_term_gradient,
-        // src/beyondRTA_MC2d.cpp:597-676): a homogeneous <gradient> on every
-        // box that is neither a reservoir nor periodic, or the least-squares
-        // gradients of the boxes' Teq (calculate_gradientT, the reference's
-        // default, src/beyondRTA_MC2d.cpp:1441-1458); Nabla_T rows at each
-        // box's Teq for the boxes with a gradient, built once as the
-        // reference's static generators are
-        GradGenerators grad = p->gradient_mode == 1
-                                  ? build_gradient_generators(m, g, p->gradient[0], p->gradient[1])
-                                  : build_gradient_generators_boxes(m, g, calculate_gradientT(g));
-        if (!grad.box.empty()) {
-            std::vector<float> gp(grad.alias.size());
-            std::vector<int> ga(grad.alias.size());
-            for (std::size_t i = 0; i < grad.alias.size(); ++i) {
-                gp[i] = grad.alias[i].prob;
-                ga[i] = grad.alias[i].alt;
-            }
-            B.d_gprob.upload(gp, s);
-            B.d_galt.upload(ga, s);
-            B.d_gsign.upload(grad.sign, s);
-        }
-        // generate the sources in `descs` (alias rows in aprob/aalt) at A[base..)
-        // the isothermal walls' alias rows do not change during a run
-        {
-            std::vector<float> ip(iso.alias.size());
-            std::vector<int> ia(iso.alias.size());
-            for (std::size_t i = 0; i < iso.alias.size(); ++i) {
-                ip[i] = iso.alias[i].prob;
-                ia[i] = iso.alias[i].alt;
-            }
-            B.d_isoprob.upload(ip, s);
-            B.d_isoalt.upload(ia, s);
-            // FP32 copies for the adiabatic walls' pmf (omega = 0 where
-            // almost_equal(0, omega): those modes take no part)
-            std::vector<float> omf(m.omega.size()), vxf(m.omega.size()), vyf(m.omega.size());
-            for (std::size_t k = 0; k < omf.size(); ++k) {
-                omf[k] = almost_equal(0., m.omega[k]) ? 0.f : float(m.omega[k]);
-                vxf[k] = float(m.vx[k]);
-                vyf[k] = float(m.vy[k]);
-            }
-            B.d_om.upload(omf, s);
-            B.d_vx.upload(vxf, s);
-            B.d_vy.upload(vyf, s);
-        }
         // generate the sources in `descs` at A[base..): alias rows from
         // aprob/aalt (uploaded here) or from a table already on the device
         // (rprob/ralt, with per-mode signs rsign), CDF rows from B.d_cdf
@@ -1663,66 +1790,11 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             B.d_igenf.upload(igenf, s);
             B.d_icnt.alloc(std::size_t(nid) * sizeof(long long));
         }
-        // adiabatic re-emission per void border: segment, inward normal, Teq
-        // and the J(T) -> T spline of its wall (one per normal and Teq)
-        std::vector<AdiBorder> adi(static_cast<std::size_t>(nborders));
-        std::vector<double> sa, sb, sc, sd, sx0, sxs;
-        std::map<std::tuple<double, double, double>, int> spline_of;
-        int spl_nk = 0;
-        std::vector<double> pmf;
-        for (int gb = 0; gb < nborders; ++gb) {
-            AdiBorder& A = adi[std::size_t(gb)];
-            const int b = border_box[std::size_t(gb)];
-            const GBorder& br = g.borders[std::size_t(gb)];
-            A.x0 = br.p1.x;
-            A.y0 = br.p1.y;
-            A.dx = br.nd.x;
-            A.dy = br.nd.y;
-            A.nx = -br.np.x;
-            A.ny = -br.np.y;
-            A.len = norm(sub(br.p2, br.p1));
-            A.box = b;
-            A.spline = -1;
-            if (b < 0 || g.reservoir[std::size_t(b)] || g.tto[std::size_t(b)] >= 0) continue;
-            const double Teq = g.Teq[std::size_t(b)];
-            A.Teq = Teq;
-            const auto key = std::make_tuple(A.nx, A.ny, Teq);
-            auto it = spline_of.find(key);
-            if (it == spline_of.end()) {
-                std::vector<double> J(100), Tv(100);
-                for (int t = 0; t < 100; ++t) {
-                    const double T = 10.0 + 10.0 * t;
-                    Tv[std::size_t(t)] = T;
-                    const double cs = wall_pmf(m, v2(A.nx, A.ny), T, Teq, pmf);
-                    J[std::size_t(t)] = ((T - Teq) >= 0 ? 1 : -1) * (cs / (double(m.nq) * vuc));
-                }
-                Spline1D sp;
-                sp.build(J, Tv);
-                spl_nk = int(sp.a.size());
-                sa.insert(sa.end(), sp.a.begin(), sp.a.end());
-                sb.insert(sb.end(), sp.b.begin(), sp.b.end());
-                sc.insert(sc.end(), sp.c.begin(), sp.c.end());
-                sd.insert(sd.end(), sp.d.begin(), sp.d.end());
-                sx0.insert(sx0.end(), sp.x0.begin(), sp.x0.end());
-                sxs.insert(sxs.end(), sp.xs.begin(), sp.xs.end());
-                it = spline_of.emplace(key, int(spline_of.size())).first;
-            }
-            A.spline = it->second;
-        }
-        B.d_adi.upload(adi, s);
+        // adiabatic re-emission per void border (plan_adiabatic_borders)
         B.d_adesc.alloc(std::size_t(nborders) * sizeof(GenDesc));
         B.d_acnt.alloc(std::size_t(nborders) * sizeof(long long));
-        SplineDev SP{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, spl_nk};
-        if (!sa.empty()) {
-            B.d_sa.upload(sa, s);
-            B.d_sb.upload(sb, s);
-            B.d_sc.upload(sc, s);
-            B.d_sd.upload(sd, s);
-            B.d_sx0.upload(sx0, s);
-            B.d_sxs.upload(sxs, s);
-            SP = SplineDev{B.d_sa.as<double>(), B.d_sb.as<double>(), B.d_sc.as<double>(), B.d_sd.as<double>(),
-                           B.d_sx0.as<double>(), B.d_sxs.as<double>(), spl_nk};
-        }
+        const SplineDev SP{B.d_sa.as<double>(), B.d_sb.as<double>(), B.d_sc.as<double>(), B.d_sd.as<double>(),
+                           B.d_sx0.as<double>(), B.d_sxs.as<double>(), PL.nk};
         const int nch = (n + WCDF_CHUNK - 1) / WCDF_CHUNK;
         const unsigned pblocks = unsigned(c->nsm) * 8u;  // persistent grids of the step kernels
         const BoxProp* bprop = p->rta ? nullptr : B.d_boxprop.as<BoxProp>();
@@ -1732,15 +1804,18 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         // borders of every step, read at the end
         enum { PH_ADV, PH_CANCEL, PH_GEN, PH_HIST, PH_PROPS, PH_READ, PH_SAVE, PH_SCAT };
         double phase[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        std::vector<cudaEvent_t> pev(std::size_t(nsteps) * 7, nullptr);
-        struct EvGuard {
+        std::vector<cudaEvent_t>& pev = B.events;
+        struct EvGuard {  // a long run's events beyond a few thousand are given back
             std::vector<cudaEvent_t>* e;
             ~EvGuard() {
-                for (auto ev : *e)
-                    if (ev) cudaEventDestroy(ev);
+                for (; e->size() > 4096; e->pop_back()) cudaEventDestroy(e->back());
             }
         } pe_guard{&pev};
-        for (auto& e : pev) ck(cudaEventCreate(&e), "cudaEventCreate");
+        while (pev.size() < std::size_t(nsteps) * 7) {
+            cudaEvent_t e = nullptr;
+            ck(cudaEventCreate(&e), "cudaEventCreate");
+            pev.push_back(e);
+        }
         phase[PH_READ] = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
         std::vector<int> hH;
         const int cancel_every = p->cancel_every > 0 ? p->cancel_every : 4;
@@ -1821,7 +1896,7 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             if (istep % cancel_every == 0) {
                 ck(cudaMemsetAsync(B.d_cnt.p, 0, hbytes, s), "memset");
                 be_cancel_dev<<<pblocks, 256, 0, s>>>(arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc + DC_NOUT, cap,
-                                                      B.d_H.as<int>(), B.d_cnt.as<int>(), n, d_res.as<int>(),
+                                                      B.d_H.as<int>(), B.d_cnt.as<int>(), n, B.d_res.as<int>(),
                                                       mix_key(p->seed, istep, 77));
                 ck(cudaMemsetAsync(dc + DC_NP, 0, sizeof(unsigned long long), s), "memset");
                 be_compact_dev<<<pblocks, 256, 0, s>>>(arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc + DC_NOUT, cap,
