@@ -8,13 +8,13 @@
 //   2 gradient source term: Nabla_T particles at random points of every box
 //     with a gradient, random sub-step (source_term_gradient :597-676,
 //     Nabla_T_distribution src/sampling.cpp:118-187)
-//                                           be_plan_sources, be_generate_dev
+//                                                   be_plan, be_generate_dev
 //   3 isothermal-wall injection, random sub-step (Isothermal_walls :446-585,
 //     Ntogenerate src/sampling.cpp:243-260)
-//                                           be_plan_sources, be_generate_dev
+//                                                   be_plan, be_generate_dev
 //   4 adiabatic diffuse re-emission of |Eborder| at the wall temperature from
 //     the J(T) cubic spline (adiabatic_diffuse_walls :281-435)
-//                  be_plan_adiabatic, be_wall_cdf1/2_dev, be_generate_dev
+//                                      be_plan, be_wall_cdf, be_generate_dev
 //   5 deletion of the absorbed particles, 6 propagator scattering with sign
 //     branching (Scattering :1073-1210, propagator_H::get
 //     src/collision_operator.cpp:892-903), each parent's branching attempts
@@ -127,13 +127,13 @@ struct BertaState {
     DBuf a_x, a_y, a_mode, a_box, a_sign;   // particles
     DBuf b_x, b_y, b_mode, b_box, b_sign;   // compaction / scattering output
     DBuf d_H, d_cnt, d_Eb, d_props, d_boxwall, d_gens, d_alias, d_rvx, d_rvy;
-    DBuf d_om, d_vx, d_vy, d_req, d_cdf, d_cdftot, d_isoprob, d_isoalt;
+    DBuf d_om, d_vx, d_vy, d_req, d_cdf, d_isoprob, d_isoalt;
     DBuf d_gprob, d_galt, d_gsign;          // gradient source rows
     DBuf d_ctot;                            // wall-CDF chunk sums
     Pinned h_gens[1];                       // staging: descriptors of the initial particles
     // device-resident step loop: counters, planned sources, per-step records
     DBuf d_dc, d_span, d_gdesc, d_ggenf, d_gcnt, d_idesc, d_igenf, d_icnt, d_adi, d_adesc, d_acnt;
-    DBuf d_phist, d_nhist, d_res, d_sa, d_sb, d_sc, d_sd, d_sx0, d_sxs;
+    DBuf d_phist, d_nhist, d_res, d_rank, d_pscat, d_sa, d_sb, d_sc, d_sd, d_sx0, d_sxs;
 
     // what a run takes from the tables alone, kept while they stay: sources,
     // adiabatic borders and their splines (BertaPlan); the phase events
@@ -222,11 +222,8 @@ struct AdvectArgs {
     const int4* boxwall;
     int* Eb;
     double dt;
-    unsigned long long key;  // Philox key of the random sub-steps
-    int random_substep;
     // boxes that do not tile a grid (or periodic boxes): the convex-box
     // tables and the key of the geometric choices
-    int general;
     unsigned long long gkey;
     int* err;
     DevTables T;
@@ -447,65 +444,70 @@ __global__ void __launch_bounds__(256) be_wall_sums(const double* om, const doub
     }
 }
 
-// pass 1: the chunk's running sums in place and its total
-__device__ __forceinline__ void wall_cdf1_body(const float* om, const float* vx, const float* vy, int n,
-                                               const WallReq* req, double* cdf, double* chunk_tot) {
-    __shared__ double part[256];
+// One chunk of a request's row: the running sums of its pmf and its total.
+// Threads take segments, and the segments' totals are scanned by warps (one
+// thread adding 256 totals in a row took 9 of this kernel's 22 us).
+__device__ __forceinline__ void wall_cdf_body(const float* om, const float* vx, const float* vy, int n,
+                                              const WallReq* req, double* cdf, double* chunk_tot) {
+    __shared__ double wsum[8];
     const int nch = (n + WCDF_CHUNK - 1) / WCDF_CHUNK;
     const int r = blockIdx.x / nch, ch = blockIdx.x % nch;
     const WallReq R = req[r];
     double* row = cdf + (long long)r * n;
     const int c0 = ch * WCDF_CHUNK, c1 = min(n, c0 + WCDF_CHUNK);
-    const int seg = (c1 - c0 + blockDim.x - 1) / blockDim.x;
-    const int k0 = c0 + threadIdx.x * seg, k1 = min(c1, k0 + seg);
+    constexpr int SEG = WCDF_CHUNK / 256;
+    const int k0 = c0 + threadIdx.x * SEG;
     constexpr double pre = 1e12 * 1.054571726e-34 / 1.3806488e-23;
     const float ce = float(pre / R.Te), q = float(R.Te / R.Tw), rr = float((R.Tw - R.Te) / R.Tw);
     const float nx = float(R.nx), ny = float(R.ny);
-    double acc = 0.;
-    for (int k = k0; k < k1; ++k) {
-        const float w = __ldg(om + k);  // 0 where almost_equal(0, omega)
-        const float vn = nx * __ldg(vx + k) + ny * __ldg(vy + k);
-        const float p = (vn > 0.f && w != 0.f) ? wall_pmf_f(w, vn, ce, q, rr) : 0.f;
-        acc += double(p);
-        row[k] = acc;  // running sum within the thread's segment
-    }
-    part[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {  // exclusive offsets of the segments
-        double sum = 0.;
-        for (int t = 0; t < blockDim.x; ++t) {
-            const double v = part[t];
-            part[t] = sum;
-            sum += v;
+    double run[SEG], acc = 0.;
+#pragma unroll
+    for (int j = 0; j < SEG; ++j) {
+        const int k = k0 + j;
+        float p = 0.f;
+        if (k < c1) {
+            const float w = __ldg(om + k);  // 0 where almost_equal(0, omega)
+            const float vn = nx * __ldg(vx + k) + ny * __ldg(vy + k);
+            if (vn > 0.f && w != 0.f) p = wall_pmf_f(w, vn, ce, q, rr);
         }
-        chunk_tot[blockIdx.x] = sum;
+        acc += double(p);
+        run[j] = acc;
     }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double inc = acc;
+    for (int o = 1; o < 32; o <<= 1) {
+        const double t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) wsum[warp] = inc;
     __syncthreads();
-    const double off = part[threadIdx.x];
-    for (int k = k0; k < k1; ++k) row[k] += off;
+    double off = inc - acc;
+    for (int w = 0; w < warp; ++w) off += wsum[w];
+#pragma unroll
+    for (int j = 0; j < SEG; ++j)
+        if (k0 + j < c1) row[k0 + j] = run[j] + off;
+    if (threadIdx.x == 255) chunk_tot[blockIdx.x] = off + acc;
 }
 
-// pass 2: offsets of the chunks, normalisation, the request's total
-__device__ __forceinline__ void wall_cdf2_body(int n, const double* chunk_tot, double* cdf, double* tot) {
+// A mode of row r by inversion: u times the row's total, its chunk, and the
+// first running sum in it that is not below; -1 where the row is empty.
+__device__ __forceinline__ int wall_cdf_draw(const double* cdf, const double* chunk_tot, int r, int n, double u) {
     const int nch = (n + WCDF_CHUNK - 1) / WCDF_CHUNK;
-    const int r = blockIdx.x / nch, ch = blockIdx.x % nch;
-    double off = 0., total = 0.;
-    for (int c = 0; c < nch; ++c) {
-        const double v = chunk_tot[(long long)r * nch + c];
-        if (c < ch) off += v;
-        total += v;
-    }
-    if (ch == 0 && threadIdx.x == 0) tot[r] = total;
-    if (!(total > 0.)) return;
-    double* row = cdf + (long long)r * n;
+    const double* t = chunk_tot + (long long)r * nch;
+    double total = 0.;
+    for (int c = 0; c < nch; ++c) total += t[c];
+    if (!(total > 0.)) return -1;
+    double x = u * total;
+    int ch = 0;
+    for (; ch < nch - 1 && x > t[ch]; ++ch) x -= t[ch];
     const int c0 = ch * WCDF_CHUNK, c1 = min(n, c0 + WCDF_CHUNK);
-    for (int k = c0 + threadIdx.x; k < c1; k += blockDim.x) row[k] = (row[k] + off) / total;
+    const int k = lower_bound_d(cdf + (long long)r * n + c0, c1 - c0, x);
+    return min(c0 + k, c1 - 1);
 }
 
 // New particles [base, base + n) from the step's sources.
 __global__ void be_generate(PArr P, long long base, long long n, const GenDesc* gens, int ngen,
-                            const float* aprob, const int* aalt, const signed char* asign,
-                            const double* cdfs, const double* cdftot, int nmodes, unsigned long long key,
+                            const float* aprob, const int* aalt, int nmodes, unsigned long long key,
                             const GBox* boxes, const V2* hull) {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
          k += (long long)gridDim.x * blockDim.x) {
@@ -518,12 +520,11 @@ __global__ void be_generate(PArr P, long long base, long long n, const GenDesc* 
         Philox g;
         g.init(key, (uint64_t)k);
         double x, y;
-        bool placed = true;
         if (gd.rect == 2) {
             // a box that is not a grid cell: bounding box and rejection
             // (geometry_2d::get_random_point, include/geometry_2d.hpp:338-356)
             const GBox& Bx = boxes[gd.box];
-            placed = false;
+            bool placed = false;
             for (int tries = 0; tries < 100000 && !placed; ++tries) {
                 x = gd.x0 + g.uniform() * gd.dx;
                 y = gd.y0 + g.uniform() * gd.dy;
@@ -537,35 +538,33 @@ __global__ void be_generate(PArr P, long long base, long long n, const GenDesc* 
             x = gd.x0 + u * gd.dx;
             y = gd.y0 + u * gd.dy;
         }
-        int mode;
-        if (gd.cdf >= 0) {
-            // lower_bound over the border's CDF row (Grid_distribution::sample)
-            const double* row = cdfs + (long long)gd.cdf * nmodes;
-            mode = cdftot[gd.cdf] > 0. ? lower_bound_d(row, nmodes, g.uniform()) : -1;
-            if (mode >= nmodes) mode = nmodes - 1;
-            if (!placed) mode = -1;
-        } else {
-            const float* pr = aprob + gd.alias_off;
-            const int* al = aalt + gd.alias_off;
-            const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
-            const float acc = float(g.next32() >> 8) * 0x1p-24f;
-            mode = acc < __ldg(pr + j) ? j : __ldg(al + j);
-        }
+        const float* pr = aprob + gd.alias_off;
+        const int* al = aalt + gd.alias_off;
+        const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
+        const float acc = float(g.next32() >> 8) * 0x1p-24f;
+        const int mode = acc < __ldg(pr + j) ? j : __ldg(al + j);
         const long long i = base + k;
         P.x[i] = x;
         P.y[i] = y;
         P.box[i] = gd.box;
         P.mode[i] = mode;
-        P.sign[i] = (gd.msign && mode >= 0) ? int(__ldg(asign + gd.alias_off + mode)) : gd.sign;
+        P.sign[i] = gd.sign;
     }
 }
 
-// Append the live particles of [0, n) to `out` (warp-aggregated).
-// Compaction of [0, n): each block takes tiles of 4 x blockDim particles,
-// counts its survivors with warp ballots and claims their places with one
-// atomic per tile (the order inside a tile is kept).
+// Compaction of the survivors of a cancellation: each block takes tiles of
+// 4 x blockDim particles, counts its survivors with warp ballots and claims
+// their places with one atomic per tile (the order inside a tile is kept).
+//
+// rank: a particle's rank among the cnt[key] particles of the majority sign at
+// its (box, mode), -1: none of them.  |H| of them survive: those whose rank
+// falls in the |H| ranks from a random one on, modulo cnt.  Ranks follow the
+// order in which warps happened to arrive; turned by an offset that does
+// not depend on it, every particle survives with probability |H| / cnt.
 constexpr int COMPACT_ITEMS = 4;
-__device__ __forceinline__ void compact_body(PArr in, long long n, PArr out, unsigned long long* count) {
+__device__ __forceinline__ void compact_body(PArr in, long long n, PArr out, unsigned long long* count,
+                                             const int* rank, const int* H, const int* cnt, int nmodes,
+                                             unsigned long long key) {
     __shared__ unsigned wcnt[COMPACT_ITEMS][32];
     __shared__ unsigned long long tile_base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -576,7 +575,19 @@ __device__ __forceinline__ void compact_body(PArr in, long long n, PArr out, uns
 #pragma unroll
         for (int k = 0; k < COMPACT_ITEMS; ++k) {
             const long long i = base + (long long)k * blockDim.x + threadIdx.x;
-            live[k] = i < n && in.mode[i] >= 0;
+            const int r = i < n ? rank[i] : -1;
+            live[k] = r >= 0;
+            if (live[k]) {
+                const long long q = (long long)in.box[i] * nmodes + in.mode[i];
+                const unsigned h = unsigned(abs(H[q])), c = unsigned(cnt[q]);
+                if (h < c) {
+                    Philox g;
+                    g.init(key, (uint64_t)q);
+                    unsigned t = unsigned(r) + mulhi32(g.next32(), c);
+                    if (t >= c) t -= c;
+                    live[k] = t < h;
+                }
+            }
             m[k] = __ballot_sync(0xffffffffu, live[k]);
             if (lane == 0) wcnt[k][warp] = __popc(m[k]);
         }
@@ -642,14 +653,14 @@ __global__ void be_hist(PArr P, long long n, int* H, int nmodes) {
         atomicAdd(H + (long long)P.box[i] * nmodes + P.mode[i], P.sign[i]);
 }
 
-// Cancellation: a particle survives when its sign is the sign of H at its
-// (box, mode) and its rank among those particles is below |H|.  Warps visit
-// the particles in chunks of 32 consecutive ones: chunk c in the order of a
-// random affine permutation w -> (a w + b) mod nchunks (a coprime to
+// Cancellation: the particles whose sign is the sign of H at their (box,
+// mode) are ranked, and |H| of each such group survive (compact_body).  Warps
+// visit the particles in chunks of 32 consecutive ones: chunk c in the order of
+// a random affine permutation w -> (a w + b) mod nchunks (a coprime to
 // nchunks), and the lanes the chunk's particles in the order of a random
-// XOR mask of the chunk, so the ranks, and with them the survivors, do not
-// follow the order of the particle list, while every read stays coalesced.
-__device__ __forceinline__ void cancel_body(PArr P, long long n, const int* H, int* cnt, int nmodes,
+// XOR mask of the chunk, so neighbouring ranks are not neighbours in the
+// particle list, while every read stays coalesced.
+__device__ __forceinline__ void cancel_body(PArr P, long long n, const int* H, int* cnt, int* rank, int nmodes,
                                             const int* reservoir, unsigned long long pa, unsigned long long pb,
                                             unsigned mkey) {
     const unsigned long long nch = (unsigned long long)((n + 31) >> 5);
@@ -664,41 +675,66 @@ __device__ __forceinline__ void cancel_body(PArr P, long long n, const int* H, i
         const long long key = (long long)P.box[i] * nmodes + P.mode[i];
         const int h = H[key];
         const int s = P.sign[i];
-        bool keep = !reservoir[P.box[i]] && h != 0 && ((s < 0) == (h < 0));
-        if (keep) keep = atomicAdd(cnt + key, 1) < (h < 0 ? -h : h);
-        if (!keep) P.mode[i] = -1;
+        int r = -1;
+        if (!reservoir[P.box[i]] && h != 0 && ((s < 0) == (h < 0))) r = atomicAdd(cnt + key, 1);
+        rank[i] = r;
     }
 }
 
-// ed, flux_x, flux_y sums of one box (raw velocities, as calculate_prop).
-__global__ void be_props(const int* H, int nmodes, const double* vx, const double* vy, double* out) {
-    const int box = blockIdx.x;
-    double e = 0., fx = 0., fy = 0.;
-    for (int k = threadIdx.x; k < nmodes; k += blockDim.x) {
-        const double h = double(H[(long long)box * nmodes + k]);
-        e += h;
-        fx += h * vx[k];
-        fy += h * vy[k];
-    }
-    __shared__ double red[3][256];
-    red[0][threadIdx.x] = e;
-    red[1][threadIdx.x] = fx;
-    red[2][threadIdx.x] = fy;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int q = 0; q < 3; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 3; ++q) out[3 * box + q] = red[q][0];
-}
+// ed, flux_x, flux_y sums of every box (raw velocities, as calculate_prop)
+// into a cleared row, PROPS_PARTS blocks per box (one block per box took 25 us
+// of a step); the first thread closes the step (close_step).
+constexpr int PROPS_PARTS = 8;
 
 // ------------------------------------------------ device-resident step
 // Counters of the step loop, kept on the device between kernels.
 // DC_IN and DC_OUTT sum the particles read and written by be_advance over
 // the run (the algorithmic traffic of its roofline).
-enum { DC_NP = 0, DC_NOUT, DC_WORK, DC_FLIPS, DC_PSTEPS, DC_NGEN, DC_IN, DC_OUTT, DC_COUNT = 8 };
+enum { DC_NP = 0, DC_NOUT, DC_NGEN, DC_FLIPS, DC_PSTEPS, DC_IN, DC_OUTT, DC_COUNT = 8 };
+
+// The end of a step: without a cancellation its output is the population;
+// records the particles alive, adds up the outputs, and clears the step's
+// counters for the next one.
+__device__ __forceinline__ void close_step(unsigned long long* dc, int swap, long long* record) {
+    if (swap) dc[DC_NP] = dc[DC_NOUT];
+    *record = (long long)dc[DC_NP];
+    dc[DC_OUTT] += dc[DC_NOUT];
+    dc[DC_NOUT] = dc[DC_NGEN] = 0;
+}
+
+__global__ void __launch_bounds__(256) be_props(const int* H, int nmodes, const double* vx, const double* vy, double* out,
+                                                unsigned long long* dc, int swap, long long* record) {
+    const int box = blockIdx.x / PROPS_PARTS, part = blockIdx.x % PROPS_PARTS;
+    const int len = (nmodes + PROPS_PARTS - 1) / PROPS_PARTS, k1 = min(nmodes, (part + 1) * len);
+    long long e = 0;
+    double fx = 0., fy = 0.;
+    for (int k = part * len + threadIdx.x; k < k1; k += 256) {
+        const int hi = H[(long long)box * nmodes + k];
+        if (hi == 0) continue;
+        const double h = double(hi);
+        e += hi;
+        fx += h * vx[k];
+        fy += h * vy[k];
+    }
+    __shared__ double red[3][8];
+    for (int o = 16; o > 0; o >>= 1) {
+        e += __shfl_down_sync(0xffffffffu, e, o);
+        fx += __shfl_down_sync(0xffffffffu, fx, o);
+        fy += __shfl_down_sync(0xffffffffu, fy, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = double(e);
+        red[1][threadIdx.x >> 5] = fx;
+        red[2][threadIdx.x >> 5] = fy;
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double v = 0.;
+        for (int w = 0; w < 8; ++w) v += red[threadIdx.x][w];
+        if (v != 0.) atomicAdd(out + 3 * box + threadIdx.x, v);
+    }
+    if (record && blockIdx.x == 0 && threadIdx.x == 0) close_step(dc, swap, record);
+}
 
 // A source planned on the device: where its particles start in the
 // particle arrays and how many there are.
@@ -723,128 +759,147 @@ constexpr unsigned BRANCH_CAP = 1u << 20;
 // step (advect = 1; particles born in this step were advected when they were
 // made), then the scattering of the survivors -- RTA (ScatteringRTA,
 // src/beyondRTA_MC2d.cpp:983-1062, a resampling with probability
-// 1 - exp(-w dt)) or the propagator with sign branching as above -- and the
-// histogram H[box][mode] += sign of every outgoing particle, appended to
-// `out` warp by warp.  Persistent warps: a lane whose parent owes no more
-// attempts takes the next parent from a counter; a parent absorbed during
-// its advection owes none.  Each particle is read once and each outgoing
-// particle written once.
-__global__ void __launch_bounds__(256) be_advance(PArr in, const unsigned long long* n_in, PArr out,
-                                                  unsigned long long* dc, long long ocap, int advect,
-                                                  AdvectArgs aa, int rta, const PAlias* pal, const BoxProp* bprop,
-                                                  int nm, const double* w, const int2* resample,
-                                                  int nmodes, unsigned long long skey, int* H, int* err) {
+// 1 - exp(-w dt), as a 53-bit threshold per mode) or the propagator with sign
+// branching as above -- and the histogram H[box][mode] += sign of every
+// outgoing particle, appended to `out`.  Each warp takes an equal run of the
+// particles; a lane whose parent owes no more attempts takes the run's next
+// one, a parent absorbed during its advection owes none.  Outgoing particles
+// gather in the warp's part of shared memory and leave 128 or more at a time,
+// with one claim of places: claims of parents and places 32 at a time, on
+// two counters of one cache line, came to 82 000 atomics on it per launch of
+// 1.3e6 particles and bounded the kernel (103 us a launch).
+constexpr int ADV_BUF = 160;
+struct AdvBuf {
+    double x[ADV_BUF], y[ADV_BUF];
+    int mode[ADV_BUF], box[ADV_BUF], sign[ADV_BUF];
+};
+template <bool GENERAL, bool RTA>
+__global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
+    be_advance(PArr in, const unsigned long long* n_in, PArr out, unsigned long long* dc, long long ocap, int advect,
+               const __grid_constant__ AdvectArgs aa, const PAlias* pal, const BoxProp* bprop, int nm,
+               const unsigned long long* pscat, const int2* resample, int nmodes, unsigned long long skey, int* H, int* err) {
+    __shared__ AdvBuf bufs[8];
+    AdvBuf& buf = bufs[threadIdx.x >> 5];
     const long long n = min((long long)*n_in, ocap);  // places beyond the buffers (an overflow) are not read
     const int lane = threadIdx.x & 31;
     if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
         if (advect) atomicAdd(dc + DC_PSTEPS, (unsigned long long)n);
         atomicAdd(dc + DC_IN, (unsigned long long)n);
     }
+    // the warp's run, in whole chunks of 32
+    const long long warps = (long long)gridDim.x * 8, per = ((n + 31) / 32 + warps - 1) / warps * 32;
+    long long next = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * per;
+    const long long end = min(n, next + per);
     unsigned long long flips = 0;
-    int mode = 0, sign = 1, box = 0, col = 0;
+    int mode = 0, sign = 1, box = 0, col = 0, cnt = 0;
     double x = 0., y = 0.;
     unsigned todo = 0, made = 0;
-    bool done = false, valid = false;
+    bool valid = false;
     Philox g;
     g.init(skey, 0);
-    for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, todo == 0 && !done);
-        if (idle) {
-            unsigned long long base = 0;
-            const int leader = __ffs(idle) - 1;
-            if (lane == leader) base = atomicAdd(dc + DC_WORK, (unsigned long long)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (todo == 0 && !done) {
-                const long long i = (long long)base + __popc(idle & ((1u << lane) - 1u));
-                if (i < n) {
-                    mode = in.mode[i];
-                    if (mode >= 0) {
-                        sign = in.sign[i];
-                        box = in.box[i];
-                        x = in.x[i];
-                        y = in.y[i];
-                        bool alive = true;
-                        if (advect) {
-                            if (aa.general) {
-                                BePol pol;
-                                pol.g.init(aa.gkey, (uint64_t)i);
-                                int e = 0;
-                                alive = advect_general(aa.T, pol, aa.Eb, x, y, box, mode, sign, aa.dt, e);
-                                if (e && aa.err) atomicCAS(aa.err, 0, e);
-                            } else {
-                                alive = advect_one(aa.G, aa.boxcell, aa.mv, aa.boxwall, aa.Eb, x, y, box, mode,
-                                                   sign, aa.dt);
-                            }
-                        }
-                        if (alive) {
-                            col = mode - 3;
-                            valid = rta ? true : (col >= 0 && col < nm);
-                            if (!valid) atomicCAS(err, 0, E_VALUE);
-                            g.init(skey, (uint64_t)i);
-                            todo = 1;
-                            made = 0;
-                        }
-                    }
-                } else {
-                    done = true;
-                }
-            }
-        }
-        if (__all_sync(0xffffffffu, done)) break;
-        const bool act = todo > 0;
-        // the warp's output places, claimed before the draws so that the
-        // atomic's round trip overlaps the propagator read
-        const unsigned m1 = __ballot_sync(0xffffffffu, act);
-        unsigned long long wo = 0;
-        if (lane == 0 && m1) wo = atomicAdd(dc + DC_NOUT, (unsigned long long)__popc(m1));
-        int nmode = mode, nsign = sign;
-        if (act && rta) {
-            const double u = g.uniform();
-            if (u < 1. - exp(-__ldg(w + mode) * aa.dt)) {
-                const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
-                const float acc = float(g.next32() >> 8) * 0x1p-24f;
-                const int2 e = __ldg(resample + j);
-                nmode = acc < __int_as_float(e.x) ? j : e.y;
-            }
-        } else if (act && valid) {
-            // one table for every box (pal), or the box's own
-            const PAlias* tab = pal ? pal : bprop[box].alias;
-            if (tab) {
-                const int j = int(mulhi32(g.next32(), uint32_t(nm)));
-                const float acc = float(g.next32() >> 8) * 0x1p-24f;
-                const PAlias e = tab[(long long)col * nm + j];
-                const bool keep = acc < e.prob;
-                const int slot = keep ? j : int(e.alt & 0x3fffffffu);
-                const bool neg = keep ? (e.alt >> 31) != 0u : ((e.alt >> 30) & 1u) != 0u;
-                nmode = slot + 3;
-                nsign = neg ? -sign : sign;
-            } else {
-                const BoxProp bp = bprop[box];
-                if (bp.c1) {
-                    const long long off = (long long)col * nm;
-                    const int im = lower_bound_abs_lirp(bp.c1 + off, bp.c2 + off, nm, g.uniform(), bp.T, bp.T1, bp.T2);
-                    nmode = im + 3;
-                    nsign = lirp_at(bp.c1 + off, bp.c2 + off, im, bp.T, bp.T1, bp.T2) > 0. ? sign : -sign;
-                } else {
-                    atomicCAS(err, 0, E_VALUE);  // a particle where nothing scatters
-                }
-            }
-        }
-        wo = __shfl_sync(0xffffffffu, wo, 0);
-        if (act) {
-            const long long o = (long long)wo + __popc(m1 & ((1u << lane) - 1u));
+    auto flush = [&] {
+        __syncwarp();
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(dc + DC_NOUT, (unsigned long long)cnt);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int j = lane; j < cnt; j += 32) {
+            const long long o = (long long)base + j;
             if (o < ocap) {
-                out.x[o] = x;
-                out.y[o] = y;
-                out.box[o] = box;
-                out.mode[o] = nmode;
-                out.sign[o] = nsign;
-                atomicAdd(H + (long long)box * nmodes + nmode, nsign);
+                out.x[o] = buf.x[j];
+                out.y[o] = buf.y[j];
+                out.mode[o] = buf.mode[j];
+                out.box[o] = buf.box[j];
+                out.sign[o] = buf.sign[j];
+                atomicAdd(H + (long long)buf.box[j] * nmodes + buf.mode[j], buf.sign[j]);
             } else {
                 atomicCAS(err, 0, E_LIMIT);
             }
+        }
+        cnt = 0;
+        __syncwarp();
+    };
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, todo == 0);
+        if (todo == 0) {
+            const long long i = next + __popc(idle & ((1u << lane) - 1u));
+            if (i < end) {
+                mode = in.mode[i];
+                if (mode >= 0) {
+                    sign = in.sign[i];
+                    box = in.box[i];
+                    x = in.x[i];
+                    y = in.y[i];
+                    bool alive = true;
+                    if (advect) {
+                        if (GENERAL) {
+                            BePol pol;
+                            pol.g.init(aa.gkey, (uint64_t)i);
+                            int e = 0;
+                            alive = advect_general(aa.T, pol, aa.Eb, x, y, box, mode, sign, aa.dt, e);
+                            if (e && aa.err) atomicCAS(aa.err, 0, e);
+                        } else {
+                            alive = advect_one(aa.G, aa.boxcell, aa.mv, aa.boxwall, aa.Eb, x, y, box, mode, sign, aa.dt);
+                        }
+                    }
+                    if (alive) {
+                        col = mode - 3;
+                        valid = RTA ? true : (col >= 0 && col < nm);
+                        if (!valid) atomicCAS(err, 0, E_VALUE);
+                        g.init(skey, (uint64_t)i);
+                        todo = 1;
+                        made = 0;
+                    }
+                }
+            }
+        }
+        next += __popc(idle);
+        const bool act = todo > 0;
+        const unsigned m1 = __ballot_sync(0xffffffffu, act);
+        if (!m1) {
+            if (next >= end) break;
+            continue;
+        }
+        if (act) {
+            int nmode = mode, nsign = sign;
+            if (RTA) {
+                if ((g.next() >> 11) < __ldg(pscat + mode)) {
+                    const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
+                    const float acc = float(g.next32() >> 8) * 0x1p-24f;
+                    const int2 e = __ldg(resample + j);
+                    nmode = acc < __int_as_float(e.x) ? j : e.y;
+                }
+            } else if (valid) {
+                // one table for every box (pal), or the box's own
+                const PAlias* tab = pal ? pal : bprop[box].alias;
+                if (tab) {
+                    const int j = int(mulhi32(g.next32(), uint32_t(nm)));
+                    const float acc = float(g.next32() >> 8) * 0x1p-24f;
+                    const PAlias e = tab[(long long)col * nm + j];
+                    const bool keep = acc < e.prob;
+                    const int slot = keep ? j : int(e.alt & 0x3fffffffu);
+                    const bool neg = keep ? (e.alt >> 31) != 0u : ((e.alt >> 30) & 1u) != 0u;
+                    nmode = slot + 3;
+                    nsign = neg ? -sign : sign;
+                } else {
+                    const BoxProp bp = bprop[box];
+                    if (bp.c1) {
+                        const long long off = (long long)col * nm;
+                        const int im = lower_bound_abs_lirp(bp.c1 + off, bp.c2 + off, nm, g.uniform(), bp.T, bp.T1, bp.T2);
+                        nmode = im + 3;
+                        nsign = lirp_at(bp.c1 + off, bp.c2 + off, im, bp.T, bp.T1, bp.T2) > 0. ? sign : -sign;
+                    } else {
+                        atomicCAS(err, 0, E_VALUE);  // a particle where nothing scatters
+                    }
+                }
+            }
+            const int o = cnt + __popc(m1 & ((1u << lane) - 1u));
+            buf.x[o] = x;
+            buf.y[o] = y;
+            buf.box[o] = box;
+            buf.mode[o] = nmode;
+            buf.sign[o] = nsign;
             --todo;
-            if (!rta && nsign != sign) {
+            if (!RTA && nsign != sign) {
                 todo += 2;
                 ++flips;
             }
@@ -853,9 +908,18 @@ __global__ void __launch_bounds__(256) be_advance(PArr in, const unsigned long l
                 todo = 0;
             }
         }
+        cnt += __popc(m1);
+        if (cnt > ADV_BUF - 32) flush();
     }
+    if (cnt) flush();
     for (int o = 16; o > 0; o >>= 1) flips += __shfl_down_sync(0xffffffffu, flips, o);
     if (lane == 0 && flips) atomicAdd(dc + DC_FLIPS, flips);
+}
+
+// u < 1 - exp(-w dt) for u = k 2^-53 as k < pscat.
+__global__ void be_thresholds(const double* w, double dt, int n, unsigned long long* pscat) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) pscat[k] = (unsigned long long)ceil((1. - exp(-w[k] * dt)) * 0x1p53);
 }
 
 // Exclusive scan of cnt[0..n) into descs[k].first, by one warp; returns the
@@ -892,26 +956,6 @@ __device__ void claim_span(unsigned long long total, unsigned long long* dc, Src
     dc[DC_NGEN] = base + total;
 }
 
-// Particle numbers of the gradient and isothermal-wall sources of one step:
-// Ntogenerate's stochastic rounding (src/sampling.cpp:166-183, :243-260) of
-// the expected numbers genf[k], from one Philox block per source.  One warp.
-__global__ void be_plan_sources(GenDesc* descs, const double* genf, long long* cnt, int ngen,
-                                unsigned long long key, unsigned long long* dc, SrcSpan* span, long long cap,
-                                int* err) {
-    if (threadIdx.x >= 32) return;
-    for (int k = threadIdx.x; k < ngen; k += 32) {
-        Philox q;
-        q.init(key, (uint64_t)k);
-        const double gen = genf[k];
-        long long c = (long long)gen;
-        if (q.uniform() <= gen - floor(gen)) ++c;
-        cnt[k] = c;
-    }
-    __syncwarp();
-    const unsigned long long total = warp_scan_first(cnt, ngen, descs);
-    if (threadIdx.x == 0) claim_span(total, dc, span, cap, err);
-}
-
 // A void border's adiabatic re-emission, tabulated per run: its segment,
 // the inward normal, its box and the box's Teq, its length and the spline
 // J(T) -> T of its wall (-1: not re-emitting: reservoirs, periodic boxes).
@@ -945,16 +989,42 @@ __device__ __forceinline__ double spline_eval(const SplineDev& S, int id, double
     return S.a[o + idx] + dx * (S.b[o + idx] + dx * (S.c[o + idx] + S.d[o + idx] * dx));
 }
 
-// The adiabatic walls of one step (src/beyondRTA_MC2d.cpp:294-350): each
-// re-emitting border re-emits |Eborder| particles at the temperature whose
-// isothermal flux carries its absorbed energy (spline of J), one
-// distribution request per border; Eborder starts again from zero.  One
-// warp.
-__global__ void be_plan_adiabatic(int* Eb, const AdiBorder* ab, int nborders, SplineDev S, double Eeff, double dtstep,
-                                  double thickness, WallReq* req, long long* cnt, GenDesc* descs,
-                                  unsigned long long* dc, SrcSpan* span, long long cap, int* err) {
-    if (threadIdx.x >= 32) return;
-    for (int k = threadIdx.x; k < nborders; k += 32) {
+// One source of a step: its descriptors and numbers, the alias rows its modes
+// come from (or CDF rows), and the Philox keys of its draws.
+struct SourceSet {
+    GenDesc* descs;
+    const double* genf;          // expected numbers (gradient, isothermal)
+    long long* cnt;
+    int ngen;
+    const float* prob;
+    const int* alt;
+    const signed char* sign;
+    unsigned long long key, akey, gkey;  // the new particles', their sub-steps', their geometric choices'
+};
+struct SourceSets {
+    SourceSet s[3];              // gradient boxes, isothermal walls, adiabatic walls
+    unsigned long long pkey[2];  // of the stochastic rounding
+};
+
+// The step's sources, one block.  Gradient and isothermal walls: the numbers by
+// Ntogenerate's stochastic rounding (src/sampling.cpp:166-183, :243-260), one
+// Philox block per source.  Adiabatic walls (src/beyondRTA_MC2d.cpp:294-350):
+// each re-emitting border re-emits |Eborder| particles at the temperature
+// whose isothermal flux carries its absorbed energy (spline of J), one
+// distribution request per border; Eborder starts again from zero.
+__global__ void __launch_bounds__(256) be_plan(const __grid_constant__ SourceSets Q, int* Eb, const AdiBorder* ab, SplineDev S,
+                                               double Eeff, double dtstep, double thickness, WallReq* req,
+                                               unsigned long long* dc, SrcSpan* span, long long cap, int* err) {
+    for (int q = 0; q < 2; ++q)
+        for (int k = threadIdx.x; k < Q.s[q].ngen; k += 256) {
+            Philox g;
+            g.init(Q.pkey[q], (uint64_t)k);
+            const double gen = Q.s[q].genf[k];
+            long long c = (long long)gen;
+            if (g.uniform() <= gen - floor(gen)) ++c;
+            Q.s[q].cnt[k] = c;
+        }
+    for (int k = threadIdx.x; k < Q.s[2].ngen; k += 256) {
         const int E = Eb[k];
         Eb[k] = 0;
         const AdiBorder A = ab[k];
@@ -973,33 +1043,45 @@ __global__ void be_plan_adiabatic(int* Eb, const AdiBorder* ab, int nborders, Sp
             d.sign = (Tb - A.Teq) >= 0 ? 1 : -1;
             c = (long long)(fabs((double)E) + 1.0e-6);
         }
-        cnt[k] = c;
+        Q.s[2].cnt[k] = c;
         d.first = 0;
-        descs[k] = d;
+        Q.s[2].descs[k] = d;
     }
-    __syncwarp();
-    const unsigned long long total = warp_scan_first(cnt, nborders, descs);
-    if (threadIdx.x == 0) claim_span(total, dc, span, cap, err);
+    __syncthreads();
+    __shared__ unsigned long long total[3];
+    const int w = threadIdx.x >> 5;
+    if (w < 3) {
+        const unsigned long long t = warp_scan_first(Q.s[w].cnt, Q.s[w].ngen, Q.s[w].descs);
+        if ((threadIdx.x & 31) == 0) total[w] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int q = 0; q < 3; ++q) claim_span(total[q], dc, span + q, cap, err);
 }
 
-// New particles of one planned source at A[span.base + k), k < span.total,
+// The step's new particles at A[span.base + k), k < span.total of each source,
 // each advected for a random part of the step as it is made (the sources
 // of steps 2-4 of the reference's loop); an absorbed one keeps mode -1.
-__global__ void be_generate_dev(PArr P, const SrcSpan* span, const GenDesc* gens, int ngen, const float* aprob,
-                                const int* aalt, const signed char* asign, const double* cdfs,
-                                const double* cdftot, int nmodes, unsigned long long key, const GBox* boxes,
-                                const V2* hull, AdvectArgs aa) {
-    const SrcSpan sp = *span;
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < (long long)sp.total;
-         k += (long long)gridDim.x * blockDim.x) {
-        int lo = 0, hi = ngen;
+template <bool GENERAL>
+__global__ void be_generate_dev(PArr P, const SrcSpan* span, const __grid_constant__ SourceSets Q, const double* cdfs,
+                                const double* ctot, int nmodes, const GBox* boxes, const V2* hull,
+                                const __grid_constant__ AdvectArgs aa) {
+    const SrcSpan s0 = span[0], s1 = span[1], s2 = span[2];
+    const long long total = (long long)(s0.total + s1.total + s2.total);
+    for (long long kk = blockIdx.x * (long long)blockDim.x + threadIdx.x; kk < total;
+         kk += (long long)gridDim.x * blockDim.x) {
+        const int q = kk < (long long)s0.total ? 0 : kk < (long long)(s0.total + s1.total) ? 1 : 2;
+        const long long k = kk - (q > 0 ? (long long)s0.total : 0) - (q > 1 ? (long long)s1.total : 0);
+        const SourceSet& Z = Q.s[q];
+        const GenDesc* gens = Z.descs;
+        int lo = 0, hi = Z.ngen;
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (gens[mid].first <= k) lo = mid; else hi = mid;
         }
         const GenDesc gd = gens[lo];
         Philox g;
-        g.init(key, (uint64_t)k);
+        g.init(Z.key, (uint64_t)k);
         double x, y;
         bool placed = true;
         if (gd.rect == 2) {
@@ -1020,28 +1102,26 @@ __global__ void be_generate_dev(PArr P, const SrcSpan* span, const GenDesc* gens
         }
         int mode;
         if (gd.cdf >= 0) {
-            const double* row = cdfs + (long long)gd.cdf * nmodes;
-            mode = cdftot[gd.cdf] > 0. ? lower_bound_d(row, nmodes, g.uniform()) : -1;
-            if (mode >= nmodes) mode = nmodes - 1;
+            mode = wall_cdf_draw(cdfs, ctot, gd.cdf, nmodes, g.uniform());
             if (!placed) mode = -1;
         } else {
-            const float* pr = aprob + gd.alias_off;
-            const int* al = aalt + gd.alias_off;
+            const float* pr = Z.prob + gd.alias_off;
+            const int* al = Z.alt + gd.alias_off;
             const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
             const float acc = float(g.next32() >> 8) * 0x1p-24f;
             mode = acc < __ldg(pr + j) ? j : __ldg(al + j);
         }
         int box = gd.box;
-        const int sign = (gd.msign && mode >= 0) ? int(__ldg(asign + gd.alias_off + mode)) : gd.sign;
-        const long long i = (long long)sp.base + k;
+        const int sign = (gd.msign && mode >= 0) ? int(__ldg(Z.sign + gd.alias_off + mode)) : gd.sign;
+        const long long i = (long long)(q == 0 ? s0.base : q == 1 ? s1.base : s2.base) + k;
         if (mode >= 0) {  // a random part of the step
             Philox h;
-            h.init(aa.key, (uint64_t)i);
+            h.init(Z.akey, (uint64_t)i);
             const double dt = aa.dt * h.uniform();
             bool alive;
-            if (aa.general) {
+            if (GENERAL) {
                 BePol pol;
-                pol.g.init(aa.gkey, (uint64_t)i);
+                pol.g.init(Z.gkey, (uint64_t)i);
                 int e = 0;
                 alive = advect_general(aa.T, pol, aa.Eb, x, y, box, mode, sign, dt, e);
                 if (e && aa.err) atomicCAS(aa.err, 0, e);
@@ -1058,20 +1138,14 @@ __global__ void be_generate_dev(PArr P, const SrcSpan* span, const GenDesc* gens
     }
 }
 
-// The wall-CDF passes over every border, for the borders the step planned
-// (cnt > 0); rows of the others are left as they are.
-__global__ void __launch_bounds__(256) be_wall_cdf1_dev(const float* om, const float* vx, const float* vy, int n,
-                                                        const WallReq* req, const long long* cnt, double* cdf,
-                                                        double* chunk_tot) {
+// The wall CDFs of every border, for the borders the step planned (cnt > 0);
+// rows of the others are left as they are.
+__global__ void __launch_bounds__(256) be_wall_cdf(const float* om, const float* vx, const float* vy, int n,
+                                                   const WallReq* req, const long long* cnt, double* cdf,
+                                                   double* chunk_tot) {
     const int nch = (n + WCDF_CHUNK - 1) / WCDF_CHUNK;
     if (cnt[blockIdx.x / nch] == 0) return;
-    wall_cdf1_body(om, vx, vy, n, req, cdf, chunk_tot);
-}
-__global__ void __launch_bounds__(256) be_wall_cdf2_dev(int n, const long long* cnt, const double* chunk_tot,
-                                                        double* cdf, double* tot) {
-    const int nch = (n + WCDF_CHUNK - 1) / WCDF_CHUNK;
-    if (cnt[blockIdx.x / nch] == 0) return;
-    wall_cdf2_body(n, chunk_tot, cdf, tot);
+    wall_cdf_body(om, vx, vy, n, req, cdf, chunk_tot);
 }
 
 // Cancellation on the device over [0, *n_in) with the random affine
@@ -1084,10 +1158,10 @@ __device__ __forceinline__ unsigned long long gcd_u64(unsigned long long a, unsi
     }
     return a;
 }
-__global__ void be_cancel_dev(PArr P, const unsigned long long* n_in, long long cap, const int* H, int* cnt,
-                              int nmodes,
-                              const int* reservoir, unsigned long long key) {
-    const long long n = min((long long)*n_in, cap);
+__global__ void be_cancel_dev(PArr P, unsigned long long* dc, long long cap, const int* H, int* cnt, int* rank,
+                              int nmodes, const int* reservoir, unsigned long long key) {
+    const long long n = min((long long)dc[DC_NOUT], cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) dc[DC_NP] = 0;  // counted by the compaction
     if (n <= 0) return;
     // the permutation's a, b and the XOR key, drawn by one thread per block
     __shared__ unsigned long long s_ab[2];
@@ -1106,22 +1180,13 @@ __global__ void be_cancel_dev(PArr P, const unsigned long long* n_in, long long 
         s_mkey = q.next32();
     }
     __syncthreads();
-    cancel_body(P, n, H, cnt, nmodes, reservoir, s_ab[0], s_ab[1], s_mkey);
+    cancel_body(P, n, H, cnt, rank, nmodes, reservoir, s_ab[0], s_ab[1], s_mkey);
 }
 
-// Compaction of [0, *n_in) with the survivors counted into *count.
-__global__ void be_compact_dev(PArr in, const unsigned long long* n_in, long long cap, PArr out,
-                               unsigned long long* count) {
-    compact_body(in, min((long long)*n_in, cap), out, count);
-}
-
-// dc[to] = dc[from]; record[step] = dc[DC_NP] after it.
-__global__ void be_counters(unsigned long long* dc, int to, int from, long long* record, int step) {
-    if (to >= 0) dc[to] = dc[from];
-    if (record) {  // the end of a step: its particles alive, and the outputs of its be_advance launches
-        record[step] = (long long)dc[DC_NP];
-        dc[DC_OUTT] += dc[DC_NOUT];
-    }
+// The survivors of a cancellation from `in` to `out`, counted into dc[DC_NP].
+__global__ void be_compact_dev(PArr in, PArr out, unsigned long long* dc, long long cap, const int* rank, const int* H,
+                               const int* cnt, int nmodes, unsigned long long key) {
+    compact_body(in, min((long long)dc[DC_NOUT], cap), out, dc + DC_NP, rank, H, cnt, nmodes, key);
 }
 
 PArr arr(DBuf& x, DBuf& y, DBuf& m, DBuf& b, DBuf& s, long long off = 0) {
@@ -1133,7 +1198,7 @@ void alloc_particles(BertaState& B, long long cap) {
     if (B.cap >= cap) return;
     for (DBuf* d : {&B.a_x, &B.a_y, &B.b_x, &B.b_y})
         d->alloc(size_t(cap) * sizeof(double));
-    for (DBuf* d : {&B.a_mode, &B.a_box, &B.a_sign, &B.b_mode, &B.b_box, &B.b_sign})
+    for (DBuf* d : {&B.a_mode, &B.a_box, &B.a_sign, &B.b_mode, &B.b_box, &B.b_sign, &B.d_rank})
         d->alloc(size_t(cap) * sizeof(int));
     B.cap = cap;
 }
@@ -1586,7 +1651,6 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         // so that no step reallocates
         B.d_req.alloc(std::size_t(nborders) * sizeof(WallReq));
         B.d_cdf.alloc(std::size_t(nborders) * std::size_t(m.n()) * sizeof(double));
-        B.d_cdftot.alloc(std::size_t(nborders) * sizeof(double));
         B.d_ctot.alloc(std::size_t(nborders) * ((m.n() + WCDF_CHUNK - 1) / WCDF_CHUNK) * sizeof(double));
         ck(cudaMemsetAsync(B.d_Eb.p, 0, std::size_t(nborders) * sizeof(int), s), "memset");
         B.d_H.alloc(std::size_t(nbx) * n * sizeof(int));
@@ -1677,8 +1741,7 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             }
             PArr A = arr(B.a_x, B.a_y, B.a_mode, B.a_box, B.a_sign);
             be_generate<<<launch_blocks(total, c->nsm), 256, 0, s>>>(
-                A, base, total, B.d_gens.as<GenDesc>(), int(descs.size()), dprob, dalt, nullptr,
-                B.d_cdf.as<double>(), B.d_cdftot.as<double>(), n, mix_key(p->seed, step, phase),
+                A, base, total, B.d_gens.as<GenDesc>(), int(descs.size()), dprob, dalt, n, mix_key(p->seed, step, phase),
                 c->d_boxes.as<GBox>(), c->d_hull.as<V2>());
         };
         std::vector<double> hprops(std::size_t(nbx) * 3);
@@ -1689,8 +1752,9 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             if (nn > 0)
                 be_hist<<<launch_blocks(nn, c->nsm), 256, 0, s>>>(arr(B.a_x, B.a_y, B.a_mode, B.a_box, B.a_sign),
                                                                   nn, B.d_H.as<int>(), n);
-            be_props<<<nbx, 256, 0, s>>>(B.d_H.as<int>(), n, B.d_rvx.as<double>(), B.d_rvy.as<double>(),
-                                          B.d_props.as<double>());
+            ck(cudaMemsetAsync(B.d_props.p, 0, std::size_t(nbx) * 3 * sizeof(double), s), "memset");
+            be_props<<<nbx * PROPS_PARTS, 256, 0, s>>>(B.d_H.as<int>(), n, B.d_rvx.as<double>(), B.d_rvy.as<double>(),
+                                                        B.d_props.as<double>(), nullptr, 0, nullptr);
             ck(cudaMemcpyAsync(hprops.data(), B.d_props.p, hprops.size() * sizeof(double), cudaMemcpyDeviceToHost, s), "d2h");
             sync(c);
             for (int b = 0; b < nbx; ++b) {
@@ -1750,7 +1814,13 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             B.d_dc.upload(h0, s);
         }
         B.d_phist.alloc(std::size_t(nsteps + 1) * std::size_t(nbx) * 3 * sizeof(double));
+        ck(cudaMemsetAsync(B.d_phist.p, 0, std::size_t(nsteps + 1) * std::size_t(nbx) * 3 * sizeof(double), s), "memset");
         B.d_nhist.alloc(std::size_t(nsteps + 1) * sizeof(long long));
+        if (p->rta) {
+            B.d_pscat.alloc(std::size_t(n) * sizeof(unsigned long long));
+            be_thresholds<<<unsigned((n + 255) / 256), 256, 0, s>>>(c->d_w.as<double>(), p->dt, n,
+                                                                    B.d_pscat.as<unsigned long long>());
+        }
         // sources with fixed descriptors: gradient boxes and isothermal walls,
         // with the expected particle numbers of a step
         std::vector<GenDesc> gdesc, idesc;
@@ -1827,89 +1897,78 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             std::swap(B.a_box.p, B.b_box.p);
             std::swap(B.a_sign.p, B.b_sign.p);
         };
+        // the advection and scattering of particles `in` into B
+        const unsigned ablocks = unsigned(c->nsm) * (general ? 2u : 3u);
+        auto advance = [&](PArr in, const unsigned long long* n_in, int advect, const AdvectArgs& aa,
+                           unsigned long long key) {
+            const auto f = general ? (p->rta ? be_advance<true, true> : be_advance<true, false>)
+                                   : (p->rta ? be_advance<false, true> : be_advance<false, false>);
+            f<<<ablocks, 256, 0, s>>>(in, n_in, arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc, cap, advect, aa, pal,
+                                      bprop, B.nm, B.d_pscat.as<unsigned long long>(), c->d_resample.as<int2>(), n, key,
+                                      B.d_H.as<int>(), err);
+        };
+        SourceSets Q{};
+        Q.s[0] = SourceSet{B.d_gdesc.as<GenDesc>(), B.d_ggenf.as<double>(), B.d_gcnt.as<long long>(), ngd,
+                           B.d_gprob.as<float>(), B.d_galt.as<int>(), B.d_gsign.as<signed char>(), 0, 0, 0};
+        Q.s[1] = SourceSet{B.d_idesc.as<GenDesc>(), B.d_igenf.as<double>(), B.d_icnt.as<long long>(), nid,
+                           B.d_isoprob.as<float>(), B.d_isoalt.as<int>(), nullptr, 0, 0, 0};
+        Q.s[2] = SourceSet{B.d_adesc.as<GenDesc>(), nullptr, B.d_acnt.as<long long>(), nborders, nullptr, nullptr, nullptr,
+                           0, 0, 0};
         while (time <= p->maxtime && istep < nsteps) {
             cudaEvent_t* ev = pev.data() + std::size_t(istep) * 7;
             ck(cudaEventRecord(ev[0], s), "event");
             // 1 + 6 + 7 for the particles of the last step: advection,
             // scattering and histogram in one pass, into B
             ck(cudaMemsetAsync(B.d_H.p, 0, hbytes, s), "memset");
-            ck(cudaMemsetAsync(dc + DC_NOUT, 0, 2 * sizeof(unsigned long long), s), "memset");
-            const AdvectArgs a_step{GA.G, GA.boxcell, GA.mv, B.d_boxwall.as<int4>(), B.d_Eb.as<int>(), p->dt, 0ull, 0,
-                                    general, mix_key(p->seed, istep, 31), err, TT};
-            be_advance<<<pblocks, 256, 0, s>>>(arr(B.a_x, B.a_y, B.a_mode, B.a_box, B.a_sign), dc + DC_NP,
-                                               arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc, cap, 1, a_step,
-                                               p->rta, pal, bprop, B.nm, c->d_w.as<double>(),
-                                               c->d_resample.as<int2>(), n,
-                                               mix_key(p->seed, istep, 64), B.d_H.as<int>(), err);
+            const AdvectArgs a_step{GA.G, GA.boxcell, GA.mv, B.d_boxwall.as<int4>(), B.d_Eb.as<int>(), p->dt,
+                                    mix_key(p->seed, istep, 31), err, TT};
+            const PArr A = arr(B.a_x, B.a_y, B.a_mode, B.a_box, B.a_sign);
+            advance(A, dc + DC_NP, 1, a_step, mix_key(p->seed, istep, 64));
             ck(cudaEventRecord(ev[1], s), "event");
             // 2-4 the step's sources, made at A[0..) (A is free now) and each
             // advected for a random part of the step as it is made
-            ck(cudaMemsetAsync(dc + DC_NGEN, 0, sizeof(unsigned long long), s), "memset");
-            const PArr A = arr(B.a_x, B.a_y, B.a_mode, B.a_box, B.a_sign);
-            auto gen_args = [&](int ph) {
-                return AdvectArgs{GA.G, GA.boxcell, GA.mv, B.d_boxwall.as<int4>(), B.d_Eb.as<int>(), p->dt,
-                                  mix_key(p->seed, istep, ph + 1), 1, general, mix_key(p->seed, istep, ph + 17), err,
-                                  TT};
+            auto keys = [&](SourceSet& q, int ph) {
+                q.key = mix_key(p->seed, istep, ph);
+                q.akey = mix_key(p->seed, istep, ph + 1);
+                q.gkey = mix_key(p->seed, istep, ph + 17);
             };
-            if (ngd) {
-                be_plan_sources<<<1, 32, 0, s>>>(B.d_gdesc.as<GenDesc>(), B.d_ggenf.as<double>(), B.d_gcnt.as<long long>(),
-                                                 ngd, mix_key(p->seed, istep, 40), dc, span + 0, cap, err);
-                be_generate_dev<<<pblocks, 256, 0, s>>>(A, span + 0, B.d_gdesc.as<GenDesc>(), ngd, B.d_gprob.as<float>(),
-                                                        B.d_galt.as<int>(), B.d_gsign.as<signed char>(),
-                                                        B.d_cdf.as<double>(), B.d_cdftot.as<double>(), n,
-                                                        mix_key(p->seed, istep, 8), c->d_boxes.as<GBox>(),
-                                                        c->d_hull.as<V2>(), gen_args(8));
-            }
-            if (nid) {
-                be_plan_sources<<<1, 32, 0, s>>>(B.d_idesc.as<GenDesc>(), B.d_igenf.as<double>(), B.d_icnt.as<long long>(),
-                                                 nid, mix_key(p->seed, istep, 41), dc, span + 1, cap, err);
-                be_generate_dev<<<pblocks, 256, 0, s>>>(A, span + 1, B.d_idesc.as<GenDesc>(), nid, B.d_isoprob.as<float>(),
-                                                        B.d_isoalt.as<int>(), nullptr, B.d_cdf.as<double>(),
-                                                        B.d_cdftot.as<double>(), n, mix_key(p->seed, istep, 2),
-                                                        c->d_boxes.as<GBox>(), c->d_hull.as<V2>(), gen_args(2));
-            }
-            if (nborders > 0) {
-                be_plan_adiabatic<<<1, 32, 0, s>>>(B.d_Eb.as<int>(), B.d_adi.as<AdiBorder>(), nborders, SP, p->Eeff,
-                                                   p->dt, g.thickness, B.d_req.as<WallReq>(), B.d_acnt.as<long long>(),
-                                                   B.d_adesc.as<GenDesc>(), dc, span + 2, cap, err);
-                be_wall_cdf1_dev<<<unsigned(nborders) * unsigned(nch), 256, 0, s>>>(
+            keys(Q.s[0], 8);
+            keys(Q.s[1], 2);
+            keys(Q.s[2], 4);
+            Q.pkey[0] = mix_key(p->seed, istep, 40);
+            Q.pkey[1] = mix_key(p->seed, istep, 41);
+            be_plan<<<1, 256, 0, s>>>(Q, B.d_Eb.as<int>(), B.d_adi.as<AdiBorder>(), SP, p->Eeff, p->dt, g.thickness,
+                                      B.d_req.as<WallReq>(), dc, span, cap, err);
+            if (nborders > 0)
+                be_wall_cdf<<<unsigned(nborders) * unsigned(nch), 256, 0, s>>>(
                     B.d_om.as<float>(), B.d_vx.as<float>(), B.d_vy.as<float>(), n, B.d_req.as<WallReq>(),
                     B.d_acnt.as<long long>(), B.d_cdf.as<double>(), B.d_ctot.as<double>());
-                be_wall_cdf2_dev<<<unsigned(nborders) * unsigned(nch), 256, 0, s>>>(
-                    n, B.d_acnt.as<long long>(), B.d_ctot.as<double>(), B.d_cdf.as<double>(), B.d_cdftot.as<double>());
-                be_generate_dev<<<pblocks, 256, 0, s>>>(A, span + 2, B.d_adesc.as<GenDesc>(), nborders, nullptr, nullptr,
-                                                        nullptr, B.d_cdf.as<double>(), B.d_cdftot.as<double>(), n,
-                                                        mix_key(p->seed, istep, 4), c->d_boxes.as<GBox>(),
-                                                        c->d_hull.as<V2>(), gen_args(4));
-            }
+            const auto gen_kernel = general ? be_generate_dev<true> : be_generate_dev<false>;
+            gen_kernel<<<pblocks, 256, 0, s>>>(A, span, Q, B.d_cdf.as<double>(), B.d_ctot.as<double>(), n,
+                                               c->d_boxes.as<GBox>(), c->d_hull.as<V2>(), a_step);
             ck(cudaEventRecord(ev[2], s), "event");
             // 5-7 for the new particles: the absorbed ones dropped, the others
             // scattered and counted in the histogram, appended to B
-            ck(cudaMemsetAsync(dc + DC_WORK, 0, sizeof(unsigned long long), s), "memset");
-            be_advance<<<pblocks, 256, 0, s>>>(A, dc + DC_NGEN, arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc,
-                                               cap, 0, a_step, p->rta, pal, bprop, B.nm, c->d_w.as<double>(),
-                                               c->d_resample.as<int2>(), n,
-                                               mix_key(p->seed, istep, 65), B.d_H.as<int>(), err);
+            advance(A, dc + DC_NGEN, 0, a_step, mix_key(p->seed, istep, 65));
             ck(cudaEventRecord(ev[3], s), "event");
             ck(cudaEventRecord(ev[4], s), "event");  // the histogram is made in the passes above
             // 8. cancellation every cancel_every steps: B -> A; otherwise B is the population
-            if (istep % cancel_every == 0) {
+            const bool cancel = istep % cancel_every == 0;
+            if (cancel) {
+                const PArr Bp = arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign);
                 ck(cudaMemsetAsync(B.d_cnt.p, 0, hbytes, s), "memset");
-                be_cancel_dev<<<pblocks, 256, 0, s>>>(arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc + DC_NOUT, cap,
-                                                      B.d_H.as<int>(), B.d_cnt.as<int>(), n, B.d_res.as<int>(),
-                                                      mix_key(p->seed, istep, 77));
-                ck(cudaMemsetAsync(dc + DC_NP, 0, sizeof(unsigned long long), s), "memset");
-                be_compact_dev<<<pblocks, 256, 0, s>>>(arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc + DC_NOUT, cap,
-                                                       arr(B.a_x, B.a_y, B.a_mode, B.a_box, B.a_sign), dc + DC_NP);
+                be_cancel_dev<<<pblocks, 256, 0, s>>>(Bp, dc, cap, B.d_H.as<int>(), B.d_cnt.as<int>(), B.d_rank.as<int>(),
+                                                      n, B.d_res.as<int>(), mix_key(p->seed, istep, 77));
+                be_compact_dev<<<pblocks, 256, 0, s>>>(Bp, A, dc, cap, B.d_rank.as<int>(), B.d_H.as<int>(),
+                                                       B.d_cnt.as<int>(), n, mix_key(p->seed, istep, 78));
             } else {
-                be_counters<<<1, 1, 0, s>>>(dc, DC_NP, DC_NOUT, nullptr, 0);
                 swap_ab();
             }
             ck(cudaEventRecord(ev[5], s), "event");
             // 9. properties of the step (calculate_prop), recorded on the device
-            be_props<<<nbx, 256, 0, s>>>(B.d_H.as<int>(), n, B.d_rvx.as<double>(), B.d_rvy.as<double>(),
-                                          B.d_phist.as<double>() + std::size_t(istep + 1) * nbx * 3);
-            be_counters<<<1, 1, 0, s>>>(dc, -1, 0, B.d_nhist.as<long long>(), istep + 1);
+            be_props<<<nbx * PROPS_PARTS, 256, 0, s>>>(B.d_H.as<int>(), n, B.d_rvx.as<double>(), B.d_rvy.as<double>(),
+                                                        B.d_phist.as<double>() + std::size_t(istep + 1) * nbx * 3, dc,
+                                                        cancel ? 0 : 1, B.d_nhist.as<long long>() + istep + 1);
             ck(cudaGetLastError(), "step launch");
             ck(cudaEventRecord(ev[6], s), "event");
             if (p->on_step) {
