@@ -407,16 +407,34 @@ __device__ __noinline__ int link_begin(const DevTables& T, const SteadyArgs& S, 
     return e;
 }
 
+// A mode's velocities with time in units of 2^k ticks: as large as a flight of
+// `dt` ps needs to fit one piece and the faster component allows, so that a
+// slow mode's long flight takes as few pieces as a fast one's.  (The flight
+// keeps 2^-59 of its length.)
+__device__ __forceinline__ int slow_down(ModeFix& m, double dt, int kt) {
+    const uint64_t vx = m.vx & ~FIX_DOWN, vy = m.vy & ~FIX_DOWN, v = vx > vy ? vx : vy;
+    int k = v ? __clzll((long long)v) - 1 : 34;  // (without velocity: 96 bits of ticks into few pieces)
+    const int need = int((dbits(dt) >> 52) & 0x7ff) - 1023 + kt - 59;
+    k = k > 34 ? 34 : k;
+    k = k > need ? need : k;
+    k = k < 0 ? 0 : k;
+    m.vx = (vx << k) | (m.vx & FIX_DOWN);
+    m.vy = (vy << k) | (m.vy & FIX_DOWN);
+    if (vx) m.rx -= uint64_t(k);  // the exponent in its low bits
+    if (vy) m.ry -= uint64_t(k);
+    return k;
+}
+
 // One steady-state generation over linked cells: the flights, draws and
 // outcomes of rta_steady_poly, a box visit tallied when it ends.  A flight is
-// walked in pieces below 2^60 ticks.  Where the particle is in a row of cells
-// that a translation closes to a period and the rest of its flight crosses
-// that period twice or more before it leaves the row, the whole periods are
-// taken at once: every box of the row gets its share of their time and
-// displacement.  Flights that run along the periodic direction cross hundreds
-// of boxes, one after the other on one lane, and were what a generation
-// waited for (3.6e6 crossings of 3.6e5 flights; 37 ms for a ribbon of 2e5
-// particles, 42 generations).
+// walked in pieces below 2^60 of its time units.  Where the particle is in a
+// row of cells that a translation closes to a period and the rest of its
+// flight crosses that period twice or more before it leaves the row, the whole
+// periods are taken at once: every box of the row gets its share of their
+// time and displacement.  Flights that run along the periodic direction cross
+// hundreds of boxes, one after the other on one lane, and were what a
+// generation waited for (3.6e6 crossings of 3.6e5 flights; 37 ms for a ribbon
+// of 2e5 particles, 42 generations, 2.0 ms now).
 __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant__ DevTables T,
                                                           const __grid_constant__ SteadyArgs S,
                                                           const __grid_constant__ LinkArgs A, double* tally,
@@ -436,6 +454,7 @@ __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant_
     uint64_t dt_lo = 0, pt = 0;
     uint32_t dt_hi = 0, nseg = 0;
     int64_t px = 0, py = 0;
+    double unit = 1.;  // ticks per time unit of the flight
     long long slot = -1;
     bool active = false, done = false;
     auto fail = [&](int e) {
@@ -493,10 +512,12 @@ __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant_
                             px = py = 0;
                             locate(A, p.box, p.pos, cp);
                             mv.vx = mv.vy = 0;
-                            const ModeFix m = A.mf[p.mode];
+                            ModeFix m = A.mf[p.mode];
+                            const int k = slow_down(m, dt, F.kt);
                             turn(A, cp, mv, m);
                             mv = m;
-                            dt_lo = fix_ticks(dt, F.kt, dt_hi);
+                            unit = bitsd(uint64_t(1023 + k) << 52);
+                            dt_lo = fix_ticks(dt, F.kt - k, dt_hi);
                         }
                     }
                 } else {
@@ -523,30 +544,38 @@ __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant_
             if (first >= 0) {
                 const long long* line = q.cross_x ? A.gxf : A.gyf;
                 const uint64_t P = uint64_t(line[last + 1] - line[first]);
-                const uint64_t side = fix_exit(q.cross_x ? cp.ay : cp.ax, q.cross_x ? mv.ry : mv.rx);
-                uint64_t lim = dt_hi || dt_lo > PIECE ? PIECE : dt_lo;
-                lim = side < lim ? side : lim;
-                const uint64_t D = mulhi_low2(lim, (q.cross_x ? mv.vx : mv.vy) & ~FIX_DOWN);
-                if (D >= 2 * P) {
-                    const uint64_t n = whole_widths(D, P) - 1;
-                    const uint64_t t = fix_exit(n * P, q.cross_x ? mv.rx : mv.ry);
-                    uint64_t o = mulhi_low2(t, (q.cross_x ? mv.vy : mv.vx) & ~FIX_DOWN);  // sideways
-                    uint64_t& beside = q.cross_x ? cp.ay : cp.ax;
-                    o = o < beside ? o : beside;
-                    beside -= o;
+                const uint64_t along = (q.cross_x ? mv.vx : mv.vy) & ~FIX_DOWN, ra = q.cross_x ? mv.rx : mv.ry;
+                const uint64_t across = (q.cross_x ? mv.vy : mv.vx) & ~FIX_DOWN, rb = q.cross_x ? mv.ry : mv.rx;
+                uint64_t& beside = q.cross_x ? cp.ay : cp.ax;
+                uint64_t n = 0, o = 0;  // periods, and how far sideways
+                double time = 0.;
+                for (;;) {
+                    const uint64_t out = fix_exit(beside, rb);
+                    uint64_t lim = dt_hi || dt_lo > PIECE ? PIECE : dt_lo;
+                    lim = out < lim ? out : lim;
+                    const uint64_t D = mulhi_low2(lim, along);
+                    if (D < 2 * P) break;
+                    const uint64_t w = whole_widths(D, P) - 1, t = fix_exit(w * P, ra);
+                    uint64_t d = mulhi_low2(t, across);
+                    d = d < beside ? d : beside;
+                    beside -= d;
+                    o += d;
                     dt_hi -= dt_lo < t ? 1u : 0u;
                     dt_lo -= t;
+                    time += double((long long)t);
+                    n += w;
+                }
+                if (n) {
                     const double perP = 1.0 / double((long long)P);
-                    const double dt_s = (flip ? -1. : 1.) * double((long long)t);
+                    const double dt_s = (flip ? -unit : unit) * time;
                     const double o_s = ((q.cross_x ? fy : fx) ? -1. : 1.) * double((long long)o);
-                    const double a_s = (q.cross_x ? fx : fy) ? -1. : 1.;
+                    const double a_s = ((q.cross_x ? fx : fy) ? -1. : 1.) * double((long long)n);
                     for (int k = first; k <= last; ++k) {
                         const int cell = q.cross_x ? k * A.ny + cp.cj : cp.ci * A.ny + k;
-                        const long long w = line[k + 1] - line[k];
-                        const double f = double(w) * perP;
+                        const double w = double(line[k + 1] - line[k]), f = w * perP;
                         double* b = tally + 3ll * __ldg(A.cellbox + cell);
                         atomicAdd(b, dt_s * f);
-                        atomicAdd(b + (q.cross_x ? 1 : 2), a_s * double((long long)n * w));
+                        atomicAdd(b + (q.cross_x ? 1 : 2), a_s * w);
                         atomicAdd(b + (q.cross_x ? 2 : 1), o_s * f);
                         if (!(__ldg(&A.side[4 * cell + (q.cross_x ? 0 : 2)].z) & LK_INNER)) c.crossings += unsigned(n);
                     }
@@ -572,7 +601,7 @@ __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant_
         }
         {  // the box visit ends, or a piece of the flight (the sums hold a few)
             double* b = tally + 3ll * p.box;
-            const double t = double((long long)pt), ts = flip ? -t : t;
+            const double t = double((long long)pt) * unit, ts = flip ? -t : t;
             if (pt) atomicAdd(b + 0, ts);
             if (px) atomicAdd(b + 1, double((long long)px));
             if (py) atomicAdd(b + 2, double((long long)py));

@@ -24,9 +24,12 @@ namespace bte {
 struct SteadyState {
     DBuf walls, wcum, gcdf, gprob, galt;          // wall generators
     DBuf sbox, scum, scdf, sprob, salt, ssign;    // gradient generators
-    DBuf pin, ptmp, flag, pos, sums, rank, phi;   // particles and scan scratch
-    DBuf bfirst, bbox, bsign;                     // births
-    DBuf tally, counters, err, work;
+    DBuf pin, ptmp, flag, pos, sums, rank;        // particles and scan scratch
+    DBuf births;                                  // first slot, box and sign of each birth box
+    // what a generation hands the host in one copy: the error words, the
+    // number of particles carried over, the work counter, phi, the tally
+    DBuf report, counters;
+    Pinned h_report, h_births;
 };
 
 namespace {
@@ -86,25 +89,40 @@ __global__ void scan_add(unsigned* out, const unsigned* sums, long long n) {
     if (i < n) out[i] += sums[i / SCAN_B];
 }
 
-__global__ void compact(const SteadyP* src, const unsigned* flag, const unsigned* pos, SteadyP* dst,
-                        long long n) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && flag[i]) dst[pos[i]] = src[i];
+// The reflected particles, in slot order, become the next input: each block of
+// SCAN_B slots adds up the blocks before it (at most LOOK_BACK of them).
+constexpr long long LOOK_BACK = 4096;
+__global__ void __launch_bounds__(SCAN_B) compact(const SteadyP* src, const unsigned* flag, const unsigned* pos,
+                                                  const unsigned* sums, bool scanned, long long nb, SteadyP* dst,
+                                                  long long n, unsigned long long* total) {
+    __shared__ unsigned base;
+    unsigned mine = 0;
+    if (!scanned) {
+        for (int k = threadIdx.x; k < int(blockIdx.x); k += SCAN_B) mine += sums[k];
+        for (int o = 16; o > 0; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
+        if (threadIdx.x == 0) base = 0;
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&base, mine);
+    } else if (threadIdx.x == 0) {
+        base = sums[blockIdx.x];
+    }
+    __syncthreads();
+    const long long i = (long long)blockIdx.x * SCAN_B + threadIdx.x;
+    if (i < n && flag[i]) dst[base + pos[i]] = src[i];
+    if (blockIdx.x == nb - 1 && threadIdx.x == 0) *total = scanned ? sums[nb] : base + sums[nb - 1];
 }
 
-// Exclusive scan of n flags into pos; returns the total (synchronises).
-unsigned long long scan_flags(SteadyState& S, const unsigned* flag, unsigned* pos, long long n,
-                              cudaStream_t s) {
+// Block-wise exclusive scan of n flags into pos; with `all`, or beyond
+// LOOK_BACK blocks, the block sums are scanned too (and added with `all`).
+bool scan_flags(SteadyState& S, const unsigned* flag, unsigned* pos, long long n, bool all, cudaStream_t s) {
     const long long nb = (n + SCAN_B - 1) / SCAN_B;
     unsigned* sums = S.sums.as<unsigned>();
     scan_blocks<<<unsigned(nb), SCAN_B, 0, s>>>(flag, pos, sums, n);
-    scan_sums<<<1, SCAN_B, 0, s>>>(sums, nb, sums + nb);
-    scan_add<<<unsigned((n + 255) / 256), 256, 0, s>>>(pos, sums, n);
+    const bool scanned = all || nb > LOOK_BACK;
+    if (scanned) scan_sums<<<1, SCAN_B, 0, s>>>(sums, nb, sums + nb);
+    if (all) scan_add<<<unsigned((n + 255) / 256), 256, 0, s>>>(pos, sums, n);
     ck(cudaGetLastError(), "scan launch");
-    unsigned tot = 0;
-    ck(cudaMemcpyAsync(&tot, sums + nb, sizeof(unsigned), cudaMemcpyDeviceToHost, s), "d2h");
-    ck(cudaStreamSynchronize(s), "scan");
-    return tot;
+    return scanned;
 }
 
 double norm_of(const std::vector<double>& a) {
@@ -244,15 +262,22 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
         S.pos.alloc(size_t(N) * sizeof(unsigned));
         S.rank.alloc(size_t(N) * sizeof(unsigned));
         S.sums.alloc(size_t((N + SCAN_B - 1) / SCAN_B + 1) * sizeof(unsigned));
-        S.phi.alloc(size_t(nbx) * sizeof(unsigned long long));
         const size_t tally_bytes = replay ? size_t(nbx) * 6 * sizeof(unsigned long long)
                                           : size_t(nbx) * 3 * sizeof(double);
-        S.tally.alloc(tally_bytes);
+        // report: err 0, carried over 16, work 24, phi 32, then the tally
+        const size_t phi_bytes = size_t(nbx) * sizeof(unsigned long long), rep_tally = 32 + phi_bytes;
+        const size_t rep_bytes = rep_tally + tally_bytes;
+        S.report.alloc(rep_bytes);
+        S.h_report.reserve(rep_bytes);
         S.counters.alloc(16 * sizeof(unsigned long long));
-        S.err.alloc(4 * sizeof(int));
-        ck(cudaMemsetAsync(S.tally.p, 0, tally_bytes, st), "memset");
+        ck(cudaMemsetAsync(S.report.p, 0, rep_bytes, st), "memset");
         ck(cudaMemsetAsync(S.counters.p, 0, 16 * sizeof(unsigned long long), st), "memset");
-        ck(cudaMemsetAsync(S.err.p, 0, 4 * sizeof(int), st), "memset");
+        char* rep = S.report.as<char>();
+        const char* hrep = static_cast<const char*>(S.h_report.p);
+        int* err = reinterpret_cast<int*>(rep);
+        auto* carried = reinterpret_cast<unsigned long long*>(rep + 16);
+        auto* counters = S.counters.as<unsigned long long>();
+        char* tally = rep + rep_tally;
 
         DevTables T{};
         fill_static_tables(c, T);
@@ -303,9 +328,8 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
         A.in = S.pin.as<SteadyP>();
         A.out = S.ptmp.as<SteadyP>();
         A.flag = S.flag.as<unsigned>();
-        A.phi = S.phi.as<unsigned long long>();
-        S.work.alloc(sizeof(unsigned long long));
-        A.work = S.work.as<unsigned long long>();
+        A.work = reinterpret_cast<unsigned long long*>(rep + 24);
+        A.phi = reinterpret_cast<unsigned long long*>(rep + 32);
 
         const PolyArgs PA{c->d_pborders.as<PolyBorder>(), c->d_ppieces.as<PolyPiece>(), c->d_mv.as<ModeVel>(),
                           nullptr, nullptr,
@@ -328,7 +352,6 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
         const int max_gen = p->max_generations > 0 ? p->max_generations : 100000;
         std::vector<double> oldv(size_t(3) * nbx, 0.), cur(size_t(3) * nbx, 0.);
         std::vector<unsigned long long> hex, hphi(static_cast<size_t>(nbx));
-        std::vector<double> htal;
         std::vector<long long> bfirst;
         std::vector<int> bbox, bsign;
         long long nin = 0, nbirth = 0, births_total = 0;
@@ -344,31 +367,35 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
                 else
                     launch_steady_prod(T, A, nullptr, nullptr, nullptr, A.flag, c->nsm, st);
                 ck(cudaGetLastError(), "select launch");
-                scan_flags(S, A.flag, S.rank.as<unsigned>(), A.n, st);
+                scan_flags(S, A.flag, S.rank.as<unsigned>(), A.n, true, st);
             }
-            ck(cudaMemsetAsync(S.phi.p, 0, size_t(nbx) * sizeof(unsigned long long), st), "memset");
+            ck(cudaMemsetAsync(A.work, 0, 8 + phi_bytes, st), "memset");
             ck(cudaEventRecord(c->ev0, st), "cudaEventRecord");
             if (replay)
-                launch_steady_replay(T, A, S.tally.as<unsigned long long>(), S.counters.as<unsigned long long>(),
-                                     S.err.as<int>(), nullptr, c->nsm, st);
+                launch_steady_replay(T, A, reinterpret_cast<unsigned long long*>(tally), counters, err, nullptr, c->nsm, st);
             else if (p->flags & BTE_FLAG_GENERAL)
-                launch_steady_prod(T, A, S.tally.as<double>(), S.counters.as<unsigned long long>(),
-                                   S.err.as<int>(), nullptr, c->nsm, st);
+                launch_steady_prod(T, A, reinterpret_cast<double*>(tally), counters, err, nullptr, c->nsm, st);
             else if (linked) {
-                if (!launch_steady_link(T, A, LA, S.tally.as<double>(), S.counters.as<unsigned long long>(),
-                                        S.err.as<int>(), c->nsm, st))
+                if (!launch_steady_link(T, A, LA, reinterpret_cast<double*>(tally), counters, err, c->nsm, st))
                     throw Error(BTE_ERR_CUDA, "steady linked-cell kernel does not fit on the device");
-            } else if (!launch_steady_poly(T, A, PA, S.tally.as<double>(), S.counters.as<unsigned long long>(),
-                                         S.err.as<int>(), c->nsm, st))
+            } else if (!launch_steady_poly(T, A, PA, reinterpret_cast<double*>(tally), counters, err, c->nsm, st))
                 throw Error(BTE_ERR_CUDA, "steady polygon kernel does not fit on the device");
             ck(cudaGetLastError(), "steady launch");
             ck(cudaEventRecord(c->ev1, st), "cudaEventRecord");
-            int herr[4];
-            ck(cudaMemcpyAsync(herr, S.err.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st), "d2h");
+            // reflected particles, in slot order, become the next input; phi
+            // and the cumulative tallies come back with their number
+            const bool scanned = scan_flags(S, A.flag, S.pos.as<unsigned>(), A.n, false, st);
+            const long long nb = (A.n + SCAN_B - 1) / SCAN_B;
+            compact<<<unsigned(nb), SCAN_B, 0, st>>>(A.out, A.flag, S.pos.as<unsigned>(), S.sums.as<unsigned>(), scanned, nb,
+                                                     S.pin.as<SteadyP>(), A.n, carried);
+            ck(cudaGetLastError(), "compact launch");
+            ck(cudaMemcpyAsync(S.h_report.p, rep, rep_bytes, cudaMemcpyDeviceToHost, st), "d2h");
             ck(cudaStreamSynchronize(st), "steady generation");
             float ms = 0.f;
             ck(cudaEventElapsedTime(&ms, c->ev0, c->ev1), "cudaEventElapsedTime");
             kms += ms;
+            int herr[4];
+            std::memcpy(herr, hrep, sizeof herr);
             if (herr[0] != 0) {
                 const long long slot = (long long)herr[1] | ((long long)herr[2] << 31);
                 char msg[160];
@@ -378,22 +405,14 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
                                                           : "geometry error");
                 throw Error(bte_status(herr[0]), msg);
             }
-            // reflected particles, in slot order, become the next input
-            const unsigned long long nref = scan_flags(S, A.flag, S.pos.as<unsigned>(), A.n, st);
-            compact<<<unsigned((A.n + 255) / 256), 256, 0, st>>>(A.out, A.flag, S.pos.as<unsigned>(),
-                                                                 S.pin.as<SteadyP>(), A.n);
-            ck(cudaGetLastError(), "compact launch");
-            // phi and the cumulative tallies
-            ck(cudaMemcpyAsync(hphi.data(), S.phi.p, size_t(nbx) * sizeof(unsigned long long),
-                               cudaMemcpyDeviceToHost, st), "d2h");
+            unsigned long long nref = 0;
+            std::memcpy(&nref, hrep + 16, sizeof nref);
+            std::memcpy(hphi.data(), hrep + 32, phi_bytes);
+            const double* htal = reinterpret_cast<const double*>(hrep + rep_tally);
             if (replay) {
                 hex.resize(size_t(nbx) * 6);
-                ck(cudaMemcpyAsync(hex.data(), S.tally.p, tally_bytes, cudaMemcpyDeviceToHost, st), "d2h");
-            } else {
-                htal.resize(size_t(nbx) * 3);
-                ck(cudaMemcpyAsync(htal.data(), S.tally.p, tally_bytes, cudaMemcpyDeviceToHost, st), "d2h");
+                std::memcpy(hex.data(), hrep + rep_tally, tally_bytes);
             }
-            ck(cudaStreamSynchronize(st), "steady readback");
             for (int b = 0; b < nbx; ++b)
                 for (int q = 0; q < 3; ++q) {
                     double v;
@@ -422,13 +441,23 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
             births_total += nbirth;
             nin = (long long)nref;
             if (nin + nbirth > N) throw Error(BTE_ERR_LIMIT, "generation larger than the particle buffers");
-            S.bfirst.upload(bfirst, st);
-            S.bbox.upload(bbox, st);
-            S.bsign.upload(bsign, st);
-            A.nbirth = int(bbox.size());
-            A.birth_first = S.bfirst.as<long long>();
-            A.birth_box = S.bbox.as<int>();
-            A.birth_sign = S.bsign.as<int>();
+            {
+                // [first slots, one more than boxes][boxes][signs]
+                const size_t m = bbox.size(), f = (m + 1) * sizeof(long long), b = f + 2 * m * sizeof(int);
+                S.h_births.reserve(b);
+                char* h = static_cast<char*>(S.h_births.p);
+                std::memcpy(h, bfirst.data(), f);
+                if (m) {
+                    std::memcpy(h + f, bbox.data(), m * sizeof(int));
+                    std::memcpy(h + f + m * sizeof(int), bsign.data(), m * sizeof(int));
+                }
+                S.births.alloc(b);
+                ck(cudaMemcpyAsync(S.births.p, h, b, cudaMemcpyHostToDevice, st), "upload");
+                A.nbirth = int(m);
+                A.birth_first = S.births.as<long long>();
+                A.birth_box = reinterpret_cast<const int*>(S.births.as<char>() + f);
+                A.birth_sign = A.birth_box + m;
+            }
             // convergence, src/RTA_MC2D.cpp:2661-2694
             auto slice = [&](const std::vector<double>& v, int q) {
                 return std::vector<double>(v.begin() + size_t(q) * nbx, v.begin() + size_t(q + 1) * nbx);
