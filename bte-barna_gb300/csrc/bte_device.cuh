@@ -369,6 +369,19 @@ struct GBox {
     int tto;  // periodic box: the box it translates to (<Translate_to id>); -1 otherwise
 };
 
+// A double as a signed integer with the same order (no NaN; the two zeros are
+// one value), so that comparisons run on the integer units.
+BTE_HD long long order_key(double x) {
+    const long long b = (long long)dbits(x);
+    return (b << 1) == 0 ? 0 : b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+
+// An axis-aligned rectangular box as order keys of its bounds; x0 > x1: any
+// other box.
+struct RectKey {
+    long long x0, x1, y0, y1;
+};
+
 // Inside or on the border of a counter-clockwise convex hull.
 BTE_HD bool inside_hull(const V2* hull, int n, V2 p) {
     for (int i = 0; i < n; ++i) {

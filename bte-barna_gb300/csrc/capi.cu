@@ -58,6 +58,8 @@ void ensure_static(bte_ctx* c) {
         c->d_tau.upload(tau, c->stream);
         c->d_mv.upload(mv, c->stream);
         c->d_mf.alloc(n * sizeof(bte::ModeFix));
+        c->d_eps.alloc(n * sizeof(bte::V2));
+        bte::launch_mode_eps(c->d_vxc.as<double>(), c->d_vyc.as<double>(), int(n), c->d_eps.as<bte::V2>(), c->stream);
         c->vmax = 0.;
         for (std::size_t k = 0; k < n; ++k) c->vmax = std::max({c->vmax, std::fabs(m.vxc[k]), std::fabs(m.vyc[k])});
         c->fix_dev = false;
@@ -71,6 +73,12 @@ void ensure_static(bte_ctx* c) {
         c->d_contacts.upload(g.contacts, c->stream);
         c->d_cseg.upload(g.contact_seg, c->stream);
         c->d_transl.upload(g.translation, c->stream);
+        {
+            std::vector<bte::RectKey> rk(g.boxes.size());
+            for (std::size_t b = 0; b < rk.size(); ++b) rk[b] = bte::rect_key(g, b);
+            c->d_rkey.upload(rk, c->stream);
+            sync(c);
+        }
         c->d_boxmat.upload(g.mat, c->stream);
         {
             const bte::TranslationFast tf = bte::build_translation_fast(g);
@@ -1227,6 +1235,8 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         T.mirror = c->have_mirror ? c->d_mirror.as<int>() : nullptr;
         T.box_mat = c->nmat > 0 ? c->d_boxmat.as<int>() : nullptr;
         bte::set_crystal_tables(c, T);
+        T.rkey = c->d_rkey.as<bte::RectKey>();
+        T.eps = c->d_eps.as<bte::V2>();
         T.ntime = int(ntime);
         T.timegrid = c->d_time.as<double>();
         T.maxtime = maxtime;
@@ -1272,7 +1282,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         bte::PostUnits units;
         ck(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
         if (replay) {
-            bte::launch_replay(T, reinterpret_cast<unsigned long long*>(tally), counters, err, c->nsm, c->stream);
+            bte::launch_replay(T, reinterpret_cast<unsigned long long*>(tally), counters, err, work, c->nsm, c->stream);
         } else if (grid_run) {
             if (!bte::launch_prod_grid(T, A, tally, counters, err, work, c->tune, c->nsm, c->stream))
                 throw Error(BTE_ERR_INPUT, "tuning not supported by the grid kernel");
@@ -1620,6 +1630,8 @@ bte_status prepared_grid_run(bte_ctx* c, const bte_rta_params* p, PreparedRun* r
     T.mirror = c->have_mirror ? c->d_mirror.as<int>() : nullptr;
     T.box_mat = c->nmat > 0 ? c->d_boxmat.as<int>() : nullptr;
     set_crystal_tables(c, T);
+    T.rkey = c->d_rkey.as<bte::RectKey>();
+    T.eps = c->d_eps.as<bte::V2>();
     T.ntime = r->ntime;
     T.timegrid = nullptr;  // set by the caller
     T.maxtime = r->maxtime;
@@ -1815,6 +1827,8 @@ void fill_static_tables(bte_ctx* c, DevTables& T) {
     T.mirror = c->have_mirror ? c->d_mirror.as<int>() : nullptr;
     T.box_mat = c->nmat > 0 ? c->d_boxmat.as<int>() : nullptr;
     set_crystal_tables(c, T);
+    T.rkey = c->d_rkey.as<bte::RectKey>();
+    T.eps = c->d_eps.as<bte::V2>();
 }
 
 // The interface tables of crystals joined by mismatch interfaces (null

@@ -105,6 +105,7 @@ struct bte_ctx {
     bte::DBuf d_boxes, d_hull, d_borders, d_contacts, d_cseg, d_transl;
     bte::DBuf d_tfast, d_tfast_rng, d_tfast_u;  // translations without a search
     bool have_tfast = false;
+    bte::DBuf d_rkey, d_eps;                      // evolparticle short cuts
     bte::DBuf d_invden;                           // 1 / (n.v) per normal class and mode
     bte::DBuf d_prect;                            // PolyRect per box
     // several crystals (bte_load_mode_tables): their own mode tables, the

@@ -23,8 +23,10 @@ struct ProdTuning {
     int particles_per_thread;  // accepted; every lane carries one
 };
 
+// (`work` is a zeroed particle counter)
 void launch_replay(const DevTables& T, unsigned long long* ex, unsigned long long* counters,
-                   int* err, int nsm, cudaStream_t s);
+                   int* err, unsigned long long* work, int nsm, cudaStream_t s);
+void launch_mode_eps(const double* vx, const double* vy, int n, V2* eps, cudaStream_t s);
 
 // General convex-box production kernel (any geometry); `work` is a zeroed
 // particle counter.

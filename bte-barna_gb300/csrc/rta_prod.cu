@@ -19,12 +19,12 @@
 
 namespace bte {
 
-// Any convex-box geometry, the flight logic of rta_flight.cuh (run_particle
-// unrolled into one evolparticle step per loop pass).  Warps are persistent
+// Any convex-box geometry, the flight logic of rta_flight.cuh, one
+// evolparticle step per loop pass.  Warps are persistent
 // and a lane whose particle has finished takes the next one from a global
 // counter (one atomic per warp), so lanes stay busy while particles of very
 // different lifetimes run out; each particle keeps its own Philox stream,
-// so its trajectory is the one run_particle would draw.
+// so its trajectory does not depend on the lane.
 __global__ void __launch_bounds__(128) rta_prod_general(DevTables T, double* tally,
                                                         unsigned long long* counters, int* err,
                                                         unsigned long long* work) {
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(128) rta_prod_general(DevTables T, double* tal
         }
         if (__all_sync(0xffffffffu, done)) break;
         if (!active) continue;
-        if (need_flight) {  // the body of run_particle's outer loop
+        if (need_flight) {  // draw the next free flight
             if (!(time < T.maxtime)) {
                 active = false;
                 continue;

@@ -37,10 +37,10 @@ struct ReplayPolicy {
         return -bte_log(uu) / T.w[k];  // k: material offset + mode
     }
     __device__ int resample(const DevTables& T, int mo) {
-        return lower_bound_d(T.resample_cdf + mo, T.n, u());
+        return lower_bound_key(T.resample_cdf + mo, T.n, u());
     }
     __device__ int gen_mode(const DevTables& T, int gi) {
-        return lower_bound_d(T.gen_cdf + (long long)gi * T.n, T.n, u());
+        return lower_bound_key(T.gen_cdf + (long long)gi * T.n, T.n, u());
     }
     __device__ int bounce(const DevTables& T, int cls, int mode) {
         const long long a = T.row_ptr[(long long)cls * (T.n + 1) + mode];
@@ -48,13 +48,13 @@ struct ReplayPolicy {
         const int len = int(b - a);
         if (len <= 0) return -1;
         const double s = u();
-        int j = lower_bound_d(T.lcdf + a, len, s);
+        int j = lower_bound_key(T.lcdf + a, len, s);
         if (j == len) j = len - 1;
         return T.lcol[a + j];
     }
     // Grid_distribution::sample over a CDF (the alias arguments are unused)
     __device__ int dist(const double* cdf, const float*, const int*, int n) {
-        return lower_bound_d(cdf, n, u());
+        return lower_bound_key(cdf, n, u());
     }
     // process_segment (periodic), src/RTA_MC2D.cpp:784-834: one value per box;
     // at a spectral location also the mode's time and its signed segment
@@ -81,8 +81,8 @@ struct ReplayPolicy {
     __device__ int tally(const DevTables& T, int box, double t0, double t1, int sign, V2 v, int mode) {
         const int loc = T.spec_loc ? T.spec_loc[box] : -1;
         const double* g = T.timegrid;
-        int sb = lower_bound_d(g, T.ntime, t0) - 1;
-        int eb = lower_bound_d(g, T.ntime, t1) - 1;
+        int sb = lower_bound_key(g, T.ntime, t0) - 1;
+        int eb = lower_bound_key(g, T.ntime, t1) - 1;
         sb = sb < 0 ? 0 : (sb > T.ntime - 2 ? T.ntime - 2 : sb);
         eb = eb < 0 ? 0 : (eb > T.ntime - 2 ? T.ntime - 2 : eb);
         const double delta_t = t1 - t0;
@@ -116,38 +116,122 @@ __device__ __forceinline__ void flush_counters(const Counters& c, unsigned long 
     }
 }
 
-__global__ void __launch_bounds__(128) rta_replay_kernel(DevTables T, unsigned long long* ex,
-                                                         unsigned long long* counters, int* err) {
-    Counters c = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    // every lane runs the same trip count so the closing shuffles see a full warp
-    const long long n = T.pend - T.pbegin;
-    const long long trips = (n + stride - 1) / stride;
-    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    for (long long it = 0; it < trips; ++it) {
-        const long long pid = T.pbegin + it * stride + tid;
-        if (pid >= T.pend) continue;
-        ReplayPolicy pol;
-        pol.g.seed(T.seed, (uint64_t)pid);
-        pol.ex = ex;
-        pol.ntally = 0;
-        const int e = run_particle(T, pol, pid, c);
-        c.tallies += pol.ntally;
-        if (e) {
-            if (atomicCAS(err, 0, e) == 0) {
-                err[1] = int(pid & 0x7fffffff);
-                err[2] = int(pid >> 31);
-            }
-        }
-    }
-    flush_counters(c, counters);
-}
-
 __device__ __forceinline__ void record_error_r(int* err, int e, long long pid) {
     if (atomicCAS(err, 0, e) == 0) {
         err[1] = int(pid & 0x7fffffff);
         err[2] = int(pid >> 31);
     }
+}
+
+// The particle lives of a run, one evolparticle step per
+// pass, as rta_prod_general: persistent warps whose finished lanes take the
+// next particle from a counter, so that particles of very different lives share
+// a warp.  Bound by the FP64 pipe, where an instruction costs the same for one
+// active lane as for 32: with one particle per thread two lanes of a warp were
+// active on average.  1e5 particles on a ribbon of 20 cells and 1536 modes took
+// 58.2 ms; with this loop and evolparticle's comparisons on the integer units,
+// 9.5.
+__global__ void __launch_bounds__(128) rta_replay_kernel(const __grid_constant__ DevTables T, unsigned long long* ex,
+                                                         unsigned long long* counters, int* err,
+                                                         unsigned long long* work) {
+    Counters c = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    const int lane = threadIdx.x & 31;
+    const long long total = T.pend - T.pbegin;
+    ReplayPolicy pol;
+    pol.g.seed(0, 0);
+    pol.ex = ex;
+    pol.ntally = 0;
+    Particle p;
+    p.pos = v2(0., 0.);
+    p.mode = p.box = p.mo = 0;
+    p.sign = 1;
+    p.t = 0.;
+    V2 v = v2(0., 0.);
+    double dt = 0., time = 0.;
+    int nudges = 0, guard = 0, fate = FATE_LOST;
+    long long nev = 0, pid = -1;
+    bool active = false, done = false, need_flight = false;
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, !active && !done);
+        if (idle) {
+            unsigned long long base = 0;
+            const int leader = __ffs(idle) - 1;
+            if (lane == leader) base = atomicAdd(work, (unsigned long long)__popc(idle));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (!active && !done) {
+                const long long mine = (long long)base + __popc(idle & ((1u << lane) - 1u));
+                if (mine < total) {
+                    pid = T.pbegin + mine;
+                    pol.g.seed(T.seed, (uint64_t)pid);
+                    const int e = generate(T, pol, pid, p);
+                    if (e) {
+                        record_error_r(err, e, pid);
+                    } else {
+                        active = true;
+                        need_flight = true;
+                        time = 0.;
+                        nudges = 0;
+                        nev = 0;
+                    }
+                } else {
+                    done = true;
+                }
+            }
+        }
+        if (__all_sync(0xffffffffu, done)) break;
+        if (!active) continue;
+        if (need_flight) {  // draw the next free flight
+            const int k = p.mode;
+            int e = 0;
+            if (!(time < T.maxtime)) e = -1;
+            else if (++nev > T.flight_cap) e = E_LIMIT;
+            else if (T.w[p.mo + k] == 0.) e = E_VALUE;
+            if (e) {
+                if (e > 0) record_error_r(err, e, pid);
+                active = false;
+                continue;
+            }
+            v = v2(T.vxc[k], T.vyc[k]);
+            dt = pol.flight(T, p.mo + k);
+            c.events++;
+            if (time + dt > T.maxtime) dt = T.maxtime - time + 1.0e-8;
+            guard = 0;
+            fate = FATE_LOST;
+            need_flight = false;
+        }
+        if (!almost_equal(dt, 0.)) {
+            int e = ++guard > FLIGHT_CAP ? E_LIMIT : 0;
+            if (!e) e = evolparticle(T, pol, p, v, dt, c, nudges, fate);
+            if (e) {
+                record_error_r(err, e, pid);
+                active = false;
+                continue;
+            }
+        }
+        if (almost_equal(dt, 0.)) {  // the flight is over
+            if (p.mode == 0) {       // absorbed
+                active = false;
+                continue;
+            }
+            time = p.t;
+            need_flight = true;
+        }
+    }
+    c.tallies += pol.ntally;
+    flush_counters(c, counters);
+}
+
+// 1e-6 v / |v| of every mode, rounded as evolparticle rounds it.
+__global__ void mode_eps(const double* vx, const double* vy, int n, V2* eps) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) {
+        const V2 v = v2(vx[k], vy[k]);
+        eps[k] = divs(scal(1.0e-6, v), norm(v));
+    }
+}
+
+void launch_mode_eps(const double* vx, const double* vy, int n, V2* eps, cudaStream_t s) {
+    mode_eps<<<(n + 255) / 256, 256, 0, s>>>(vx, vy, n, eps);
 }
 
 // Generation 0: 1 per slot whose first draw picks a gradient generator.
@@ -199,13 +283,13 @@ void launch_steady_replay(const DevTables& T, const SteadyArgs& A, unsigned long
 }
 
 void launch_replay(const DevTables& T, unsigned long long* ex, unsigned long long* counters,
-                   int* err, int nsm, cudaStream_t s) {
+                   int* err, unsigned long long* work, int nsm, cudaStream_t s) {
     const long long n = T.pend - T.pbegin;
     if (n <= 0) return;
     long long blocks = (n + 127) / 128;
-    const long long cap = (long long)nsm * 16;
+    const long long cap = (long long)nsm * 4;  // resident blocks (128 registers x 128 threads)
     if (blocks > cap) blocks = cap;
-    rta_replay_kernel<<<unsigned(blocks), 128, 0, s>>>(T, ex, counters, err);
+    rta_replay_kernel<<<unsigned(blocks), 128, 0, s>>>(T, ex, counters, err, work);
 }
 
 }  // namespace bte

@@ -883,6 +883,22 @@ TranslationFast build_translation_fast(const HostGeometry& g, double margin) {
     return R;
 }
 
+RectKey rect_key(const HostGeometry& g, std::size_t b) {
+    const RectKey none{1, 0, 0, 0};
+    const GBox& B = g.boxes[b];
+    const std::vector<V2> hull(g.hull.begin() + B.hull_off, g.hull.begin() + B.hull_off + B.nhull);
+    double x0, y0, x1, y1;
+    if (!as_rect(hull, x0, y0, x1, y1) || !(x0 < x1 && y0 < y1)) return none;
+    for (int i = 0; i < 4; ++i)  // four corners, counter-clockwise
+        if (!(cross(sub(hull[(i + 1) % 4], hull[i]), sub(hull[(i + 2) % 4], hull[(i + 1) % 4])) > 0.)) return none;
+    for (int k = 0; k < B.nborders; ++k) {
+        const GBorder& r = g.borders[std::size_t(B.border_off + k)];
+        const bool vert = std::fabs(r.np.x) == 1. && r.np.y == 0., hor = r.np.x == 0. && std::fabs(r.np.y) == 1.;
+        if (!(vert ? r.la.x == r.lb.x && r.la.y != r.lb.y : hor && r.la.y == r.lb.y && r.la.x != r.lb.x)) return none;
+    }
+    return RectKey{order_key(x0), order_key(x1), order_key(y0), order_key(y1)};
+}
+
 LinkGrid build_link_grid(const HostGeometry& g) {
     LinkGrid L;
     const std::size_t nbx = g.boxes.size();

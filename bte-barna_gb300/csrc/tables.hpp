@@ -71,6 +71,10 @@ struct TranslationFast {
 };
 TranslationFast build_translation_fast(const HostGeometry& g, double margin = 1.0e-2);
 
+// The bounds of box b as order keys where it is an axis-aligned rectangle with
+// axis-aligned border lines, else x0 > x1.
+RectKey rect_key(const HostGeometry& g, std::size_t b);
+
 // Boxes that are all axis-aligned rectangles, cut into the cells of the lines
 // through all their edges: what lies across each side of each cell.  `ok`
 // only where every side has one definite answer (no sliver between lines, a
