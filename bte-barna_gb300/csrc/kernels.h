@@ -62,6 +62,7 @@ struct GridArgs {
     const unsigned long long* wxf;  // and the widths between them
     const unsigned long long* wyf;
     const int* map;          // the cells with a void rim: [nx + 2][ny + 2], as G.cell
+    int lanes;               // lanes of a warp that take particles (set by the launch)
     int refill;              // idle lanes of a warp before new particles are generated
     int cls[4];              // normal classes of the +x, -x, +y, -y walls (-1: none)
 };

@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
     long long pid = -1;
     uint32_t nev = 0, npass = 0;
     double* tgrp = tally;  // the tally of the particle's replica group
-    bool active = false, done = false;
+    bool active = false, done = lane >= A.lanes;
     // adjoint state: Phi so far, the particle's total, pending score terms
     double phi_run = 0., phi_tot = 0., spec_score = 0.;
     double sum_r = 0., g_p = 0., phi_all = 0.;
@@ -413,8 +413,8 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
             return;
         }
         const ModeFix m = A.mf[mode];
-        const float ef = -logf((float(word >> 9) + 0.5f) * 0x1p-23f);
         const double tau_k = __ldg(T.tau + mo + mode);
+        const float ef = -logf((float(word >> 9) + 0.5f) * 0x1p-23f);
         if ((m.vx ^ mv.vx) & FIX_DOWN) ax = __ldg(A.wxf + ci) - ax;
         if ((m.vy ^ mv.vy) & FIX_DOWN) ay = __ldg(A.wyf + cj) - ay;
         mv = m;
@@ -501,6 +501,17 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
             // this pass's random words (used at its end); computed ahead of
             // the segment, with which it shares no data
             const uint4 rr = pass_block(npass++, (uint64_t)pid, T.seed);
+            // the mode a scattering at the end of this segment would draw: its
+            // table read runs under the segment's arithmetic (1e4 particles
+            // 0.51 -> 0.48 ms, 1e6 3.13 -> 3.06; the 64-register variant
+            // reads it in place: 114.5 ms there, 116.6 ahead)
+            constexpr bool AHEAD = MINB < 4;
+            int cand = mode;
+            if (AHEAD && !T.ballistic) {
+                const int k = int(mulhi32(rr.y, uint32_t(T.n)));
+                const int2 e = __ldg(T.resample + mo + k);
+                cand = float(rr.z >> 8) * 0x1p-24f < __int_as_float(e.x) ? k : e.y;
+            }
             if (CHECK && (ci < 0 || ci >= A.G.nx || cj < 0 || cj >= A.G.ny || box < 0 || box >= T.nboxes || bin < 0 ||
                           bin > last_bin)) {
                 stop(E_CHECK);
@@ -618,10 +629,14 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
                     }
                     c.wall_hits++;
                 } else if (!T.ballistic) {
-                    keep = int(mulhi32(rr.y, uint32_t(T.n)));
-                    const int2 e = __ldg(T.resample + mo + keep);
-                    pr = __int_as_float(e.x);
-                    alt = e.y;
+                    if (AHEAD) {
+                        keep = alt = cand;
+                    } else {
+                        keep = int(mulhi32(rr.y, uint32_t(T.n)));
+                        const int2 e = __ldg(T.resample + mo + keep);
+                        pr = __int_as_float(e.x);
+                        alt = e.y;
+                    }
                     if (ADJ == 2) pend_kind |= 1;
                 }
                 const float acc = float(rr.z >> 8) * 0x1p-24f;
@@ -1340,14 +1355,14 @@ bool launch_steady_poly(const DevTables& T, const SteadyArgs& A, const PolyArgs&
     return true;
 }
 
-bool launch_prod_grid(const DevTables& T, const GridArgs& A, double* tally,
+bool launch_prod_grid(const DevTables& T, const GridArgs& A0, double* tally,
                       unsigned long long* counters, int* err, unsigned long long* work,
                       const ProdTuning& tune, int nsm, cudaStream_t s, int adj_pass,
                       const AdjArgs* adj) {
     const long long n = T.pend - T.pbegin;
     if (n <= 0) return true;
-    const int threads = tune.block_threads > 0 ? tune.block_threads : 256;
-    if (threads > 256 || threads % 32) return false;
+    GridArgs A = A0;
+    A.lanes = 32;
     const size_t smem = size_t(3) * T.nboxes * T.nbins * sizeof(double);
     // the adjoint passes run with the tally in global memory
     const bool use_smem = tune.smem_tally != 0 && smem <= 200 * 1024 && adj_pass == 0 && T.ngroups <= 1;
@@ -1357,6 +1372,18 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A, double* tally,
     // several particles in turn (2e6 on 36864 modes: 111 ms against 118 with
     // three), three leave fewer lanes idle at the end of a short run (2e5:
     // 0.53 ms against 0.61; 1e6: 3.36 and 3.38, the same).
+    // A run too small to fill the GPU is bound by the passes of its longest
+    // particles, and a pass takes as long as its warp's branches together: the
+    // particles are spread over one lane of up to 16 warps per SM, then over
+    // as few lanes of 8 warps as hold them.  Kernel times of 1e3, 2e3, 1e4 and
+    // 3e4 particles with all lanes in use 0.126, 0.62, 0.64 and 0.65 ms, so
+    // 0.089, 0.35, 0.48 and 0.56 (16 warps at 1e4: 0.55; 4: 0.54).
+    const bool tuned = tune.block_threads > 0 || tune.blocks_per_sm > 0 || use_smem;
+    if (!tuned && !T.checks)
+        A.lanes = n <= 16ll * nsm ? 1 : int(std::min<long long>(32, (n + 8ll * nsm - 1) / (8ll * nsm)));
+    const bool small = A.lanes < 32;
+    const int threads = tune.block_threads > 0 ? tune.block_threads : small ? 64 : 256;
+    if (threads > 256 || threads % 32) return false;
     const bool long_run = n >= 8ll * 1024 * nsm;
     int bps = tune.blocks_per_sm > 0 ? tune.blocks_per_sm : (use_smem ? 1 : long_run ? 4 : 3);
     const AdjArgs none{};
@@ -1392,8 +1419,8 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A, double* tally,
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, fn, threads, use_smem ? smem : 0);
     if (maxb < 1) return false;
     if (bps > maxb) bps = maxb;
-    long long blocks = (long long)nsm * bps;
-    const long long need = (n + threads - 1) / threads;
+    long long blocks = (long long)nsm * (small ? maxb : bps);
+    const long long per = threads / 32 * A.lanes, need = (n + per - 1) / per;
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
     const unsigned nb = unsigned(blocks);
