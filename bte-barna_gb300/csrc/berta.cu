@@ -1496,16 +1496,16 @@ namespace {
 // sum, each with the sign of its entry.
 std::vector<double> signed_cumm(const std::vector<double>& P, int nm) {
     std::vector<double> c(P.size());
-    for (int j = 0; j < nm; ++j) {
-        const double* col = P.data() + std::size_t(j) * nm;
+    bte::host_parallel(std::size_t(nm), bte::hw_threads(), [&](std::size_t j) {
+        const double* col = P.data() + j * std::size_t(nm);
         double abssum = 0.;
         for (int i = 0; i < nm; ++i) abssum += std::fabs(col[i]);
         double acc = 0.;
         for (int i = 0; i < nm; ++i) {
             acc += std::fabs(col[i]);
-            c[std::size_t(j) * nm + i] = col[i] < 0. ? -acc / abssum : acc / abssum;
+            c[j * std::size_t(nm) + std::size_t(i)] = col[i] < 0. ? -acc / abssum : acc / abssum;
         }
-    }
+    });
     return c;
 }
 
@@ -1515,20 +1515,25 @@ std::vector<bte::PAlias> propagator_alias(const std::vector<double>& P, int nm) 
     using namespace bte;
     const std::size_t nn = std::size_t(nm) * std::size_t(nm);
     std::vector<PAlias> tab(nn);
-    std::vector<double> w(static_cast<std::size_t>(nm));
-    std::vector<Alias> al(static_cast<std::size_t>(nm));
-    for (int j = 0; j < nm; ++j) {
-        const double* col = P.data() + std::size_t(j) * nm;
-        for (int i = 0; i < nm; ++i) w[std::size_t(i)] = std::fabs(col[i]);
-        alias_table(w.data(), nm, al.data());
-        for (int i = 0; i < nm; ++i) {
-            PAlias e;
-            e.prob = al[std::size_t(i)].prob;
-            const int alt = al[std::size_t(i)].alt;
-            e.alt = unsigned(alt) | (col[alt] < 0. ? (1u << 30) : 0u) | (col[i] < 0. ? (1u << 31) : 0u);
-            tab[std::size_t(j) * nm + std::size_t(i)] = e;
+    // (columns on all host threads: 375 ms for 6141 modes on one, 55 on 16)
+    const std::size_t nblk = std::min(nn ? std::size_t(nm) : 0, std::size_t(hw_threads()) * 8);
+    host_parallel(nblk, hw_threads(), [&](std::size_t blk) {
+        std::vector<double> w(static_cast<std::size_t>(nm));
+        std::vector<Alias> al(static_cast<std::size_t>(nm));
+        AliasScratch scratch;
+        for (std::size_t j = std::size_t(nm) * blk / nblk; j < std::size_t(nm) * (blk + 1) / nblk; ++j) {
+            const double* col = P.data() + j * std::size_t(nm);
+            for (int i = 0; i < nm; ++i) w[std::size_t(i)] = std::fabs(col[i]);
+            alias_table(w.data(), nm, al.data(), scratch);
+            for (int i = 0; i < nm; ++i) {
+                PAlias e;
+                e.prob = al[std::size_t(i)].prob;
+                const int alt = al[std::size_t(i)].alt;
+                e.alt = unsigned(alt) | (col[alt] < 0. ? (1u << 30) : 0u) | (col[i] < 0. ? (1u << 31) : 0u);
+                tab[j * std::size_t(nm) + std::size_t(i)] = e;
+            }
         }
-    }
+    });
     return tab;
 }
 

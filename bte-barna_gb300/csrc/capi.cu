@@ -422,16 +422,18 @@ void ensure_resample(bte_ctx* c, double T0) {
     std::vector<double> cdf;
     std::vector<bte::Alias> al;
     if (c->nmat > 0) {
-        bte::HostModes mm = c->modes;
-        const std::size_t n = mm.n();
-        for (int k = 0; k < c->nmat; ++k) {
+        const std::size_t n = c->modes.n(), nmat = std::size_t(c->nmat);
+        cdf.resize(nmat * n);
+        al.resize(nmat * n);
+        bte::host_parallel(nmat, hw_threads(), [&](std::size_t k) {
+            bte::HostModes mm = c->modes;
             std::vector<double> ck;
             std::vector<bte::Alias> ak;
             mm.w.assign(c->mat_w.begin() + std::ptrdiff_t(k * n), c->mat_w.begin() + std::ptrdiff_t((k + 1) * n));
-            bte::build_resample(mm, c->mat_T0[std::size_t(k)], ck, ak);
-            cdf.insert(cdf.end(), ck.begin(), ck.end());
-            al.insert(al.end(), ak.begin(), ak.end());
-        }
+            bte::build_resample(mm, c->mat_T0[k], ck, ak);
+            std::copy(ck.begin(), ck.end(), cdf.begin() + std::ptrdiff_t(k * n));
+            std::copy(ak.begin(), ak.end(), al.begin() + std::ptrdiff_t(k * n));
+        });
     } else {
         bte::build_resample(c->modes, T0, cdf, al);
     }
@@ -514,10 +516,13 @@ void ensure_generators(bte_ctx* c, const bte_rta_params* p) {
     }
     std::vector<float> prob(c->gens.alias.size());
     std::vector<int> alt(c->gens.alias.size());
-    for (std::size_t i = 0; i < prob.size(); ++i) {
-        prob[i] = c->gens.alias[i].prob;
-        alt[i] = c->gens.alias[i].alt;
-    }
+    const std::size_t chunk = std::size_t(1) << 20;
+    bte::host_parallel((prob.size() + chunk - 1) / chunk, hw_threads(), [&](std::size_t b) {
+        for (std::size_t i = b * chunk; i < std::min(prob.size(), (b + 1) * chunk); ++i) {
+            prob[i] = c->gens.alias[i].prob;
+            alt[i] = c->gens.alias[i].alt;
+        }
+    });
     c->d_gcdf.upload(c->gens.cdf, c->stream);
     c->d_gprob.upload(prob, c->stream);
     c->d_galt.upload(alt, c->stream);

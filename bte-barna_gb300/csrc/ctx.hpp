@@ -74,11 +74,6 @@ struct PostUnits {
     double t = 1., x = 1.;
 };
 
-inline int hw_threads() {
-    unsigned n = std::thread::hardware_concurrency();
-    return n ? int(n < 64u ? n : 64u) : 4;
-}
-
 struct BertaState;   // berta.cu
 struct SteadyState;  // steady.cu
 struct SpectralState;  // spectral.cu

@@ -4,6 +4,7 @@
 // generators.
 #pragma once
 
+#include <functional>
 #include <cstdint>
 #include <stdexcept>
 #include <string>
@@ -207,6 +208,16 @@ double initial_counts(Generators& G, int64_t nparticles, uint64_t seed);
 
 // Walker/Vose alias table of unnormalised non-negative weights.
 void alias_table(const double* w, int n, Alias* out);
+struct AliasScratch {
+    std::vector<double> p;
+    std::vector<int> small, large;
+};
+void alias_table(const double* w, int n, Alias* out, AliasScratch& scratch);
+
+// f(0) .. f(n - 1) on up to nthreads host threads, each taking the next index;
+// returns when all are done and rethrows the first exception.
+void host_parallel(std::size_t n, int nthreads, const std::function<void(std::size_t)>& f);
+int hw_threads();
 
 // Mode-mirror maps for specular reflection on the q grid: for each wall
 // normal class, the mode with v_n reversed (or -1 when the class is not
