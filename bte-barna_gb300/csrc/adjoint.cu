@@ -40,7 +40,10 @@ bte_status bte_rta_adjoint(bte_ctx* c, const bte_rta_params* p, const double* we
         const long long np = r.T.pend - r.T.pbegin;
         DBuf dW, dphi, dg, ds, dcnt, derr, dwork;
         std::vector<double> W(weights, weights + nk * 3);  // in the walk's units
+        int comps = 0;
         for (std::size_t k = 0; k < nk; ++k) {
+            for (int q = 0; q < 3; ++q)
+                if (W[3 * k + std::size_t(q)] != 0.) comps |= 1 << q;
             W[3 * k] *= r.A.fx.per_tick();
             W[3 * k + 1] *= r.A.fx.per_unit();
             W[3 * k + 2] *= r.A.fx.per_unit();
@@ -56,7 +59,7 @@ bte_status bte_rta_adjoint(bte_ctx* c, const bte_rta_params* p, const double* we
         ck(cudaMemsetAsync(dg.p, 0, n * sizeof(double), s), "memset");
         ck(cudaMemsetAsync(ds.p, 0, 4 * sizeof(double), s), "memset");
         ck(cudaMemsetAsync(derr.p, 0, 4 * sizeof(int), s), "memset");
-        AdjArgs a{dW.as<double>(), dphi.as<double>(), dg.as<double>(), ds.as<double>()};
+        AdjArgs a{dW.as<double>(), dphi.as<double>(), dg.as<double>(), ds.as<double>(), comps};
         float ms_total = 0.f;
         unsigned long long ev = 0;
         for (int pass = 1; pass <= 2; ++pass) {
@@ -95,7 +98,7 @@ bte_status bte_rta_adjoint(bte_ctx* c, const bte_rta_params* p, const double* we
         const double sumR = p->ballistic ? 0. : sc[1];
         for (std::size_t k = 0; k < n; ++k) {
             const double tau = m.w[k] > 0. ? 1.0 / m.w[k] : 0.;
-            out->dphi_dtau[k] = g[k] + (tau > 0. && Z > 0. ? (pm[k] / Z) / tau * sumR : 0.);
+            out->dphi_dtau[k] = g[k] * m.w[k] + (tau > 0. && Z > 0. ? (pm[k] / Z) / tau * sumR : 0.);
         }
         out->phi = sc[2];
         out->dphi_dp = sc[0];

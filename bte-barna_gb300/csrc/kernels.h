@@ -149,8 +149,9 @@ bool launch_prod_link(const DevTables& T, const LinkArgs& A, double* tally, unsi
 struct AdjArgs {
     const double* W;      // [nboxes * nbins][3]
     double* phi_total;    // [particles]
-    double* g_tau;        // [nmodes]
+    double* g_tau;        // [nmodes], times tau
     double* g_scalar;     // [3]
+    int comps;            // bit q: W has a component q that is not zero
 };
 
 // Axis-aligned grid production kernel (persistent, warp-refilled work).

@@ -212,7 +212,8 @@ __global__ void __launch_bounds__(256, 2) rta_prod_link(const __grid_constant__ 
         dt_lo = fix_flight(ef, tau_k, F.kt, dt_hi);
         nseg = 0;
         c.events++;
-        if (++nev > cap || tau_k <= 0.) stop(tau_k > 0. ? E_LIMIT : E_VALUE);
+        const long long tau_b = __double_as_longlong(tau_k);  // (its sign without the FP64 lanes)
+        if (++nev > cap || tau_b <= 0) stop(tau_b > 0 ? E_LIMIT : E_VALUE);
     };
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, !active && !done);
@@ -321,8 +322,7 @@ __global__ void __launch_bounds__(256, 2) rta_prod_link(const __grid_constant__ 
             }
             if (leave || q.bin_end) {
                 double* b = tally + 3ll * (box * T.nbins + bin);
-                const double t = double((long long)pt);
-                if (pt) atomicAdd(b + 0, flip ? -t : t);
+                if (pt) atomicAdd(b + 0, double(flip ? -(long long)pt : (long long)pt));
                 if (px) atomicAdd(b + 1, double((long long)px));
                 if (py) atomicAdd(b + 2, double((long long)py));
                 if (leave || part == last_part) c.tallies++;

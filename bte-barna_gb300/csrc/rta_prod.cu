@@ -318,7 +318,10 @@ __device__ int grid_generate(const DevTables& T, const DevGrid& G, const int2* b
 // busy; now the FP64 pipe only turns the three pending sums into doubles
 // (17 cycles each), and the kernel is bound by instruction issue: 2e6
 // particles of the porous transient (36864 modes, 2422 cells, 200 bins) take
-// 115 ms instead of 151, the 1e6-particle ribbon 4.04 instead of 4.51.  A lane
+// 106-111 ms instead of 144-152, the 1e6-particle ribbon 3.06 instead of 4.78.
+// Of 32 lanes 20 are active (57 % of the passes end in a draw, the others in a
+// flush, and a warp issues both), 456 instructions a pass, 62 % of the issue
+// slots taken.  A lane
 // flushes at most once per pass; a sum of zero (a mode without velocity) adds
 // nothing and is not sent.  The tally is left in the walk's units (ticks, and
 // position units), which the reader scales by powers of two.
@@ -329,7 +332,9 @@ __device__ int grid_generate(const DevTables& T, const DevGrid& G, const int2* b
 // alias table) and draws the next flight length there.
 //
 // ADJ selects the two passes of the adjoint (ADJ = 0 is the plain kernel),
-// which need no tally:
+// which need no tally.  Their FP64 sums bound them (84 % of the pipe in pass
+// 2) while every component of the functional was converted and weighted: a
+// functional of one component, 1e6 particles: 4.2 and 7.0 ms, now 3.3 and 4.0.
 // 1 forward: accumulates each particle's contribution to a linear functional
 //   Phi = sum W[box][bin][q] tally[box][bin][q] (W in the walk's units);
 // 2 adjoint: replays every particle from its Philox counter (the same draws
@@ -385,8 +390,8 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
     uint32_t nev = 0, npass = 0;
     double* tgrp = tally;  // the tally of the particle's replica group
     bool active = false, done = lane >= A.lanes;
-    // adjoint state: Phi so far, the particle's total, pending score terms
-    double phi_run = 0., phi_tot = 0., spec_score = 0.;
+    // adjoint state: Phi so far (pass 1) or still to come (pass 2), pending score terms
+    double phi_run = 0., spec_score = 0.;
     double sum_r = 0., g_p = 0., phi_all = 0.;
     long long slot = 0;
     int pend_kind = 0;
@@ -396,12 +401,19 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
         active = false;
         done = true;
     };
-    // The functional's part of the pending sums.
-    auto weighted = [&]() -> double {
+    // x plus or minus the functional's part of the pending sums: one conversion
+    // and one FMA for each component that has a weight at all (a loop: as three
+    // conditions they were predicated, and held the FP64 lanes all the same).
+    auto weighted = [&](double x, bool minus) -> double {
         const double* Wk = adj.W + 3ll * (box * T.nbins + bin);
-        const double t = double((long long)pt);
-        return __ldg(Wk) * (flip ? -t : t) + __ldg(Wk + 1) * double((long long)px) +
-               __ldg(Wk + 2) * double((long long)py);
+        const long long t = (flip != 0) != minus ? -(long long)pt : (long long)pt;
+#pragma unroll 1
+        for (int m = adj.comps; m; m &= m - 1) {
+            const int q = __ffs(m) - 1;
+            const long long d = q == 1 ? px : py;
+            x = fma(__ldg(Wk + q), double(q == 0 ? t : minus ? -d : d), x);
+        }
+        return x;
     };
     // A new free flight of the current mode from one random word:
     // dt = -tau ln u (FP32 log), u = (k + 1/2) 2^-23 from 23 bits, never 0
@@ -421,18 +433,21 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
         dt_lo = fix_flight(ef, tau_k, F.kt, dt_hi);
         c.events++;
         if (ADJ == 2) {
-            // future contribution from here: Phi_total - (flushed + pending part)
-            const double R = phi_tot - (phi_run + weighted());
+            // future contribution from here: what the flushes left of Phi_total
+            // less the pending part
+            const double R = weighted(phi_run, true);
             // the flight's (e - 1) / tau and, for a mode from a
-            // post-scattering draw, that draw's -1 / tau
-            const double gk = (widen_pos(ef) - ((pend_kind & 1) ? 2.0 : 1.0)) * (R * __ldg(T.w + mo + mode));
+            // post-scattering draw, that draw's -1 / tau (the 1 / tau of all a
+            // mode's flights: the reader's)
+            const double gk = (widen_pos(ef) - ((pend_kind & 1) ? 2.0 : 1.0)) * R;
             if (pend_kind & 1) sum_r += R;
             if (pend_kind & 2) g_p += spec_score * R;
             pend_kind = 0;
             atomicAdd(adj.g_tau + mode, gk);
         }
         // zero rate or runaway particle
-        if (++nev > cap || tau_k <= 0.) stop(tau_k > 0. ? E_LIMIT : E_VALUE);
+        const long long tau_b = __double_as_longlong(tau_k);  // (its sign without the FP64 lanes)
+        if (++nev > cap || tau_b <= 0) stop(tau_b > 0 ? E_LIMIT : E_VALUE);
     };
     for (;;) {
         // refill idle lanes of the warp with new particles; a lane is done when
@@ -469,9 +484,8 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
                         nev = npass = 0;
                         if (ADJ) {
                             slot = mine;
-                            phi_run = 0.;
+                            phi_run = ADJ == 2 ? adj.phi_total[mine] : 0.;
                             pend_kind = 0;
-                            if (ADJ == 2) phi_tot = adj.phi_total[mine];
                         }
                         bin = part = 0;
                         rb = __ldg(binw);
@@ -549,11 +563,10 @@ __global__ void __launch_bounds__(256, MINB) rta_prod_grid(DevTables T, GridArgs
             }
             if (leave || q.bin_end) {
                 if (ADJ) {
-                    phi_run += weighted();
+                    phi_run = weighted(phi_run, ADJ == 2);
                 } else {
                     double* b = tgrp + 3ll * (box * T.nbins + bin);
-                    const double t = double((long long)pt);
-                    if (pt) atomicAdd(b + 0, flip ? -t : t);
+                    if (pt) atomicAdd(b + 0, double(flip ? -(long long)pt : (long long)pt));
                     if (px) atomicAdd(b + 1, double((long long)px));
                     if (py) atomicAdd(b + 2, double((long long)py));
                 }
@@ -1405,9 +1418,9 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A0, double* tally,
                                  int(smem)) != cudaSuccess)
             return false;
     } else if (adj_pass == 1) {
-        fn = reinterpret_cast<const void*>(rta_prod_grid<false, 2, 1>);
+        fn = reinterpret_cast<const void*>(rta_prod_grid<false, 3, 1>);
     } else if (adj_pass == 2) {
-        fn = reinterpret_cast<const void*>(rta_prod_grid<false, 2, 2>);
+        fn = reinterpret_cast<const void*>(rta_prod_grid<false, 3, 2>);
     } else if (threads * bps > 768) {  // the register cap follows the resident threads
         fn = reinterpret_cast<const void*>(rta_prod_grid<false, 4, 0>);
     } else if (threads * bps > 512) {
@@ -1427,9 +1440,9 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A0, double* tally,
     if (use_smem)
         rta_prod_grid<true, 1, 0><<<nb, threads, smem, s>>>(T, A, tally, counters, err, work, aa);
     else if (adj_pass == 1)
-        rta_prod_grid<false, 2, 1><<<nb, threads, 0, s>>>(T, A, tally, counters, err, work, aa);
+        rta_prod_grid<false, 3, 1><<<nb, threads, 0, s>>>(T, A, tally, counters, err, work, aa);
     else if (adj_pass == 2)
-        rta_prod_grid<false, 2, 2><<<nb, threads, 0, s>>>(T, A, tally, counters, err, work, aa);
+        rta_prod_grid<false, 3, 2><<<nb, threads, 0, s>>>(T, A, tally, counters, err, work, aa);
     else if (fn == reinterpret_cast<const void*>(rta_prod_grid<false, 4, 0>))
         rta_prod_grid<false, 4, 0><<<nb, threads, 0, s>>>(T, A, tally, counters, err, work, aa);
     else if (fn == reinterpret_cast<const void*>(rta_prod_grid<false, 3, 0>))
