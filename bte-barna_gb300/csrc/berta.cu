@@ -166,37 +166,52 @@ __device__ __forceinline__ int grid_at(const DevGrid& G, int i, int j) {
 
 // Ballistic advection of one particle for time `dt` on the grid.  Returns
 // false when it was absorbed (mode set to -1): at a void wall its signed
-// count goes to the wall's Eborder, at a reservoir it is dropped.
+// count goes to the wall's Eborder, at a reservoir it is dropped.  The end of
+// the flight is tried first and its coordinates compared with the cell's
+// borders as integers; only a crossing computes an exit time, and two only
+// where both coordinates leave: 12 FP64 instructions a warp and step where
+// both exit times at every cell were 21 (17 cycles of the SM's FP64 lanes
+// each).
 __device__ bool advect_one(const DevGrid& G, const int2* boxcell, const ModeVel* mv, const int4* boxwall,
                            int* Eb, double& x, double& y, int& box, int mode, int sign, double dt) {
     const ModeVel v = mv[mode];
     const int2 ij = __ldg(boxcell + box);
     int i = ij.x, j = ij.y;
+    const int upx = obits(v.vx) >= 0 ? 1 : 0, upy = obits(v.vy) >= 0 ? 1 : 0;
     for (int guard = 0; guard < (1 << 20); ++guard) {
-        const int upx = obits(v.vx) >= 0 ? 1 : 0, upy = obits(v.vy) >= 0 ? 1 : 0;
         const double xw = __ldg(G.gx + i + upx), yw = __ldg(G.gy + j + upy);
-        const double tx = (xw - x) * v.ivx, ty = (yw - y) * v.ivy;
-        const bool xfirst = obits(tx) <= obits(ty);
-        const long long te_b = xfirst ? obits(tx) : obits(ty);
-        if (!(obits(dt) > te_b)) {  // stays in the cell
-            x = fma(dt, v.vx, x);
-            y = fma(dt, v.vy, y);
+        const double xe = fma(dt, v.vx, x), ye = fma(dt, v.vy, y);
+        const bool outx = upx ? order_key(xe) > order_key(xw) : order_key(xe) < order_key(xw);
+        const bool outy = upy ? order_key(ye) > order_key(yw) : order_key(ye) < order_key(yw);
+        if (!(outx || outy)) {  // stays in the cell
+            x = xe;
+            y = ye;
             return true;
         }
-        const double seg = __longlong_as_double(te_b > 0 ? te_b : 0);
-        double nx = fma(seg, v.vx, x), ny = fma(seg, v.vy, y);
+        double seg = ((outx ? xw : yw) - (outx ? x : y)) * (outx ? v.ivx : v.ivy);
+        bool xfirst = outx;
+        if (outx && outy) {
+            const double ty = (yw - y) * v.ivy;
+            if (obits(ty) < obits(seg)) {
+                xfirst = false;
+                seg = ty;
+            }
+        }
+        if (obits(seg) < 0) seg = 0.;
+        if (obits(seg) > obits(dt)) seg = dt;
+        const double along = fma(seg, xfirst ? v.vy : v.vx, xfirst ? y : x);
         int ni = i, nj = j, wall;
         if (xfirst) {
-            nx = xw;
+            x = xw;
+            y = along;
             ni = i + (upx ? 1 : -1);
             wall = upx ? 0 : 1;
         } else {
-            ny = yw;
+            x = along;
+            y = yw;
             nj = j + (upy ? 1 : -1);
             wall = upy ? 2 : 3;
         }
-        x = nx;
-        y = ny;
         dt -= seg;
         const int nb = grid_at(G, ni, nj);
         if (nb >= 0) {
@@ -764,15 +779,29 @@ constexpr unsigned BRANCH_CAP = 1u << 20;
 // outgoing particle, appended to `out`.  Each warp takes an equal run of the
 // particles; a lane whose parent owes no more attempts takes the run's next
 // one, a parent absorbed during its advection owes none.  Outgoing particles
-// gather in the warp's part of shared memory and leave 128 or more at a time,
+// gather in the warp's part of shared memory and leave 97 or more at a time,
 // with one claim of places: claims of parents and places 32 at a time, on
 // two counters of one cache line, came to 82 000 atomics on it per launch of
 // 1.3e6 particles and bounded the kernel (103 us a launch).
-constexpr int ADV_BUF = 160;
+//
+// Bound by the latency of its reads: a lane's next particle, its mode's
+// velocity and its column's alias slot (one of 301 MB for 6141 modes).  The
+// particles arrive in shared memory a chunk of 32 ahead (cp.async), and the
+// first draw of a parent, which needs only its mode, is read before the
+// advection: 70 -> 61 us for 1.3e6 particles, with the exits of advect_one.
+constexpr int ADV_BUF = 128, ADV_IN = 64;
 struct AdvBuf {
     double x[ADV_BUF], y[ADV_BUF];
     int mode[ADV_BUF], box[ADV_BUF], sign[ADV_BUF];
+    double ix[ADV_IN], iy[ADV_IN];
+    int imode[ADV_IN], ibox[ADV_IN], isign[ADV_IN];
 };
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(BYTES)
+                 : "memory");
+}
 template <bool GENERAL, bool RTA>
 __global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
     be_advance(PArr in, const unsigned long long* n_in, PArr out, unsigned long long* dc, long long ocap, int advect,
@@ -788,8 +817,23 @@ __global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
     }
     // the warp's run, in whole chunks of 32
     const long long warps = (long long)gridDim.x * 8, per = ((n + 31) / 32 + warps - 1) / warps * 32;
-    long long next = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * per;
-    const long long end = min(n, next + per);
+    const long long start = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * per, end = min(n, start + per);
+    // of the run: taken, asked for (the ring holds the last ADV_IN) and arrived
+    long long next = start, asked = start, here = start;
+    auto ask = [&] {
+        const long long i = asked + lane;
+        if (i < end) {
+            const int k = int(i & (ADV_IN - 1));
+            copy_async<8>(buf.ix + k, in.x + i);
+            copy_async<8>(buf.iy + k, in.y + i);
+            copy_async<4>(buf.imode + k, in.mode + i);
+            copy_async<4>(buf.ibox + k, in.box + i);
+            copy_async<4>(buf.isign + k, in.sign + i);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asked += 32;
+    };
+    for (int k = 0; k < ADV_IN / 32; ++k) ask();
     unsigned long long flips = 0;
     int mode = 0, sign = 1, box = 0, col = 0, cnt = 0;
     double x = 0., y = 0.;
@@ -797,6 +841,17 @@ __global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
     bool valid = false;
     Philox g;
     g.init(skey, 0);
+    int slot = 0;
+    float acc = 0.f, eprob = 0.f;
+    unsigned ealt = 0;
+    // one attempt's alias slot of the parent's column
+    auto draw_slot = [&](const PAlias* tab) {
+        slot = int(mulhi32(g.next32(), uint32_t(nm)));
+        acc = float(g.next32() >> 8) * 0x1p-24f;
+        const PAlias e = tab[(long long)col * nm + slot];
+        eprob = e.prob;
+        ealt = e.alt;
+    };
     auto flush = [&] {
         __syncwarp();
         unsigned long long base = 0;
@@ -820,15 +875,40 @@ __global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
     };
     for (;;) {
         const unsigned idle = __ballot_sync(0xffffffffu, todo == 0);
+        const long long upto = next + __popc(idle);
+        if (upto > here) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            here = asked;
+            __syncwarp();
+        }
         if (todo == 0) {
             const long long i = next + __popc(idle & ((1u << lane) - 1u));
             if (i < end) {
-                mode = in.mode[i];
+                const int k = int(i & (ADV_IN - 1));
+                mode = buf.imode[k];
                 if (mode >= 0) {
-                    sign = in.sign[i];
-                    box = in.box[i];
-                    x = in.x[i];
-                    y = in.y[i];
+                    sign = buf.isign[k];
+                    box = buf.ibox[k];
+                    x = buf.ix[k];
+                    y = buf.iy[k];
+                    g.init(skey, (uint64_t)i);
+                    if (RTA) {
+                        slot = mode;
+                        if ((g.next() >> 11) < __ldg(pscat + mode)) {
+                            slot = int(mulhi32(g.next32(), uint32_t(nmodes)));
+                            acc = float(g.next32() >> 8) * 0x1p-24f;
+                            const int2 e = __ldg(resample + slot);
+                            eprob = __int_as_float(e.x);
+                            ealt = unsigned(e.y);
+                        } else {
+                            acc = 0.f;
+                            eprob = 1.f;
+                        }
+                    } else {
+                        col = mode - 3;
+                        valid = col >= 0 && col < nm;
+                        if (pal && valid) draw_slot(pal);
+                    }
                     bool alive = true;
                     if (advect) {
                         if (GENERAL) {
@@ -842,17 +922,16 @@ __global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
                         }
                     }
                     if (alive) {
-                        col = mode - 3;
-                        valid = RTA ? true : (col >= 0 && col < nm);
-                        if (!valid) atomicCAS(err, 0, E_VALUE);
-                        g.init(skey, (uint64_t)i);
+                        if (!RTA && !valid) atomicCAS(err, 0, E_VALUE);
                         todo = 1;
                         made = 0;
                     }
                 }
             }
         }
-        next += __popc(idle);
+        __syncwarp();
+        if (upto >= asked - (ADV_IN - 32)) ask();  // the older chunk has been taken
+        next = upto;
         const bool act = todo > 0;
         const unsigned m1 = __ballot_sync(0xffffffffu, act);
         if (!m1) {
@@ -862,23 +941,16 @@ __global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
         if (act) {
             int nmode = mode, nsign = sign;
             if (RTA) {
-                if ((g.next() >> 11) < __ldg(pscat + mode)) {
-                    const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
-                    const float acc = float(g.next32() >> 8) * 0x1p-24f;
-                    const int2 e = __ldg(resample + j);
-                    nmode = acc < __int_as_float(e.x) ? j : e.y;
-                }
+                nmode = acc < eprob ? slot : int(ealt);
             } else if (valid) {
                 // one table for every box (pal), or the box's own
                 const PAlias* tab = pal ? pal : bprop[box].alias;
                 if (tab) {
-                    const int j = int(mulhi32(g.next32(), uint32_t(nm)));
-                    const float acc = float(g.next32() >> 8) * 0x1p-24f;
-                    const PAlias e = tab[(long long)col * nm + j];
-                    const bool keep = acc < e.prob;
-                    const int slot = keep ? j : int(e.alt & 0x3fffffffu);
-                    const bool neg = keep ? (e.alt >> 31) != 0u : ((e.alt >> 30) & 1u) != 0u;
-                    nmode = slot + 3;
+                    if (!pal || made) draw_slot(tab);
+                    const bool keep = acc < eprob;
+                    const int to = keep ? slot : int(ealt & 0x3fffffffu);
+                    const bool neg = keep ? (ealt >> 31) != 0u : ((ealt >> 30) & 1u) != 0u;
+                    nmode = to + 3;
                     nsign = neg ? -sign : sign;
                 } else {
                     const BoxProp bp = bprop[box];

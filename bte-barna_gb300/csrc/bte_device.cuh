@@ -371,9 +371,25 @@ struct GBox {
 
 // A double as a signed integer with the same order (no NaN; the two zeros are
 // one value), so that comparisons run on the integer units.
+// The halves are taken apart: on the whole word the compiler finds the absolute
+// value, or a test for zero, and makes an FP64 instruction of it.
+BTE_HD uint64_t magnitude_bits(double x) {
+#if defined(__CUDA_ARCH__)
+    return (uint64_t(uint32_t(__double2hiint(x)) & 0x7fffffffu) << 32) | uint32_t(__double2loint(x));
+#else
+    return dbits(x) & 0x7fffffffffffffffULL;
+#endif
+}
+BTE_HD int sign_mask(double x) {  // 0 or -1
+#if defined(__CUDA_ARCH__)
+    return __double2hiint(x) >> 31;
+#else
+    return int(int64_t(dbits(x)) >> 63);
+#endif
+}
 BTE_HD long long order_key(double x) {
-    const long long b = (long long)dbits(x);
-    return (b << 1) == 0 ? 0 : b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+    const long long s = sign_mask(x);
+    return ((long long)magnitude_bits(x) ^ s) - s;
 }
 
 // An axis-aligned rectangular box as order keys of its bounds; x0 > x1: any

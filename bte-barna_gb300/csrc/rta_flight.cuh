@@ -283,20 +283,22 @@ static __device__ __noinline__ bool get_inter_rect(const DevTables& T, int box, 
     bool found = false;
     for (int id = 0; id < B.nborders; ++id) {
         const GBorder& b = T.borders[B.border_off + id];
-        const bool vert = (dbits(b.np.x) << 1) != 0;  // a line of constant x
-        const uint64_t nv = vert ? dbits(b.np.x) ^ dbits(v.x) : dbits(b.np.y) ^ dbits(v.y);
-        const uint64_t va = vert ? dbits(v.x) : dbits(v.y);
-        if ((nv >> 63) || (va << 1) == 0) continue;  // n.v > 0 only
+        const bool vert = magnitude_bits(b.np.x) != 0;  // a line of constant x
+        const double nn = vert ? b.np.x : b.np.y, vn = vert ? v.x : v.y;
+        if (sign_mask(nn) != sign_mask(vn) || magnitude_bits(vn) == 0) continue;  // n.v > 0 only
         const V2 w = sub(b.la, r0);
         const double d2 = vert ? b.lb.y - b.la.y : b.lb.x - b.la.x;
         const double wn = vert ? w.x : w.y;
         const double a = (vert ? d1.x : d1.y) * d2, c = wn * d2;
         const double den = vert ? a : -a, nt = vert ? c : -c;  // cross(d1, d2), cross(w, d2)
-        if ((dbits(den) << 1) == 0) continue;
+        const uint64_t md = magnitude_bits(den);
+        if (md == 0) continue;
         // 0 <= nt / den <= 1
-        if ((dbits(nt) << 1) != 0 && (((dbits(nt) ^ dbits(den)) >> 63) || (dbits(nt) << 1) > (dbits(den) << 1))) continue;
+        const uint64_t mt = magnitude_bits(nt);
+        if (mt != 0 && (sign_mask(nt) != sign_mask(den) || mt > md)) continue;
         const double nu = cross(w, d1);
-        if ((dbits(nu) << 1) != 0 && (((dbits(nu) ^ dbits(den)) >> 63) || (dbits(nu) << 1) > (dbits(den) << 1))) continue;
+        const uint64_t mu = magnitude_bits(nu);
+        if (mu != 0 && (sign_mask(nu) != sign_mask(den) || mu > md)) continue;
         // r0 on the border line: the general test
         if (order_key(vert ? r0.x : r0.y) == order_key(vert ? b.la.x : b.la.y) && on_segment(r0, b.la, b.lb)) continue;
         const double u = nu / den;

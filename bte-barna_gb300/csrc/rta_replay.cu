@@ -130,7 +130,7 @@ __device__ __forceinline__ void record_error_r(int* err, int e, long long pid) {
 // active lane as for 32: with one particle per thread two lanes of a warp were
 // active on average.  1e5 particles on a ribbon of 20 cells and 1536 modes took
 // 58.2 ms; with this loop and evolparticle's comparisons on the integer units,
-// 9.5.
+// 8.4.
 __global__ void __launch_bounds__(128) rta_replay_kernel(const __grid_constant__ DevTables T, unsigned long long* ex,
                                                          unsigned long long* counters, int* err,
                                                          unsigned long long* work) {
