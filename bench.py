@@ -338,7 +338,7 @@ def run_berta(args, rank, world, local):
                 "d2h_bytes_per_step": (nsteps + 1) * (nbx * 3 + 1) * 8},
         "kernel_ms_per_step": kern_ms / args.steps,
         # device time of the reference's timer buckets per 100-step run
-        # (CUDA events at the phase borders of every step)
+        # (clock stamps at the phase borders of every step)
         "phase_ms_per_step": {ph: v / args.steps for ph, v in phase_sum.items()},
         "roofline": {"bound": "hbm", "kernel": "be_advance", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind + " (copy burst)",

@@ -8,13 +8,13 @@
 //   2 gradient source term: Nabla_T particles at random points of every box
 //     with a gradient, random sub-step (source_term_gradient :597-676,
 //     Nabla_T_distribution src/sampling.cpp:118-187)
-//                                                   be_plan, be_generate_dev
+//                                                   be_plan, be_advance
 //   3 isothermal-wall injection, random sub-step (Isothermal_walls :446-585,
 //     Ntogenerate src/sampling.cpp:243-260)
-//                                                   be_plan, be_generate_dev
+//                                                   be_plan, be_advance
 //   4 adiabatic diffuse re-emission of |Eborder| at the wall temperature from
 //     the J(T) cubic spline (adiabatic_diffuse_walls :281-435)
-//                                      be_plan, be_wall_cdf, be_generate_dev
+//                                                   be_plan, be_advance
 //   5 deletion of the absorbed particles, 6 propagator scattering with sign
 //     branching (Scattering :1073-1210, propagator_H::get
 //     src/collision_operator.cpp:892-903), each parent's branching attempts
@@ -127,19 +127,19 @@ struct BertaState {
     DBuf a_x, a_y, a_mode, a_box, a_sign;   // particles
     DBuf b_x, b_y, b_mode, b_box, b_sign;   // compaction / scattering output
     DBuf d_H, d_cnt, d_Eb, d_props, d_boxwall, d_gens, d_alias, d_rvx, d_rvy;
-    DBuf d_om, d_vx, d_vy, d_req, d_cdf, d_isoprob, d_isoalt;
+    DBuf d_om, d_vx, d_vy, d_cdf, d_isoprob, d_isoalt;
     DBuf d_gprob, d_galt, d_gsign;          // gradient source rows
     DBuf d_ctot;                            // wall-CDF chunk sums
     Pinned h_gens[1];                       // staging: descriptors of the initial particles
     // device-resident step loop: counters, planned sources, per-step records
     DBuf d_dc, d_span, d_gdesc, d_ggenf, d_gcnt, d_idesc, d_igenf, d_icnt, d_adi, d_adesc, d_acnt;
+    DBuf d_H2, d_stamps;
     DBuf d_phist, d_nhist, d_res, d_rank, d_pscat, d_sa, d_sb, d_sc, d_sd, d_sx0, d_sxs;
 
     // what a run takes from the tables alone, kept while they stay: sources,
-    // adiabatic borders and their splines (BertaPlan); the phase events
+    // adiabatic borders and their splines (BertaPlan)
     BertaPlan* plan = nullptr;
     DBuf d_wallreq, d_wallsum;
-    std::vector<cudaEvent_t> events;
     ~BertaState();
 };
 
@@ -463,11 +463,9 @@ __global__ void __launch_bounds__(256) be_wall_sums(const double* om, const doub
 // Threads take segments, and the segments' totals are scanned by warps (one
 // thread adding 256 totals in a row took 9 of this kernel's 22 us).
 __device__ __forceinline__ void wall_cdf_body(const float* om, const float* vx, const float* vy, int n,
-                                              const WallReq* req, double* cdf, double* chunk_tot) {
+                                              const WallReq& R, int r, int ch, double* cdf, double* chunk_tot) {
     __shared__ double wsum[8];
     const int nch = (n + WCDF_CHUNK - 1) / WCDF_CHUNK;
-    const int r = blockIdx.x / nch, ch = blockIdx.x % nch;
-    const WallReq R = req[r];
     double* row = cdf + (long long)r * n;
     const int c0 = ch * WCDF_CHUNK, c1 = min(n, c0 + WCDF_CHUNK);
     constexpr int SEG = WCDF_CHUNK / 256;
@@ -501,7 +499,7 @@ __device__ __forceinline__ void wall_cdf_body(const float* om, const float* vx, 
 #pragma unroll
     for (int j = 0; j < SEG; ++j)
         if (k0 + j < c1) row[k0 + j] = run[j] + off;
-    if (threadIdx.x == 255) chunk_tot[blockIdx.x] = off + acc;
+    if (threadIdx.x == 255) chunk_tot[r * nch + ch] = off + acc;
 }
 
 // A mode of row r by inversion: u times the row's total, its chunk, and the
@@ -696,6 +694,39 @@ __device__ __forceinline__ void cancel_body(PArr P, long long n, const int* H, i
     }
 }
 
+// The device's clock in ns, written at the phase borders of a step: an event
+// between two kernels kept the stream for 2 us (seven were 14 of a step's 150).
+struct Stamps {
+    // the starts of the advance, the plan, the new particles' pass, the
+    // cancellation and the properties; the histogram read; the step's end
+    unsigned long long t[7];
+};
+// A step's kernels follow one another without a gap: each is launched as its
+// predecessor's blocks end (after_previous) and reads nothing before that one
+// is done.  With the 4 or 6 launches of a step 3.72 -> 3.37 ms for 30 steps of
+// the propagator, 2.89 -> 2.45 for 40 of RTA; launched as soon as all the
+// predecessor's blocks run (launch_dependents), 4.0 and 2.58: the waiting
+// blocks take room on the SMs from the ones that work.
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+void after_previous(void (*f)(P...), unsigned blocks, cudaStream_t s, A&&... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    ck(cudaLaunchKernelEx(&cfg, f, P(args)...), "step launch");
+}
+__device__ __forceinline__ void stamp(unsigned long long* t) {
+    unsigned long long v;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(v));
+    *t = v;
+}
+
 // ed, flux_x, flux_y sums of every box (raw velocities, as calculate_prop)
 // into a cleared row, PROPS_PARTS blocks per box (one block per box took 25 us
 // of a step); the first thread closes the step (close_step).
@@ -718,19 +749,28 @@ __device__ __forceinline__ void close_step(unsigned long long* dc, int swap, lon
 }
 
 __global__ void __launch_bounds__(256) be_props(const int* H, int nmodes, const double* vx, const double* vy, double* out,
-                                                unsigned long long* dc, int swap, long long* record) {
+                                                unsigned long long* dc, int swap, long long* record, int* next_H,
+                                                int* next_cnt, int* old_Eb, int nborders, Stamps* st) {
+    await_previous();
+    if (st && blockIdx.x == 0 && threadIdx.x == 0) stamp(st->t + 4);
+    for (int k = blockIdx.x * 256 + threadIdx.x; k < nborders; k += gridDim.x * 256) old_Eb[k] = 0;
     const int box = blockIdx.x / PROPS_PARTS, part = blockIdx.x % PROPS_PARTS;
     const int len = (nmodes + PROPS_PARTS - 1) / PROPS_PARTS, k1 = min(nmodes, (part + 1) * len);
     long long e = 0;
     double fx = 0., fy = 0.;
     for (int k = part * len + threadIdx.x; k < k1; k += 256) {
         const int hi = H[(long long)box * nmodes + k];
+        if (next_H) {  // the next step's histogram and ranks start from zero
+            next_H[(long long)box * nmodes + k] = 0;
+            next_cnt[(long long)box * nmodes + k] = 0;
+        }
         if (hi == 0) continue;
         const double h = double(hi);
         e += hi;
         fx += h * vx[k];
         fy += h * vy[k];
     }
+    if (st && blockIdx.x == 0 && threadIdx.x == 0) stamp(st->t + 5);
     __shared__ double red[3][8];
     for (int o = 16; o > 0; o >>= 1) {
         e += __shfl_down_sync(0xffffffffu, e, o);
@@ -748,7 +788,10 @@ __global__ void __launch_bounds__(256) be_props(const int* H, int nmodes, const 
         for (int w = 0; w < 8; ++w) v += red[threadIdx.x][w];
         if (v != 0.) atomicAdd(out + 3 * box + threadIdx.x, v);
     }
-    if (record && blockIdx.x == 0 && threadIdx.x == 0) close_step(dc, swap, record);
+    if (record && blockIdx.x == 0 && threadIdx.x == 0) {
+        close_step(dc, swap, record);
+        stamp(st->t + 6);
+    }
 }
 
 // A source planned on the device: where its particles start in the
@@ -756,237 +799,6 @@ __global__ void __launch_bounds__(256) be_props(const int* H, int nmodes, const 
 struct SrcSpan {
     unsigned long long base, total;
 };
-
-// Propagator scattering with sign branching (Scattering,
-// src/beyondRTA_MC2d.cpp:1073-1210): every scattering attempt of a parent
-// draws its next mode from the parent's column (an alias table over |P|
-// with the signs in the alias word, or, for an interpolated propagator, the
-// signed CDF probed as propagator_H::lower_bound does) and emits one
-// outgoing particle; when the drawn sign differs from the parent's, the
-// reference puts two copies of the parent back into the queue, and each
-// copy makes an attempt of its own.  The copies are identical to the
-// parent, so a thread keeps only the number of attempts its parent still
-// owes and makes them in place, with fresh draws.  BRANCH_CAP bounds the
-// attempts of one parent (a supercritical propagator never stops).
-constexpr unsigned BRANCH_CAP = 1u << 20;
-
-// One step of the particles [0, *n_in) of `in`, fused: advection by the
-// step (advect = 1; particles born in this step were advected when they were
-// made), then the scattering of the survivors -- RTA (ScatteringRTA,
-// src/beyondRTA_MC2d.cpp:983-1062, a resampling with probability
-// 1 - exp(-w dt), as a 53-bit threshold per mode) or the propagator with sign
-// branching as above -- and the histogram H[box][mode] += sign of every
-// outgoing particle, appended to `out`.  Each warp takes an equal run of the
-// particles; a lane whose parent owes no more attempts takes the run's next
-// one, a parent absorbed during its advection owes none.  Outgoing particles
-// gather in the warp's part of shared memory and leave 97 or more at a time,
-// with one claim of places: claims of parents and places 32 at a time, on
-// two counters of one cache line, came to 82 000 atomics on it per launch of
-// 1.3e6 particles and bounded the kernel (103 us a launch).
-//
-// Bound by the latency of its reads: a lane's next particle, its mode's
-// velocity and its column's alias slot (one of 301 MB for 6141 modes).  The
-// particles arrive in shared memory a chunk of 32 ahead (cp.async), and the
-// first draw of a parent, which needs only its mode, is read before the
-// advection: 70 -> 61 us for 1.3e6 particles, with the exits of advect_one.
-constexpr int ADV_BUF = 128, ADV_IN = 64;
-struct AdvBuf {
-    double x[ADV_BUF], y[ADV_BUF];
-    int mode[ADV_BUF], box[ADV_BUF], sign[ADV_BUF];
-    double ix[ADV_IN], iy[ADV_IN];
-    int imode[ADV_IN], ibox[ADV_IN], isign[ADV_IN];
-};
-template <int BYTES>
-__device__ __forceinline__ void copy_async(void* dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
-                 "n"(BYTES)
-                 : "memory");
-}
-template <bool GENERAL, bool RTA>
-__global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
-    be_advance(PArr in, const unsigned long long* n_in, PArr out, unsigned long long* dc, long long ocap, int advect,
-               const __grid_constant__ AdvectArgs aa, const PAlias* pal, const BoxProp* bprop, int nm,
-               const unsigned long long* pscat, const int2* resample, int nmodes, unsigned long long skey, int* H, int* err) {
-    __shared__ AdvBuf bufs[8];
-    AdvBuf& buf = bufs[threadIdx.x >> 5];
-    const long long n = min((long long)*n_in, ocap);  // places beyond the buffers (an overflow) are not read
-    const int lane = threadIdx.x & 31;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
-        if (advect) atomicAdd(dc + DC_PSTEPS, (unsigned long long)n);
-        atomicAdd(dc + DC_IN, (unsigned long long)n);
-    }
-    // the warp's run, in whole chunks of 32
-    const long long warps = (long long)gridDim.x * 8, per = ((n + 31) / 32 + warps - 1) / warps * 32;
-    const long long start = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * per, end = min(n, start + per);
-    // of the run: taken, asked for (the ring holds the last ADV_IN) and arrived
-    long long next = start, asked = start, here = start;
-    auto ask = [&] {
-        const long long i = asked + lane;
-        if (i < end) {
-            const int k = int(i & (ADV_IN - 1));
-            copy_async<8>(buf.ix + k, in.x + i);
-            copy_async<8>(buf.iy + k, in.y + i);
-            copy_async<4>(buf.imode + k, in.mode + i);
-            copy_async<4>(buf.ibox + k, in.box + i);
-            copy_async<4>(buf.isign + k, in.sign + i);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asked += 32;
-    };
-    for (int k = 0; k < ADV_IN / 32; ++k) ask();
-    unsigned long long flips = 0;
-    int mode = 0, sign = 1, box = 0, col = 0, cnt = 0;
-    double x = 0., y = 0.;
-    unsigned todo = 0, made = 0;
-    bool valid = false;
-    Philox g;
-    g.init(skey, 0);
-    int slot = 0;
-    float acc = 0.f, eprob = 0.f;
-    unsigned ealt = 0;
-    // one attempt's alias slot of the parent's column
-    auto draw_slot = [&](const PAlias* tab) {
-        slot = int(mulhi32(g.next32(), uint32_t(nm)));
-        acc = float(g.next32() >> 8) * 0x1p-24f;
-        const PAlias e = tab[(long long)col * nm + slot];
-        eprob = e.prob;
-        ealt = e.alt;
-    };
-    auto flush = [&] {
-        __syncwarp();
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(dc + DC_NOUT, (unsigned long long)cnt);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        for (int j = lane; j < cnt; j += 32) {
-            const long long o = (long long)base + j;
-            if (o < ocap) {
-                out.x[o] = buf.x[j];
-                out.y[o] = buf.y[j];
-                out.mode[o] = buf.mode[j];
-                out.box[o] = buf.box[j];
-                out.sign[o] = buf.sign[j];
-                atomicAdd(H + (long long)buf.box[j] * nmodes + buf.mode[j], buf.sign[j]);
-            } else {
-                atomicCAS(err, 0, E_LIMIT);
-            }
-        }
-        cnt = 0;
-        __syncwarp();
-    };
-    for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, todo == 0);
-        const long long upto = next + __popc(idle);
-        if (upto > here) {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            here = asked;
-            __syncwarp();
-        }
-        if (todo == 0) {
-            const long long i = next + __popc(idle & ((1u << lane) - 1u));
-            if (i < end) {
-                const int k = int(i & (ADV_IN - 1));
-                mode = buf.imode[k];
-                if (mode >= 0) {
-                    sign = buf.isign[k];
-                    box = buf.ibox[k];
-                    x = buf.ix[k];
-                    y = buf.iy[k];
-                    g.init(skey, (uint64_t)i);
-                    if (RTA) {
-                        slot = mode;
-                        if ((g.next() >> 11) < __ldg(pscat + mode)) {
-                            slot = int(mulhi32(g.next32(), uint32_t(nmodes)));
-                            acc = float(g.next32() >> 8) * 0x1p-24f;
-                            const int2 e = __ldg(resample + slot);
-                            eprob = __int_as_float(e.x);
-                            ealt = unsigned(e.y);
-                        } else {
-                            acc = 0.f;
-                            eprob = 1.f;
-                        }
-                    } else {
-                        col = mode - 3;
-                        valid = col >= 0 && col < nm;
-                        if (pal && valid) draw_slot(pal);
-                    }
-                    bool alive = true;
-                    if (advect) {
-                        if (GENERAL) {
-                            BePol pol;
-                            pol.g.init(aa.gkey, (uint64_t)i);
-                            int e = 0;
-                            alive = advect_general(aa.T, pol, aa.Eb, x, y, box, mode, sign, aa.dt, e);
-                            if (e && aa.err) atomicCAS(aa.err, 0, e);
-                        } else {
-                            alive = advect_one(aa.G, aa.boxcell, aa.mv, aa.boxwall, aa.Eb, x, y, box, mode, sign, aa.dt);
-                        }
-                    }
-                    if (alive) {
-                        if (!RTA && !valid) atomicCAS(err, 0, E_VALUE);
-                        todo = 1;
-                        made = 0;
-                    }
-                }
-            }
-        }
-        __syncwarp();
-        if (upto >= asked - (ADV_IN - 32)) ask();  // the older chunk has been taken
-        next = upto;
-        const bool act = todo > 0;
-        const unsigned m1 = __ballot_sync(0xffffffffu, act);
-        if (!m1) {
-            if (next >= end) break;
-            continue;
-        }
-        if (act) {
-            int nmode = mode, nsign = sign;
-            if (RTA) {
-                nmode = acc < eprob ? slot : int(ealt);
-            } else if (valid) {
-                // one table for every box (pal), or the box's own
-                const PAlias* tab = pal ? pal : bprop[box].alias;
-                if (tab) {
-                    if (!pal || made) draw_slot(tab);
-                    const bool keep = acc < eprob;
-                    const int to = keep ? slot : int(ealt & 0x3fffffffu);
-                    const bool neg = keep ? (ealt >> 31) != 0u : ((ealt >> 30) & 1u) != 0u;
-                    nmode = to + 3;
-                    nsign = neg ? -sign : sign;
-                } else {
-                    const BoxProp bp = bprop[box];
-                    if (bp.c1) {
-                        const long long off = (long long)col * nm;
-                        const int im = lower_bound_abs_lirp(bp.c1 + off, bp.c2 + off, nm, g.uniform(), bp.T, bp.T1, bp.T2);
-                        nmode = im + 3;
-                        nsign = lirp_at(bp.c1 + off, bp.c2 + off, im, bp.T, bp.T1, bp.T2) > 0. ? sign : -sign;
-                    } else {
-                        atomicCAS(err, 0, E_VALUE);  // a particle where nothing scatters
-                    }
-                }
-            }
-            const int o = cnt + __popc(m1 & ((1u << lane) - 1u));
-            buf.x[o] = x;
-            buf.y[o] = y;
-            buf.box[o] = box;
-            buf.mode[o] = nmode;
-            buf.sign[o] = nsign;
-            --todo;
-            if (!RTA && nsign != sign) {
-                todo += 2;
-                ++flips;
-            }
-            if (++made >= BRANCH_CAP) {
-                atomicCAS(err, 0, E_LIMIT);
-                todo = 0;
-            }
-        }
-        cnt += __popc(m1);
-        if (cnt > ADV_BUF - 32) flush();
-    }
-    if (cnt) flush();
-    for (int o = 16; o > 0; o >>= 1) flips += __shfl_down_sync(0xffffffffu, flips, o);
-    if (lane == 0 && flips) atomicAdd(dc + DC_FLIPS, flips);
-}
 
 // u < 1 - exp(-w dt) for u = k 2^-53 as k < pscat.
 __global__ void be_thresholds(const double* w, double dt, int n, unsigned long long* pscat) {
@@ -1078,15 +890,41 @@ struct SourceSets {
     unsigned long long pkey[2];  // of the stochastic rounding
 };
 
-// The step's sources, one block.  Gradient and isothermal walls: the numbers by
-// Ntogenerate's stochastic rounding (src/sampling.cpp:166-183, :243-260), one
-// Philox block per source.  Adiabatic walls (src/beyondRTA_MC2d.cpp:294-350):
-// each re-emitting border re-emits |Eborder| particles at the temperature
-// whose isothermal flux carries its absorbed energy (spline of J), one
-// distribution request per border; Eborder starts again from zero.
-__global__ void __launch_bounds__(256) be_plan(const __grid_constant__ SourceSets Q, int* Eb, const AdiBorder* ab, SplineDev S,
-                                               double Eeff, double dtstep, double thickness, WallReq* req,
-                                               unsigned long long* dc, SrcSpan* span, long long cap, int* err) {
+// The temperature whose isothermal flux carries the energy that border A
+// absorbed in E particles (spline of J, src/beyondRTA_MC2d.cpp:294-350).
+struct WallPlan {
+    double Eeff, dtstep, thickness;
+    SplineDev S;
+    const AdiBorder* ab;
+    const float *om, *vx, *vy;   // the modes, in FP32
+    double *cdf, *chunk_tot;     // the borders' rows
+};
+__device__ __forceinline__ double wall_temperature(const WallPlan& W, const AdiBorder& A, int E) {
+    return spline_eval(W.S, A.spline, W.Eeff * E / W.dtstep / (A.len * W.thickness));
+}
+
+// The step's sources, by the first block.  Gradient and isothermal walls: the
+// numbers by Ntogenerate's stochastic rounding (src/sampling.cpp:166-183,
+// :243-260), one Philox block per source.  Adiabatic walls: each re-emitting
+// border re-emits |Eborder| particles at its wall temperature.  The other
+// blocks make the CDF rows of the borders that re-emit, a chunk of modes each;
+// they find their border's temperature themselves (as a launch of their own
+// after the plan the two took 16 us of a step, together 9).
+__global__ void __launch_bounds__(256) be_plan(const __grid_constant__ SourceSets Q, const int* Eb,
+                                               const __grid_constant__ WallPlan W, int nmodes, unsigned long long* dc,
+                                               SrcSpan* span, long long cap, int* err, Stamps* st) {
+    await_previous();
+    if (blockIdx.x > 0) {
+        const int nch = (nmodes + WCDF_CHUNK - 1) / WCDF_CHUNK;
+        const int r = int(blockIdx.x - 1) / nch, ch = int(blockIdx.x - 1) % nch;
+        const int E = Eb[r];
+        const AdiBorder A = W.ab[r];
+        if (A.spline < 0 || E == 0) return;
+        const WallReq R{A.nx, A.ny, wall_temperature(W, A, E), A.Teq};
+        wall_cdf_body(W.om, W.vx, W.vy, nmodes, R, r, ch, W.cdf, W.chunk_tot);
+        return;
+    }
+    if (threadIdx.x == 0) stamp(st->t + 1);
     for (int q = 0; q < 2; ++q)
         for (int k = threadIdx.x; k < Q.s[q].ngen; k += 256) {
             Philox g;
@@ -1098,16 +936,13 @@ __global__ void __launch_bounds__(256) be_plan(const __grid_constant__ SourceSet
         }
     for (int k = threadIdx.x; k < Q.s[2].ngen; k += 256) {
         const int E = Eb[k];
-        Eb[k] = 0;
-        const AdiBorder A = ab[k];
+        const AdiBorder A = W.ab[k];
         long long c = 0;
         GenDesc d{};
         d.cdf = k;
         d.box = A.box >= 0 ? A.box : 0;
         if (A.spline >= 0 && E != 0) {
-            const double Jb = Eeff * E / dtstep / (A.len * thickness);
-            const double Tb = spline_eval(S, A.spline, Jb);
-            req[k] = WallReq{A.nx, A.ny, Tb, A.Teq};
+            const double Tb = wall_temperature(W, A, E);
             d.x0 = A.x0;
             d.y0 = A.y0;
             d.dx = A.dx;
@@ -1131,93 +966,312 @@ __global__ void __launch_bounds__(256) be_plan(const __grid_constant__ SourceSet
         for (int q = 0; q < 3; ++q) claim_span(total[q], dc, span + q, cap, err);
 }
 
-// The step's new particles at A[span.base + k), k < span.total of each source,
-// each advected for a random part of the step as it is made (the sources
-// of steps 2-4 of the reference's loop); an absorbed one keeps mode -1.
+// New particle i of a step (the sources of steps 2-4 of the reference's loop),
+// advected for a random part of the step; false where it is absorbed on the
+// way or has no place or mode.
+struct MakeArgs {
+    const SrcSpan* span;
+    SourceSets Q;
+    const double* cdfs;
+    const double* ctot;
+    const GBox* boxes;
+    const V2* hull;
+};
 template <bool GENERAL>
-__global__ void be_generate_dev(PArr P, const SrcSpan* span, const __grid_constant__ SourceSets Q, const double* cdfs,
-                                const double* ctot, int nmodes, const GBox* boxes, const V2* hull,
-                                const __grid_constant__ AdvectArgs aa) {
-    const SrcSpan s0 = span[0], s1 = span[1], s2 = span[2];
-    const long long total = (long long)(s0.total + s1.total + s2.total);
-    for (long long kk = blockIdx.x * (long long)blockDim.x + threadIdx.x; kk < total;
-         kk += (long long)gridDim.x * blockDim.x) {
-        const int q = kk < (long long)s0.total ? 0 : kk < (long long)(s0.total + s1.total) ? 1 : 2;
-        const long long k = kk - (q > 0 ? (long long)s0.total : 0) - (q > 1 ? (long long)s1.total : 0);
-        const SourceSet& Z = Q.s[q];
-        const GenDesc* gens = Z.descs;
-        int lo = 0, hi = Z.ngen;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (gens[mid].first <= k) lo = mid; else hi = mid;
-        }
-        const GenDesc gd = gens[lo];
-        Philox g;
-        g.init(Z.key, (uint64_t)k);
-        double x, y;
-        bool placed = true;
-        if (gd.rect == 2) {
-            const GBox& Bx = boxes[gd.box];
-            placed = false;
-            for (int tries = 0; tries < 100000 && !placed; ++tries) {
-                x = gd.x0 + g.uniform() * gd.dx;
-                y = gd.y0 + g.uniform() * gd.dy;
-                placed = inside_hull(hull + Bx.hull_off, Bx.nhull, v2(x, y));
-            }
-        } else if (gd.rect) {
+__device__ __forceinline__ bool make_particle(const MakeArgs& M, const AdvectArgs& aa, int nmodes, long long i, double& x,
+                                              double& y, int& box, int& mode, int& sign) {
+    const long long t0 = (long long)M.span[0].total, t1 = t0 + (long long)M.span[1].total;
+    const int q = i < t0 ? 0 : i < t1 ? 1 : 2;
+    const long long k = i - (q == 0 ? 0 : q == 1 ? t0 : t1);
+    const SourceSet& Z = M.Q.s[q];
+    const GenDesc* gens = Z.descs;
+    int lo = 0, hi = Z.ngen;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (gens[mid].first <= k) lo = mid; else hi = mid;
+    }
+    const GenDesc gd = gens[lo];
+    Philox g;
+    g.init(Z.key, (uint64_t)k);
+    bool placed = true;
+    if (gd.rect == 2) {
+        const GBox& Bx = M.boxes[gd.box];
+        placed = false;
+        for (int tries = 0; tries < 100000 && !placed; ++tries) {
             x = gd.x0 + g.uniform() * gd.dx;
             y = gd.y0 + g.uniform() * gd.dy;
-        } else {
-            const double u = g.uniform();
-            x = gd.x0 + u * gd.dx;
-            y = gd.y0 + u * gd.dy;
+            placed = inside_hull(M.hull + Bx.hull_off, Bx.nhull, v2(x, y));
         }
-        int mode;
-        if (gd.cdf >= 0) {
-            mode = wall_cdf_draw(cdfs, ctot, gd.cdf, nmodes, g.uniform());
-            if (!placed) mode = -1;
-        } else {
-            const float* pr = Z.prob + gd.alias_off;
-            const int* al = Z.alt + gd.alias_off;
-            const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
-            const float acc = float(g.next32() >> 8) * 0x1p-24f;
-            mode = acc < __ldg(pr + j) ? j : __ldg(al + j);
-        }
-        int box = gd.box;
-        const int sign = (gd.msign && mode >= 0) ? int(__ldg(Z.sign + gd.alias_off + mode)) : gd.sign;
-        const long long i = (long long)(q == 0 ? s0.base : q == 1 ? s1.base : s2.base) + k;
-        if (mode >= 0) {  // a random part of the step
-            Philox h;
-            h.init(Z.akey, (uint64_t)i);
-            const double dt = aa.dt * h.uniform();
-            bool alive;
-            if (GENERAL) {
-                BePol pol;
-                pol.g.init(Z.gkey, (uint64_t)i);
-                int e = 0;
-                alive = advect_general(aa.T, pol, aa.Eb, x, y, box, mode, sign, dt, e);
-                if (e && aa.err) atomicCAS(aa.err, 0, e);
-            } else {
-                alive = advect_one(aa.G, aa.boxcell, aa.mv, aa.boxwall, aa.Eb, x, y, box, mode, sign, dt);
-            }
-            if (!alive) mode = -1;
-        }
-        P.x[i] = x;
-        P.y[i] = y;
-        P.box[i] = box;
-        P.mode[i] = mode;
-        P.sign[i] = sign;
+    } else if (gd.rect) {
+        x = gd.x0 + g.uniform() * gd.dx;
+        y = gd.y0 + g.uniform() * gd.dy;
+    } else {
+        const double u = g.uniform();
+        x = gd.x0 + u * gd.dx;
+        y = gd.y0 + u * gd.dy;
     }
+    if (gd.cdf >= 0) {
+        mode = wall_cdf_draw(M.cdfs, M.ctot, gd.cdf, nmodes, g.uniform());
+        if (!placed) mode = -1;
+    } else {
+        const float* pr = Z.prob + gd.alias_off;
+        const int* al = Z.alt + gd.alias_off;
+        const int j = int(mulhi32(g.next32(), uint32_t(nmodes)));
+        const float acc = float(g.next32() >> 8) * 0x1p-24f;
+        mode = acc < __ldg(pr + j) ? j : __ldg(al + j);
+    }
+    if (mode < 0) return false;
+    box = gd.box;
+    sign = gd.msign ? int(__ldg(Z.sign + gd.alias_off + mode)) : gd.sign;
+    // a random part of the step
+    Philox h;
+    h.init(Z.akey, (uint64_t)i);
+    const double dt = aa.dt * h.uniform();
+    if (!GENERAL) return advect_one(aa.G, aa.boxcell, aa.mv, aa.boxwall, aa.Eb, x, y, box, mode, sign, dt);
+    BePol pol;
+    pol.g.init(Z.gkey, (uint64_t)i);
+    int e = 0;
+    const bool alive = advect_general(aa.T, pol, aa.Eb, x, y, box, mode, sign, dt, e);
+    if (e && aa.err) atomicCAS(aa.err, 0, e);
+    return alive;
 }
 
-// The wall CDFs of every border, for the borders the step planned (cnt > 0);
-// rows of the others are left as they are.
-__global__ void __launch_bounds__(256) be_wall_cdf(const float* om, const float* vx, const float* vy, int n,
-                                                   const WallReq* req, const long long* cnt, double* cdf,
-                                                   double* chunk_tot) {
-    const int nch = (n + WCDF_CHUNK - 1) / WCDF_CHUNK;
-    if (cnt[blockIdx.x / nch] == 0) return;
-    wall_cdf_body(om, vx, vy, n, req, cdf, chunk_tot);
+// Propagator scattering with sign branching (Scattering,
+// src/beyondRTA_MC2d.cpp:1073-1210): every scattering attempt of a parent
+// draws its next mode from the parent's column (an alias table over |P|
+// with the signs in the alias word, or, for an interpolated propagator, the
+// signed CDF probed as propagator_H::lower_bound does) and emits one
+// outgoing particle; when the drawn sign differs from the parent's, the
+// reference puts two copies of the parent back into the queue, and each
+// copy makes an attempt of its own.  The copies are identical to the
+// parent, so a thread keeps only the number of attempts its parent still
+// owes and makes them in place, with fresh draws.  BRANCH_CAP bounds the
+// attempts of one parent (a supercritical propagator never stops).
+constexpr unsigned BRANCH_CAP = 1u << 20;
+
+// One step of the particles [0, *n_in) of `in`, fused: advection by the
+// step, or with MAKE the step's new particles [0, *n_in), each made (and
+// advected for a part of the step) by the lane that takes it; then the scattering of the survivors -- RTA (ScatteringRTA,
+// src/beyondRTA_MC2d.cpp:983-1062, a resampling with probability
+// 1 - exp(-w dt), as a 53-bit threshold per mode) or the propagator with sign
+// branching as above -- and the histogram H[box][mode] += sign of every
+// outgoing particle, appended to `out`.  Each warp takes an equal run of the
+// particles; a lane whose parent owes no more attempts takes the run's next
+// one, a parent absorbed during its advection owes none.  Outgoing particles
+// gather in the warp's part of shared memory and leave 97 or more at a time,
+// with one claim of places: claims of parents and places 32 at a time, on
+// two counters of one cache line, came to 82 000 atomics on it per launch of
+// 1.3e6 particles and bounded the kernel (103 us a launch).
+//
+// Bound by the latency of its reads: a lane's next particle, its mode's
+// velocity and its column's alias slot (one of 301 MB for 6141 modes).  The
+// particles arrive in shared memory a chunk of 32 ahead (cp.async), and the
+// first draw of a parent, which needs only its mode, is read before the
+// advection: 70 -> 61 us for 1.3e6 particles, with the exits of advect_one.
+constexpr int ADV_BUF = 128, ADV_IN = 64;
+struct AdvBuf {
+    double x[ADV_BUF], y[ADV_BUF];
+    int mode[ADV_BUF], box[ADV_BUF], sign[ADV_BUF];
+    double ix[ADV_IN], iy[ADV_IN];
+    int imode[ADV_IN], ibox[ADV_IN], isign[ADV_IN];
+};
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "n"(BYTES)
+                 : "memory");
+}
+template <bool GENERAL, bool RTA, bool MAKE>
+__global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
+    be_advance(PArr in, const unsigned long long* n_in, PArr out, unsigned long long* dc, long long ocap,
+               const __grid_constant__ AdvectArgs aa, const __grid_constant__ MakeArgs ma, const PAlias* pal, const BoxProp* bprop, int nm,
+               const unsigned long long* pscat, const int2* resample, int nmodes, unsigned long long skey, int* H, int* err,
+               Stamps* st) {
+    await_previous();
+    if (blockIdx.x == 0 && threadIdx.x == 0) stamp(st->t + (MAKE ? 2 : 0));
+    __shared__ AdvBuf bufs[8];
+    AdvBuf& buf = bufs[threadIdx.x >> 5];
+    const long long n = min((long long)*n_in, ocap);  // places beyond the buffers (an overflow) are not read
+    const int lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
+        if (!MAKE) atomicAdd(dc + DC_PSTEPS, (unsigned long long)n);
+        atomicAdd(dc + DC_IN, (unsigned long long)n);
+    }
+    // the warp's run
+    const long long warps = (long long)gridDim.x * 8, per = max(32ll, ((n + warps - 1) / warps + 7) / 8 * 8);
+    const long long start = ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)) * per, end = min(n, start + per);
+    // of the run: taken, asked for (the ring holds the last ADV_IN) and arrived
+    long long next = start, asked = start, here = start;
+    auto ask = [&] {
+        const long long i = asked + lane;
+        if (!MAKE && i < end) {
+            const int k = int(i & (ADV_IN - 1));
+            copy_async<8>(buf.ix + k, in.x + i);
+            copy_async<8>(buf.iy + k, in.y + i);
+            copy_async<4>(buf.imode + k, in.mode + i);
+            copy_async<4>(buf.ibox + k, in.box + i);
+            copy_async<4>(buf.isign + k, in.sign + i);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asked += 32;
+    };
+    for (int k = 0; k < (MAKE ? 0 : ADV_IN / 32); ++k) ask();
+    unsigned long long flips = 0;
+    int mode = 0, sign = 1, box = 0, col = 0, cnt = 0;
+    double x = 0., y = 0.;
+    unsigned todo = 0, made = 0;
+    bool valid = false;
+    Philox g;
+    g.init(skey, 0);
+    int slot = 0;
+    float acc = 0.f, eprob = 0.f;
+    unsigned ealt = 0;
+    // one attempt's alias slot of the parent's column
+    auto draw_slot = [&](const PAlias* tab) {
+        slot = int(mulhi32(g.next32(), uint32_t(nm)));
+        acc = float(g.next32() >> 8) * 0x1p-24f;
+        const PAlias e = tab[(long long)col * nm + slot];
+        eprob = e.prob;
+        ealt = e.alt;
+    };
+    auto flush = [&] {
+        __syncwarp();
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(dc + DC_NOUT, (unsigned long long)cnt);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int j = lane; j < cnt; j += 32) {
+            const long long o = (long long)base + j;
+            if (o < ocap) {
+                out.x[o] = buf.x[j];
+                out.y[o] = buf.y[j];
+                out.mode[o] = buf.mode[j];
+                out.box[o] = buf.box[j];
+                out.sign[o] = buf.sign[j];
+                atomicAdd(H + (long long)buf.box[j] * nmodes + buf.mode[j], buf.sign[j]);
+            } else {
+                atomicCAS(err, 0, E_LIMIT);
+            }
+        }
+        cnt = 0;
+        __syncwarp();
+    };
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, todo == 0);
+        const long long upto = next + __popc(idle);
+        if (!MAKE && upto > here) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            here = asked;
+            __syncwarp();
+        }
+        if (todo == 0) {
+            const long long i = next + __popc(idle & ((1u << lane) - 1u));
+            if (i < end) {
+                if (MAKE) {
+                    if (!make_particle<GENERAL>(ma, aa, nmodes, i, x, y, box, mode, sign)) mode = -1;
+                } else {
+                    const int k = int(i & (ADV_IN - 1));
+                    mode = buf.imode[k];
+                    sign = buf.isign[k];
+                    box = buf.ibox[k];
+                    x = buf.ix[k];
+                    y = buf.iy[k];
+                }
+                if (mode >= 0) {
+                    g.init(skey, (uint64_t)i);
+                    if (RTA) {
+                        slot = mode;
+                        if ((g.next() >> 11) < __ldg(pscat + mode)) {
+                            slot = int(mulhi32(g.next32(), uint32_t(nmodes)));
+                            acc = float(g.next32() >> 8) * 0x1p-24f;
+                            const int2 e = __ldg(resample + slot);
+                            eprob = __int_as_float(e.x);
+                            ealt = unsigned(e.y);
+                        } else {
+                            acc = 0.f;
+                            eprob = 1.f;
+                        }
+                    } else {
+                        col = mode - 3;
+                        valid = col >= 0 && col < nm;
+                        if (pal && valid) draw_slot(pal);
+                    }
+                    bool alive = true;
+                    if (!MAKE) {
+                        if (GENERAL) {
+                            BePol pol;
+                            pol.g.init(aa.gkey, (uint64_t)i);
+                            int e = 0;
+                            alive = advect_general(aa.T, pol, aa.Eb, x, y, box, mode, sign, aa.dt, e);
+                            if (e && aa.err) atomicCAS(aa.err, 0, e);
+                        } else {
+                            alive = advect_one(aa.G, aa.boxcell, aa.mv, aa.boxwall, aa.Eb, x, y, box, mode, sign, aa.dt);
+                        }
+                    }
+                    if (alive) {
+                        if (!RTA && !valid) atomicCAS(err, 0, E_VALUE);
+                        todo = 1;
+                        made = 0;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (!MAKE && upto >= asked - (ADV_IN - 32)) ask();  // the older chunk has been taken
+        next = upto;
+        const bool act = todo > 0;
+        const unsigned m1 = __ballot_sync(0xffffffffu, act);
+        if (!m1) {
+            if (next >= end) break;
+            continue;
+        }
+        if (act) {
+            int nmode = mode, nsign = sign;
+            if (RTA) {
+                nmode = acc < eprob ? slot : int(ealt);
+            } else if (valid) {
+                // one table for every box (pal), or the box's own
+                const PAlias* tab = pal ? pal : bprop[box].alias;
+                if (tab) {
+                    if (!pal || made) draw_slot(tab);
+                    const bool keep = acc < eprob;
+                    const int to = keep ? slot : int(ealt & 0x3fffffffu);
+                    const bool neg = keep ? (ealt >> 31) != 0u : ((ealt >> 30) & 1u) != 0u;
+                    nmode = to + 3;
+                    nsign = neg ? -sign : sign;
+                } else {
+                    const BoxProp bp = bprop[box];
+                    if (bp.c1) {
+                        const long long off = (long long)col * nm;
+                        const int im = lower_bound_abs_lirp(bp.c1 + off, bp.c2 + off, nm, g.uniform(), bp.T, bp.T1, bp.T2);
+                        nmode = im + 3;
+                        nsign = lirp_at(bp.c1 + off, bp.c2 + off, im, bp.T, bp.T1, bp.T2) > 0. ? sign : -sign;
+                    } else {
+                        atomicCAS(err, 0, E_VALUE);  // a particle where nothing scatters
+                    }
+                }
+            }
+            const int o = cnt + __popc(m1 & ((1u << lane) - 1u));
+            buf.x[o] = x;
+            buf.y[o] = y;
+            buf.box[o] = box;
+            buf.mode[o] = nmode;
+            buf.sign[o] = nsign;
+            --todo;
+            if (!RTA && nsign != sign) {
+                todo += 2;
+                ++flips;
+            }
+            if (++made >= BRANCH_CAP) {
+                atomicCAS(err, 0, E_LIMIT);
+                todo = 0;
+            }
+        }
+        cnt += __popc(m1);
+        if (cnt > ADV_BUF - 32) flush();
+    }
+    if (cnt) flush();
+    for (int o = 16; o > 0; o >>= 1) flips += __shfl_down_sync(0xffffffffu, flips, o);
+    if (lane == 0 && flips) atomicAdd(dc + DC_FLIPS, flips);
 }
 
 // Cancellation on the device over [0, *n_in) with the random affine
@@ -1231,8 +1285,10 @@ __device__ __forceinline__ unsigned long long gcd_u64(unsigned long long a, unsi
     return a;
 }
 __global__ void be_cancel_dev(PArr P, unsigned long long* dc, long long cap, const int* H, int* cnt, int* rank,
-                              int nmodes, const int* reservoir, unsigned long long key) {
+                              int nmodes, const int* reservoir, unsigned long long key, Stamps* st) {
+    await_previous();
     const long long n = min((long long)dc[DC_NOUT], cap);
+    if (blockIdx.x == 0 && threadIdx.x == 0) stamp(st->t + 3);
     if (blockIdx.x == 0 && threadIdx.x == 0) dc[DC_NP] = 0;  // counted by the compaction
     if (n <= 0) return;
     // the permutation's a, b and the XOR key, drawn by one thread per block
@@ -1258,6 +1314,7 @@ __global__ void be_cancel_dev(PArr P, unsigned long long* dc, long long cap, con
 // The survivors of a cancellation from `in` to `out`, counted into dc[DC_NP].
 __global__ void be_compact_dev(PArr in, PArr out, unsigned long long* dc, long long cap, const int* rank, const int* H,
                                const int* cnt, int nmodes, unsigned long long key) {
+    await_previous();
     compact_body(in, min((long long)dc[DC_NOUT], cap), out, dc + DC_NP, rank, H, cnt, nmodes, key);
 }
 
@@ -1350,7 +1407,6 @@ struct BertaPlan {
 
 BertaState::~BertaState() {
     delete plan;
-    for (auto e : events) cudaEventDestroy(e);
 }
 
 namespace {
@@ -1723,14 +1779,14 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         const Generators &iso = PL.iso, &ini = PL.ini;
         const GradGenerators& grad = PL.grad;
         const bool have_ini = PL.have_ini;
-        B.d_Eb.alloc(std::size_t(nborders) * sizeof(int));
+        B.d_Eb.alloc(2 * std::size_t(nborders) * sizeof(int));
         // per-step buffers at their largest size (one request per border),
         // so that no step reallocates
-        B.d_req.alloc(std::size_t(nborders) * sizeof(WallReq));
         B.d_cdf.alloc(std::size_t(nborders) * std::size_t(m.n()) * sizeof(double));
         B.d_ctot.alloc(std::size_t(nborders) * ((m.n() + WCDF_CHUNK - 1) / WCDF_CHUNK) * sizeof(double));
-        ck(cudaMemsetAsync(B.d_Eb.p, 0, std::size_t(nborders) * sizeof(int), s), "memset");
+        ck(cudaMemsetAsync(B.d_Eb.p, 0, 2 * std::size_t(nborders) * sizeof(int), s), "memset");
         B.d_H.alloc(std::size_t(nbx) * n * sizeof(int));
+        B.d_H2.alloc(std::size_t(nbx) * n * sizeof(int));
         B.d_cnt.alloc(std::size_t(nbx) * n * sizeof(int));
         B.d_props.alloc(std::size_t(nbx) * 3 * sizeof(double));
         c->d_err.alloc(4 * sizeof(int));
@@ -1831,7 +1887,8 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
                                                                   nn, B.d_H.as<int>(), n);
             ck(cudaMemsetAsync(B.d_props.p, 0, std::size_t(nbx) * 3 * sizeof(double), s), "memset");
             be_props<<<nbx * PROPS_PARTS, 256, 0, s>>>(B.d_H.as<int>(), n, B.d_rvx.as<double>(), B.d_rvy.as<double>(),
-                                                        B.d_props.as<double>(), nullptr, 0, nullptr);
+                                                        B.d_props.as<double>(), nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0,
+                                                        nullptr);
             ck(cudaMemcpyAsync(hprops.data(), B.d_props.p, hprops.size() * sizeof(double), cudaMemcpyDeviceToHost, s), "d2h");
             sync(c);
             for (int b = 0; b < nbx; ++b) {
@@ -1940,29 +1997,21 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         // adiabatic re-emission per void border (plan_adiabatic_borders)
         B.d_adesc.alloc(std::size_t(nborders) * sizeof(GenDesc));
         B.d_acnt.alloc(std::size_t(nborders) * sizeof(long long));
-        const SplineDev SP{B.d_sa.as<double>(), B.d_sb.as<double>(), B.d_sc.as<double>(), B.d_sd.as<double>(),
-                           B.d_sx0.as<double>(), B.d_sxs.as<double>(), PL.nk};
         const int nch = (n + WCDF_CHUNK - 1) / WCDF_CHUNK;
+        const WallPlan WP{p->Eeff, p->dt, g.thickness,
+                          SplineDev{B.d_sa.as<double>(), B.d_sb.as<double>(), B.d_sc.as<double>(), B.d_sd.as<double>(),
+                                    B.d_sx0.as<double>(), B.d_sxs.as<double>(), PL.nk},
+                          B.d_adi.as<AdiBorder>(), B.d_om.as<float>(), B.d_vx.as<float>(), B.d_vy.as<float>(),
+                          B.d_cdf.as<double>(), B.d_ctot.as<double>()};
         const unsigned pblocks = unsigned(c->nsm) * 8u;  // persistent grids of the step kernels
         const BoxProp* bprop = p->rta ? nullptr : B.d_boxprop.as<BoxProp>();
         int istep = 0;
         double time = 0.;
-        // phase timing (the reference's timer buckets): events at the phase
+        // phase timing (the reference's timer buckets): stamps at the phase
         // borders of every step, read at the end
         enum { PH_ADV, PH_CANCEL, PH_GEN, PH_HIST, PH_PROPS, PH_READ, PH_SAVE, PH_SCAT };
         double phase[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        std::vector<cudaEvent_t>& pev = B.events;
-        struct EvGuard {  // a long run's events beyond a few thousand are given back
-            std::vector<cudaEvent_t>* e;
-            ~EvGuard() {
-                for (; e->size() > 4096; e->pop_back()) cudaEventDestroy(e->back());
-            }
-        } pe_guard{&pev};
-        while (pev.size() < std::size_t(nsteps) * 7) {
-            cudaEvent_t e = nullptr;
-            ck(cudaEventCreate(&e), "cudaEventCreate");
-            pev.push_back(e);
-        }
+        B.d_stamps.alloc(std::size_t(nsteps) * sizeof(Stamps));
         phase[PH_READ] = 1e3 * std::chrono::duration<double>(std::chrono::steady_clock::now() - t_start).count();
         std::vector<int> hH;
         const int cancel_every = p->cancel_every > 0 ? p->cancel_every : 4;
@@ -1976,13 +2025,17 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         };
         // the advection and scattering of particles `in` into B
         const unsigned ablocks = unsigned(c->nsm) * (general ? 2u : 3u);
-        auto advance = [&](PArr in, const unsigned long long* n_in, int advect, const AdvectArgs& aa,
+        int *H = B.d_H.as<int>(), *next_H = B.d_H2.as<int>();  // this step's histogram and the next one's
+        // the walls' counts of this step's plan and of the next one's
+        int *Eb = B.d_Eb.as<int>(), *next_Eb = Eb + nborders;
+        Stamps* st = nullptr;
+        ck(cudaMemsetAsync(next_H, 0, hbytes, s), "memset");
+        ck(cudaMemsetAsync(B.d_cnt.p, 0, hbytes, s), "memset");
+        auto advance = [&](auto f, unsigned blocks, PArr in, const unsigned long long* n_in, const AdvectArgs& aa, const MakeArgs& ma,
                            unsigned long long key) {
-            const auto f = general ? (p->rta ? be_advance<true, true> : be_advance<true, false>)
-                                   : (p->rta ? be_advance<false, true> : be_advance<false, false>);
-            f<<<ablocks, 256, 0, s>>>(in, n_in, arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc, cap, advect, aa, pal,
+            after_previous(f, blocks, s, in, n_in, arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign), dc, cap, aa, ma, pal,
                                       bprop, B.nm, B.d_pscat.as<unsigned long long>(), c->d_resample.as<int2>(), n, key,
-                                      B.d_H.as<int>(), err);
+                                      H, err, st);
         };
         SourceSets Q{};
         Q.s[0] = SourceSet{B.d_gdesc.as<GenDesc>(), B.d_ggenf.as<double>(), B.d_gcnt.as<long long>(), ngd,
@@ -1992,18 +2045,17 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         Q.s[2] = SourceSet{B.d_adesc.as<GenDesc>(), nullptr, B.d_acnt.as<long long>(), nborders, nullptr, nullptr, nullptr,
                            0, 0, 0};
         while (time <= p->maxtime && istep < nsteps) {
-            cudaEvent_t* ev = pev.data() + std::size_t(istep) * 7;
-            ck(cudaEventRecord(ev[0], s), "event");
+            st = B.d_stamps.as<Stamps>() + istep;
+            std::swap(H, next_H);
             // 1 + 6 + 7 for the particles of the last step: advection,
             // scattering and histogram in one pass, into B
-            ck(cudaMemsetAsync(B.d_H.p, 0, hbytes, s), "memset");
-            const AdvectArgs a_step{GA.G, GA.boxcell, GA.mv, B.d_boxwall.as<int4>(), B.d_Eb.as<int>(), p->dt,
-                                    mix_key(p->seed, istep, 31), err, TT};
+            AdvectArgs a_step{GA.G, GA.boxcell, GA.mv, B.d_boxwall.as<int4>(), Eb, p->dt,
+                              mix_key(p->seed, istep, 31), err, TT};
             const PArr A = arr(B.a_x, B.a_y, B.a_mode, B.a_box, B.a_sign);
-            advance(A, dc + DC_NP, 1, a_step, mix_key(p->seed, istep, 64));
-            ck(cudaEventRecord(ev[1], s), "event");
-            // 2-4 the step's sources, made at A[0..) (A is free now) and each
-            // advected for a random part of the step as it is made
+            advance(general ? (p->rta ? be_advance<true, true, false> : be_advance<true, false, false>)
+                            : (p->rta ? be_advance<false, true, false> : be_advance<false, false, false>),
+                    ablocks, A, dc + DC_NP, a_step, MakeArgs{}, mix_key(p->seed, istep, 64));
+            // 2-4 the step's sources
             auto keys = [&](SourceSet& q, int ph) {
                 q.key = mix_key(p->seed, istep, ph);
                 q.akey = mix_key(p->seed, istep, ph + 1);
@@ -2014,45 +2066,37 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             keys(Q.s[2], 4);
             Q.pkey[0] = mix_key(p->seed, istep, 40);
             Q.pkey[1] = mix_key(p->seed, istep, 41);
-            be_plan<<<1, 256, 0, s>>>(Q, B.d_Eb.as<int>(), B.d_adi.as<AdiBorder>(), SP, p->Eeff, p->dt, g.thickness,
-                                      B.d_req.as<WallReq>(), dc, span, cap, err);
-            if (nborders > 0)
-                be_wall_cdf<<<unsigned(nborders) * unsigned(nch), 256, 0, s>>>(
-                    B.d_om.as<float>(), B.d_vx.as<float>(), B.d_vy.as<float>(), n, B.d_req.as<WallReq>(),
-                    B.d_acnt.as<long long>(), B.d_cdf.as<double>(), B.d_ctot.as<double>());
-            const auto gen_kernel = general ? be_generate_dev<true> : be_generate_dev<false>;
-            gen_kernel<<<pblocks, 256, 0, s>>>(A, span, Q, B.d_cdf.as<double>(), B.d_ctot.as<double>(), n,
-                                               c->d_boxes.as<GBox>(), c->d_hull.as<V2>(), a_step);
-            ck(cudaEventRecord(ev[2], s), "event");
-            // 5-7 for the new particles: the absorbed ones dropped, the others
-            // scattered and counted in the histogram, appended to B
-            advance(A, dc + DC_NGEN, 0, a_step, mix_key(p->seed, istep, 65));
-            ck(cudaEventRecord(ev[3], s), "event");
-            ck(cudaEventRecord(ev[4], s), "event");  // the histogram is made in the passes above
+            after_previous(be_plan, 1u + unsigned(nborders) * unsigned(nch), s, Q, Eb, WP, n, dc, span, cap, err, st);
+            // the new particles made; 5-7 for them: the absorbed ones dropped, the
+            // others scattered and counted in the histogram, appended to B
+            a_step.Eb = next_Eb;  // (what they leave on the walls is planned in the next step)
+            const MakeArgs ma{span, Q, B.d_cdf.as<double>(), B.d_ctot.as<double>(), c->d_boxes.as<GBox>(), c->d_hull.as<V2>()};
+            advance(general ? (p->rta ? be_advance<true, true, true> : be_advance<true, false, true>)
+                            : (p->rta ? be_advance<false, true, true> : be_advance<false, false, true>),
+                    pblocks, A, dc + DC_NGEN, a_step, ma, mix_key(p->seed, istep, 65));
             // 8. cancellation every cancel_every steps: B -> A; otherwise B is the population
             const bool cancel = istep % cancel_every == 0;
             if (cancel) {
                 const PArr Bp = arr(B.b_x, B.b_y, B.b_mode, B.b_box, B.b_sign);
-                ck(cudaMemsetAsync(B.d_cnt.p, 0, hbytes, s), "memset");
-                be_cancel_dev<<<pblocks, 256, 0, s>>>(Bp, dc, cap, B.d_H.as<int>(), B.d_cnt.as<int>(), B.d_rank.as<int>(),
-                                                      n, B.d_res.as<int>(), mix_key(p->seed, istep, 77));
-                be_compact_dev<<<pblocks, 256, 0, s>>>(Bp, A, dc, cap, B.d_rank.as<int>(), B.d_H.as<int>(),
+                after_previous(be_cancel_dev, pblocks, s, Bp, dc, cap, H, B.d_cnt.as<int>(), B.d_rank.as<int>(),
+                                                      n, B.d_res.as<int>(), mix_key(p->seed, istep, 77), st);
+                after_previous(be_compact_dev, pblocks, s, Bp, A, dc, cap, B.d_rank.as<int>(), H,
                                                        B.d_cnt.as<int>(), n, mix_key(p->seed, istep, 78));
             } else {
                 swap_ab();
             }
-            ck(cudaEventRecord(ev[5], s), "event");
             // 9. properties of the step (calculate_prop), recorded on the device
-            be_props<<<nbx * PROPS_PARTS, 256, 0, s>>>(B.d_H.as<int>(), n, B.d_rvx.as<double>(), B.d_rvy.as<double>(),
+            after_previous(be_props, unsigned(nbx * PROPS_PARTS), s, H, n, B.d_rvx.as<double>(), B.d_rvy.as<double>(),
                                                         B.d_phist.as<double>() + std::size_t(istep + 1) * nbx * 3, dc,
-                                                        cancel ? 0 : 1, B.d_nhist.as<long long>() + istep + 1);
+                                                        cancel ? 0 : 1, B.d_nhist.as<long long>() + istep + 1, next_H,
+                                                        B.d_cnt.as<int>(), Eb, nborders, st);
+            std::swap(Eb, next_Eb);
             ck(cudaGetLastError(), "step launch");
-            ck(cudaEventRecord(ev[6], s), "event");
             if (p->on_step) {
                 hH.resize(std::size_t(nbx) * n);
                 int herr[4];
                 long long hnp = 0;
-                ck(cudaMemcpyAsync(hH.data(), B.d_H.p, hbytes, cudaMemcpyDeviceToHost, s), "d2h");
+                ck(cudaMemcpyAsync(hH.data(), H, hbytes, cudaMemcpyDeviceToHost, s), "d2h");
                 ck(cudaMemcpyAsync(hprops.data(), B.d_phist.as<double>() + std::size_t(istep + 1) * nbx * 3,
                                    hprops.size() * sizeof(double), cudaMemcpyDeviceToHost, s), "d2h");
                 ck(cudaMemcpyAsync(&hnp, B.d_nhist.as<long long>() + istep + 1, sizeof hnp, cudaMemcpyDeviceToHost, s),
@@ -2080,6 +2124,9 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             std::vector<long long> nh(std::size_t(nsteps + 1));
             std::vector<unsigned long long> hdc(DC_COUNT);
             ck(cudaMemcpyAsync(ph.data(), B.d_phist.p, ph.size() * sizeof(double), cudaMemcpyDeviceToHost, s), "d2h");
+            std::vector<Stamps> hst(static_cast<std::size_t>(istep));
+            if (istep > 0)
+                ck(cudaMemcpyAsync(hst.data(), B.d_stamps.p, hst.size() * sizeof(Stamps), cudaMemcpyDeviceToHost, s), "d2h");
             ck(cudaMemcpyAsync(nh.data(), B.d_nhist.p, nh.size() * sizeof(long long), cudaMemcpyDeviceToHost, s), "d2h");
             ck(cudaMemcpyAsync(hdc.data(), dc, DC_COUNT * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s), "d2h");
             ck(cudaMemcpyAsync(herr, err, sizeof herr, cudaMemcpyDeviceToHost, s), "d2h");
@@ -2102,21 +2149,22 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             branchings = (long long)hdc[DC_FLIPS];
             adv_in = (long long)hdc[DC_IN];
             adv_out = (long long)hdc[DC_OUTT];
-            const int bucket[6] = {PH_ADV, PH_GEN, PH_SCAT, PH_HIST, PH_CANCEL, PH_PROPS};
-            for (int st = 0; st < istep; ++st)
-                for (int k = 0; k < 6; ++k) {
-                    float pms = 0.f;
-                    if (cudaEventElapsedTime(&pms, pev[std::size_t(st) * 7 + k], pev[std::size_t(st) * 7 + k + 1]) ==
-                        cudaSuccess)
-                        phase[bucket[k]] += pms;
-                }
+            // (scattering: the pass that makes and scatters the new particles;
+            // histogram: its reading, both passes having counted it)
+            for (int k = 0; k < istep; ++k) {
+                const unsigned long long* t = hst[std::size_t(k)].t;
+                const unsigned long long made = k % cancel_every == 0 ? t[3] : t[4];
+                const unsigned long long at[7] = {t[0], t[1], t[2], made, t[4], t[5], t[6]};
+                const int bucket[6] = {PH_ADV, PH_GEN, PH_SCAT, PH_CANCEL, PH_HIST, PH_PROPS};
+                for (int q = 0; q < 6; ++q) phase[bucket[q]] += 1e-6 * double((long long)(at[q + 1] - at[q]));
+            }
         }
         ck(cudaEventRecord(c->ev1, s), "event");
         sync(c);
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->ev0, c->ev1);
         if (out->histogram)
-            ck(cudaMemcpy(out->histogram, B.d_H.p, std::size_t(nbx) * n * sizeof(int), cudaMemcpyDeviceToHost), "d2h");
+            ck(cudaMemcpy(out->histogram, H, hbytes, cudaMemcpyDeviceToHost), "d2h");
         out->nboxes = nbx;
         out->nsteps = istep;
         out->particle_steps = psteps;
