@@ -127,6 +127,7 @@ struct LinkArgs {
     const unsigned long long* wxf;
     const unsigned long long* wyf;
     int ny, refill;
+    int lanes;                   // lanes of a warp that take particles (set by the launch)
     const int4* side;            // [cell = i ny + j][4] LinkEntry
     const int4* range;           // [box] columns [x, y) and rows [z, w)
     const unsigned char* per;    // [box] 1: spans the period in x, 2: in y
@@ -153,6 +154,19 @@ struct AdjArgs {
     double* g_scalar;     // [3]
     int comps;            // bit q: W has a component q that is not zero
 };
+
+// Lanes of a warp that take particles, of a run of n.
+// A run too small to fill the GPU is bound by the passes of its longest
+// particles, and a pass takes as long as its warp's branches together: the
+// particles are spread over one lane of up to 16 warps per SM, then over
+// as few lanes of 8 warps as hold them.  Kernel times of 1e3, 2e3, 1e4 and
+// 3e4 particles with all lanes in use 0.126, 0.62, 0.64 and 0.65 ms, so
+// 0.089, 0.35, 0.48 and 0.56 on a ribbon (16 warps at 1e4: 0.55; 4: 0.54).
+inline int particle_lanes(long long n, int nsm) {
+    if (n <= 16ll * nsm) return 1;
+    const long long l = (n + 8ll * nsm - 1) / (8ll * nsm);
+    return l < 32 ? int(l) : 32;
+}
 
 // Axis-aligned grid production kernel (persistent, warp-refilled work).
 // adj_pass 1 / 2 runs the forward / adjoint pass of the adjoint with `adj`

@@ -168,8 +168,8 @@ __device__ __noinline__ int link_generate(const DevTables& T, long long pid, Phi
 //   pending displacement goes on.
 // In doubles the polygon kernel took 160 registers (one block of 256 threads
 // per SM) and 42 to 124 FP64 operations per event.  GB300: periodic bar
-// (2e6 particles, 10 strips, 100 bins) 10.1 -> 1.87 ms, two-crystal ribbon (3e5
-// particles) 1.79 -> 0.77 ms.
+// (2e6 particles, 10 strips, 100 bins) 10.1 -> 1.80 ms, two-crystal ribbon (3e5
+// particles) 1.79 -> 0.71 ms, of 2e3 particles 0.17.
 template <bool CORNER>
 __global__ void __launch_bounds__(256, 2) rta_prod_link(const __grid_constant__ DevTables T,
                                                         const __grid_constant__ LinkArgs A, double* gtally,
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(256, 2) rta_prod_link(const __grid_constant__ 
     uint32_t dt_hi = 0, nev = 0, npass = 0, nseg = 0;
     int64_t px = 0, py = 0;
     long long pid = -1;
-    bool active = false, done = false;
+    bool active = false, done = lane >= A.lanes;
     auto stop = [&](int e) {
         record_error(err, e, pid);
         active = false;
@@ -257,6 +257,12 @@ __global__ void __launch_bounds__(256, 2) rta_prod_link(const __grid_constant__ 
         }
         if (active) {
             const uint4 rr = pass_block(npass, (uint64_t)pid, T.seed);
+            int cand = mode;  // the mode a scattering would draw, read ahead as in rta_prod_grid
+            if (!T.ballistic) {
+                const int j = int(mulhi32(rr.y, uint32_t(T.n)));
+                const int2 e = __ldg(T.resample + mo + j);
+                cand = float(rr.z >> 8) * 0x1p-24f < __int_as_float(e.x) ? j : e.y;
+            }
             ModeFix m = mv;
             if (per & 1) m.rx = ~0ull;
             if (per & 2) m.ry = ~0ull;
@@ -378,11 +384,8 @@ __global__ void __launch_bounds__(256, 2) rta_prod_link(const __grid_constant__ 
                         alt = e.z;
                     }
                     c.wall_hits++;
-                } else if (!T.ballistic) {
-                    keep = int(mulhi32(rr.y, uint32_t(T.n)));
-                    const int2 e = __ldg(T.resample + mo + keep);
-                    pr = __int_as_float(e.x);
-                    alt = e.y;
+                } else {
+                    keep = alt = cand;
                 }
                 const float acc = float(rr.z >> 8) * 0x1p-24f;
                 mode = acc < pr ? keep : alt;
@@ -456,7 +459,7 @@ __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant_
     int64_t px = 0, py = 0;
     double unit = 1.;  // ticks per time unit of the flight
     long long slot = -1;
-    bool active = false, done = false;
+    bool active = false, done = lane >= A.lanes;
     auto fail = [&](int e) {
         record_error(err, e, slot);
         S.flag[slot] = 0;
@@ -680,35 +683,41 @@ __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant_
 
 }  // namespace
 
-bool launch_steady_link(const DevTables& T, const SteadyArgs& S, const LinkArgs& A, double* tally,
+bool launch_steady_link(const DevTables& T, const SteadyArgs& S, const LinkArgs& A0, double* tally,
                         unsigned long long* counters, int* err, int nsm, cudaStream_t s) {
     if (S.n <= 0) return true;
+    LinkArgs A = A0;
+    A.lanes = particle_lanes(S.n, nsm);
+    const int threads = A.lanes < 32 ? 64 : 128;
     int maxb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, rta_steady_link, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, rta_steady_link, threads, 0);
     if (maxb < 1) return false;
     long long blocks = (long long)nsm * maxb;
-    const long long need = (S.n + 127) / 128;
+    const long long per = threads / 32 * A.lanes, need = (S.n + per - 1) / per;
     if (blocks > need) blocks = need;
     cudaMemsetAsync(S.work, 0, sizeof(unsigned long long), s);
-    rta_steady_link<<<unsigned(blocks), 128, 0, s>>>(T, S, A, tally, counters, err);
+    rta_steady_link<<<unsigned(blocks), unsigned(threads), 0, s>>>(T, S, A, tally, counters, err);
     return true;
 }
 
-bool launch_prod_link(const DevTables& T, const LinkArgs& A, double* tally, unsigned long long* counters, int* err,
+bool launch_prod_link(const DevTables& T, const LinkArgs& A0, double* tally, unsigned long long* counters, int* err,
                       unsigned long long* work, int nsm, cudaStream_t s) {
     const long long n = T.pend - T.pbegin;
     if (n <= 0) return true;
+    LinkArgs A = A0;
+    A.lanes = particle_lanes(n, nsm);
     int maxb = 0;
     // two blocks of 256 threads per SM: with three (80 registers, spills) the
     // bar takes 1.96 ms instead of 1.85, the crystals 0.82 instead of 0.77
     const void* f = A.pbox ? (const void*)rta_prod_link<true> : (const void*)rta_prod_link<false>;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, f, 256, 0);
+    const int threads = A.lanes < 32 ? 64 : 256;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&maxb, f, threads, 0);
     if (maxb < 1) return false;
     long long blocks = (long long)nsm * maxb;
-    const long long need = (n + 255) / 256;
+    const long long per = threads / 32 * A.lanes, need = (n + per - 1) / per;
     if (blocks > need) blocks = need;
     void* args[] = {(void*)&T, (void*)&A, &tally, &counters, &err, &work};
-    return cudaLaunchKernel(f, dim3(unsigned(blocks)), dim3(256), args, 0, s) == cudaSuccess;
+    return cudaLaunchKernel(f, dim3(unsigned(blocks)), dim3(unsigned(threads)), args, 0, s) == cudaSuccess;
 }
 
 }  // namespace bte

@@ -1385,15 +1385,9 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A0, double* tally,
     // several particles in turn (2e6 on 36864 modes: 111 ms against 118 with
     // three), three leave fewer lanes idle at the end of a short run (2e5:
     // 0.53 ms against 0.61; 1e6: 3.36 and 3.38, the same).
-    // A run too small to fill the GPU is bound by the passes of its longest
-    // particles, and a pass takes as long as its warp's branches together: the
-    // particles are spread over one lane of up to 16 warps per SM, then over
-    // as few lanes of 8 warps as hold them.  Kernel times of 1e3, 2e3, 1e4 and
-    // 3e4 particles with all lanes in use 0.126, 0.62, 0.64 and 0.65 ms, so
-    // 0.089, 0.35, 0.48 and 0.56 (16 warps at 1e4: 0.55; 4: 0.54).
     const bool tuned = tune.block_threads > 0 || tune.blocks_per_sm > 0 || use_smem;
     if (!tuned && !T.checks)
-        A.lanes = n <= 16ll * nsm ? 1 : int(std::min<long long>(32, (n + 8ll * nsm - 1) / (8ll * nsm)));
+        A.lanes = particle_lanes(n, nsm);
     const bool small = A.lanes < 32;
     const int threads = tune.block_threads > 0 ? tune.block_threads : small ? 64 : 256;
     if (threads > 256 || threads % 32) return false;

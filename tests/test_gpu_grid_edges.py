@@ -7,6 +7,9 @@
   in another order, agree to M 2^-53 of the sum of their magnitudes: with
   fewer than 2^20 flushes per entry and sums of one sign per wall, 2^-33 of
   the largest entry; 1e-9 leaves a factor of ten for cancellation.
+- The linked-cell and the replay kernel spread a small run in the same way:
+  the counters of a run are the sums over the parts of its particle range,
+  whose sizes lie on both sides of each border of the rule.
 - A time bin much longer than a flight across the domain is walked in equal
   parts.  Its means must be those of the replay mode, which knows no parts:
   five standard errors over independent seeds."""
@@ -36,6 +39,21 @@ def test_lanes_of_a_small_run(engine, N):
         assert small[k] == full[k], k
     for k in ("gz", "gz_jx", "gz_jy"):
         assert np.abs(small[k] - full[k]).max() <= 1e-9 * np.abs(full[k]).max(), k
+
+
+@pytest.mark.parametrize("mode", [btegpu.MODE_PRODUCTION, btegpu.MODE_REPLAY])
+@pytest.mark.parametrize("part", [1, 16 * 152, 16 * 152 + 1, 8 * 31 * 152 + 1])
+def test_parts_of_a_run_add_up(engine, mode, part):
+    engine.load_modes(synth.mode_table(8, 3, 3, 300.0, config=100))
+    engine.load_geometry(synth.periodic_bar_geometry())
+    N = part + 8 * 32 * 152 + 1
+    args = dict(T0=300.0, dt=10.0, maxtime=50.0, N=N, seed=9, source=btegpu.SOURCE_WALLS, mode=mode)
+    whole = engine.rta_run(**args)
+    parts = [engine.rta_run(begin=0, end=part, **args), engine.rta_run(begin=part, end=N, **args)]
+    for k in KEYS:
+        assert whole[k] == sum(p[k] for p in parts), k
+    for k in ("gz", "gz_jx", "gz_jy"):
+        assert np.abs(whole[k] - sum(p[k] for p in parts)).max() <= 1e-9 * np.abs(whole[k]).max(), k
 
 
 @pytest.mark.parametrize("dt", [200.0, 4000.0])
