@@ -1082,7 +1082,7 @@ __device__ __forceinline__ void copy_async(void* dst, const void* src) {
                  : "memory");
 }
 template <bool GENERAL, bool RTA, bool MAKE>
-__global__ void __launch_bounds__(256, GENERAL ? 2 : 3)
+__global__ void __launch_bounds__(256, GENERAL ? 2 : MAKE && !RTA ? 4 : 3)
     be_advance(PArr in, const unsigned long long* n_in, PArr out, unsigned long long* dc, long long ocap,
                const __grid_constant__ AdvectArgs aa, const __grid_constant__ MakeArgs ma, const PAlias* pal, const BoxProp* bprop, int nm,
                const unsigned long long* pscat, const int2* resample, int nmodes, unsigned long long skey, int* H, int* err,
