@@ -168,7 +168,7 @@ def nsm_of_device():
 def profile_figures():
     """ncu figures of the grid kernel from the committed capture summary:
     DRAM bytes per launch = fixed (tables, first touch) + per event, and the
-    FP64 thread operations per event."""
+    warp instructions per event."""
     p = os.path.join(REPO, "profiles", "rta_prod_grid_c1.json")
     if os.path.exists(p):
         try:
@@ -960,14 +960,14 @@ def main():
         traffic = None
         if "dram_bytes_per_event" in prof:
             traffic = prof.get("dram_fixed_bytes", 0.0) + prof["dram_bytes_per_event"] * ev_launch
-        fp64 = None
-        if "fp64_thread_ops_per_event" in prof:
+        issue = None
+        if "warp_inst_per_event" in prof:
             mhz = clk.get("sm_mhz") or clk.get("sm_max_mhz") or 2070.0
-            lane_peak = prof.get("fp64_lane_ops_per_sm_cycle", 2) * nsm_of_device() * mhz * 1e6
-            ops = prof["fp64_thread_ops_per_event"] * value
-            fp64 = {"pipe": "fp64", "ops_per_event": prof["fp64_thread_ops_per_event"],
-                    "achieved": ops / 1e9, "peak": lane_peak / 1e9, "unit": "Gop/s",
-                    "frac": ops / lane_peak, "pipe_busy_pct_ncu": prof.get("fp64_pipe_busy_pct")}
+            slots = 4 * nsm_of_device() * mhz * 1e6
+            inst = prof["warp_inst_per_event"] * value
+            issue = {"pipe": "issue", "ops_per_event": prof["warp_inst_per_event"],
+                     "achieved": inst / 1e9, "peak": slots / 1e9, "unit": "Gop/s",
+                     "frac": inst / slots, "pipe_busy_pct_ncu": prof.get("issue_active_pct")}
         l2red = None
         if "l2_red_sectors_per_event" in prof and "l2_red_peak_sectors_per_s" in prof:
             red = prof["l2_red_sectors_per_event"] * value
@@ -993,7 +993,7 @@ def main():
                          "frac": achieved / peak, "peak_source": peak_kind,
                          "traffic": traffic,
                          "bytes_per_event": per_launch_bytes / max(ev_launch, 1)},
-            "co_bound": fp64,
+            "co_bound": issue,
             "l2_reductions": l2red,
             "clocks": clk,
             "tuning": {"block_threads": choice[0], "blocks_per_sm": choice[1],
