@@ -21,6 +21,8 @@ constexpr std::size_t PDF_BYTES = std::size_t(64) << 20;
 // Gamma pdf of mode k0 + k (shape w^2 / sigma, scale sigma / w: gamma_pdf,
 // :61-63) at every tick; 0 where it is negligible or sigma is 0 (a NaN).
 // par: per mode {shape, scale, lgamma(shape), log(scale)}.
+// FP64 logarithms and exponentials bound it: 32 us for 1536 modes at 200 ticks,
+// once for all the locations of a crystal.
 __global__ void spec_pdf(const double4* par, const double* om, int k0, int nk, const double* ticks, int nw,
                          double* pdf) {
     const long long total = (long long)nk * nw;
@@ -41,9 +43,10 @@ __global__ void spec_pdf(const double4* par, const double* om, int k0, int nk, c
 // out[q][bin][tick] += sum over modes of {1, vx, vy}[q] time[bin][mode]
 // pdf[mode][tick], for the modes [k0, k0 + nk).  A block takes one bin, 128
 // ticks and 128 modes, whose weighted times it first puts in shared memory;
-// blocks over the modes add with FP64 atomics.  Three FMAs per term on the two
-// FP64 lanes of an SM bound it; the host loops took 42 ms for 3 boxes, 40 bins, 1536
-// modes and 200 ticks, this takes 0.3 ms in all.
+// blocks over the modes add with FP64 atomics.  Bound by three FMAs per term on
+// the two FP64 lanes of an SM, so a warp passes over the modes whose pdf is
+// zero at all its 32 ticks (more than half of them): 133 us per location of 40
+// bins, 1536 modes and 200 ticks, now 55.  (The host loops took 42 ms for three.)
 __global__ void __launch_bounds__(SPEC_T) spec_contract(const double* time, double unit, long long tstride, int nbins,
                                                          const double* vx, const double* vy, int k0, int nk,
                                                          const double* pdf, int nw, double* out) {
@@ -58,16 +61,23 @@ __global__ void __launch_bounds__(SPEC_T) spec_contract(const double* time, doub
         w[2][threadIdx.x] = vy[k] * t;
     }
     __syncthreads();
-    if (i >= nw) return;
     double s[3] = {0., 0., 0.};
-    for (int k = 0; k < n; ++k) {
-        const double t = w[0][k];
-        if (t == 0.) continue;  // (the same for the whole block)
-        const double g = pdf[(long long)(c0 + k) * nw + i];
-        s[0] += t * g;
-        s[1] += w[1][k] * g;
-        s[2] += w[2][k] * g;
+    const double* col = pdf + (long long)c0 * nw + i;
+    for (int k4 = 0; k4 < n; k4 += 4) {
+        double g[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) g[j] = i < nw && k4 + j < n ? col[(long long)(k4 + j) * nw] : 0.;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!__any_sync(0xffffffffu, __double2hiint(g[j]) | __double2loint(g[j]))) continue;
+            const double t = w[0][k4 + j];
+            if (t == 0.) continue;  // (the same for the whole block)
+            s[0] += t * g[j];
+            s[1] += w[1][k4 + j] * g[j];
+            s[2] += w[2][k4 + j] * g[j];
+        }
     }
+    if (i >= nw) return;
     for (int q = 0; q < 3; ++q)
         if (s[q] != 0.) atomicAdd(out + ((long long)q * nbins + b) * nw + i, s[q]);
 }
@@ -90,11 +100,19 @@ __global__ void spec_fdq(const double* time, double unit, const long long* count
     }
 }
 
-// v[bin][i] times `scale`, summed over the bins so far (integrate), divided
-// by `div`; one thread per i, eight bins read ahead.
-__global__ void spec_finish(double* v, int nbins, int n, double scale, double div, int integrate) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// The four arrays of a location: v[bin][i] times `scale`, summed over the bins
+// so far (integrate), divided by `div`; one thread per i, eight bins read ahead,
+// a warp per block so that the divisions spread over the SMs (as four launches of
+// 128 threads a block 80 us per location, now 20).
+struct SpecFinish {
+    double scale[4], div[4];
+    int n[4];
+};
+__global__ void __launch_bounds__(32) spec_finish(double* v, int nbins, int nw, SpecFinish f, int integrate) {
+    const int q = blockIdx.y, n = f.n[q], i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    const double scale = f.scale[q], div = f.div[q];
+    v += (long long)q * nbins * nw;
     double run = 0.;
     for (int b0 = 0; b0 < nbins; b0 += 8) {
         double x[8];
@@ -103,7 +121,7 @@ __global__ void spec_finish(double* v, int nbins, int n, double scale, double di
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             run = integrate ? run + x[j] : x[j];
-            if (b0 + j < nbins) v[(long long)(b0 + j) * n + i] = run / div;
+            if (b0 + j < nbins) v[(long long)(b0 + j) * n + i] = div == 1.0 ? run : run / div;
         }
     }
 }
@@ -169,6 +187,7 @@ extern "C" bte_status bte_get_spectral(bte_ctx* c, bte_spectral_result* out) {
             S.out.alloc(nloc * per * sizeof(double));
             ck(cudaMemsetAsync(S.out.p, 0, nloc * per * sizeof(double), s), "memset");
         }
+        int pdf_of = -2;  // the crystal whose whole pdf is in S.pdf
         for (std::size_t l = 0; l < nloc; ++l) {
             const int kc = crystal_of(l);
             const HostModes& m = modes_of(kc);
@@ -207,8 +226,10 @@ extern "C" bte_status bte_get_spectral(bte_ctx* c, bte_spectral_result* out) {
             double* o = S.out.as<double>() + l * per;
             const double* time = c->d_spec.as<double>() + l * nbins * n + off;
             if (want_w) {
-                S.ticks.upload(grid, s);
-                sync(c);
+                if (pdf_of != kc) {
+                    S.ticks.upload(grid, s);
+                    sync(c);
+                }
                 // (at most 65535 blocks over the modes)
                 const int chunk = int(std::max<std::size_t>(
                     1, std::min({nk, PDF_BYTES / (nw * sizeof(double)), std::size_t(65535) * SPEC_K})));
@@ -216,9 +237,10 @@ extern "C" bte_status bte_get_spectral(bte_ctx* c, bte_spectral_result* out) {
                 for (std::size_t k0 = 0; k0 < nk; k0 += std::size_t(chunk)) {
                     const int kn = int(std::min(std::size_t(chunk), nk - k0));
                     const long long cells = (long long)kn * (long long)nw;
-                    spec_pdf<<<unsigned(std::min<long long>((cells + 255) / 256, 8ll * c->nsm)), 256, 0, s>>>(
-                        S.par.as<double4>(), S.om.as<double>(), int(k0), kn, S.ticks.as<double>(), int(nw),
-                        S.pdf.as<double>());
+                    if (pdf_of != kc)
+                        spec_pdf<<<unsigned(std::min<long long>((cells + 255) / 256, 8ll * c->nsm)), 256, 0, s>>>(
+                            S.par.as<double4>(), S.om.as<double>(), int(k0), kn, S.ticks.as<double>(), int(nw),
+                            S.pdf.as<double>());
                     for (std::size_t b0 = 0; b0 < nbins; b0 += 32768) {  // (grid limit in y)
                         const unsigned bn = unsigned(std::min<std::size_t>(32768, nbins - b0));
                         spec_contract<<<dim3(unsigned((nw + SPEC_T - 1) / SPEC_T), bn, unsigned((kn + SPEC_K - 1) / SPEC_K)),
@@ -227,6 +249,7 @@ extern "C" bte_status bte_get_spectral(bte_ctx* c, bte_spectral_result* out) {
                                                         o + b0 * nw);
                     }
                 }
+                pdf_of = std::size_t(chunk) == nk ? kc : -2;
             }
             if (out->fd_q)
                 spec_fdq<<<unsigned(std::min<std::size_t>((nbins * nq + 255) / 256, std::size_t(8 * c->nsm))), 256, 0, s>>>(
@@ -241,14 +264,10 @@ extern "C" bte_status bte_get_spectral(bte_ctx* c, bte_spectral_result* out) {
             const double Eeff = c->spec_Eeff;
             const double sdT = Eeff / vbox, sj = Eeff * 1e12 * 1e9 * 1e9 / vbox;
             const double sq = Eeff * vcorr * double(nq) / (vbox * 1.0e+12 * hbar);
-            if (want_w)
-                for (int q = 0; q < 3; ++q)
-                    spec_finish<<<unsigned((nw + 127) / 128), 128, 0, s>>>(o + std::size_t(q) * nbins * nw, int(nbins), int(nw),
-                                                                           q == 0 ? sdT : sj, q == 0 ? cv / vcorr : 1.0,
-                                                                           steady ? 0 : 1);
-            if (out->fd_q)
-                spec_finish<<<unsigned((nq + 127) / 128), 128, 0, s>>>(o + 3 * nbins * nw, int(nbins), int(nq), sq, 1.0,
-                                                                       steady ? 0 : 1);
+            SpecFinish f{{sdT, sj, sj, sq}, {cv / vcorr, 1.0, 1.0, 1.0}, {}};
+            for (int q = 0; q < 4; ++q) f.n[q] = q < 3 ? (want_w ? int(nw) : 0) : (out->fd_q ? int(nq) : 0);
+            const std::size_t widest = std::max(nw, nq);
+            spec_finish<<<dim3(unsigned((widest + 31) / 32), 4), 32, 0, s>>>(o, int(nbins), int(nw), f, steady ? 0 : 1);
             ck(cudaGetLastError(), "spectral launch");
         }
         const std::size_t raw_vals = nloc * nbins * n, cnt_vals = nloc * n;
