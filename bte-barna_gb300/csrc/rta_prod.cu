@@ -1379,12 +1379,12 @@ bool launch_prod_grid(const DevTables& T, const GridArgs& A0, double* tally,
     const size_t smem = size_t(3) * T.nboxes * T.nbins * sizeof(double);
     // the adjoint passes run with the tally in global memory
     const bool use_smem = tune.smem_tally != 0 && smem <= 200 * 1024 && adj_pass == 0 && T.ngroups <= 1;
-    // residency variants: 4 blocks of 256 threads per SM (64 registers), 3 (76
+    // residency variants: 4 blocks of 256 threads per SM (64 registers), 3 (79
     // registers) or 2 (no register cap); the shared-memory tally allows one
     // block per SM.  Four hide the table reads better once every lane carries
-    // several particles in turn (2e6 on 36864 modes: 111 ms against 118 with
-    // three), three leave fewer lanes idle at the end of a short run (2e5:
-    // 0.53 ms against 0.61; 1e6: 3.36 and 3.38, the same).
+    // several particles in turn (2e6 on 36864 modes: 112.6 ms against 115.0
+    // with three; 4e6 on 6144 modes 17.2 against 16.9), three leave fewer lanes
+    // idle at the end of a short run (1e6: 3.03 ms against 3.17).
     const bool tuned = tune.block_threads > 0 || tune.blocks_per_sm > 0 || use_smem;
     if (!tuned && !T.checks)
         A.lanes = particle_lanes(n, nsm);
