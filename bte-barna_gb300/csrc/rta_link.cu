@@ -440,8 +440,9 @@ __device__ __forceinline__ int slow_down(ModeFix& m, double dt, int kt) {
 // of 2e5 particles, 42 generations, 2.0 ms now).
 __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant__ DevTables T,
                                                           const __grid_constant__ SteadyArgs S,
-                                                          const __grid_constant__ LinkArgs A, double* tally,
+                                                          const __grid_constant__ LinkArgs A, double* gtally,
                                                           unsigned long long* counters, int* err) {
+    double* tally = gtally + (long long)(blockIdx.x % T.ncopies) * T.group_stride;
     Counters c = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     const int lane = threadIdx.x & 31;
     const FixScale& F = A.fx;
