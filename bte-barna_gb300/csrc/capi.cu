@@ -1179,25 +1179,6 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         const int ngroups = c->ngroups > 1 ? c->ngroups : 1;
         const std::size_t tally_bytes =
             replay ? nk * 6 * sizeof(unsigned long long) : nk * 3 * sizeof(double) * std::size_t(ngroups);
-        // A small tally is hit by all SMs at few places (the cells next to the
-        // reservoirs, the first bins), and reductions on one address serialise
-        // in L2: 1.25e5 B took 4.25 ms with one copy, 3.54 with two, 3.41 with
-        // four, 3.38 with eight and no less with more (1e6 particles, 5200
-        // keys; 2e5 particles, 1080 keys: 1.17, 0.75, 0.58, 0.53).  Copies
-        // beyond 16 MB in all only fill L2 (11.6 MB: 118.0 ms with one, 118.8
-        // with eight).
-        int ncopies = 1;
-        if ((grid_run || link_run) && ngroups == 1)
-            ncopies = int(std::clamp<std::size_t>((std::size_t(16) << 20) / tally_bytes, 1, 8));
-        const std::size_t run_bytes = RUN_HEAD + tally_bytes * std::size_t(ncopies);
-        c->d_run.alloc(run_bytes);
-        ck(cudaMemsetAsync(c->d_run.p, 0, run_bytes, c->stream), "memset");
-        char* base = c->d_run.as<char>();
-        auto* counters = reinterpret_cast<unsigned long long*>(base);
-        auto* work = reinterpret_cast<unsigned long long*>(base + 128);
-        auto* err = reinterpret_cast<int*>(base + RUN_ERR);
-        auto* tally = reinterpret_cast<double*>(base + RUN_HEAD);
-
         // Eeff (src/RTA_MC2D.cpp:2177) and the particle range
         double Eeff;
         long long total;
@@ -1211,6 +1192,28 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         long long pbeg = std::max<long long>(0, p->particle_begin);
         long long pend = p->particle_end > 0 ? std::min<long long>(p->particle_end, total) : total;
         if (pend < pbeg) pend = pbeg;
+
+        // A small tally is hit by all SMs at few places (the cells next to the
+        // reservoirs, the first bins), and reductions on one address serialise
+        // in L2: 1.25e5 B took 4.25 ms with one copy, 3.54 with two, 3.41 with
+        // four, 3.38 with eight (1e6 particles, 5200 keys; 2e5 particles, 1080
+        // keys: 1.17, 0.75, 0.58, 0.53), and of that 1 % less with 32; a periodic
+        // bar of 14 boxes (2e6 particles, 1400 keys) 1.79 with eight, 1.45 with
+        // 32.  A run too small to fill the GPU takes four (2e4 particles: 658 us
+        // with one, 628 with four, 634 with 32).  Copies beyond 16 MB in all only
+        // fill L2 (11.6 MB: 118.0 ms with one, 118.8 with eight).
+        int ncopies = 1;
+        if ((grid_run || link_run) && ngroups == 1)
+            ncopies = int(std::clamp<std::size_t>((std::size_t(16) << 20) / tally_bytes, 1,
+                                                  bte::particle_lanes(pend - pbeg, c->nsm) < 32 ? 4 : 32));
+        const std::size_t run_bytes = RUN_HEAD + tally_bytes * std::size_t(ncopies);
+        c->d_run.alloc(run_bytes);
+        ck(cudaMemsetAsync(c->d_run.p, 0, run_bytes, c->stream), "memset");
+        char* base = c->d_run.as<char>();
+        auto* counters = reinterpret_cast<unsigned long long*>(base);
+        auto* work = reinterpret_cast<unsigned long long*>(base + 128);
+        auto* err = reinterpret_cast<int*>(base + RUN_ERR);
+        auto* tally = reinterpret_cast<double*>(base + RUN_HEAD);
 
         bte::DevTables T{};
         T.n = int(m.n());

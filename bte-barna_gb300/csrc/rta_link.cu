@@ -168,8 +168,8 @@ __device__ __noinline__ int link_generate(const DevTables& T, long long pid, Phi
 //   pending displacement goes on.
 // In doubles the polygon kernel took 160 registers (one block of 256 threads
 // per SM) and 42 to 124 FP64 operations per event.  GB300: periodic bar
-// (2e6 particles, 10 strips, 100 bins) 10.1 -> 1.80 ms, two-crystal ribbon (3e5
-// particles) 1.79 -> 0.71 ms, of 2e3 particles 0.17.
+// (2e6 particles, 10 strips, 100 bins) 10.1 -> 1.45 ms, two-crystal ribbon (3e5
+// particles) 1.79 -> 0.70 ms, of 2e3 particles 0.17.
 template <bool CORNER>
 __global__ void __launch_bounds__(256, 2) rta_prod_link(const __grid_constant__ DevTables T,
                                                         const __grid_constant__ LinkArgs A, double* gtally,
@@ -436,8 +436,8 @@ __device__ __forceinline__ int slow_down(ModeFix& m, double dt, int kt) {
 // periods are taken at once: every box of the row gets its share of their
 // time and displacement.  Flights that run along the periodic direction cross
 // hundreds of boxes, one after the other on one lane, and were what a
-// generation waited for (3.6e6 crossings of 3.6e5 flights; 37 ms for a ribbon
-// of 2e5 particles, 42 generations, 2.0 ms now).
+// generation waited for (3.6e6 crossings of 3.6e5 flights: 30 ms in doubles for a
+// ribbon of 2e5 particles, 42 generations, now 1.25).
 __global__ void __launch_bounds__(128, 4) rta_steady_link(const __grid_constant__ DevTables T,
                                                           const __grid_constant__ SteadyArgs S,
                                                           const __grid_constant__ LinkArgs A, double* gtally,
