@@ -13,8 +13,9 @@
 //     Ntogenerate src/sampling.cpp:243-260)
 //                                                   be_plan, be_advance
 //   4 adiabatic diffuse re-emission of |Eborder| at the wall temperature from
-//     the J(T) cubic spline (adiabatic_diffuse_walls :281-435)
-//                                                   be_plan, be_advance
+//     the J(T) cubic spline (adiabatic_diffuse_walls :281-435), Eborder with
+//     what 1 to 3 left there in this step and the re-emitted particles of the
+//     last one                                      be_plan, be_advance
 //   5 deletion of the absorbed particles, 6 propagator scattering with sign
 //     branching (Scattering :1073-1210, propagator_H::get
 //     src/collision_operator.cpp:892-903), each parent's branching attempts
@@ -697,16 +698,20 @@ __device__ __forceinline__ void cancel_body(PArr P, long long n, const int* H, i
 // The device's clock in ns, written at the phase borders of a step: an event
 // between two kernels kept the stream for 2 us (seven were 14 of a step's 150).
 struct Stamps {
-    // the starts of the advance, the plan, the new particles' pass, the
-    // cancellation and the properties; the histogram read; the step's end
-    unsigned long long t[7];
+    // the starts of the advance, the plan, the re-emitted particles' pass, the
+    // cancellation and the properties; the histogram read; the step's end;
+    // the start of the sources' pass (where there are any)
+    unsigned long long t[8];
 };
+constexpr int STAMP_SOURCES = 7;
 // A step's kernels follow one another without a gap: each is launched as its
 // predecessor's blocks end (after_previous) and reads nothing before that one
-// is done.  With the 4 or 6 launches of a step 3.72 -> 3.37 ms for 30 steps of
-// the propagator, 2.89 -> 2.45 for 40 of RTA; launched as soon as all the
-// predecessor's blocks run (launch_dependents), 4.0 and 2.58: the waiting
-// blocks take room on the SMs from the ones that work.
+// is done.  With one pass for all new particles (4 or 6 launches a step) that
+// made 3.37 of 3.72 ms for 30 steps of the propagator and 2.45 of 2.89 for 40 of
+// RTA; launched as soon as all the predecessor's blocks run (launch_dependents),
+// 4.0 and 2.58: the waiting blocks take room on the SMs from the ones that work.
+// With the sources' particles in a pass before the walls' plan (5 or 7
+// launches) 3.59 and 2.96.
 __device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <class... P, class... A>
 void after_previous(void (*f)(P...), unsigned blocks, cudaStream_t s, A&&... args) {
@@ -736,7 +741,9 @@ constexpr int PROPS_PARTS = 8;
 // Counters of the step loop, kept on the device between kernels.
 // DC_IN and DC_OUTT sum the particles read and written by be_advance over
 // the run (the algorithmic traffic of its roofline).
-enum { DC_NP = 0, DC_NOUT, DC_NGEN, DC_FLIPS, DC_PSTEPS, DC_IN, DC_OUTT, DC_COUNT = 8 };
+// DC_NSRC: the new particles of the gradient source and the isothermal walls,
+// DC_NGEN: of the adiabatic walls.
+enum { DC_NP = 0, DC_NOUT, DC_NGEN, DC_FLIPS, DC_PSTEPS, DC_IN, DC_OUTT, DC_NSRC, DC_COUNT = 8 };
 
 // The end of a step: without a cancellation its output is the population;
 // records the particles alive, adds up the outputs, and clears the step's
@@ -745,7 +752,7 @@ __device__ __forceinline__ void close_step(unsigned long long* dc, int swap, lon
     if (swap) dc[DC_NP] = dc[DC_NOUT];
     *record = (long long)dc[DC_NP];
     dc[DC_OUTT] += dc[DC_NOUT];
-    dc[DC_NOUT] = dc[DC_NGEN] = 0;
+    dc[DC_NOUT] = 0;
 }
 
 __global__ void __launch_bounds__(256) be_props(const int* H, int nmodes, const double* vx, const double* vy, double* out,
@@ -794,7 +801,7 @@ __global__ void __launch_bounds__(256) be_props(const int* H, int nmodes, const 
     }
 }
 
-// A source planned on the device: how many particles it makes.
+// The gradient source's particles of a step, planned on the device.
 struct SrcSpan {
     unsigned long long total;
 };
@@ -822,19 +829,6 @@ __device__ unsigned long long warp_scan_first(const long long* cnt, int n, GenDe
         carry += __shfl_sync(0xffffffffu, incl, 31);
     }
     return carry;
-}
-
-// Adds `total` to the step's new particles, within the capacity (a source that
-// would overflow it sets BTE_ERR_LIMIT and makes nothing).
-__device__ void claim_span(unsigned long long total, unsigned long long* dc, SrcSpan* span, long long cap,
-                           int* err) {
-    const unsigned long long base = dc[DC_NGEN];
-    if ((long long)(base + total) > cap) {
-        atomicCAS(err, 0, E_LIMIT);
-        total = 0;
-    }
-    span->total = total;
-    dc[DC_NGEN] = base + total;
 }
 
 // A void border's adiabatic re-emission, tabulated per run: its segment,
@@ -884,7 +878,7 @@ struct SourceSet {
 };
 struct SourceSets {
     SourceSet s[3];              // gradient boxes, isothermal walls, adiabatic walls
-    unsigned long long pkey[2];  // of the stochastic rounding
+    unsigned long long pkey[2];  // of the next step's stochastic rounding
 };
 
 // The temperature whose isothermal flux carries the energy that border A
@@ -900,13 +894,18 @@ __device__ __forceinline__ double wall_temperature(const WallPlan& W, const AdiB
     return spline_eval(W.S, A.spline, W.Eeff * E / W.dtstep / (A.len * W.thickness));
 }
 
-// The step's sources, by the first block.  Gradient and isothermal walls: the
-// numbers by Ntogenerate's stochastic rounding (src/sampling.cpp:166-183,
-// :243-260), one Philox block per source.  Adiabatic walls: each re-emitting
-// border re-emits |Eborder| particles at its wall temperature.  The other
-// blocks make the CDF rows of the borders that re-emit, a chunk of modes each;
-// they find their border's temperature themselves (as a launch of their own
-// after the plan the two took 16 us of a step, together 9).
+// By the first block, the re-emission of this step's adiabatic walls and the
+// sources of the next step.  Adiabatic walls: each re-emitting border re-emits
+// |Eborder| particles at its wall temperature, |Eborder| with what the step's
+// other particles left there, so the plan comes after the pass that makes
+// them.  Gradient and isothermal walls: the numbers by Ntogenerate's stochastic
+// rounding (src/sampling.cpp:166-183, :243-260), one Philox block per source;
+// they depend on nothing else and are drawn a step ahead, so that their pass
+// needs no plan of its own in front (step 0's by a launch without borders).
+// More of them than the particle buffers hold fail in the step that makes
+// them.  The other blocks make the CDF rows of the borders that re-emit, a
+// chunk of modes each; they find their border's temperature themselves (as a
+// launch of their own after the plan the two took 16 us of a step, together 9).
 __global__ void __launch_bounds__(256) be_plan(const __grid_constant__ SourceSets Q, const int* Eb,
                                                const __grid_constant__ WallPlan W, int nmodes, unsigned long long* dc,
                                                SrcSpan* span, long long cap, int* err, Stamps* st) {
@@ -921,7 +920,7 @@ __global__ void __launch_bounds__(256) be_plan(const __grid_constant__ SourceSet
         wall_cdf_body(W.om, W.vx, W.vy, nmodes, R, r, ch, W.cdf, W.chunk_tot);
         return;
     }
-    if (threadIdx.x == 0) stamp(st->t + 1);
+    if (st && threadIdx.x == 0) stamp(st->t + 1);
     for (int q = 0; q < 2; ++q)
         for (int k = threadIdx.x; k < Q.s[q].ngen; k += 256) {
             Philox g;
@@ -959,15 +958,23 @@ __global__ void __launch_bounds__(256) be_plan(const __grid_constant__ SourceSet
         if ((threadIdx.x & 31) == 0) total[w] = t;
     }
     __syncthreads();
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 3; ++q) claim_span(total[q], dc, span + q, cap, err);
+    if (threadIdx.x == 0) {
+        if (dc[DC_NSRC] + total[2] > (unsigned long long)cap) {
+            atomicCAS(err, 0, E_LIMIT);
+            total[2] = 0;
+        }
+        dc[DC_NGEN] = total[2];
+        dc[DC_NSRC] = total[0] + total[1];
+        span->total = total[0];
+    }
 }
 
-// New particle i of a step (the sources of steps 2-4 of the reference's loop),
-// advected for a random part of the step; false where it is absorbed on the
-// way or has no place or mode.
+// New particle i of a pass (the sources of steps 2 and 3 of the reference's
+// loop, or with `walls` of step 4), advected for a random part of the step;
+// false where it is absorbed on the way or has no place or mode.
 struct MakeArgs {
-    const SrcSpan* span;
+    bool walls;
+    const SrcSpan* span;  // of the gradient source; the isothermal walls' particles follow
     SourceSets Q;
     const double* cdfs;
     const double* ctot;
@@ -977,9 +984,9 @@ struct MakeArgs {
 template <bool GENERAL>
 __device__ __forceinline__ bool make_particle(const MakeArgs& M, const AdvectArgs& aa, int nmodes, long long i, double& x,
                                               double& y, int& box, int& mode, int& sign) {
-    const long long t0 = (long long)M.span[0].total, t1 = t0 + (long long)M.span[1].total;
-    const int q = i < t0 ? 0 : i < t1 ? 1 : 2;
-    const long long k = i - (q == 0 ? 0 : q == 1 ? t0 : t1);
+    const long long t0 = M.walls ? 0 : (long long)M.span->total;
+    const int q = M.walls ? 2 : i < t0 ? 0 : 1;
+    const long long k = i - (q == 1 ? t0 : 0);
     const SourceSet& Z = M.Q.s[q];
     const GenDesc* gens = Z.descs;
     int lo = 0, hi = Z.ngen;
@@ -1047,8 +1054,9 @@ __device__ __forceinline__ bool make_particle(const MakeArgs& M, const AdvectArg
 constexpr unsigned BRANCH_CAP = 1u << 20;
 
 // One step of the particles [0, *n_in) of `in`, fused: advection by the
-// step, or with MAKE the step's new particles [0, *n_in), each made (and
-// advected for a part of the step) by the lane that takes it; then the scattering of the survivors -- RTA (ScatteringRTA,
+// step, or with MAKE the new particles [0, *n_in) of the step's sources or of
+// its walls, each made (and advected for a part of the step) by the lane that
+// takes it; then the scattering of the survivors -- RTA (ScatteringRTA,
 // src/beyondRTA_MC2d.cpp:983-1062, a resampling with probability
 // 1 - exp(-w dt), as a 53-bit threshold per mode) or the propagator with sign
 // branching as above -- and the histogram H[box][mode] += sign of every
@@ -1088,14 +1096,17 @@ __global__ void __launch_bounds__(256, GENERAL ? 2 : MAKE && !RTA ? 4 : 3)
                const BoxProp* bprop, int nm, const unsigned long long* pscat, const int2* resample, int nmodes, unsigned long long skey, int* H, int* err,
                Stamps* st) {
     await_previous();
-    if (blockIdx.x == 0 && threadIdx.x == 0) stamp(st->t + (MAKE ? 2 : 0));
+    if (blockIdx.x == 0 && threadIdx.x == 0) stamp(st->t + (!MAKE ? 0 : ma.walls ? 2 : STAMP_SOURCES));
     __shared__ AdvBuf bufs[8];
     AdvBuf& buf = bufs[threadIdx.x >> 5];
-    const long long n = min((long long)*n_in, ocap);  // places beyond the buffers (an overflow) are not read
+    // places beyond the buffers (an overflow) are not read, nor as many made
+    const unsigned long long number = *n_in;
+    const long long n = number <= (unsigned long long)ocap ? (long long)number : MAKE ? 0 : ocap;
     const int lane = threadIdx.x & 31;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) {
-        if (!MAKE) atomicAdd(dc + DC_PSTEPS, (unsigned long long)n);
-        atomicAdd(dc + DC_IN, (unsigned long long)n);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (MAKE && number > (unsigned long long)ocap) atomicCAS(err, 0, E_LIMIT);
+        if (!MAKE && n > 0) atomicAdd(dc + DC_PSTEPS, (unsigned long long)n);
+        if (n > 0) atomicAdd(dc + DC_IN, (unsigned long long)n);
     }
     // the warp's run
     const long long warps = (long long)gridDim.x * 8, per = max(32ll, ((n + warps - 1) / warps + 7) / 8 * 8);
@@ -1940,7 +1951,7 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
         for (double t = 0.; t <= p->maxtime; t += p->dt) ++nsteps;
         B.d_dc.alloc(DC_COUNT * sizeof(unsigned long long));
         auto* dc = B.d_dc.as<unsigned long long>();
-        B.d_span.alloc(3 * sizeof(SrcSpan));
+        B.d_span.alloc(sizeof(SrcSpan));
         SrcSpan* span = B.d_span.as<SrcSpan>();
         {
             std::vector<unsigned long long> h0(DC_COUNT, 0ull);
@@ -2044,6 +2055,20 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
                            B.d_isoprob.as<float>(), B.d_isoalt.as<int>(), nullptr, 0, 0, 0};
         Q.s[2] = SourceSet{B.d_adesc.as<GenDesc>(), nullptr, B.d_acnt.as<long long>(), nborders, nullptr, nullptr, nullptr,
                            0, 0, 0};
+        const bool sources = ngd + nid > 0;
+        // the walls' re-emission in a step (none before the first) and the
+        // numbers of the next one's gradient and isothermal particles (none
+        // after the last)
+        auto plan = [&](bool walls, int next) {
+            SourceSets q = Q;
+            if (!walls) q.s[2].ngen = 0;
+            if (next >= nsteps) q.s[0].ngen = q.s[1].ngen = 0;
+            q.pkey[0] = mix_key(p->seed, next, 40);
+            q.pkey[1] = mix_key(p->seed, next, 41);
+            after_previous(be_plan, 1u + (walls ? unsigned(nborders) * unsigned(nch) : 0u), s, q, Eb, WP, n, dc, span, cap,
+                           err, st);
+        };
+        if (sources) plan(false, 0);
         while (time <= p->maxtime && istep < nsteps) {
             st = B.d_stamps.as<Stamps>() + istep;
             std::swap(H, next_H);
@@ -2055,7 +2080,6 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             advance(general ? (p->rta ? be_advance<true, true, false> : be_advance<true, false, false>)
                             : (p->rta ? be_advance<false, true, false> : be_advance<false, false, false>),
                     ablocks, A, dc + DC_NP, a_step, MakeArgs{}, mix_key(p->seed, istep, 64));
-            // 2-4 the step's sources
             auto keys = [&](SourceSet& q, int ph) {
                 q.key = mix_key(p->seed, istep, ph);
                 q.akey = mix_key(p->seed, istep, ph + 1);
@@ -2064,16 +2088,21 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             keys(Q.s[0], 8);
             keys(Q.s[1], 2);
             keys(Q.s[2], 4);
-            Q.pkey[0] = mix_key(p->seed, istep, 40);
-            Q.pkey[1] = mix_key(p->seed, istep, 41);
-            after_previous(be_plan, 1u + unsigned(nborders) * unsigned(nch), s, Q, Eb, WP, n, dc, span, cap, err, st);
+            MakeArgs ma{false, span, Q, B.d_cdf.as<double>(), B.d_ctot.as<double>(), c->d_boxes.as<GBox>(), c->d_hull.as<V2>()};
             // the new particles made; 5-7 for them: the absorbed ones dropped, the
             // others scattered and counted in the histogram, appended to B
-            a_step.Eb = next_Eb;  // (what they leave on the walls is planned in the next step)
-            const MakeArgs ma{span, Q, B.d_cdf.as<double>(), B.d_ctot.as<double>(), c->d_boxes.as<GBox>(), c->d_hull.as<V2>()};
-            advance(general ? (p->rta ? be_advance<true, true, true> : be_advance<true, false, true>)
-                            : (p->rta ? be_advance<false, true, true> : be_advance<false, false, true>),
-                    pblocks, A, dc + DC_NGEN, a_step, ma, mix_key(p->seed, istep, 65));
+            auto make = [&](const unsigned long long* number, int phase_key) {
+                advance(general ? (p->rta ? be_advance<true, true, true> : be_advance<true, false, true>)
+                                : (p->rta ? be_advance<false, true, true> : be_advance<false, false, true>),
+                        pblocks, A, number, a_step, ma, mix_key(p->seed, istep, phase_key));
+            };
+            // 2 and 3, into the walls' counts of this step
+            if (sources) make(dc + DC_NSRC, 65);
+            // 4
+            plan(true, istep + 1);
+            a_step.Eb = next_Eb;  // what the re-emitted particles leave on the walls is for the next step
+            ma.walls = true;
+            make(dc + DC_NGEN, 66);
             // 8. cancellation every cancel_every steps: B -> A; otherwise B is the population
             const bool cancel = istep % cancel_every == 0;
             if (cancel) {
@@ -2149,14 +2178,15 @@ extern "C" bte_status bte_berta_run(bte_ctx* c, const bte_berta_params* p, bte_b
             branchings = (long long)hdc[DC_FLIPS];
             adv_in = (long long)hdc[DC_IN];
             adv_out = (long long)hdc[DC_OUTT];
-            // (scattering: the pass that makes and scatters the new particles;
-            // histogram: its reading, both passes having counted it)
+            // (scattering: the passes that make and scatter the new particles;
+            // histogram: its reading, all passes having counted it)
             for (int k = 0; k < istep; ++k) {
                 const unsigned long long* t = hst[std::size_t(k)].t;
                 const unsigned long long made = k % cancel_every == 0 ? t[3] : t[4];
-                const unsigned long long at[7] = {t[0], t[1], t[2], made, t[4], t[5], t[6]};
-                const int bucket[6] = {PH_ADV, PH_GEN, PH_SCAT, PH_CANCEL, PH_HIST, PH_PROPS};
-                for (int q = 0; q < 6; ++q) phase[bucket[q]] += 1e-6 * double((long long)(at[q + 1] - at[q]));
+                const unsigned long long src = sources ? t[STAMP_SOURCES] : t[1];
+                const unsigned long long at[8] = {t[0], src, t[1], t[2], made, t[4], t[5], t[6]};
+                const int bucket[7] = {PH_ADV, PH_SCAT, PH_GEN, PH_SCAT, PH_CANCEL, PH_HIST, PH_PROPS};
+                for (int q = 0; q < 7; ++q) phase[bucket[q]] += 1e-6 * double((long long)(at[q + 1] - at[q]));
             }
         }
         ck(cudaEventRecord(c->ev1, s), "event");
