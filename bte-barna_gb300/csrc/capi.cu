@@ -893,7 +893,7 @@ bte_status bte_set_tuning(bte_ctx* c, const bte_tuning* t) {
 
 bte_status bte_load_modes(bte_ctx* c, const bte_mode_table* mt) {
     if (!c) return BTE_ERR_INPUT;
-    c->group_valid = false;
+    c->group_valid = c->spec_valid = false;
     try {
         ck(cudaSetDevice(c->device), "cudaSetDevice");
         c->modes = bte::build_modes(mt);
@@ -920,7 +920,7 @@ bte_status bte_load_modes(bte_ctx* c, const bte_mode_table* mt) {
 
 bte_status bte_load_geometry(bte_ctx* c, const bte_geometry* g) {
     if (!c) return BTE_ERR_INPUT;
-    c->group_valid = false;
+    c->group_valid = c->spec_valid = false;
     try {
         ck(cudaSetDevice(c->device), "cudaSetDevice");
         bte::HostGeometry ng = bte::build_geometry(g);
@@ -947,7 +947,7 @@ bte_status bte_load_geometry(bte_ctx* c, const bte_geometry* g) {
 bte_status bte_load_mode_tables(bte_ctx* c, int32_t ntables, const bte_mode_table* tables,
                                 const double* thickness) {
     if (!c) return BTE_ERR_INPUT;
-    c->group_valid = false;
+    c->group_valid = c->spec_valid = false;
     try {
         if (ntables < 1 || !tables) throw Error(BTE_ERR_INPUT, "no mode tables");
         std::vector<double> th;
@@ -1054,6 +1054,8 @@ bte_status bte_load_materials(bte_ctx* c, int32_t nmat, const double* w, const d
             c->shares_dirty = true;
             return BTE_OK;
         }
+        // (the spectral outputs are formed with the run's materials)
+        if (!same_rates && (nmat > 0 || c->nmat > 0)) c->spec_valid = false;
         c->nmat = nmat;
         c->mat_w.assign(w ? w : nullptr, w ? w + size_t(nmat) * n : nullptr);
         c->mat_T0.assign(T0 ? T0 : nullptr, T0 ? T0 + nmat : nullptr);
@@ -1271,6 +1273,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         T.group_stride = (long long)(nk * 3);
         T.ncopies = ncopies;
         // spectral decomposition: per-mode time at the selected boxes
+        c->spec_valid = false;
         const std::size_t nloc = c->spec_boxes.size();
         const std::size_t spec_vals = nloc * std::size_t(nbins) * m.n();
         if (nloc > 0) {
@@ -1285,7 +1288,6 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
             T.spec = c->d_spec.as<double>();
             T.spec_ex = c->d_spec.as<unsigned long long>();
         }
-        c->spec_valid = false;
 
         bte::PostUnits units;
         ck(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
@@ -1326,14 +1328,6 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         int herr[4];
         std::memcpy(hc, c->h_out.p, sizeof hc);
         std::memcpy(herr, static_cast<const char*>(c->h_out.p) + RUN_ERR, sizeof herr);
-        if (nloc > 0) {  // the tally stays on the device for bte_get_spectral
-            if (replay) bte::spec_from_exact(c, spec_vals);
-            c->spec_unit = grid_run || link_run ? A.fx.per_tick() : 1.;
-            c->spec_nbins = nbins;
-            c->spec_T0 = p->T0;
-            c->spec_steady = false;
-            c->spec_valid = true;
-        }
         float ms = 0;
         ck(cudaEventElapsedTime(&ms, c->ev0, c->ev1), "cudaEventElapsedTime");
         out->kernel_ms = ms;
@@ -1346,6 +1340,15 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
                           : herr[0] == BTE_ERR_CHECK ? "index check failed"
                                                       : "geometry error");
             throw Error(bte_status(herr[0]), msg);
+        }
+        if (nloc > 0) {  // the tally stays on the device for bte_get_spectral
+            if (replay) bte::spec_from_exact(c, spec_vals);
+            c->spec_unit = grid_run || link_run ? A.fx.per_tick() : 1.;
+            c->spec_nbins = nbins;
+            c->spec_T0 = p->T0;
+            c->spec_Eeff = Eeff;
+            c->spec_steady = false;
+            c->spec_valid = true;
         }
         if (ngroups > 1) {  // the groups' tallies stay on the device
             c->group_n = ngroups;
@@ -1376,7 +1379,6 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         out->nboxes = nbx;
         out->nbins = nbins;
         out->Eeff = Eeff;
-        c->spec_Eeff = Eeff;
         out->energy_rate = c->gens.total_energy;
         out->events = (int64_t)hc[0];
         out->wall_hits = (int64_t)hc[1];

@@ -456,7 +456,9 @@ bte_status bte_set_spectral(bte_ctx* ctx, int32_t nloc, const int32_t* boxes, in
  *   fd_q      the distribution per q point (fd_q_*.csv); after a steady run
  *             the reference adds sign / omega per segment, not per time
  * with omega[nloc][nomega] the tick centres and q1bz[nq][2] the q points.
- * Any pointer may be NULL. */
+ * Any pointer may be NULL.  Formed with the tables of the run: other modes,
+ * boxes or materials loaded since, or a last run that failed, make it
+ * BTE_ERR_STATE. */
 typedef struct bte_spectral_result {
     int32_t nloc, nbins, nomega, nq;   /* out */
     double* omega;

@@ -1,0 +1,62 @@
+"""bte_get_spectral forms the last run's outputs from a tally on the device,
+with the tables it was made with: once other modes, crystals, boxes or
+materials are loaded, or the last run failed, there is nothing to form."""
+import numpy as np
+import pytest
+
+import btegpu
+import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def run(engine):
+    case = synth.small_case(n_particles=2000)
+    bins = int(round(case["maxtime"] / case["dt"]))
+
+    def go(**kw):
+        engine.load_modes(case["modes"])
+        engine.load_geometry(case["geom"])
+        engine.set_spectral([1, 3], nomega=50)
+        engine.rta_run(case["T0"], case["dt"], case["maxtime"], case["N"], seed=4, **kw)
+        return engine.get_spectral(bins)
+
+    yield case, bins, go
+    engine.load_modes(case["modes"])
+    engine.load_geometry(case["geom"])
+    engine.set_spectral([])
+
+
+LOADS = {
+    "larger mode table": lambda e, c: e.load_modes(synth.mode_table(32, 3, 3, 300.0, config=100)),
+    "smaller mode table": lambda e, c: e.load_modes(synth.mode_table(5, 3, 3, 300.0, config=100)),
+    "crystals": lambda e, c: e.load_mode_tables([c["modes"], c["modes"]]),
+    "geometry": lambda e, c: e.load_geometry(synth.ribbon_geometry(100.0, 50.0, 2)),
+    "materials": lambda e, c: e.load_materials([c["modes"]["w"]] * 2, [c["T0"], c["T0"] + 10.0]),
+}
+
+
+@pytest.mark.parametrize("what", sorted(LOADS))
+def test_other_tables_end_the_spectral_outputs(engine, run, what):
+    case, bins, go = run
+    first = go()
+    LOADS[what](engine, case)
+    with pytest.raises(btegpu.BteError) as ex:
+        engine.get_spectral(bins)
+    assert ex.value.code == btegpu.BTE_ERR_STATE
+    again = go()
+    assert again["raw"].shape == first["raw"].shape
+    assert np.allclose(again["raw"], first["raw"], rtol=1e-9, atol=1e-12 * np.abs(first["raw"]).max())
+
+
+@pytest.mark.parametrize("mode", [btegpu.MODE_PRODUCTION, btegpu.MODE_REPLAY])
+def test_a_failed_run_leaves_no_spectral_outputs(engine, run, mode):
+    case, bins, go = run
+    go()
+    with pytest.raises(btegpu.BteError) as ex:
+        go(mode=mode, flight_cap=3)
+    assert ex.value.code == btegpu.BTE_ERR_LIMIT
+    with pytest.raises(btegpu.BteError) as ex:
+        engine.get_spectral(bins)
+    assert ex.value.code == btegpu.BTE_ERR_STATE
