@@ -1277,10 +1277,7 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         const std::size_t nloc = c->spec_boxes.size();
         const std::size_t spec_vals = nloc * std::size_t(nbins) * m.n();
         if (nloc > 0) {
-            std::vector<int>& loc = c->h_specloc;  // (stays until the copy is done)
-            loc.assign(std::size_t(nbx), -1);
-            for (std::size_t i = 0; i < nloc; ++i) loc[std::size_t(c->spec_boxes[i])] = int(i);
-            c->d_specloc.upload(loc, c->stream);
+            bte::upload_spectral_locations(c);
             const std::size_t bytes = spec_vals * (replay ? 2 * sizeof(unsigned long long) : sizeof(double));
             c->d_spec.alloc(bytes);
             ck(cudaMemsetAsync(c->d_spec.p, 0, bytes, c->stream), "memset");
@@ -1794,6 +1791,17 @@ std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step
         g[std::size_t(2 * ntime - 1 + i)] = bitsd(uint64_t(std::llrint(std::ldexp(w, tick_exp))));
     }
     return g;
+}
+
+void upload_spectral_locations(bte_ctx* c) {
+    std::vector<int>& loc = c->h_specloc;  // (stays until the copy is done)
+    loc.assign(c->geom.boxes.size(), -1);
+    for (std::size_t i = 0; i < c->spec_boxes.size(); ++i) {
+        const std::size_t b = std::size_t(c->spec_boxes[i]);  // (of the geometry of bte_set_spectral)
+        if (b >= loc.size()) throw Error(BTE_ERR_INPUT, "spectral location is not a box of the loaded geometry");
+        loc[b] = int(i);
+    }
+    c->d_specloc.upload(loc, c->stream);
 }
 
 // A replay run's 128-bit per-mode tally in c->d_spec, replaced by its values

@@ -199,6 +199,8 @@ void reset_propagators(bte_ctx* c);
 void destroy_steady(bte_ctx* c);
 void destroy_spectral(bte_ctx* c);
 void spec_from_exact(bte_ctx* c, std::size_t vals);
+// The spectral locations as an index per box, into c->d_specloc.
+void upload_spectral_locations(bte_ctx* c);
 // T0 of box b's material (the run's T0 without materials).
 double box_T0(const bte_ctx* c, int b, double T0);
 // Validation and tables of one RTA run (capi.cu).

@@ -316,10 +316,7 @@ bte_status bte_steady_run(bte_ctx* c, const bte_steady_params* p, bte_steady_res
         const size_t spec_vals = nloc * size_t(n);
         c->spec_valid = false;
         if (nloc > 0) {
-            std::vector<int>& loc = c->h_specloc;  // (stays until the copy is done)
-            loc.assign(size_t(nbx), -1);
-            for (size_t i = 0; i < nloc; ++i) loc[size_t(c->spec_boxes[i])] = int(i);
-            c->d_specloc.upload(loc, st);
+            upload_spectral_locations(c);
             const size_t bytes = spec_vals * (replay ? 2 * sizeof(unsigned long long) : sizeof(double));
             c->d_spec.alloc(bytes);
             c->d_speccnt.alloc(spec_vals * sizeof(unsigned long long));

@@ -50,6 +50,24 @@ def test_other_tables_end_the_spectral_outputs(engine, run, what):
     assert np.allclose(again["raw"], first["raw"], rtol=1e-9, atol=1e-12 * np.abs(first["raw"]).max())
 
 
+@pytest.mark.parametrize("steady", [False, True])
+def test_locations_beyond_a_smaller_geometry_are_refused(engine, run, steady):
+    """Location 7 of eight boxes, then a geometry of five: no run starts."""
+    case, bins, go = run
+    engine.load_modes(case["modes"])
+    engine.load_geometry(synth.periodic_cell_geometry(40.0, 40.0, 2, 2))
+    engine.set_spectral([7], nomega=50)
+    engine.load_geometry(synth.periodic_cell_geometry(40.0, 40.0, 1, 1))
+    with pytest.raises(btegpu.BteError) as ex:
+        if steady:
+            engine.steady_run(300.0, (0.01, 0.0), 1000)
+        else:
+            engine.load_geometry(synth.ribbon_geometry(100.0, 50.0, 3))
+            engine.rta_run(300.0, 10.0, 100.0, 1000)
+    assert ex.value.code == btegpu.BTE_ERR_INPUT and "spectral" in str(ex.value)
+    go()
+
+
 @pytest.mark.parametrize("mode", [btegpu.MODE_PRODUCTION, btegpu.MODE_REPLAY])
 def test_a_failed_run_leaves_no_spectral_outputs(engine, run, mode):
     case, bins, go = run
