@@ -1176,8 +1176,8 @@ bte_status bte_rta_run(bte_ctx* c, const bte_rta_params* p, bte_rta_result* out)
         const int nbx = int(g.boxes.size());
         const std::size_t nk = std::size_t(nbx) * std::size_t(nbins);
         c->group_valid = false;
-        if (c->ngroups > 1 && (replay || !g.rect_grid))
-            throw Error(BTE_ERR_INPUT, "replica groups need production mode on boxes that tile a grid");
+        if (c->ngroups > 1 && !grid_run)  // (no other kernel knows the groups)
+            throw Error(BTE_ERR_INPUT, "replica groups need production mode on boxes of one mode table that tile a grid");
         const int ngroups = c->ngroups > 1 ? c->ngroups : 1;
         const std::size_t tally_bytes =
             replay ? nk * 6 * sizeof(unsigned long long) : nk * 3 * sizeof(double) * std::size_t(ngroups);

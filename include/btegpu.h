@@ -482,7 +482,8 @@ bte_status bte_get_spectral(bte_ctx* ctx, bte_spectral_result* out);
  * reference estimates errors from independent runs (nruns,
  * src/RTA_MC2D.cpp:2099-2101, :2188); a group is one such run made with
  * 1/ngroups of the particles.  ngroups = 0 or 1 switches it off; a replay
- * run or a geometry off a grid fails with BTE_ERR_INPUT while it is on. */
+ * run, a geometry off a grid or several crystals (bte_load_mode_tables) fail
+ * with BTE_ERR_INPUT while it is on. */
 bte_status bte_set_groups(bte_ctx* ctx, int32_t ngroups);
 
 /* Outputs of group `group` of the last run with replica groups, scaled to
