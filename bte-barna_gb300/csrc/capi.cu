@@ -1575,6 +1575,10 @@ bte_status prepared_grid_run(bte_ctx* c, const bte_rta_params* p, PreparedRun* r
         *why = "the allocation-free run needs boxes that tile an axis-aligned grid";
         return BTE_ERR_INPUT;
     }
+    if (c->ncrys > 0 && c->ndmm > 0) {  // (the grid kernel knows no interfaces)
+        *why = "the allocation-free run takes no interfaces between crystals";
+        return BTE_ERR_INPUT;
+    }
     if (c->resample_T0 != (c->nmat > 0 ? -2.0 : p->T0) || c->gen_key_source != p->source ||
         (p->source == BTE_SOURCE_INITIAL &&
          (c->gen_key_n != p->nparticles || c->gen_key_seed != p->seed))) {
