@@ -1336,6 +1336,7 @@ PArr arr(DBuf& x, DBuf& y, DBuf& m, DBuf& b, DBuf& s, long long off = 0) {
 
 void alloc_particles(BertaState& B, long long cap) {
     if (B.cap >= cap) return;
+    B.cap = 0;  // (until all of them are there)
     for (DBuf* d : {&B.a_x, &B.a_y, &B.b_x, &B.b_y})
         d->alloc(size_t(cap) * sizeof(double));
     for (DBuf* d : {&B.a_mode, &B.a_box, &B.a_sign, &B.b_mode, &B.b_box, &B.b_sign, &B.d_rank})

@@ -43,6 +43,11 @@ long long btegpu_debug_fixwalk(const double* gx, int nx, const double* gy, int n
                                const double* tau, const double* vx, const double* vy, int* scales, long long* out,
                                long long cap);
 
+/* What a buffer is kept by (Keyed, ctx.hpp): n updates to keys[i], whose fill
+ * fails where fails[i]; filled[i]: whether the fill ran.  Returns whether the
+ * buffer counts as filled at the end. */
+int btegpu_debug_keyed(const int* keys, const int* fails, int n, int* filled);
+
 /* The host build of bte_log. */
 int btegpu_debug_log(const double* x, double* y, long long n);
 

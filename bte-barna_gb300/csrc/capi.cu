@@ -438,6 +438,7 @@ void ensure_resample(bte_ctx* c, double T0) {
         bte::build_resample(c->modes, T0, cdf, al);
     }
     static_assert(sizeof(bte::Alias) == sizeof(int2) && offsetof(bte::Alias, alt) == 4, "an alias slot is an int2");
+    c->resample_T0 = -1;  // (until all of it is there)
     c->d_rcdf.upload(cdf, c->stream);
     c->d_resample.upload(al, c->stream);
     sync(c);
@@ -457,8 +458,11 @@ using bte::sync;
 // Per-material budgets of a walls-source run: wall w of material m is drawn
 // with probability share[m] E_w / E_m (energy-weighted when no shares).
 void apply_shares(bte_ctx* c, bool upload) {
-    c->shares_dirty = false;
-    if (c->mat_share.empty()) return;
+    if (c->mat_share.empty()) {
+        c->shares_dirty = false;
+        return;
+    }
+    c->shares_dirty = true;  // (until the weights are there)
     const std::size_t nm = c->mat_share.size();
     c->mat_energy.assign(nm, 0.);
     for (auto& W : c->gens.walls) {
@@ -480,6 +484,7 @@ void apply_shares(bte_ctx* c, bool upload) {
         c->d_wcum.upload(c->gens.wall_cum, c->stream);
         sync(c);
     }
+    c->shares_dirty = false;
 }
 
 void ensure_generators(bte_ctx* c, const bte_rta_params* p) {
@@ -487,6 +492,7 @@ void ensure_generators(bte_ctx* c, const bte_rta_params* p) {
         if (p->source == BTE_SOURCE_WALLS && c->shares_dirty) apply_shares(c, true);
         if (p->source == BTE_SOURCE_INITIAL &&
             (c->gen_key_n != p->nparticles || c->gen_key_seed != p->seed)) {
+            c->gen_key_n = -1;  // (until the counts are there)
             c->gen_Eeff = bte::initial_counts(c->gens, p->nparticles, p->seed);
             c->d_ifirst.upload(c->gens.init_first, c->stream);
             sync(c);
@@ -495,6 +501,7 @@ void ensure_generators(bte_ctx* c, const bte_rta_params* p) {
         }
         return;
     }
+    c->gen_key_source = -1;  // (until all of them are there)
     if (c->ncrys > 0) {
         // each crystal's generators, rows over the concatenated modes
         std::vector<bte::Generators> G;
@@ -706,10 +713,7 @@ void device_post(bte_ctx* c, const bte_rta_params* p, int nbx, int nbins, double
         f[2] = cvm ? vcorr / (*cvm)[m] : 0.;
         f[3] = box_T0(c, b, p->T0);
     }
-    if (c->h_boxpost != bp) {
-        c->h_boxpost.swap(bp);  // (stays until the copy is done)
-        c->d_boxpost.upload(c->h_boxpost, c->stream);
-    }
+    c->boxpost.update(std::move(bp), [&](const std::vector<double>& v) { c->d_boxpost.upload(v, c->stream); });
     PostArgs a{};
     a.tally = tally;
     a.ncopies = ncopies;
@@ -1538,6 +1542,21 @@ long long btegpu_debug_fixwalk(const double* gx, int nx, const double* gy, int n
     return m;
 }
 
+int btegpu_debug_keyed(const int* keys, const int* fails, int n, int* filled) {
+    bte::Keyed<int> k;
+    for (int i = 0; i < n; ++i) {
+        filled[i] = 0;
+        try {
+            k.update(keys[i], [&](int) {
+                filled[i] = 1;
+                if (fails[i]) throw Error(BTE_ERR_CUDA, "fill");
+            });
+        } catch (const Error&) {
+        }
+    }
+    return k.valid ? 1 : 0;
+}
+
 int btegpu_debug_log(const double* x, double* y, long long n) {
     for (long long i = 0; i < n; ++i) y[i] = bte::bte_log(x[i]);
     return 0;
@@ -1777,13 +1796,10 @@ void fix_on_device(bte_ctx* c, const FixScale& f) {
 }
 
 void upload_time_grid(bte_ctx* c, int ntime, double maxtime, double step, int tick_exp) {
-    if (c->time_n == ntime && c->time_max == maxtime && c->time_step == step && c->time_exp == tick_exp) return;
-    c->h_time = time_grid_with_widths(ntime, maxtime, step, tick_exp);  // (stays until the copy is done)
-    c->d_time.upload(c->h_time, c->stream);
-    c->time_n = ntime;
-    c->time_max = maxtime;
-    c->time_step = step;
-    c->time_exp = tick_exp;
+    c->time.update(TimeKey{ntime, tick_exp, maxtime, step}, [&](const TimeKey&) {
+        c->h_time = time_grid_with_widths(ntime, maxtime, step, tick_exp);  // (stays until the copy is done)
+        c->d_time.upload(c->h_time, c->stream);
+    });
 }
 
 std::vector<double> time_grid_with_widths(int ntime, double maxtime, double step, int tick_exp) {

@@ -5,6 +5,7 @@
 
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "../../include/btegpu.h"
@@ -14,8 +15,9 @@
 namespace bte {
 
 inline void ck(cudaError_t e, const char* what) {
-    if (e != cudaSuccess)
-        throw Error(BTE_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    cudaGetLastError();  // (a failed allocation is not the next launch's error)
+    throw Error(BTE_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 // Owned device allocation.
@@ -45,6 +47,29 @@ struct DBuf {
     }
     template <class T>
     T* as() const { return static_cast<T*>(p); }
+};
+
+// What a device buffer holds, by a key that determines it.  A fill that fails
+// leaves no key, so the next call fills the buffer again whatever it asks for.
+template <class Key>
+struct Keyed {
+    Key key{};
+    bool valid = false;
+    template <class Fill>
+    void update(Key k, Fill&& fill) {
+        if (valid && key == k) return;
+        valid = false;
+        key = std::move(k);
+        fill(key);  // (a copy from the key itself may still run: it stays)
+        valid = true;
+    }
+};
+
+// A time grid: points, last point, width, and the ticks' exponent.
+struct TimeKey {
+    int n = 0, exp = 0;
+    double max = 0., step = 0.;
+    bool operator==(const TimeKey& o) const { return n == o.n && exp == o.exp && max == o.max && step == o.step; }
 };
 
 // Page-locked host memory, grown as needed and kept: device copies from or
@@ -177,9 +202,9 @@ struct bte_ctx {
     // per-box factors they take, and their page-locked readback
     bte::DBuf d_time, d_run, d_out, d_boxpost, d_err;
     bte::Pinned h_out;
-    std::vector<double> h_boxpost, h_time;   // what d_boxpost and d_time hold
-    int time_n = 0, time_exp = 0;            // and for which grid
-    double time_max = 0., time_step = 0.;
+    bte::Keyed<std::vector<double>> boxpost;  // what d_boxpost holds
+    bte::Keyed<bte::TimeKey> time;            // and the grid in d_time,
+    std::vector<double> h_time;               // copied from here
     // beyond-RTA (berta.cu)
     bte::BertaState* berta = nullptr;
     // periodic / gradient steady state (steady.cu)

@@ -203,6 +203,7 @@ extern "C" bte_status bte_get_spectral(bte_ctx* c, bte_spectral_result* out) {
             if (!compute) continue;
             if (S.crystal != kc || S.version != c->tables_version) {
                 sync(c);  // (an earlier location's kernels may still read them)
+                S.version = -1;  // (until all of them are there)
                 const std::vector<double> sig = mode_sigmas(m);
                 S.hpar.assign(4 * nk, 0.);
                 for (std::size_t k = 0; k < nk; ++k) {
