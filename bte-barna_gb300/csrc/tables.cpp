@@ -245,7 +245,8 @@ HostModes build_modes(const bte_mode_table* mt) {
         m.vz[k] = mt->vg[3 * k + 2];
         m.vxc[k] = almost_equal(m.vx[k], 0.) ? 0. : m.vx[k];
         m.vyc[k] = almost_equal(m.vy[k], 0.) ? 0. : m.vy[k];
-        if (!std::isfinite(m.omega[k]) || !std::isfinite(m.w[k]) || m.w[k] < 0.)
+        if (!std::isfinite(m.omega[k]) || !std::isfinite(m.w[k]) || m.w[k] < 0. || !std::isfinite(m.vx[k]) ||
+            !std::isfinite(m.vy[k]))
             throw Error(BTE_ERR_VALUE, "non-finite or negative mode data");
     }
     std::memcpy(m.dq, mt->dq, sizeof(m.dq));
