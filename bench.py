@@ -304,7 +304,8 @@ def run_berta(args, rank, world, local):
         ps += int(r["particle_steps"])
         kern_ms += float(r["kernel_ms"])
         alive.append(int(r["nparticles"][-1]))
-        # be_advance: the advection and scattering phases (two launches a step)
+        # be_advance: the advection and scattering phases (three launches a
+        # step: the particles, the walls' injection, the re-emission)
         adv_ms += r["phase_ms"]["advection"] + r["phase_ms"]["scattering"]
         adv_bytes += BE_IN_BYTES * r["advance_in"] + BE_OUT_BYTES * r["advance_out"]
         adv_in += int(r["advance_in"])
@@ -316,7 +317,7 @@ def run_berta(args, rank, world, local):
     clk = clocks.stop()
     nbx = int(c["geom"]["nboxes"])
     nsteps = btegpu.berta_steps(dt, maxtime)
-    launches = 2 * nsteps * args.steps
+    launches = 3 * nsteps * args.steps
     peak, peak_kind = measured_peaks()
     achieved = adv_bytes / (adv_ms * 1e-3) / 1e9
     prof = berta_profile_figures()
