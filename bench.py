@@ -998,8 +998,8 @@ def main():
             "l2_reductions": l2red,
             "clocks": clk,
             "tuning": {"block_threads": choice[0], "blocks_per_sm": choice[1],
-                       "smem_tally": choice[2], "particles_per_thread": choice[3],
-                       "ns_per_event": {f"{k[0]}x{k[1]}{'s' if k[2] else ''}{'p2' if k[3] == 2 else ''}": v
+                       "smem_tally": choice[2],
+                       "ns_per_event": {f"{k[0]}x{k[1]}{'s' if k[2] else ''}": v
                                         for k, v in tuned.items()}},
         }
         if world == 1 and not args.no_cpu_baseline:

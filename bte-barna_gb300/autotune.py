@@ -7,9 +7,8 @@ fastest setting on the engine.  Runs before any timed region.
 """
 import btegpu
 
-# (threads per block, blocks per SM, shared-memory tally, particles per thread)
-CANDIDATES = [(256, 4, 0, 1), (128, 8, 0, 1), (256, 3, 0, 1), (256, 2, 0, 1), (128, 6, 0, 1), (128, 4, 0, 1),
-              (256, 1, 1, 1)]
+# (threads per block, blocks per SM, shared-memory tally)
+CANDIDATES = [(256, 4, 0), (128, 8, 0), (256, 3, 0), (256, 2, 0), (128, 6, 0), (128, 4, 0), (256, 1, 1)]
 
 
 def tune(engine, run, trial_particles: int, smem_bytes: int, repeats: int = 2):
@@ -18,12 +17,11 @@ def tune(engine, run, trial_particles: int, smem_bytes: int, repeats: int = 2):
     Returns (best candidate, {candidate: ns per event})."""
     results = {}
     for cand in CANDIDATES:
-        threads, bps, smem, ppt = cand
+        threads, bps, smem = cand
         if smem and smem_bytes > 200 * 1024:
             continue
         try:
-            engine.set_tuning(block_threads=threads, blocks_per_sm=bps, smem_tally=smem,
-                              particles_per_thread=ppt)
+            engine.set_tuning(block_threads=threads, blocks_per_sm=bps, smem_tally=smem)
             best = None
             for r in range(repeats):
                 out = run(r * trial_particles, (r + 1) * trial_particles)
@@ -33,6 +31,5 @@ def tune(engine, run, trial_particles: int, smem_bytes: int, repeats: int = 2):
         except btegpu.BteError:
             continue
     choice = min(results, key=results.get)
-    engine.set_tuning(block_threads=choice[0], blocks_per_sm=choice[1], smem_tally=choice[2],
-                      particles_per_thread=choice[3])
+    engine.set_tuning(block_threads=choice[0], blocks_per_sm=choice[1], smem_tally=choice[2])
     return choice, results
