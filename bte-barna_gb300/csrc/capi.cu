@@ -501,7 +501,7 @@ void ensure_generators(bte_ctx* c, const bte_rta_params* p) {
         }
         return;
     }
-    c->gen_key_source = -1;  // (until all of them are there)
+    bte::Generators gens;  // (a failure up to here leaves the present ones)
     if (c->ncrys > 0) {
         // each crystal's generators, rows over the concatenated modes
         std::vector<bte::Generators> G;
@@ -511,16 +511,17 @@ void ensure_generators(bte_ctx* c, const bte_rta_params* p) {
                             ? bte::build_wall_generators(c->crys[std::size_t(k)], c->geom, false, &e)
                             : bte::build_initial_generators(c->crys[std::size_t(k)], c->geom, &e));
         }
-        c->gens = bte::merge_generators(G, p->source == BTE_SOURCE_WALLS, true);
-        if (p->source == BTE_SOURCE_INITIAL) c->gen_Eeff = bte::initial_counts(c->gens, p->nparticles, p->seed);
+        gens = bte::merge_generators(G, p->source == BTE_SOURCE_WALLS, true);
     } else if (p->source == BTE_SOURCE_WALLS) {
-        c->gens = bte::build_wall_generators(c->modes, c->geom);
-        apply_shares(c, false);
+        gens = bte::build_wall_generators(c->modes, c->geom);
     } else {
         if (!c->mat_share.empty()) throw Error(BTE_ERR_INPUT, "particle shares need the walls source");
-        c->gens = bte::build_initial_generators(c->modes, c->geom);
-        c->gen_Eeff = bte::initial_counts(c->gens, p->nparticles, p->seed);
+        gens = bte::build_initial_generators(c->modes, c->geom);
     }
+    c->gen_key_source = -1;  // (until all of them are there)
+    c->gens = std::move(gens);
+    if (p->source == BTE_SOURCE_INITIAL) c->gen_Eeff = bte::initial_counts(c->gens, p->nparticles, p->seed);
+    else if (c->ncrys == 0) apply_shares(c, false);
     std::vector<float> prob(c->gens.alias.size());
     std::vector<int> alt(c->gens.alias.size());
     const std::size_t chunk = std::size_t(1) << 20;

@@ -39,3 +39,21 @@ def test_particle_buffers_after_a_capacity_that_cannot_be_had(engine):
     after = engine.berta_run(capacity=1 << 20, **run)
     assert after["nsteps"] == before["nsteps"]
     assert abs(after["nparticles"][-1] - before["nparticles"][-1]) < 0.1 * before["nparticles"][-1]
+
+
+@pytest.mark.gpu
+def test_a_source_that_cannot_be_built_leaves_the_present_one(engine):
+    """A ribbon at one temperature has no initial deviation: asking for one
+    fails, and the walls' generators of the run before it still serve the
+    allocation-free run, which builds nothing."""
+    import torch
+    engine.load_modes(synth.mode_table(8, 3, 3, 300.0, config=100))
+    engine.load_geometry(synth.ribbon_geometry(200.0, 50.0, 5))
+    walls = engine.rta_run(300.0, 10.0, 100.0, 2000, seed=3, source=btegpu.SOURCE_WALLS)
+    with pytest.raises(btegpu.BteError):
+        engine.rta_run(300.0, 10.0, 100.0, 2000, seed=3, source=btegpu.SOURCE_INITIAL)
+    dev = torch.zeros((7, 10, 3), dtype=torch.float64, device="cuda:0")
+    params = btegpu.params_struct(300.0, 10.0, 100.0, 2000, 3)
+    r = btegpu.RtaResult()
+    st = engine.lib.bte_rta_run_noalloc(engine.ctx, C.byref(params), C.c_void_p(dev.data_ptr()), C.byref(r))
+    assert st == btegpu.BTE_OK and r.events == walls["events"]
