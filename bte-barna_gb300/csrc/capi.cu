@@ -898,12 +898,13 @@ bte_status bte_set_tuning(bte_ctx* c, const bte_tuning* t) {
 
 bte_status bte_load_modes(bte_ctx* c, const bte_mode_table* mt) {
     if (!c) return BTE_ERR_INPUT;
-    c->group_valid = c->spec_valid = false;
+    c->group_valid = false;
     try {
         ck(cudaSetDevice(c->device), "cudaSetDevice");
         c->modes = bte::build_modes(mt);
         c->have_modes = true;
         c->tables_version++;
+        c->spec_valid = false;
         bte::reset_propagators(c);
         c->ncrys = 0;
         c->crys.clear();
@@ -925,7 +926,7 @@ bte_status bte_load_modes(bte_ctx* c, const bte_mode_table* mt) {
 
 bte_status bte_load_geometry(bte_ctx* c, const bte_geometry* g) {
     if (!c) return BTE_ERR_INPUT;
-    c->group_valid = c->spec_valid = false;
+    c->group_valid = false;
     try {
         ck(cudaSetDevice(c->device), "cudaSetDevice");
         bte::HostGeometry ng = bte::build_geometry(g);
@@ -939,6 +940,7 @@ bte_status bte_load_geometry(bte_ctx* c, const bte_geometry* g) {
         c->geom = std::move(ng);
         c->have_geom = true;
         c->tables_version++;
+        c->spec_valid = false;
         c->geom_dev = false;
         c->dmm_dev = false;
         if (!same_normals) c->lambert_dev = false;
@@ -952,7 +954,7 @@ bte_status bte_load_geometry(bte_ctx* c, const bte_geometry* g) {
 bte_status bte_load_mode_tables(bte_ctx* c, int32_t ntables, const bte_mode_table* tables,
                                 const double* thickness) {
     if (!c) return BTE_ERR_INPUT;
-    c->group_valid = c->spec_valid = false;
+    c->group_valid = false;
     try {
         if (ntables < 1 || !tables) throw Error(BTE_ERR_INPUT, "no mode tables");
         std::vector<double> th;
@@ -982,6 +984,7 @@ bte_status bte_load_mode_tables(bte_ctx* c, int32_t ntables, const bte_mode_tabl
         c->ncrys = ntables;
         c->have_modes = true;
         c->tables_version++;
+        c->spec_valid = false;
         bte::reset_propagators(c);
         c->nmat = ntables;
         c->mat_w = std::move(mw);

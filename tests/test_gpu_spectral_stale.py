@@ -50,6 +50,17 @@ def test_other_tables_end_the_spectral_outputs(engine, run, what):
     assert np.allclose(again["raw"], first["raw"], rtol=1e-9, atol=1e-12 * np.abs(first["raw"]).max())
 
 
+def test_a_load_that_fails_leaves_the_spectral_outputs(engine, run):
+    case, bins, go = run
+    first = go()
+    bad = dict(case["modes"], w=-np.asarray(case["modes"]["w"]))
+    with pytest.raises(btegpu.BteError):
+        engine.load_modes(bad)
+    with pytest.raises(btegpu.BteError):
+        engine.load_materials([bad["w"]], [case["T0"]])
+    assert np.array_equal(engine.get_spectral(bins)["raw"], first["raw"])
+
+
 @pytest.mark.parametrize("steady", [False, True])
 def test_locations_beyond_a_smaller_geometry_are_refused(engine, run, steady):
     """Location 7 of eight boxes, then a geometry of five: no run starts."""
